@@ -8,16 +8,37 @@ plus the C-ABI call on the current stream -- runs at execution (and CUDA-graph c
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 NAMESPACE = "gemq_b200"
 
 
+def _plain(args) -> bool:
+    """No tracing mode is active and the first argument is an ordinary tensor: nobody but the
+    caller looks at this call, so the operator registry has nothing to add to it."""
+    return torch._C._len_torch_dispatch_stack() == 0 and type(args[0]) in (torch.Tensor, torch.nn.Parameter)
+
+
 def library_op(name: str, fake):
     """``@library_op("name", fake_fn)``: register ``fn`` as ``gemq_b200::name`` (no argument is
-    mutated, outputs are fresh tensors) with ``fake_fn`` as its shape/dtype propagation."""
+    mutated, outputs are fresh tensors) with ``fake_fn`` as its shape/dtype propagation.
+
+    A call in eager mode goes straight to ``fn``: the Python dispatch of a custom operator costs
+    20-30 us of host time, more than the kernels of a small call take.  Under ``torch.compile`` and
+    under tracing modes (fake tensors) the call is the operator."""
     def deco(fn):
         op = torch.library.custom_op(f"{NAMESPACE}::{name}", mutates_args=())(fn)
         op.register_fake(fake)
-        return op
+        overload = op._opoverload
+
+        @functools.wraps(fn)
+        def call(*args, **kwargs):
+            if torch.compiler.is_compiling() or not args or not _plain(args):
+                return overload(*args, **kwargs)
+            return fn(*args, **kwargs)
+
+        call._init_fn = fn
+        return call
     return deco
