@@ -1,0 +1,457 @@
+// Products of a few activation rows (at most 16 per tile) with packed matrices: the streaming core
+// shared by the dense linears (few_linear.cu) and the decode batches of the MoE layers (few_moe.cu).
+//
+// What bounds it.  Each weight is used for at most 16 rows, so the matrices have to stream at the
+// memory rate and the arithmetic per weight has to stay small.  The codes are not de-quantised: an
+// fp16 whose exponent field is zero is the subnormal m * 2^-24, so `word & mask` IS a pair of fp16
+// operands holding two codes (times 2^pos for codes that sit `pos` bits up), and it goes straight
+// into mma.sync.m16n8k16 as the A operand (16 weight columns x 16 k).  The B operand is the
+// activation of eight rows, scaled per row and group by a power of two and per k by 2^-pos: exact.
+// Products are summed per quantisation group in fp32; a closed group is added with its scale and its
+// offset times the group's activation sum.  Per 8192 weights (64 columns, one group) and eight rows: 144
+// to 160 ANDs and shifts -- the ALU pipe takes two cycles for each, which is the arithmetic limit -- 32
+// MMAs, and about 70 instructions to close the group on the otherwise idle FMA pipe.  (One scale per row
+// and the offsets as an extra MMA saved half of those, but the scale of a whole row needs a pass over x
+// before the first fragment can be written.)
+//
+// A CTA is four consumer warps of 64 columns each and one producer warp that keeps a ring of stages
+// filled.  A stage is 16 packed rows: TMA boxes of 32-column strips (128B swizzle: conflict-free
+// 16-byte reads), scales and offsets as cp.async, all completing on one mbarrier.  Rings in registers
+// do not work: a warp has six scoreboards, so eight loads in flight serialise (3.0 against 6.2 TB/s in
+// a copy-only probe).
+//
+// The B operands ("table") lie in shared memory in fragment order, 64 bytes per row and two k-steps;
+// MMA columns past the last row read a block of zeros.
+#pragma once
+
+#include "gemv.cuh"
+#include "ptx.cuh"
+
+namespace gemq {
+namespace few {
+
+constexpr int kCons = 4;
+constexpr int kThreads = 32 * (kCons + 1);
+constexpr int kMaxRing = 3;
+constexpr int kStageRows = 16;               // packed rows per pipeline stage
+constexpr int kTileRows = 16;                // activation rows of a tile: one or two blocks of eight MMA columns
+constexpr int kStrip = 2048;                 // 16 packed rows x 32 columns
+constexpr int kWStage = kCons * 2 * kStrip;
+constexpr int kMetaStage = kCons * 4 * 256;  // per warp and group: 64 scales, 64 offsets
+constexpr int kMaxDyn = 225 * 1024;          // dynamic shared memory: 227 KB less the static part
+
+enum { kErrFewFull = 31, kErrFewEmpty = 32 };
+
+__host__ __device__ constexpr int packed_rows(int K, int bits) { return bits == 3 ? (K + 9) / 10 : K * bits / 32; }
+__host__ __device__ constexpr int n_stages(int K, int bits) { return cdiv(packed_rows(K, bits), kStageRows); }
+// Table pieces of a stage: 16 bytes per row and lane column = the B registers of two k-steps.
+// 3-bit: three passes of five k-steps, padded to six.
+__host__ __device__ constexpr int stage_pieces(int bits) { return bits == 3 ? 9 : 16 / bits; }
+// Group slots of a stage.  3-bit: the group that ends in stage s of a run of four, and behind the run's last
+// stage the fifth group.
+__host__ __device__ constexpr int stage_slots(int bits) { return bits == 3 ? 2 : 4 / bits; }
+// Bytes of a stage of the table: pieces [piece][row][lane column], then per group slot and row (row count
+// rounded up to even) what undoes the row's scaling of the group, and the sum of its activations.
+__host__ __device__ constexpr int table_stage_bytes(int bits, int rows) {
+  return stage_pieces(bits) * 64 * rows + stage_slots(bits) * 16 * ((rows + 1) / 2);
+}
+// Bytes that hold a tile of `rows` rows at any bit width.
+__host__ __device__ constexpr size_t table_tile_bytes(int K, int rows) {
+  size_t most = 0;
+  for (int b = 1; b <= 4; ++b) {
+    const size_t n = static_cast<size_t>(n_stages(K, b)) * table_stage_bytes(b, rows);
+    most = n > most ? n : most;
+  }
+  return most;
+}
+
+__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Operand q of a packed word: two codes in place, `pos` bits up in their half.
+template <int B>
+struct Fmt {
+  static constexpr int kEps = B == 3 ? 10 : 32 / B;
+  static constexpr int kPos = 10 / B;       // operands that fit the ten mantissa bits without a shift
+  static constexpr uint32_t kMask = ((1u << B) - 1u) * 0x00010001u;
+  // 3-bit words are spread first: codes 0..4 to the lower half, 5..9 to the upper one
+  __device__ static __forceinline__ uint32_t spread(uint32_t w) {
+    return B == 3 ? ((w & 0x00007fffu) | ((w << 1) & 0x7fff0000u)) : w;
+  }
+  // codes q and q + kEps / 2
+  __device__ static __forceinline__ uint32_t operand(uint32_t w, int q) {
+    return (w >> ((q / kPos) * kPos * B)) & (kMask << (B * (q % kPos)));
+  }
+  __host__ __device__ static constexpr int pos(int q) { return B * (q % kPos); }
+  // packed row (of eight) that lane column c reads as its word r = 0, 1.  1-bit groups are four rows long.
+  __host__ __device__ static constexpr int row(int c, int r) { return B == 1 ? c + 4 * r : 2 * c + r; }
+};
+
+template <int NB>
+struct State {
+  float acc[2][2][NB][4];   // open group: [strip][column pair][row block][C fragment]
+  float out[2][2][NB][4];   // closed groups: scale * sum(code * x) + offset * sum(x)
+};
+
+template <int NB>
+__device__ __forceinline__ void clear(State<NB>& S) {
+#pragma unroll
+  for (int st = 0; st < 2; ++st)
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S.acc[st][s][nb][e] = S.out[st][s][nb][e] = 0.f;
+}
+
+__device__ __forceinline__ void half4(const unsigned char* p, float (&f)[4]) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x));
+  const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+
+// Close a group.  `meta` = its scales and offsets of the warp's 64 columns, `ft` = its (unscale, sum) pairs.
+template <int NB>
+__device__ __forceinline__ void fold(State<NB>& S, const unsigned char* meta, const unsigned char* ft, int rows, int lane) {
+  const int g = lane >> 2, c = lane & 3;
+  float4 fx[NB];  // (unscale, sum) of rows 8 nb + 2 c and the next; rows past the last repeat a valid pair, nobody reads them
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb) {
+    const int pair = min(4 * nb + c, (rows - 1) >> 1);
+    fx[nb] = *reinterpret_cast<const float4*>(ft + 16 * pair);
+  }
+#pragma unroll
+  for (int st = 0; st < 2; ++st) {
+    float sc[4], zr[4];
+    half4(meta + 64 * st + 8 * g, sc);
+    half4(meta + 128 + 64 * st + 8 * g, zr);
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float f = (e & 1) ? fx[nb].z : fx[nb].x, xs = (e & 1) ? fx[nb].w : fx[nb].y;
+          const int k = 2 * s + (e >> 1);
+          S.out[st][s][nb][e] = fmaf(sc[k], S.acc[st][s][nb][e] * f, fmaf(zr[k], xs, S.out[st][s][nb][e]));
+          S.acc[st][s][nb][e] = 0.f;
+        }
+  }
+}
+
+// Where a lane finds its B operands: MMA column g of block nb is row g + 8 nb; columns past the last
+// row stay on the zero block.
+template <int NB>
+struct TablePtr {
+  const unsigned char* p[NB];
+  int step[NB];  // bytes from a piece to the next
+};
+template <int NB>
+__device__ __forceinline__ TablePtr<NB> table_ptr(const unsigned char* T, const unsigned char* zero, int rows, int lane) {
+  TablePtr<NB> t;
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb) {
+    const int r = (lane >> 2) + 8 * nb;
+    t.p[nb] = r < rows ? T + r * 64 + (lane & 3) * 16 : zero;
+    t.step[nb] = r < rows ? rows * 64 : 0;
+  }
+  return t;
+}
+
+// Word r of the lane in block j (eight packed rows), both strips (STEP bytes apart).
+template <int B, int STEP>
+__device__ __forceinline__ void load_words(uint4 (&w)[2], const unsigned char* W, int j, int r, int g, int c) {
+  const int row = Fmt<B>::row(c, r);
+#pragma unroll
+  for (int st = 0; st < 2; ++st)
+    w[st] = *reinterpret_cast<const uint4*>(W + st * STEP + (8 * j + row) * 128 + ((g ^ row) << 4));
+}
+
+// A stage (16 packed rows) of a 1/2/4-bit matrix: 4 / B groups, each eight k-steps of 16.
+template <int B, int NB, int STEP>
+__device__ __forceinline__ void stage_pow2(State<NB>& S, const unsigned char* W, const unsigned char* T, const unsigned char* zero,
+                                           const unsigned char* meta, int rows, int groups, int lane) {
+  using F = Fmt<B>;
+  const int g = lane >> 2, c = lane & 3;
+  constexpr int QW = F::kEps / 8;  // pieces per packed word
+  TablePtr<NB> t = table_ptr<NB>(T, zero, rows, lane);
+  // one group per trip: two blocks of rows leave no registers for more in flight
+#pragma unroll 1
+  for (int gi = 0; gi < groups; ++gi) {
+#pragma unroll
+    for (int wl = 0; wl < B; ++wl) {
+      uint4 w[2];
+      // the group's words: 1-bit row gi (block gi / 2), 2-bit block gi, 4-bit both blocks
+      load_words<B, STEP>(w, W, B == 1 ? gi >> 1 : (B == 2 ? gi : wl >> 1), B == 1 ? gi & 1 : wl & 1, g, c);
+#pragma unroll
+      for (int q = 0; q < QW; ++q) {
+        uint4 b[NB];
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) {
+          b[nb] = *reinterpret_cast<const uint4*>(t.p[nb]);
+          t.p[nb] += t.step[nb];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = 2 * (2 * q + h);
+#pragma unroll
+          for (int st = 0; st < 2; ++st) {
+            const uint32_t wv[4] = {w[st].x, w[st].y, w[st].z, w[st].w};
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+              const uint32_t a0 = F::operand(wv[2 * s], m), a1 = F::operand(wv[2 * s + 1], m);
+              const uint32_t a2 = F::operand(wv[2 * s], m + 1), a3 = F::operand(wv[2 * s + 1], m + 1);
+#pragma unroll
+              for (int nb = 0; nb < NB; ++nb)
+                mma16816(S.acc[st][s][nb], a0, a1, a2, a3, h ? b[nb].z : b[nb].x, h ? b[nb].w : b[nb].y);
+            }
+          }
+        }
+      }
+    }
+    fold<NB>(S, meta + gi * 256, T + stage_pieces(B) * 64 * rows + gi * 16 * ((rows + 1) >> 1), rows, lane);
+  }
+}
+
+// Five k-steps over an 8-row block of 3-bit words; `t` moves on by the pass's three pieces.
+template <int NB, int STEP>
+__device__ __forceinline__ void pass_b3(State<NB>& S, const unsigned char* W, TablePtr<NB>& t, int j, int lane) {
+  using F = Fmt<3>;
+  const int g = lane >> 2, c = lane & 3;
+  uint4 wa[2], wb[2];
+  load_words<3, STEP>(wa, W, j, 0, g, c);
+  load_words<3, STEP>(wb, W, j, 1, g, c);
+  uint32_t v[2][2][4];
+#pragma unroll
+  for (int st = 0; st < 2; ++st) {
+    v[st][0][0] = F::spread(wa[st].x); v[st][0][1] = F::spread(wa[st].y);
+    v[st][0][2] = F::spread(wa[st].z); v[st][0][3] = F::spread(wa[st].w);
+    v[st][1][0] = F::spread(wb[st].x); v[st][1][1] = F::spread(wb[st].y);
+    v[st][1][2] = F::spread(wb[st].z); v[st][1][3] = F::spread(wb[st].w);
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    uint4 b[NB];
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb) {
+      b[nb] = *reinterpret_cast<const uint4*>(t.p[nb]);
+      t.p[nb] += t.step[nb];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int m = 2 * q + h;
+      if (m < 5) {
+        const int s0 = 2 * m, s1 = 2 * m + 1;  // operand slots: five of the first word, five of the second
+#pragma unroll
+        for (int st = 0; st < 2; ++st)
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            const uint32_t a0 = F::operand(v[st][s0 / 5][2 * s], s0 % 5), a1 = F::operand(v[st][s0 / 5][2 * s + 1], s0 % 5);
+            const uint32_t a2 = F::operand(v[st][s1 / 5][2 * s], s1 % 5), a3 = F::operand(v[st][s1 / 5][2 * s + 1], s1 % 5);
+#pragma unroll
+            for (int nb = 0; nb < NB; ++nb)
+              mma16816(S.acc[st][s][nb], a0, a1, a2, a3, h ? b[nb].z : b[nb].x, h ? b[nb].w : b[nb].y);
+          }
+      }
+    }
+  }
+}
+
+// A stage of a 3-bit matrix.  64 packed rows = 640 k = five groups = four stages; a group ends inside
+// blocks 1, 3, 4, 6 of the run and at its end.  A block with two groups takes two passes whose table
+// entries hold only the one or the other.  `s4` = stage of the run, `left` = groups from the run's first on.
+template <int NB, int STEP>
+__device__ __forceinline__ void stage_b3(State<NB>& S, const unsigned char* W, const unsigned char* T, const unsigned char* zero,
+                                         const unsigned char* meta, int rows, int s4, int left, int lane) {
+  const unsigned char* ft = T + stage_pieces(3) * 64 * rows;
+  const bool late = s4 >= 2;  // the group ends in the stage's first block, not in its second
+  TablePtr<NB> t = table_ptr<NB>(T, zero, rows, lane);
+#pragma unroll 1
+  for (int p = 0; p < 3; ++p) {
+    pass_b3<NB, STEP>(S, W, t, late ? p >> 1 : (p + 1) >> 1, lane);
+    if (p == (late ? 0 : 1) && s4 < left) fold<NB>(S, meta, ft, rows, lane);
+  }
+  if (s4 == 3 && left > 4) fold<NB>(S, meta + 256, ft + 16 * ((rows + 1) >> 1), rows, lane);
+}
+
+template <int B, int NB, int STEP>
+__device__ __forceinline__ void stage_any(State<NB>& S, const unsigned char* W, const unsigned char* T, const unsigned char* zero,
+                                          const unsigned char* meta, int rows, int sg, int ngroups, int lane) {
+  if (B == 3) stage_b3<NB, STEP>(S, W, T, zero, meta, rows, sg & 3, ngroups - 5 * (sg >> 2), lane);
+  else stage_pow2<B == 3 ? 2 : B, NB, STEP>(S, W, T, zero, meta, rows, min(4 / B, ngroups - (4 / B) * sg), lane);
+}
+
+// Columns 4g .. 4g + 3 of strip st for row 8 nb + 2 c + o.
+template <int NB>
+__device__ __forceinline__ float4 result4(const State<NB>& S, int st, int nb, int o) {
+  return make_float4(S.out[st][0][nb][o], S.out[st][0][nb][2 + o], S.out[st][1][nb][o], S.out[st][1][nb][2 + o]);
+}
+
+// Bounded wait without sleeping: the hardware suspends the warp inside try_wait.
+__device__ __forceinline__ void wait_bar(unsigned long long* bar, uint32_t parity, int* err, int code) {
+  for (int i = 0; i < kSpinLimit; ++i)
+    if (mbar_try_wait(bar, parity)) return;
+  atomicExch(err, code);
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(unsigned long long* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, unsigned long long* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+// Box of a strip map (tma.cu): (column 0 of 32, packed row, strip); strips and rows past the end are zero-filled.
+__device__ __forceinline__ void tma_load_strips(void* dst, const CUtensorMap* map, int row, int strip, unsigned long long* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(0), "r"(row), "r"(strip), "r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Part p of n of a matrix's stages: whole stages, for 3-bit whole runs of four.
+__device__ __forceinline__ void stage_range(int bits, int K, int p, int n, int& lo, int& hi) {
+  const int st = n_stages(K, bits);
+  const int unit = bits == 3 ? 4 : 1;
+  const int u = cdiv(st, unit);
+  lo = min(st, (u * p / n) * unit);
+  hi = min(st, (u * (p + 1) / n) * unit);
+}
+
+template <typename T> __device__ __forceinline__ float to_f(T v);
+template <> __device__ __forceinline__ float to_f<__half>(__half v) { return __half2float(v); }
+template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <typename T> __device__ __forceinline__ T from_f(float v);
+template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+__device__ __forceinline__ float round_h(float v) { return __half2float(__float2half_rn(v)); }
+
+// Exponent that puts the largest |x| of a group into [2^14, 2^15): no bit of x is lost down to 2^-20 of it.
+__device__ __forceinline__ int group_exponent(float mx) {
+  const int ce = 14 - (static_cast<int>((__float_as_uint(mx) >> 23) & 0xffu) - 127);
+  return ce < -100 ? -100 : (ce > 100 ? 100 : ce);
+}
+// (unscale, sum) of a group and the factor its activations are written with.
+__device__ __forceinline__ float2 group_pair(int ce, float sum) { return make_float2(pow2i(24 - ce), sum); }
+
+// The pieces of one packed word of a 1/2/4-bit matrix: x = its activations, f = the group's factor.
+template <int B>
+__device__ __forceinline__ void word_pieces(const float (&x)[32 / B], float f, unsigned char* dst, int step) {
+  using F = Fmt<B>;
+  constexpr int EPS = F::kEps;
+#pragma unroll
+  for (int q = 0; q < EPS / 8; ++q) {
+    __half2 h[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const float s = f * pow2i(-F::pos(4 * q + p));
+      h[p] = __floats2half2_rn(x[4 * q + p] * s, x[4 * q + p + EPS / 2] * s);
+    }
+    *reinterpret_cast<uint4*>(dst + q * step) = *reinterpret_cast<const uint4*>(h);
+  }
+}
+
+// 3-bit: piece q (0..8) of stage sg for lane column c.  x(k) = activation k, 0 past the end; f(group) = factor.
+template <typename X, typename G>
+__device__ __forceinline__ uint4 piece_b3(int sg, int q, int c, X x, G factor) {
+  const int pass = q / 3, s4 = sg & 3;
+  // pass -> block of the stage, and which of its two groups (0: it has one, 1: the first, 2: the second)
+  const int blk = 2 * sg + (s4 < 2 ? (pass > 0) : (pass == 2));
+  const int part = s4 < 2 ? pass : (pass == 2 ? 0 : pass + 1);
+  const int end = 5 * (sg >> 2) + s4;  // the group that ends in this stage
+  const int grp = part == 0 ? (s4 < 2 ? end : end + 1) : end + part - 1;
+  const float f = factor(grp);
+  __half v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int slot = 4 * (q % 3) + (e >> 1);  // operand slot 0..9, above: padding
+    const int pr = slot % 5;
+    const int k = (8 * blk + 2 * c + (slot >= 5)) * 10 + pr + 5 * (e & 1);
+    const float xv = slot < 10 && (k >> 7) == grp ? x(k) : 0.f;
+    v[e] = __float2half_rn(xv * (f * pow2i(-Fmt<3>::pos(pr))));
+  }
+  return *reinterpret_cast<const uint4*>(v);
+}
+
+// Stage and slot of a group.
+__device__ __forceinline__ void group_place(int bits, int grp, int& sg, int& slot) {
+  if (bits == 3) { sg = 4 * (grp / 5) + min(grp % 5, 3); slot = grp % 5 == 4 ? 1 : 0; }
+  else { const int n = 4 / bits; sg = grp / n; slot = grp - sg * n; }
+}
+
+// Half a warp writes one group of one row to the table: `v` = its 128 activations in shared memory, t = the
+// row's place in its tile.  All pieces of the group are written: the ones of its words, for 3-bit the ones of
+// its passes.
+template <typename T>
+__device__ __forceinline__ void group_to_table(const T* v, int bits, int grp, unsigned char* tab, int rows, int t, int lane) {
+  const int l16 = lane & 15;
+  float mx = 0.f, sm = 0.f;
+  {
+    const uint4 r = *reinterpret_cast<const uint4*>(v + 8 * l16);
+    const T* e = reinterpret_cast<const T*>(&r);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float f = to_f<T>(e[k]);
+      mx = fmaxf(mx, fabsf(f));
+      sm += f;
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    sm += __shfl_xor_sync(0xffffffffu, sm, o);
+  }
+  const int ce = group_exponent(mx);
+  const float f = pow2i(ce);
+  int sg, slot;
+  group_place(bits, grp, sg, slot);
+  const int tb = table_stage_bytes(bits, rows), re = (rows + 1) & ~1;
+  if (l16 == 0)
+    *reinterpret_cast<float2*>(tab + sg * tb + stage_pieces(bits) * 64 * rows + (slot * re + t) * 8) = group_pair(ce, sm);
+  if (bits == 3) {
+    const int i5 = grp % 5, run = grp / 5;
+    // the group's passes, counted from the run's first: 0, 1 | 2, 3, 4 | 5, 6 | 7, 8, 9 | 10, 11
+    const int first = i5 == 0 ? 0 : (i5 == 1 ? 2 : (i5 == 2 ? 5 : (i5 == 3 ? 7 : 10)));
+    const int count = (i5 == 1 || i5 == 3) ? 3 : 2;
+    for (int i = l16; i < count * 12; i += 16) {
+      const int ps = first + i / 12, q3 = (i % 12) >> 2, c = i & 3;
+      const int s3 = 4 * run + ps / 3, q = 3 * (ps % 3) + q3;
+      const uint4 o = piece_b3(s3, q, c, [&](int k) { return to_f<T>(v[k - grp * kGroup]); }, [&](int) { return f; });
+      *reinterpret_cast<uint4*>(tab + s3 * tb + (q * rows + t) * 64 + c * 16) = o;
+    }
+    return;
+  }
+  // 16 pieces: lane -> packed word of the group (eps activations), piece of the word
+  const int eps = 32 / bits, qw = 4 / bits;
+  const int w = l16 / qw, q = l16 - w * qw;
+  const int c = bits == 1 ? w : (w & 7) >> 1;
+  const int wr = bits == 1 ? slot : (bits == 2 ? 2 * slot + (w & 1) : 2 * (w >> 3) + (w & 1));
+  const int npos = bits == 1 ? 10 : (bits == 2 ? 5 : 2);
+  __half2 h[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const int pr = 4 * q + p;
+    const float sc = f * pow2i(-bits * (pr >= npos ? pr - npos : pr));  // at most two shifts per word
+    h[p] = __floats2half2_rn(to_f<T>(v[w * eps + pr]) * sc, to_f<T>(v[w * eps + pr + (eps >> 1)]) * sc);
+  }
+  *reinterpret_cast<uint4*>(tab + sg * tb + ((wr * qw + q) * rows + t) * 64 + c * 16) = *reinterpret_cast<const uint4*>(h);
+}
+
+}  // namespace few
+
+// tma.cu: packed words [rows, N] as strips of 32 columns, box 16 rows x `strips` strips, 128B swizzle.
+bool tensor_map_strips(CUtensorMap* out, const void* base, int N, long long rows, int strips);
+
+}  // namespace gemq

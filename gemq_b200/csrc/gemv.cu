@@ -717,6 +717,20 @@ extern "C" size_t gemq_gemv_workspace_bytes(int total_cols, int max_k, int token
   return gemv_workspace_bytes(total_cols, max_k, tokens);
 }
 
+// One matrix goes to the one-launch few-row kernel (few_linear.cu) for every shape that takes: 8.9 us
+// against 12.2 us for a 14336 x 4096 2-bit matrix and one row, 9.2 against 32.6 us for 13 rows of a 4-bit
+// 4096 x 4096 one (which took a pass over the weights per eight rows here).
+extern "C" int gemq_linear_rows(const void* x, int ldx, int x_is_bf16, const int32_t* wq, const void* scales, const void* zeros,
+                                const void* bias, void* y, int rows, int N, int K, int nbits, int group_size, int32_t* err,
+                                gemq_stream_t stream);
+
+namespace gemq {
+bool few_linear_takes(const void* wq, const void* scales, const void* zeros, const void* y, int N, int K, int G) {
+  return G == kGroup && K % kGroup == 0 && K <= 32768 && N % 32 == 0 && aligned16(wq) && aligned16(scales) && aligned16(zeros) &&
+         aligned16(y);
+}
+}  // namespace gemq
+
 static bool bits_ok(int b) { return b >= 1 && b <= 4; }
 
 static void job_from_stacked(GemvJob& J, const gemq_stacked_t* W, const int64_t* idx_slot, int N, int K) {
@@ -743,6 +757,11 @@ extern "C" int gemq_dequant_gemv(const void* x, int ldx, const int32_t* wq, cons
                                  void* workspace, size_t workspace_bytes, gemq_stream_t stream) {
   if (!x || !wq || !scales || !zeros || !y || tokens <= 0 || N <= 0 || K <= 0 || group_size <= 0 || !bits_ok(nbits))
     return GEMQ_ERR_BAD_ARG;
+  if (ldy == N && few_linear_takes(wq, scales, zeros, y, N, K, group_size)) {
+    if (!workspace || workspace_bytes < kMaxCounters * sizeof(int) || !aligned16(workspace)) return GEMQ_ERR_WORKSPACE;
+    return gemq_linear_rows(x, ldx, 0, wq, scales, zeros, nullptr, y, tokens, N, K, nbits, group_size,
+                            static_cast<int*>(workspace) + kErrWord, stream);
+  }
   GemvParams P = {};
   P.n_jobs = 1;
   P.T = tokens;

@@ -36,16 +36,17 @@ struct MapKey {
 
 // elem_bytes 4 -> UINT32, 2 -> UINT16 (any 16-bit type).  `inner` elements per row, row stride
 // inner * elem_bytes (a multiple of 16).  128B swizzle needs box_inner * elem_bytes <= 128.
+static std::mutex g_mu;
+static std::map<MapKey, CUtensorMap> g_cache;
+
 bool tensor_map_2d(CUtensorMap* out, const void* base, int elem_bytes, int inner, long long rows, int box_inner,
                    int box_rows, bool swizzle128) {
-  static std::mutex mu;
-  static std::map<MapKey, CUtensorMap> cache;
   int dev = 0;
   cudaGetDevice(&dev);
   const MapKey key{base, rows, inner, elem_bytes, box_inner, box_rows, swizzle128 ? 1 : 0, dev};
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find(key);
-  if (it != cache.end()) {
+  std::lock_guard<std::mutex> lock(g_mu);
+  auto it = g_cache.find(key);
+  if (it != g_cache.end()) {
     *out = it->second;
     return true;
   }
@@ -61,8 +62,38 @@ bool tensor_map_2d(CUtensorMap* out, const void* base, int elem_bytes, int inner
                          swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return false;
-  if (cache.size() > 4096) cache.clear();
-  cache[key] = m;
+  if (g_cache.size() > 4096) g_cache.clear();
+  g_cache[key] = m;
+  *out = m;
+  return true;
+}
+
+// 3-D view (32 columns, rows, strips): one box brings `strips` neighbouring 32-column strips of 16 rows,
+// each as 16 swizzled rows of 128 bytes.  One such instruction replaces a 2-D box per strip: a warp's
+// lanes issue their boxes one after the other, about 50 cycles each.
+bool tensor_map_strips(CUtensorMap* out, const void* base, int N, long long rows, int strips) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const MapKey key{base, rows, N, 4, 32, 16, 16 + strips, dev};
+  std::lock_guard<std::mutex> lock(g_mu);
+  auto it = g_cache.find(key);
+  if (it != g_cache.end()) {
+    *out = it->second;
+    return true;
+  }
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (!enc) return false;
+  const cuuint64_t dims[3] = {32, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(N / 32)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(N) * 4, 128};
+  const cuuint32_t box[3] = {32, 16, static_cast<cuuint32_t>(strips)};
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  CUtensorMap m;
+  if (enc(&m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return false;
+  if (g_cache.size() > 4096) g_cache.clear();
+  g_cache[key] = m;
   *out = m;
   return true;
 }

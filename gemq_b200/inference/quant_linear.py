@@ -11,7 +11,7 @@ import torch
 import torch.nn as nn
 from torch import Tensor
 
-from ..kernels import dequant_gemm
+from ..kernels.dequant_gemm import quant_linear
 from .packed_linear import PackedLinear
 
 
@@ -27,11 +27,6 @@ class QuantLinear(nn.Module):
     def forward(self, x: Tensor) -> Tensor:
         """``x [..., in]`` fp16 / bf16 -> ``[..., out]`` in the same dtype."""
         lead = x.shape[:-1]
-        rows = x.reshape(-1, self.in_features)
-        small = rows.shape[0] < 32 and rows.dtype != torch.float16
-        y = dequant_gemm(rows.to(torch.float16) if small else rows, self.W_q, self.scales, self.zeros, self.W_nbits,
-                         self.group_size)
-        y = y.to(x.dtype)
-        if self.bias is not None:
-            y = y + self.bias.to(y.dtype)
+        y = quant_linear(x.reshape(-1, self.in_features), self.W_q, self.scales, self.zeros, self.W_nbits, self.group_size,
+                         self.bias)
         return y.reshape(*lead, self.out_features)

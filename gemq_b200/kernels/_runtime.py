@@ -77,3 +77,23 @@ def error_word(dev: torch.device) -> torch.Tensor:
 def tc_gemm_ok(M: int, N: int, K: int, group_size: int) -> bool:
     """Shapes the tcgen05 GEMM takes; smaller row counts stay on the decode kernel."""
     return M >= 32 and N % 128 == 0 and K % 64 == 0 and group_size % 64 == 0 and K % group_size == 0
+
+
+def few_rows_ok(w_q, scales, zeros, K: int, N: int, group_size: int) -> bool:
+    """Matrices the few-row kernel takes (``gemq_linear_rows``)."""
+    return (group_size == 128 and K % 128 == 0 and K <= 32768 and N % 32 == 0 and
+            (w_q.data_ptr() | scales.data_ptr() | zeros.data_ptr()) & 15 == 0)
+
+
+def linear_rows(x, w_q, scales, zeros, nbits: int, group_size: int, bias=None):
+    """``x [M, K] @ deq(w_q) (+ bias)`` in x's dtype (fp16 or bf16) through the few-row kernel; the
+    arguments have been checked."""
+    dev = x.device
+    M, K = x.shape
+    N = w_q.shape[1]
+    out = torch.empty((M, N), dtype=x.dtype, device=dev)
+    _capi.check("gemq_linear_rows", _capi.lib.gemq_linear_rows(
+        x.data_ptr(), x.stride(0), int(x.dtype == torch.bfloat16), w_q.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
+        bias.data_ptr() if bias is not None else None, out.data_ptr(), M, N, K, nbits, group_size,
+        error_word(dev).data_ptr(), stream_ptr(dev)))
+    return out

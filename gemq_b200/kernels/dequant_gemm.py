@@ -1,12 +1,15 @@
 """Dequant-fused GEMM; same call signature as gemq/triton_kernels/dequant_gemm.py."""
 from __future__ import annotations
 
+from typing import Optional
+
 import torch
 from torch import Tensor
 
 from .. import _capi
 from ._ops import library_op
-from ._runtime import check_kernel_form, error_word, require, require_cuda, stream_ptr, tc_gemm_ok
+from ._runtime import (check_kernel_form, error_word, few_rows_ok, linear_rows, require, require_cuda, stream_ptr,
+                       tc_gemm_ok)
 from .dequant_gemv import dequant_gemv_rows
 
 _ROW_BLOCK = 64
@@ -43,6 +46,27 @@ def dequant_gemm(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: i
         return rows(x, w_q, scales, zeros, nbits, group_size)
     return torch.cat([rows(x[i:i + _ROW_BLOCK], w_q, scales, zeros, nbits, group_size)
                       for i in range(0, M, _ROW_BLOCK)])
+
+
+@library_op("quant_linear",
+            lambda x, w_q, scales, zeros, nbits, group_size, bias: x.new_empty((x.shape[0], w_q.shape[1])))
+def quant_linear(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int,
+                 bias: Optional[Tensor]) -> Tensor:
+    """``x [M, K] @ deq(w_q) + bias`` in x's dtype (fp16 or bf16): what ``QuantLinear`` computes.  Below
+    the row count of the tcgen05 GEMM, and for widths it does not take, one call of the few-row kernel
+    reads x and writes y in their own dtype; before, bf16 rows went through fp16 copies either side."""
+    dev = require_cuda(x, w_q, scales, zeros)
+    M, K = x.shape
+    N = w_q.shape[1]
+    half = x.dtype in (torch.float16, torch.bfloat16)
+    if half and not tc_gemm_ok(M, N, K, group_size) and few_rows_ok(w_q, scales, zeros, K, N, group_size):
+        check_kernel_form(w_q, scales, zeros, K, N, nbits, group_size)
+        if bias is not None:
+            bias = bias.to(device=dev, dtype=x.dtype).contiguous()
+        return linear_rows(x if x.stride(1) == 1 else x.contiguous(), w_q, scales, zeros, nbits, group_size, bias)
+    small = M < 32 and x.dtype != torch.float16
+    y = dequant_gemm._init_fn(x.to(torch.float16) if small else x, w_q, scales, zeros, nbits, group_size).to(x.dtype)
+    return y if bias is None else y + bias.to(y.dtype)
 
 
 dequant_gemm_triton = dequant_gemm

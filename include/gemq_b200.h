@@ -202,6 +202,15 @@ int gemq_dequant_gemm_tc(const void* x, const int64_t* expert, const int32_t* wq
                          const int32_t* zs_strides, int fixed_bits, void* y, int M, int N, int K,
                          int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream);
 
+/* The same product for a few rows (decode batches; any row count is taken, up to 16 rows per pass
+ * over the weights), with an optional bias: y[rows, N] = x @ deq(W) (+ bias), x rows `ldx` elements
+ * apart, x, bias and y fp16 or (x_is_bf16) bf16.  One launch; the packed codes are multiplied in
+ * place (exact products, fp32 sums in a fixed order).  Needs group_size 128, K % 128 == 0,
+ * K <= 32768, N % 32 == 0; GEMQ_ERR_ALIGN unless the packed tensors and y are 16-byte aligned. */
+int gemq_linear_rows(const void* x, int ldx, int x_is_bf16, const int32_t* wq, const void* scales,
+                     const void* zeros, const void* bias, void* y, int rows, int N, int K, int nbits,
+                     int group_size, int32_t* err, gemq_stream_t stream);
+
 /* Device scratch of gemq_moe_prefill for `tokens` rows. */
 size_t gemq_moe_prefill_scratch_bytes(const gemq_moe_layer_t* layer, int tokens);
 

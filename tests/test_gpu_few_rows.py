@@ -1,0 +1,42 @@
+"""The few-row kernels at the edges of their tiles: one to seventeen rows around the 8- and 16-row blocks,
+column counts that end inside a 64-column tile, reduction lengths that end inside a stage or a 3-bit run,
+and MoE batches whose experts get no row, one row or more than a tile."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import gemq_oracle as O
+from conftest import REL_FRO_TOL, rel_fro
+import moe_fixtures as MF
+
+pytestmark = pytest.mark.gpu
+
+# One rounding of the output: 2^-11 (fp16) or 2^-8 (bf16) of each value at most; the sums before it are fp32.
+OUT_TOL = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+@pytest.mark.parametrize("b", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(32, 128), (96, 640), (576, 1408), (160, 4096)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_linear_rows_edges(b, N, K, dtype):
+    from gemq_b200.kernels._runtime import error_word
+    from gemq_b200.kernels.dequant_gemm import quant_linear
+    rng = np.random.default_rng(b * 100 + N)
+    lin = MF.draw_linear(rng, N, K, b)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    wq, s, z = t(lin["wq"]), t(lin["s"]), t(lin["z"])
+    W = O.dequantize(lin["wq"], lin["s"], lin["z"], b, 128, K).astype(np.float64)
+    bias = torch.from_numpy(rng.standard_normal(N)).to(dtype).cuda()
+    for M in (1, 7, 8, 9, 16, 17):
+        x = torch.from_numpy(rng.standard_normal((M, K))).to(dtype).cuda()
+        y = quant_linear(x, wq, s, z, b, 128, None)
+        assert y.dtype == dtype and torch.equal(y, quant_linear(x, wq, s, z, b, 128, None))
+        want = x.double().cpu().numpy() @ W
+        # the de-quantised reference weights carry an fp16 rounding (2^-11) that the exact codes do not
+        assert rel_fro(y.double().cpu().numpy(), want) < OUT_TOL[dtype] + 2.0 ** -11, (M, rel_fro(y.double().cpu().numpy(), want))
+        yb = quant_linear(x, wq, s, z, b, 128, bias)
+        assert torch.equal(yb, y + bias)
+    # rows of a wider tensor, not 16-byte aligned
+    wide = torch.from_numpy(rng.standard_normal((5, K + 3))).to(dtype).cuda()[:, 1:K + 1]
+    assert torch.equal(quant_linear(wide, wq, s, z, b, 128, None), quant_linear(wide.contiguous(), wq, s, z, b, 128, None))
+    assert int(error_word(y.device).item()) == 0
