@@ -29,6 +29,13 @@
 
 namespace gemq {
 
+namespace few {  // few_moe.cu
+bool moe_few_rows_ok(const gemq_moe_layer_t* L, int tokens);
+size_t moe_few_rows_bytes(const gemq_moe_layer_t* L, int tokens);
+int moe_few_rows(const gemq_moe_layer_t* L, const void* x, void* out, const long long* idx, const void* w, int tokens, bool bf16,
+                 char* scratch, int* err, cudaStream_t st);
+}  // namespace few
+
 constexpr int kGemmBM = 256, kGemmBN = 128, kGemmBK = 64;  // CTA tile; two M=128 MMAs share every B tile
 constexpr int kMmaM = 128;
 constexpr int kGemmStages = 3;
@@ -607,6 +614,7 @@ struct PrefillScratch {
   void* hs;     // [T, SF]
   void* yss;    // [T, D]
   void* xh;     // [T, D] fp16 copy of bf16 activations (shared experts)
+  char* few;    // scratch of the few-row path (shares the bytes behind the error word)
   int max_tiles;
 };
 
@@ -620,6 +628,7 @@ size_t prefill_bytes(const gemq_moe_layer_t* L, int tokens, PrefillScratch* S, c
   char* cursor = take(sizeof(int) * E);
   char* offsets = take(sizeof(int) * (E + 1));
   char* ntl = take(sizeof(int) * 2);
+  const size_t few_at = off;
   char* te = take(sizeof(int) * max_tiles);
   char* tr0 = take(sizeof(int) * max_tiles);
   char* trn = take(sizeof(int) * max_tiles);
@@ -642,7 +651,12 @@ size_t prefill_bytes(const gemq_moe_layer_t* L, int tokens, PrefillScratch* S, c
     S->plan.tile_rows = reinterpret_cast<int*>(trn);
     S->plan.inv = reinterpret_cast<int*>(inv);
     S->row_w = roww; S->xs = xs; S->h = h; S->ys = ys; S->hs = hs; S->yss = yss; S->xh = xh;
+    S->few = base ? base + few_at : nullptr;
     S->max_tiles = max_tiles;
+  }
+  if (few::moe_few_rows_ok(L, tokens)) {
+    const size_t n = few_at + few::moe_few_rows_bytes(L, tokens);
+    off = n > off ? n : off;
   }
   return off;
 }
@@ -709,6 +723,8 @@ extern "C" int gemq_moe_prefill(const gemq_moe_layer_t* L, const void* x, void* 
     const int rc = gemq_moe_route(x, gate, tokens, D, E, A, route_mode, L->renorm, x_is_bf16, idx, w, logits, stream);
     if (rc) return rc;
   }
+  if (few::moe_few_rows_ok(L, tokens))
+    return few::moe_few_rows(L, x, out, reinterpret_cast<const long long*>(idx), w, tokens, bf, S.few, S.err, st);
   prefill_zero_kernel<<<cdiv(E + 2, 256), 256, 0, st>>>(S.plan, E);
   cudaMemsetAsync(S.err, 0, sizeof(int), st);
   prefill_count_kernel<<<cdiv(R, 256), 256, 0, st>>>(S.plan, reinterpret_cast<const long long*>(idx), R, E, S.err);

@@ -40,3 +40,23 @@ def test_linear_rows_edges(b, N, K, dtype):
     wide = torch.from_numpy(rng.standard_normal((5, K + 3))).to(dtype).cuda()[:, 1:K + 1]
     assert torch.equal(quant_linear(wide, wq, s, z, b, 128, None), quant_linear(wide.contiguous(), wq, s, z, b, 128, None))
     assert int(error_word(y.device).item()) == 0
+
+
+@pytest.mark.parametrize("bits", [[1, 2, 3, 4], [3, 3, 3, 3], [1, 1, 4, 1]])
+@pytest.mark.parametrize("D,Fd", [(256, 512), (640, 384), (1408, 896)])
+def test_moe_few_rows_edges(bits, D, Fd):
+    layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=4, A=2, bits=bits, seed=9, gate_std=0.02)
+    blk = MF.gpu_block(layer)
+    w1, w3, w2, _ = MF.oracle_parts(layer)
+    g = torch.Generator().manual_seed(D)
+    for T, one in ((2, False), (5, True), (9, True), (17, True), (24, False)):
+        x = torch.randn(T, D, generator=g).half()
+        # `one`: every token picks expert 2 and one other, so one expert crosses the tile sizes
+        sel = torch.stack([torch.tensor([2, int(torch.randint(0, 2, (1,), generator=g))]) if one
+                           else torch.randperm(4, generator=g)[:2] for _ in range(T)])
+        w = torch.softmax(torch.randn(T, 2, generator=g), -1).half()
+        out = blk._prefill(x.cuda(), 1, True, routing=(w.cuda(), sel.cuda()))[0]
+        assert blk.prefill_error_code(T) == 0
+        ref = O.moe_reference_fp32(x, w.float(), sel, w1, w3, w2).numpy()
+        assert rel_fro(out.float().cpu().numpy(), ref) < REL_FRO_TOL
+        assert torch.equal(out, blk._prefill(x.cuda(), 1, True, routing=(w.cuda(), sel.cuda()))[0])
