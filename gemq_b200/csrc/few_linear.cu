@@ -182,15 +182,16 @@ __device__ __forceinline__ void consume_linear(State<NB>& A, LinearShared& S, co
   if (B == 3) build_b3<T>(P, tab, x, rows, lo, hi, lane);
   else build_pow2<T, B == 3 ? 2 : B>(P, tab, x, rows, lo, hi, lane);
   __syncwarp();
+  const uint32_t zero = smem_u32(S.zero), tab32 = smem_u32(tab), ring32 = smem_u32(ring);
   int slot = 0;
   uint32_t par = 0;
 #pragma unroll 1
   for (int it = 0; it < iters; ++it) {
-    const unsigned char* st = ring + slot * kLinStage;
+    const uint32_t st = ring32 + slot * kLinStage;
     wait_bar(&S.full[slot], par, P.err, kErrFewFull);
     const int sg = lo + it;
     if (sg < hi)
-      stage_any<B, NB, kStrip>(A, st + warp * 2 * kStrip, tab + it * table_stage_bytes(B, rows), S.zero, st + kWStage + warp * 1024,
+      stage_any<B, NB, kStrip>(A, st + warp * 2 * kStrip, tab32 + it * table_stage_bytes(B, rows), zero, st + kWStage + warp * 1024,
                                rows, sg, P.K / kGroup, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive(&S.empty[slot]);

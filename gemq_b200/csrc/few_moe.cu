@@ -2,7 +2,7 @@
 // (few_rows.cuh has the arithmetic; the large grouped GEMM takes over where the rows per expert make the
 // tensor cores the better place).
 //
-//   plan     one CTA: rows grouped by expert in tiles of at most 16, experts with the most bytes first
+//   plan     one CTA: rows grouped by expert in tiles of at most 16, the longest first
 //   table    one CTA per row: the activation as tensor-core fragments of the expert's bit width.  Done once
 //            per call: every CTA of the products would otherwise convert all rows for a few columns
 //   up       128 gate and the same 128 up columns per CTA over the whole reduction length; the epilogue
@@ -60,15 +60,16 @@ struct MoeShared {
 template <int MODE> constexpr int kStripStep = MODE == kUp ? kCons * kStrip : kStrip;
 
 template <int MODE, int NB, int B>
-__device__ __forceinline__ void consume_moe(State<NB>& A, MoeShared& S, const MoeParams& P, const unsigned char* ring, int lo, int hi,
-                                            int rows, int ngroups, int warp, int lane) {
+__device__ __forceinline__ void consume_moe(State<NB>& A, MoeShared& S, const MoeParams& P, uint32_t ring, int lo, int hi, int rows,
+                                            int ngroups, int warp, int lane) {
+  const uint32_t zero = smem_u32(S.zero);
   int slot = 0;
   uint32_t par = 0;
 #pragma unroll 1
   for (int sg = lo; sg < hi; ++sg) {
-    const unsigned char* st = ring + slot * P.stage_bytes;
+    const uint32_t st = ring + slot * P.stage_bytes;
     wait_bar(&S.full[slot], par, P.err, kErrFewFull);
-    stage_any<B, NB, kStripStep<MODE>>(A, st + (MODE == kUp ? 1 : 2) * warp * kStrip, st + kWStage + kMetaStage, S.zero,
+    stage_any<B, NB, kStripStep<MODE>>(A, st + (MODE == kUp ? 1 : 2) * warp * kStrip, st + kWStage + kMetaStage, zero,
                                        st + kWStage + warp * 1024, rows, sg, ngroups, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive(&S.empty[slot]);
@@ -82,10 +83,10 @@ __device__ __forceinline__ void run_tile(MoeShared& S, const MoeParams& P, unsig
                                          int lane) {
   State<NB> A;
   clear(A);
-  if (bits == 1) consume_moe<MODE, NB, 1>(A, S, P, ring, lo, hi, rows, ngroups, warp, lane);
-  else if (bits == 2) consume_moe<MODE, NB, 2>(A, S, P, ring, lo, hi, rows, ngroups, warp, lane);
-  else if (bits == 3) consume_moe<MODE, NB, 3>(A, S, P, ring, lo, hi, rows, ngroups, warp, lane);
-  else consume_moe<MODE, NB, 4>(A, S, P, ring, lo, hi, rows, ngroups, warp, lane);
+  if (bits == 1) consume_moe<MODE, NB, 1>(A, S, P, smem_u32(ring), lo, hi, rows, ngroups, warp, lane);
+  else if (bits == 2) consume_moe<MODE, NB, 2>(A, S, P, smem_u32(ring), lo, hi, rows, ngroups, warp, lane);
+  else if (bits == 3) consume_moe<MODE, NB, 3>(A, S, P, smem_u32(ring), lo, hi, rows, ngroups, warp, lane);
+  else consume_moe<MODE, NB, 4>(A, S, P, smem_u32(ring), lo, hi, rows, ngroups, warp, lane);
   const int g = lane >> 2, c = lane & 3;
   if (MODE == kUp) {
     // h of the tile over the drained ring, then half a warp per row turns it into fragments
@@ -125,12 +126,14 @@ __device__ __forceinline__ void run_tile(MoeShared& S, const MoeParams& P, unsig
   }
 }
 
-// MAXNB = 1: tiles of at most eight rows, three CTAs per SM; 2: at most sixteen, two CTAs per SM.
+// MAXNB = 1: tiles of at most eight rows; 2: at most sixteen.
 template <int MODE, int MAXNB>
-__global__ void __launch_bounds__(kThreads, MAXNB == 1 ? 3 : 2) few_moe_kernel(const __grid_constant__ MoeParams P) {
+__global__ void __launch_bounds__(kThreads, 3) few_moe_kernel(const __grid_constant__ MoeParams P) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  __shared__ MoeShared S;
+  // barriers in the first kilobyte, then the ring (1024-byte aligned like the array): three CTAs share an SM's
+  // 228 KB to the last kilobyte
+  MoeShared& S = *reinterpret_cast<MoeShared*>(smem_raw);
+  unsigned char* ring = smem_raw + 1024;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < kMaxRing; ++s) {
@@ -255,8 +258,8 @@ __global__ void __launch_bounds__(kTabThreads) few_table_kernel(const __grid_con
 // ---- permutation of the batch: one CTA -----------------------------------------------------------
 constexpr int kPlanThreads = 512;
 
-// Sorted rows: the experts with the most bytes first (their CTAs start first); the shared expert's tokens
-// come behind the routed rows, its tiles lead the tile list.
+// Sorted rows: the experts whose tiles take longest first (the CTAs start in this order); the shared
+// expert's tokens come behind the routed rows, its tiles lead the tile list.
 template <typename T>
 __global__ void __launch_bounds__(kPlanThreads) few_plan_kernel(Plan pl, const long long* __restrict__ idx, const T* __restrict__ w,
                                                                 const int* __restrict__ nbits, int R, int A, int E, int tokens,
@@ -273,6 +276,9 @@ __global__ void __launch_bounds__(kPlanThreads) few_plan_kernel(Plan pl, const l
     if (e < 0 || e >= E) atomicExch(err, kErrBadExpertId);
     else atomicAdd(&count[static_cast<int>(e)], 1);
   }
+  __syncthreads();
+  // longest first: two blocks of eight rows take twice the MMAs of one, more bits more copying
+  for (int e = tid; e < E; e += kPlanThreads) key[e] += count[e] > 8 ? 8 : 0;
   __syncthreads();
   const int sh_tiles = shared ? cdiv(tokens, tile_rows) : 0;
   for (int e = tid; e < E; e += kPlanThreads) {
@@ -515,7 +521,7 @@ int moe_few_rows(const gemq_moe_layer_t* L, const void* x, void* out, const long
   int tab = 0;
   for (int b = 1; b <= 4; ++b) tab = table_stage_bytes(b, Y.tile_rows) > tab ? table_stage_bytes(b, Y.tile_rows) : tab;
   const int stage = (kWStage + kMetaStage + tab + 1023) / 1024 * 1024;
-  const int ring = nb == 1 ? 2 : 3;
+  const int ring = 2;  // three CTAs per SM
   const size_t smem = 1024 + static_cast<size_t>(ring) * stage;
 
   MoeParams U = {};

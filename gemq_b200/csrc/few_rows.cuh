@@ -7,12 +7,10 @@
 // operands holding two codes (times 2^pos for codes that sit `pos` bits up), and it goes straight
 // into mma.sync.m16n8k16 as the A operand (16 weight columns x 16 k).  The B operand is the
 // activation of eight rows, scaled per row and group by a power of two and per k by 2^-pos: exact.
-// Products are summed per quantisation group in fp32; a closed group is added with its scale and its
-// offset times the group's activation sum.  Per 8192 weights (64 columns, one group) and eight rows: 144
-// to 160 ANDs and shifts -- the ALU pipe takes two cycles for each, which is the arithmetic limit -- 32
-// MMAs, and about 70 instructions to close the group on the otherwise idle FMA pipe.  (One scale per row
-// and the offsets as an extra MMA saved half of those, but the scale of a whole row needs a pass over x
-// before the first fragment can be written.)
+// Products are summed per quantisation group in fp32; a closed group is added with its scale, the offsets
+// times the groups' activation sums come in as one tf32 MMA per stage.  Per 8192 weights (64 columns, one
+// group) and eight rows: 144 to 160 ANDs and shifts -- the ALU pipe takes two cycles for each -- 32 MMAs of
+// eight cycles, and about 50 instructions to close the group on the otherwise idle FMA pipe.
 //
 // A CTA is four consumer warps of 64 columns each and one producer warp that keeps a ring of stages
 // filled.  A stage is 16 packed rows: TMA boxes of 32-column strips (128B swizzle: conflict-free
@@ -72,6 +70,50 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// The first k-step of a group: no accumulators to clear.
+__device__ __forceinline__ void mma16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                               uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// d += z * (hi + lo) over four k slots; fp16 offsets are exact in tf32, the two halves carry 22 bits of a group sum
+__device__ __forceinline__ void mma_offsets(float (&d)[4], float z0, float z1, uint32_t hi, uint32_t lo) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%4,%5}, {%6,%7}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(__float_as_uint(z0)), "r"(__float_as_uint(z1)), "r"(hi), "r"(lo));
+}
+
+// Shared-memory reads by 32-bit address: pointers would be carried as 64 bits.
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+// Two fp32 lanes per instruction.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void mul_add2(float& o0, float& o1, float a0, float a1, unsigned long long f, unsigned long long sc) {
+  unsigned long long t = pack2(a0, a1), o = pack2(o0, o1);
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(t) : "l"(f));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(o) : "l"(t), "l"(sc));
+  asm("mov.b64 {%0,%1}, %2;" : "=f"(o0), "=f"(o1) : "l"(o));
+}
+
 // Operand q of a packed word: two codes in place, `pos` bits up in their half.
 template <int B>
 struct Fmt {
@@ -109,39 +151,64 @@ __device__ __forceinline__ void clear(State<NB>& S) {
         for (int e = 0; e < 4; ++e) S.acc[st][s][nb][e] = S.out[st][s][nb][e] = 0.f;
 }
 
-__device__ __forceinline__ void half4(const unsigned char* p, float (&f)[4]) {
-  const uint2 r = *reinterpret_cast<const uint2*>(p);
+__device__ __forceinline__ void half4(uint32_t p, float (&f)[4]) {
+  const uint2 r = lds64(p);
   const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x));
   const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
 }
 
-// Close a group.  `meta` = its scales and offsets of the warp's 64 columns, `ft` = its (unscale, sum) pairs.
-template <int NB>
-__device__ __forceinline__ void fold(State<NB>& S, const unsigned char* meta, const unsigned char* ft, int rows, int lane) {
+// Close a group: out += scale * acc.  `meta` = its scales and offsets of the warp's 64 columns, `ft` = its
+// (unscale, sum) pairs.  CLEAR: leave the accumulators at zero.
+template <int NB, bool CLEAR>
+__device__ __forceinline__ void fold(State<NB>& S, uint32_t meta, uint32_t ft, int rows, int lane) {
   const int g = lane >> 2, c = lane & 3;
-  float4 fx[NB];  // (unscale, sum) of rows 8 nb + 2 c and the next; rows past the last repeat a valid pair, nobody reads them
+  unsigned long long f[NB];  // of rows 8 nb + 2 c and the next; rows past the last repeat a valid one, nobody reads them
 #pragma unroll
   for (int nb = 0; nb < NB; ++nb) {
-    const int pair = min(4 * nb + c, (rows - 1) >> 1);
-    fx[nb] = *reinterpret_cast<const float4*>(ft + 16 * pair);
+    const uint4 t = lds128(ft + 16 * min(4 * nb + c, (rows - 1) >> 1));
+    f[nb] = pack2(__uint_as_float(t.x), __uint_as_float(t.z));
   }
 #pragma unroll
   for (int st = 0; st < 2; ++st) {
-    float sc[4], zr[4];
+    float sc[4];
     half4(meta + 64 * st + 8 * g, sc);
-    half4(meta + 128 + 64 * st + 8 * g, zr);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned long long s2 = pack2(sc[k], sc[k]);
+      const int s = k >> 1, e = 2 * (k & 1);
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) {
+        mul_add2(S.out[st][s][nb][e], S.out[st][s][nb][e + 1], S.acc[st][s][nb][e], S.acc[st][s][nb][e + 1], f[nb], s2);
+        if (CLEAR) S.acc[st][s][nb][e] = S.acc[st][s][nb][e + 1] = 0.f;
+      }
+    }
+  }
+}
+
+// Offset term of a stage: out += offset * sum(x), its groups in the k slots of one MMA per column pair.
+// `on`: the lane column's group slot exists.
+template <int NB>
+__device__ __forceinline__ void add_offsets(State<NB>& S, uint32_t meta, uint32_t ft, int rows, bool on, int lane) {
+  const int g = lane >> 2, c = lane & 3, re = (rows + 1) & ~1;
+  uint32_t hi[NB], lo[NB];
+#pragma unroll
+  for (int nb = 0; nb < NB; ++nb) {
+    hi[nb] = lo[nb] = 0u;
+    if (on) {
+      const uint32_t v = lds32(ft + (c * re + min(g + 8 * nb, rows - 1)) * 8 + 4);
+      hi[nb] = v & 0xffffe000u;
+      lo[nb] = __float_as_uint(__uint_as_float(v) - __uint_as_float(hi[nb]));
+    }
+  }
+#pragma unroll
+  for (int st = 0; st < 2; ++st) {
+    float zr[4] = {0.f, 0.f, 0.f, 0.f};
+    if (on) half4(meta + c * 256 + 128 + 64 * st + 8 * g, zr);
 #pragma unroll
     for (int s = 0; s < 2; ++s)
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float f = (e & 1) ? fx[nb].z : fx[nb].x, xs = (e & 1) ? fx[nb].w : fx[nb].y;
-          const int k = 2 * s + (e >> 1);
-          S.out[st][s][nb][e] = fmaf(sc[k], S.acc[st][s][nb][e] * f, fmaf(zr[k], xs, S.out[st][s][nb][e]));
-          S.acc[st][s][nb][e] = 0.f;
-        }
+      for (int nb = 0; nb < NB; ++nb) mma_offsets(S.out[st][s][nb], zr[2 * s], zr[2 * s + 1], hi[nb], lo[nb]);
   }
 }
 
@@ -149,11 +216,11 @@ __device__ __forceinline__ void fold(State<NB>& S, const unsigned char* meta, co
 // row stay on the zero block.
 template <int NB>
 struct TablePtr {
-  const unsigned char* p[NB];
-  int step[NB];  // bytes from a piece to the next
+  uint32_t p[NB];
+  uint32_t step[NB];  // bytes from a piece to the next
 };
 template <int NB>
-__device__ __forceinline__ TablePtr<NB> table_ptr(const unsigned char* T, const unsigned char* zero, int rows, int lane) {
+__device__ __forceinline__ TablePtr<NB> table_ptr(uint32_t T, uint32_t zero, int rows, int lane) {
   TablePtr<NB> t;
 #pragma unroll
   for (int nb = 0; nb < NB; ++nb) {
@@ -166,17 +233,17 @@ __device__ __forceinline__ TablePtr<NB> table_ptr(const unsigned char* T, const 
 
 // Word r of the lane in block j (eight packed rows), both strips (STEP bytes apart).
 template <int B, int STEP>
-__device__ __forceinline__ void load_words(uint4 (&w)[2], const unsigned char* W, int j, int r, int g, int c) {
+__device__ __forceinline__ void load_words(uint4 (&w)[2], uint32_t W, int j, int r, int g, int c) {
   const int row = Fmt<B>::row(c, r);
 #pragma unroll
   for (int st = 0; st < 2; ++st)
-    w[st] = *reinterpret_cast<const uint4*>(W + st * STEP + (8 * j + row) * 128 + ((g ^ row) << 4));
+    w[st] = lds128(W + st * STEP + (8 * j + row) * 128 + ((g ^ row) << 4));
 }
 
 // A stage (16 packed rows) of a 1/2/4-bit matrix: 4 / B groups, each eight k-steps of 16.
 template <int B, int NB, int STEP>
-__device__ __forceinline__ void stage_pow2(State<NB>& S, const unsigned char* W, const unsigned char* T, const unsigned char* zero,
-                                           const unsigned char* meta, int rows, int groups, int lane) {
+__device__ __forceinline__ void stage_pow2(State<NB>& S, uint32_t W, uint32_t T, uint32_t zero, uint32_t meta, int rows, int groups,
+                                           int lane) {
   using F = Fmt<B>;
   const int g = lane >> 2, c = lane & 3;
   constexpr int QW = F::kEps / 8;  // pieces per packed word
@@ -194,7 +261,7 @@ __device__ __forceinline__ void stage_pow2(State<NB>& S, const unsigned char* W,
         uint4 b[NB];
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
-          b[nb] = *reinterpret_cast<const uint4*>(t.p[nb]);
+          b[nb] = lds128(t.p[nb]);
           t.p[nb] += t.step[nb];
         }
 #pragma unroll
@@ -208,20 +275,23 @@ __device__ __forceinline__ void stage_pow2(State<NB>& S, const unsigned char* W,
               const uint32_t a0 = F::operand(wv[2 * s], m), a1 = F::operand(wv[2 * s + 1], m);
               const uint32_t a2 = F::operand(wv[2 * s], m + 1), a3 = F::operand(wv[2 * s + 1], m + 1);
 #pragma unroll
-              for (int nb = 0; nb < NB; ++nb)
-                mma16816(S.acc[st][s][nb], a0, a1, a2, a3, h ? b[nb].z : b[nb].x, h ? b[nb].w : b[nb].y);
+              for (int nb = 0; nb < NB; ++nb) {
+                if (wl == 0 && m == 0) mma16816_first(S.acc[st][s][nb], a0, a1, a2, a3, b[nb].x, b[nb].y);
+                else mma16816(S.acc[st][s][nb], a0, a1, a2, a3, h ? b[nb].z : b[nb].x, h ? b[nb].w : b[nb].y);
+              }
             }
           }
         }
       }
     }
-    fold<NB>(S, meta + gi * 256, T + stage_pieces(B) * 64 * rows + gi * 16 * ((rows + 1) >> 1), rows, lane);
+    fold<NB, false>(S, meta + gi * 256, T + stage_pieces(B) * 64 * rows + gi * 16 * ((rows + 1) >> 1), rows, lane);
   }
+  add_offsets<NB>(S, meta, T + stage_pieces(B) * 64 * rows, rows, c < groups, lane);
 }
 
 // Five k-steps over an 8-row block of 3-bit words; `t` moves on by the pass's three pieces.
 template <int NB, int STEP>
-__device__ __forceinline__ void pass_b3(State<NB>& S, const unsigned char* W, TablePtr<NB>& t, int j, int lane) {
+__device__ __forceinline__ void pass_b3(State<NB>& S, uint32_t W, TablePtr<NB>& t, int j, int lane) {
   using F = Fmt<3>;
   const int g = lane >> 2, c = lane & 3;
   uint4 wa[2], wb[2];
@@ -240,7 +310,7 @@ __device__ __forceinline__ void pass_b3(State<NB>& S, const unsigned char* W, Ta
     uint4 b[NB];
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb) {
-      b[nb] = *reinterpret_cast<const uint4*>(t.p[nb]);
+      b[nb] = lds128(t.p[nb]);
       t.p[nb] += t.step[nb];
     }
 #pragma unroll
@@ -267,22 +337,24 @@ __device__ __forceinline__ void pass_b3(State<NB>& S, const unsigned char* W, Ta
 // blocks 1, 3, 4, 6 of the run and at its end.  A block with two groups takes two passes whose table
 // entries hold only the one or the other.  `s4` = stage of the run, `left` = groups from the run's first on.
 template <int NB, int STEP>
-__device__ __forceinline__ void stage_b3(State<NB>& S, const unsigned char* W, const unsigned char* T, const unsigned char* zero,
-                                         const unsigned char* meta, int rows, int s4, int left, int lane) {
-  const unsigned char* ft = T + stage_pieces(3) * 64 * rows;
+__device__ __forceinline__ void stage_b3(State<NB>& S, uint32_t W, uint32_t T, uint32_t zero, uint32_t meta, int rows, int s4, int left,
+                                         int lane) {
+  const uint32_t ft = T + stage_pieces(3) * 64 * rows;
   const bool late = s4 >= 2;  // the group ends in the stage's first block, not in its second
   TablePtr<NB> t = table_ptr<NB>(T, zero, rows, lane);
 #pragma unroll 1
   for (int p = 0; p < 3; ++p) {
     pass_b3<NB, STEP>(S, W, t, late ? p >> 1 : (p + 1) >> 1, lane);
-    if (p == (late ? 0 : 1) && s4 < left) fold<NB>(S, meta, ft, rows, lane);
+    if (p == (late ? 0 : 1) && s4 < left) fold<NB, true>(S, meta, ft, rows, lane);
   }
-  if (s4 == 3 && left > 4) fold<NB>(S, meta + 256, ft + 16 * ((rows + 1) >> 1), rows, lane);
+  if (s4 == 3 && left > 4) fold<NB, true>(S, meta + 256, ft + 16 * ((rows + 1) >> 1), rows, lane);
+  const int c = lane & 3;
+  add_offsets<NB>(S, meta, ft, rows, (c == 0 && s4 < left) || (c == 1 && s4 == 3 && left > 4), lane);
 }
 
 template <int B, int NB, int STEP>
-__device__ __forceinline__ void stage_any(State<NB>& S, const unsigned char* W, const unsigned char* T, const unsigned char* zero,
-                                          const unsigned char* meta, int rows, int sg, int ngroups, int lane) {
+__device__ __forceinline__ void stage_any(State<NB>& S, uint32_t W, uint32_t T, uint32_t zero, uint32_t meta, int rows, int sg, int ngroups,
+                                          int lane) {
   if (B == 3) stage_b3<NB, STEP>(S, W, T, zero, meta, rows, sg & 3, ngroups - 5 * (sg >> 2), lane);
   else stage_pow2<B == 3 ? 2 : B, NB, STEP>(S, W, T, zero, meta, rows, min(4 / B, ngroups - (4 / B) * sg), lane);
 }
