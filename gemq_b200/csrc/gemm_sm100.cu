@@ -29,6 +29,10 @@
 
 namespace gemq {
 
+// route.cu
+int route_tokens(const void* x, const void* gate, bool gate_half, int tokens, int D, int E, int A, int mode, int renorm, bool bf16,
+                 int64_t* idx, void* weights, void* logits, bool logits_act, cudaStream_t stream);
+
 namespace few {  // few_moe.cu
 bool moe_few_rows_ok(const gemq_moe_layer_t* L, int tokens);
 size_t moe_few_rows_bytes(const gemq_moe_layer_t* L, int tokens);
@@ -704,7 +708,7 @@ extern "C" size_t gemq_moe_prefill_scratch_bytes(const gemq_moe_layer_t* L, int 
 }
 
 extern "C" int gemq_moe_prefill(const gemq_moe_layer_t* L, const void* x, void* out, int64_t* idx, void* w,
-                                float* logits, int tokens, int do_route, int route_mode, int x_is_bf16,
+                                void* logits, int tokens, int do_route, int route_mode, int x_is_bf16,
                                 void* scratch, size_t scratch_bytes, gemq_stream_t stream) {
   if (!L || !x || !out || !idx || !w || !scratch || tokens <= 0) return GEMQ_ERR_BAD_ARG;
   const int D = L->hidden, F = L->ffn, A = L->top_k, E = L->n_experts, SF = L->shared_ffn, G = L->group_size;
@@ -719,8 +723,7 @@ extern "C" int gemq_moe_prefill(const gemq_moe_layer_t* L, const void* x, void* 
   const int R = tokens * A;
 
   if (do_route) {
-    const void* gate = L->gate;
-    const int rc = gemq_moe_route(x, gate, tokens, D, E, A, route_mode, L->renorm, x_is_bf16, idx, w, logits, stream);
+    const int rc = route_tokens(x, L->gate, true, tokens, D, E, A, route_mode, L->renorm, bf, idx, w, logits, do_route == 2, st);
     if (rc) return rc;
   }
   if (few::moe_few_rows_ok(L, tokens))

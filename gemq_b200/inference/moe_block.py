@@ -20,7 +20,7 @@ from torch import Tensor
 
 from .. import _capi
 from ..kernels import dequant_gemm, dequant_group_gemm
-from ..kernels._ops import library_op
+from ..kernels._ops import library_op, plain_call
 from ..kernels._runtime import require_cuda, stream_ptr
 from .packed_linear import is_packed_linear
 
@@ -178,7 +178,8 @@ class _QuantFusedMoEBase(nn.Module):
         out = _moe_prefill_routed(x, routing[0], routing[1], self._handle, route_mode, renorm)
         return out, routing[0], routing[1], None
 
-    def _prefill_impl(self, x: Tensor, route_mode: int, renorm: bool, routing=None):
+    def _prefill_impl(self, x: Tensor, route_mode: int, renorm: bool, routing=None, logits_dtype=torch.float32):
+        """``logits_dtype``: fp32, x's dtype, or None (no logits are wanted)."""
         dev = require_cuda(x)
         x = x.contiguous()
         T = x.shape[0]
@@ -189,20 +190,16 @@ class _QuantFusedMoEBase(nn.Module):
         out = torch.empty_like(x)
         if routing is not None:
             w, idx = routing[0].contiguous(), routing[1].contiguous()
-            logits = torch.empty((T, self.num_experts), dtype=torch.float32, device=dev)
-            do_route = 0
-        elif bf:  # the library's router reads the fp16 gate of the layer: route here with a bf16 copy
-            w, idx, logits = self._route(x, route_mode, renorm)
-            do_route = 0
+            logits, do_route = None, 0
         else:
             idx = torch.empty((T, self.top_k), dtype=torch.int64, device=dev)
             w = torch.empty((T, self.top_k), dtype=x.dtype, device=dev)
-            logits = torch.empty((T, self.num_experts), dtype=torch.float32, device=dev)
-            do_route = 1
+            logits = torch.empty((T, self.num_experts), dtype=logits_dtype, device=dev) if logits_dtype is not None else None
+            do_route = 1 if logits_dtype == torch.float32 else 2
         sc = self._prefill_scratch
         _capi.check("gemq_moe_prefill", _capi.lib.gemq_moe_prefill(
-            C.byref(self._layer), x.data_ptr(), out.data_ptr(), idx.data_ptr(), w.data_ptr(), logits.data_ptr(),
-            T, do_route, route_mode, int(bf), sc.data_ptr(), sc.numel(), stream_ptr(dev)))
+            C.byref(self._layer), x.data_ptr(), out.data_ptr(), idx.data_ptr(), w.data_ptr(),
+            logits.data_ptr() if logits is not None else None, T, do_route, route_mode, int(bf), sc.data_ptr(), sc.numel(), stream_ptr(dev)))
         return out, w, idx, logits
 
     def prefill_error_code(self, tokens: int) -> int:
@@ -293,7 +290,10 @@ class QuantFusedMixtralMoEBlock(_QuantFusedMoEBase):
         b, s, d = hidden_states.shape
         x = hidden_states.reshape(-1, d)
         if self._prefill_ok() and x.dtype in (torch.float16, torch.bfloat16):
-            out, _, _, logits = self._prefill(x, ROUTE_FP32_SOFTMAX, True)
+            if plain_call(x):  # the router writes the logits in the activation dtype
+                out, _, _, logits = self._prefill_impl(x, ROUTE_FP32_SOFTMAX, True, logits_dtype=x.dtype)
+            else:
+                out, _, _, logits = self._prefill(x, ROUTE_FP32_SOFTMAX, True)
             return out.reshape(b, s, d), logits.to(hidden_states.dtype)
         raise self._unsupported(x)
 
@@ -376,7 +376,10 @@ class QuantFusedDeepseekV2MoEBlock(_QuantFusedMoEBase):
             out, _, _ = self._decode(xh.contiguous(), ROUTE_FP32)
             return out.to(hidden_states.dtype).reshape(b, s, d)
         if grouped:
-            out, _, _, _ = self._prefill(x, ROUTE_FP32, bool(self.norm_topk_prob))
+            if plain_call(x):
+                out = self._prefill_impl(x, ROUTE_FP32, bool(self.norm_topk_prob), logits_dtype=None)[0]
+            else:
+                out, _, _, _ = self._prefill(x, ROUTE_FP32, bool(self.norm_topk_prob))
             return out.reshape(b, s, d)
         raise self._unsupported(x)
 

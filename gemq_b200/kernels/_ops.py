@@ -15,10 +15,11 @@ import torch
 NAMESPACE = "gemq_b200"
 
 
-def _plain(args) -> bool:
-    """No tracing mode is active and the first argument is an ordinary tensor: nobody but the
+def plain_call(x) -> bool:
+    """No compiler and no tracing mode is active and ``x`` is an ordinary tensor: nobody but the
     caller looks at this call, so the operator registry has nothing to add to it."""
-    return torch._C._len_torch_dispatch_stack() == 0 and type(args[0]) in (torch.Tensor, torch.nn.Parameter)
+    return (not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0 and
+            type(x) in (torch.Tensor, torch.nn.Parameter))
 
 
 def library_op(name: str, fake):
@@ -35,7 +36,7 @@ def library_op(name: str, fake):
 
         @functools.wraps(fn)
         def call(*args, **kwargs):
-            if torch.compiler.is_compiling() or not args or not _plain(args):
+            if not args or not plain_call(args[0]):
                 return overload(*args, **kwargs)
             return fn(*args, **kwargs)
 

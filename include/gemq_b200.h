@@ -219,10 +219,10 @@ size_t gemq_moe_prefill_scratch_bytes(const gemq_moe_layer_t* layer, int tokens)
  * pairs into expert-sorted rows, grouped gate/up GEMM with the SiLU*mul epilogue, grouped down
  * GEMM scaled by the routing weight, per-token combine in expert order, shared experts.
  * x, out: [tokens, D] fp16 or bf16; idx int64 [tokens, A]; w [tokens, A] in the activation dtype;
- * logits fp32 [tokens, E] or NULL.  With do_route the gate of `layer` (fp16) is used, so bf16
- * callers route first (gemq_moe_route) and pass do_route = 0. */
+ * logits [tokens, E] or NULL: fp32 with do_route = 1, the activation type with do_route = 2.  The
+ * router uses the fp16 gate of `layer`, rounded to bf16 for bf16 activations. */
 int gemq_moe_prefill(const gemq_moe_layer_t* layer, const void* x, void* out, int64_t* idx, void* w,
-                     float* logits, int tokens, int do_route, int route_mode, int x_is_bf16,
+                     void* logits, int tokens, int do_route, int route_mode, int x_is_bf16,
                      void* scratch, size_t scratch_bytes, gemq_stream_t stream);
 
 /* Device address of the error word gemq_moe_prefill writes in `scratch` (0 = every wait was met). */
