@@ -61,6 +61,7 @@ _SIGNATURES = {
     "gemq_moe_route": (_I, [_P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P]),
     "gemq_moe_decode_scratch_bytes": (_Z, [C.POINTER(MoeLayer)]),
     "gemq_dequant_gemm_tc": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _P, _P]),
+    "gemq_linear_gemm": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P]),
     "gemq_linear_rows": (_I, [_P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P]),
     "gemq_moe_prefill_scratch_bytes": (_Z, [C.POINTER(MoeLayer), _I]),
     "gemq_moe_prefill": (_I, [C.POINTER(MoeLayer), _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _Z, _P]),

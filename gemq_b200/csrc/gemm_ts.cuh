@@ -1,0 +1,595 @@
+// De-quantising GEMM on the 5th-generation tensor cores with the weights as the TMEM operand.
+//
+//   D[128 weight columns, tokens] += W^T[128 columns, k] (tensor memory) * X^T[k, tokens] (shared memory)
+//
+// What bounds it.  With activations as the row operand both operands stood in shared memory, which
+// moved 1280 cycles' worth of bytes per 1024 cycles of MMAs (both operands written once, the weight tile
+// read once per 128 rows), and a CTA spent 390 instructions on 64 weights: 0.6 of the tensor peak.  Here
+// the producers put the de-quantised weights straight from their registers into tensor memory (tcgen05.st;
+// thread = weight column = TMEM lane) and shared memory only carries the activations.  The weights are
+// de-quantised exactly as the reference does, fp16(fma(q, s, z)): three instructions per two weights when
+// the activations come in the order in which the codes lie in a word (no byte permutes; the kernels
+// that write the activations of the MoE layers store them so), four in natural order.
+//
+// Two CTAs of a cluster (one per SM, persistent) work on a tile of 256 weight columns and up to 256 tokens as one
+// cta_group::2 MMA: each holds 128 columns of the weights and of the fp32 result in its tensor memory and
+// half of the tokens in its shared memory.  (One CTA alone on 128 columns x 256 tokens reads 64 bytes a cycle of
+// activations out of shared memory and has to bring in as many: 128 bytes a cycle, all shared memory can do;
+// 660 instead of 512 cycles per k-block.)  Tiles of the gate/up pass hold 64 gate and the same 64 up
+// columns per CTA, 16 + 16 per warp, so that a shuffle brings them together.
+//   16 producer warps  four groups that take 64-wide k-blocks in turn: fetch packed words a block of the group
+//                      ahead, de-quantise 64 k x 32 columns per warp, store them to the A ring; they
+//                      also drain the accumulators: first the next tile's first stages are produced,
+//                      so the MMAs go on while the epilogue computes and stores
+//   1 TMA warp         activation boxes of 128, 64 or 32 tokens x 64 k (128B swizzle; an instruction takes about
+//                      100 cycles to issue)
+//   1 MMA warp         (first CTA) issues tcgen05.mma and the commits that free the ring stages
+// Every wait is bounded.
+#pragma once
+
+#include <type_traits>
+
+#include "gemv.cuh"
+#include "ptx.cuh"
+
+namespace gemq {
+namespace ts {
+
+constexpr int kBK = 64;            // k-block
+constexpr int kCols = 128;         // weight columns of a CTA = TMEM lanes
+constexpr int kTokens = 256;       // most tokens of a tile
+constexpr int kStages = 8;
+constexpr int kProducers = 16;
+constexpr int kGroups = kProducers / 4;
+constexpr int kThreads = 32 * (kProducers + 2);
+constexpr int kRowBytes = kBK * 2;  // of a k-block
+constexpr int kStageBytes = kTokens / 2 * kBK * 2;  // half of the tokens
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kTmemA = 256;   // A ring behind the accumulators: 32 columns per stage
+
+enum { kErrFull = 11, kErrEmpty = 13, kErrAcc = 14, kErrDrained = 15 };
+enum { kOutUp = 0,      // silu(gate) * up, fp16, stored in the order of the down projection's words
+       kOutDown = 1,    // times the row's routing weight, fp16
+       kOutLinear = 2   // activation type
+};
+
+// One matrix family of a launch: routed experts, or the shared expert.
+struct Family {
+  const uint32_t* wq[2];
+  const __half* scales[2];
+  const __half* zeros[2];
+  const int* nbits;          // [E] or nullptr -> bits
+  const int* wq_strides;     // [E] or nullptr
+  const int* zs_strides[2];  // [E] or nullptr -> e * (K / G) * N
+  const int* out_nbits;      // up: bit widths of the matrices that read h, or nullptr -> out_bits
+  int bits, out_bits;
+  int N, K, G;               // row pitch of the packed words, reduction length, group size
+  int col_tiles;             // tiles (of a CTA pair) along N
+  void* out;                 // row 0 of the family's output rows
+  int row0;                  // first sorted row of the family: its output row 0
+};
+
+struct alignas(64) Params {
+  CUtensorMap b_map[2][3]; // activations per family, boxes of 128, 64, 32 rows x 64, 128B swizzle
+  Family fam[2];
+  const int4* tiles;       // {expert (-1: shared), first row, rows, 0}, shared tiles first; nullptr: linear
+  const int* n_tiles;
+  int shared_tiles;
+  const long long* expert; // linear: expert id read on the device, or nullptr -> 0
+  int rows, tile_rows;     // linear: rows, tokens per tile
+  const __half* row_w;     // down: routing weight per sorted row
+  const void* bias;        // linear
+  int* err;
+};
+
+struct Smem {
+  alignas(1024) unsigned char b[kStages][kStageBytes];
+  alignas(16) unsigned char out[4][64 * kCols * 2];  // result rows of a quarter of the tokens
+  alignas(8) unsigned long long full[kStages], empty[kStages], acc_full, drained;
+  uint32_t tmem_base;
+};
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(on));
+  return on != 0;
+}
+
+// ---- tcgen05 forms used here --------------------------------------------------------------------
+// D[tmem] (+)= A[tmem] * B[smem] over the CTA pair; issued by one thread of the first CTA.
+__device__ __forceinline__ void umma_ts_f16(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+      "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// 32 lanes x 32 columns from registers: thread i writes lane (base + i).
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
+      "%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+      "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
+      "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void wait_bar(unsigned long long* bar, uint32_t parity, int* err, int code) {
+  for (int i = 0; i < kSpinLimit; ++i)
+    if (mbar_try_wait(bar, parity)) return;
+  atomicExch(err, code);
+}
+
+// ---- the CTA pair --------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t pair_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void pair_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The first CTA's copy of a barrier, as a cluster address.
+__device__ __forceinline__ uint32_t first_cta(const unsigned long long* bar) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(bar)));
+  return a;
+}
+// What is handed over lies in tensor memory and is complete (tcgen05.wait) before this: a release at cluster
+// scope would also wait for the packed words in flight, 1500 cycles per k-block.
+__device__ __forceinline__ void arrive_at(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Arrive at the barrier of both CTAs once the pair's MMAs issued so far have completed.
+__device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                   smem_u32(bar)),
+               "h"(static_cast<unsigned short>(3))
+               : "memory");
+}
+// Box into this CTA's shared memory; its bytes count on a barrier of the first CTA (cluster address).
+__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+
+// ---- de-quantisation -----------------------------------------------------------------------------
+template <bool BF16>
+__device__ __forceinline__ uint32_t act2(__half2 v) {
+  if (BF16) {
+    const float2 f = __half22float2(v);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
+    return *reinterpret_cast<const uint32_t*>(&b);
+  }
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ uint32_t u32(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ __half2 h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
+
+// W^T[k, n] = fp16(fma(fp16(q), s, z)) (gemq/triton_kernels/utils.py:206-210).  `bits` = one code in each half,
+// POS bits up.  Under the exponent of 2^(10 - POS) the code counts in units of one: the half reads
+// 2^(10 - POS) + q, and one exact subtraction leaves q.
+template <int POS>
+__device__ __forceinline__ __half2 dequant2(uint32_t bits, __half2 s2, __half2 z2) {
+  constexpr uint32_t EXP = (0x6400u - (static_cast<uint32_t>(POS) << 10)) * 0x00010001u;
+  const __half2 q = __hsub2(h2(bits | EXP), __float2half2_rn(static_cast<float>(1 << (10 - POS))));
+  return __hfma2(q, s2, z2);
+}
+
+template <int B, int Q>
+__device__ __forceinline__ __half2 word_pair(uint32_t w, __half2 s2, __half2 z2) {
+  constexpr int NPOS = 10 / B, JJ = Q % NPOS, SH = (Q / NPOS) * NPOS * B;
+  constexpr uint32_t MASK = ((1u << B) - 1u) * 0x00010001u;
+  return dequant2<B * JJ>((w >> SH) & (MASK << (B * JJ)), s2, z2);
+}
+
+// 64 codes of a column as 32 TMEM words.  NAT: neighbouring k share a word; else codes q and q + eps / 2 of a
+// packed word do (the activations are stored in that order).
+template <int B, bool BF16, bool NAT, int I, int Q>
+__device__ __forceinline__ void dequant_word(uint32_t (&o)[32], uint32_t w, __half2 s2, __half2 z2) {
+  constexpr int PAIRS = 16 / B;
+  if constexpr (Q < PAIRS) {
+    const __half2 a = word_pair<B, Q>(w, s2, z2);
+    if constexpr (!NAT) {
+      o[I * PAIRS + Q] = act2<BF16>(a);
+      dequant_word<B, BF16, NAT, I, Q + 1>(o, w, s2, z2);
+    } else {
+      const __half2 b = word_pair<B, Q + 1>(w, s2, z2);
+      o[I * PAIRS + Q / 2] = act2<BF16>(h2(__byte_perm(u32(a), u32(b), 0x5410)));
+      o[I * PAIRS + PAIRS / 2 + Q / 2] = act2<BF16>(h2(__byte_perm(u32(a), u32(b), 0x7632)));
+      dequant_word<B, BF16, NAT, I, Q + 2>(o, w, s2, z2);
+    }
+  }
+}
+template <int B, bool BF16, bool NAT, int I>
+__device__ __forceinline__ void dequant_words(uint32_t (&o)[32], const uint32_t* w, __half2 s2, __half2 z2) {
+  if constexpr (I < 2 * B) {
+    dequant_word<B, BF16, NAT, I, 0>(o, w[I], s2, z2);
+    dequant_words<B, BF16, NAT, I + 1>(o, w, s2, z2);
+  }
+}
+
+// 3-bit: a 64-code window starts at an even code of its first word and spans eight words; always natural
+// order.  All 40 pairs are formed, the window is the 32 from pair (k0 mod 10) / 2 on.
+template <bool BF16>
+__device__ __forceinline__ void dequant_b3(uint32_t (&pr)[40], const uint32_t* w, __half2 s2, __half2 z2) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t m = (w[i] & 0x00007fffu) | ((w[i] << 1) & 0x7fff0000u);  // codes 0..4 | 5..9
+    const uint32_t mh = m >> 9;
+    const uint32_t v0 = u32(dequant2<0>(m & 0x00070007u, s2, z2)), v1 = u32(dequant2<3>(m & 0x00380038u, s2, z2));
+    const uint32_t v2 = u32(dequant2<6>(m & 0x01c001c0u, s2, z2)), v3 = u32(dequant2<0>(mh & 0x00070007u, s2, z2));
+    const uint32_t v4 = u32(dequant2<3>(mh & 0x00380038u, s2, z2));
+    pr[5 * i + 0] = act2<BF16>(h2(__byte_perm(v0, v1, 0x5410)));  // codes 0, 1
+    pr[5 * i + 1] = act2<BF16>(h2(__byte_perm(v2, v3, 0x5410)));  // 2, 3
+    pr[5 * i + 2] = act2<BF16>(h2(__byte_perm(v4, v0, 0x7610)));  // 4, 5
+    pr[5 * i + 3] = act2<BF16>(h2(__byte_perm(v1, v2, 0x7632)));  // 6, 7
+    pr[5 * i + 4] = act2<BF16>(h2(__byte_perm(v3, v4, 0x7632)));  // 8, 9
+  }
+}
+
+// A tile of the launch, as one CTA of the pair sees it.
+struct Tile {
+  int fam, expert, row0, rows, col0;
+  // tokens of the MMA (32, 64, ..), of which each CTA brings half
+  __device__ __forceinline__ int n() const { return (rows + 31) & ~31; }
+};
+
+template <int COLS, bool LINEAR>  // COLS: columns of a CTA along N (gate/up: 64)
+__device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Tile& t) {
+  if (LINEAR) {
+    const Family& F = P.fam[0];
+    const int mt = idx / F.col_tiles;
+    if (mt * P.tile_rows >= P.rows) return false;
+    t.fam = 0;
+    t.expert = P.expert ? static_cast<int>(*P.expert) : 0;
+    t.row0 = mt * P.tile_rows;
+    t.rows = min(P.tile_rows, P.rows - t.row0);
+    t.col0 = (2 * (idx - mt * F.col_tiles) + rank) * COLS;
+    return true;
+  }
+  const int sh = P.shared_tiles * P.fam[1].col_tiles;
+  const int fam = idx < sh ? 1 : 0;
+  const int i = fam ? idx : idx - sh;
+  const int ct = P.fam[fam].col_tiles;
+  const int mt = (fam ? 0 : P.shared_tiles) + i / ct;
+  if (mt >= *P.n_tiles) return false;
+  const int4 d = P.tiles[mt];
+  t.fam = fam;
+  t.expert = d.x;
+  t.row0 = d.y;
+  t.rows = d.z;
+  t.col0 = (2 * (i % ct) + rank) * COLS;
+  return true;
+}
+
+// ---- producer ------------------------------------------------------------------------------------
+// k-blocks [kb0, kb1) of a tile; `base` = k-blocks this CTA has handled before the tile.
+// (Out of line, like the epilogue: inlined, the 96 registers of 18 warps spill in the k loop.)
+template <bool UP, bool BF16, bool NAT, int B>
+__device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb0, int kb1, uint32_t tmem) {
+  constexpr int NW = B == 3 ? 8 : 2 * B;  // words of a 64-code window
+  const Family& F = P.fam[T.fam];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int mi = UP ? lane >> 4 : 0;
+  // columns past the end repeat the last one; their results are not stored
+  const int col = UP ? T.col0 + 16 * (warp & 3) + (lane & 15) : min(T.col0 + 32 * (warp & 3) + lane, F.N - 1);
+  const size_t N = F.N;
+  const int ngroups = F.K / F.G;
+  size_t woff = 0, zoff = 0;
+  if (T.expert >= 0 && F.wq_strides) woff = static_cast<size_t>(F.wq_strides[T.expert]);
+  if (T.expert >= 0) {
+    const int* zs = mi ? F.zs_strides[1] : F.zs_strides[0];
+    zoff = zs ? static_cast<size_t>(zs[T.expert]) : static_cast<size_t>(T.expert) * ngroups * N;
+  }
+  const uint32_t* wp = (mi ? F.wq[1] : F.wq[0]) + woff + col;
+  const __half* sp = (mi ? F.scales[1] : F.scales[0]) + zoff + col;
+  const __half* zp = (mi ? F.zeros[1] : F.zeros[0]) + zoff + col;
+  // Parameters used in the loop live in registers: through the reference every use is a load.
+  const int G = F.G, K = F.K;
+  int* const err = P.err;
+  const int gshift = (G & (G - 1)) == 0 ? __ffs(G) - 1 : -1;
+  // first k-block of this warp's group at or after kb0
+  int kb = kb0 + static_cast<int>(((warp >> 2) + kGroups - (base + kb0) % kGroups) % kGroups);
+  if (kb >= kb1) return;
+  struct Set { uint32_t w[NW]; __half s, z; };
+  Set cur, nxt;
+  if (B != 3) wp += static_cast<size_t>(kb) * (2 * B) * N;
+  auto fetch = [&](Set& R, int k) {  // blocks in order
+    const int k0 = k * kBK;
+    const int g = gshift >= 0 ? k0 >> gshift : k0 / G;
+    if (B == 3) {  // the last window of a matrix may end before its eighth word
+      const int first = k0 / 10, left = (K + 9) / 10 - first;
+      const uint32_t* q = wp + static_cast<size_t>(first) * N;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) R.w[i] = q[static_cast<size_t>(min(i, left - 1)) * N];
+    } else {
+      const uint32_t* q = wp;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        R.w[i] = *q;
+        q += N;
+      }
+      wp += static_cast<size_t>(kGroups * 2 * B) * N;
+    }
+    R.s = sp[static_cast<size_t>(g) * N];
+    R.z = zp[static_cast<size_t>(g) * N];
+  };
+  uint32_t c = base + kb;
+  uint32_t s = c % kStages, par = ((c / kStages) & 1) ^ 1;
+  const uint32_t full0 = first_cta(&S.full[0]);
+  const uint32_t dst0 = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemA;
+  fetch(cur, kb);
+#pragma unroll 1
+  for (; kb < kb1; kb += kGroups) {
+    if (kb + kGroups < kb1) fetch(nxt, kb + kGroups);
+    const __half2 s2 = __half2half2(cur.s), z2 = __half2half2(cur.z);
+    const uint32_t dst = dst0 + s * 32;
+    if (B == 3) {
+      uint32_t pr[40];
+      dequant_b3<BF16>(pr, cur.w, s2, z2);
+      wait_bar(&S.empty[s], par, err, kErrEmpty);
+      tc_fence_after_sync();
+      switch ((kb * kBK % 10) >> 1) {  // uniform
+        case 0: tmem_st32(dst, pr); break;
+        case 1: tmem_st32(dst, pr + 1); break;
+        case 2: tmem_st32(dst, pr + 2); break;
+        case 3: tmem_st32(dst, pr + 3); break;
+        default: tmem_st32(dst, pr + 4); break;
+      }
+    } else {
+      uint32_t o[32];
+      dequant_words<B == 3 ? 2 : B, BF16, NAT, 0>(o, cur.w, s2, z2);
+      wait_bar(&S.empty[s], par, err, kErrEmpty);
+      tc_fence_after_sync();
+      tmem_st32(dst, o);
+    }
+    tmem_wait_st();
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) arrive_at(full0 + s * 8);
+    s += kGroups;
+    if (s >= kStages) { s -= kStages; par ^= 1u; }
+    cur = nxt;
+  }
+}
+
+template <bool UP, bool BF16, bool NAT>
+__device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb0, int kb1, uint32_t tmem) {
+  const Family& F = P.fam[T.fam];
+  const int bits = F.nbits && T.expert >= 0 ? F.nbits[T.expert] : F.bits;
+  if (bits == 1) produce<UP, BF16, NAT, 1>(S, P, T, base, kb0, kb1, tmem);
+  else if (bits == 2) produce<UP, BF16, NAT, 2>(S, P, T, base, kb0, kb1, tmem);
+  else if (bits == 3) produce<UP, BF16, NAT, 3>(S, P, T, base, kb0, kb1, tmem);
+  else produce<UP, BF16, NAT, 4>(S, P, T, base, kb0, kb1, tmem);
+}
+
+// ---- epilogue: warp w owns TMEM lanes (= columns) 32 (w & 3) .. + 31 and tokens 64 (w >> 2) .. + 63 ----
+template <typename T> __device__ __forceinline__ float as_float(T v);
+template <> __device__ __forceinline__ float as_float<__half>(__half v) { return __half2float(v); }
+template <> __device__ __forceinline__ float as_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+template <typename T> __device__ __forceinline__ T as_act(float v);
+template <> __device__ __forceinline__ __half as_act<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 as_act<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+
+// 32 lanes x 16 columns into registers.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The four warps of a token quarter gather their columns in shared memory and store whole rows, 16 bytes a lane.
+// Short loops on purpose: the code runs once per tile, straight-line it took 7 us of instruction fetches.
+template <int OUT, typename T>
+__device__ __noinline__ void epilogue(Smem& S, const Params& P, const Tile& t, uint32_t tmem, uint32_t parity) {
+  constexpr int ROW = OUT == kOutUp ? kCols / 2 : kCols;  // columns of a staged row
+  const Family& F = P.fam[t.fam];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lq = warp & 3, tq = warp >> 2;
+  const int rows = min(64, t.rows - 64 * tq);  // valid tokens of this quarter
+  T* st = reinterpret_cast<T*>(S.out[tq]);
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + tq) : "memory");  // the rows of the tile before are out
+  wait_bar(&S.acc_full, parity, P.err, kErrAcc);
+  tc_fence_after_sync();
+  const uint32_t at = tmem + (static_cast<uint32_t>(32 * lq) << 16) + 64 * tq;
+  if (OUT == kOutUp) {
+    // Lanes 0..15 hold x1 of 16 columns, lanes 16..31 x3 of the same: per pair of tokens each half gives the
+    // other one value; the lower half forms h of the even token, the upper half of the odd one.
+    // F.silu(x1) * x3 on fp16 tensors: each step is rounded.
+    const bool up = lane >= 16;
+    const int ob = F.out_nbits && t.expert >= 0 ? F.out_nbits[t.expert] : F.out_bits;
+    const int eps = ob == 3 ? 2 : 32 / ob;  // 3-bit matrices read their rows in natural order
+    const int cc = 16 * lq + (lane & 15), j = cc & (eps - 1);
+    T* dst = st + (cc & ~(eps - 1)) + 2 * (j & (eps / 2 - 1)) + (j >= eps / 2 ? 1 : 0) + (up ? ROW : 0);
+#pragma unroll 1
+    for (int c = 0; c < rows; c += 16) {
+      uint32_t d[16];
+      tmem_ld16(at + c, d);
+#pragma unroll
+      for (int i = 0; i < 16; i += 2) {
+        const float mine = __uint_as_float(up ? d[i + 1] : d[i]), give = __uint_as_float(up ? d[i] : d[i + 1]);
+        const float got = __shfl_xor_sync(0xffffffffu, give, 16);
+        const float x1 = __half2float(__float2half_rn(up ? got : mine)), x3 = __half2float(__float2half_rn(up ? mine : got));
+        dst[(c + i) * ROW] = as_act<T>(__half2float(__float2half_rn(silu_f32(x1))) * x3);
+      }
+    }
+  } else {
+    const int col = t.col0 + 32 * lq + lane;
+    float bias = 0.f, rw0 = 1.f, rw1 = 1.f;
+    const bool has_bias = OUT == kOutLinear && P.bias != nullptr;
+    if (has_bias && col < F.N) bias = as_float<T>(static_cast<const T*>(P.bias)[col]);
+    if (OUT == kOutDown && t.fam == 0 && rows > 0) {
+      const __half* rw = P.row_w + t.row0 + 64 * tq;
+      rw0 = __half2float(rw[min(lane, rows - 1)]);
+      rw1 = __half2float(rw[min(lane + 32, rows - 1)]);
+    }
+    T* dst = st + 32 * lq + lane;
+#pragma unroll 1
+    for (int c = 0; c < rows; c += 16) {
+      uint32_t d[16];
+      tmem_ld16(at + c, d);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        T v = as_act<T>(__uint_as_float(d[i]));
+        if (OUT == kOutDown) v = as_act<T>(as_float<T>(v) * __shfl_sync(0xffffffffu, c < 32 ? rw0 : rw1, (c + i) & 31));
+        if (OUT == kOutLinear && has_bias) v = as_act<T>(as_float<T>(v) + bias);
+        dst[(c + i) * ROW] = v;
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncwarp();
+  if (lane == 0) arrive_at(first_cta(&S.drained));  // the next tile's MMAs may overwrite the accumulators
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + tq) : "memory");
+  constexpr int PIECES = ROW / 8;
+  const size_t pitch = F.N;
+  const int cols = F.N - t.col0;  // N is a multiple of 32
+  T* out = static_cast<T*>(F.out) + static_cast<size_t>(t.row0 - F.row0 + 64 * tq) * pitch + t.col0;
+#pragma unroll 2
+  for (int p = 32 * lq + lane; p < rows * PIECES; p += 128) {
+    const int r = p / PIECES, q = p % PIECES;
+    if (8 * q < cols) *reinterpret_cast<uint4*>(out + r * pitch + 8 * q) = *reinterpret_cast<const uint4*>(st + r * ROW + 8 * q);
+  }
+}
+
+template <int OUT, bool BF16>
+__global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_constant__ Params P) {
+  constexpr bool UP = OUT == kOutUp, LINEAR = OUT == kOutLinear;
+  constexpr int COLS = UP ? kCols / 2 : kCols;
+  using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  Smem& S = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const int warp = threadIdx.x >> 5;
+  const int rank = static_cast<int>(pair_rank());
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&S.full[s], 9);  // in the first CTA: a group's four warps of either CTA, the activation boxes
+      mbar_init(&S.empty[s], 1);
+    }
+    mbar_init(&S.acc_full, 1);
+    mbar_init(&S.drained, 2 * kProducers);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kProducers + 1) tmem_alloc_pair(&S.tmem_base, kTmemCols);
+  tc_fence_before_sync();
+  __syncthreads();
+  pair_sync();
+  tc_fence_after_sync();
+  const uint32_t tmem = S.tmem_base;
+  // Only now: a CTA of the next kernel must not take this SM's tensor memory first.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // The packed words are nobody's result: a linear's producers start on them at once.  Its activations are read,
+  // and with that its results written, after the TMA warp's wait.
+  if (!LINEAR || P.expert || warp == kProducers) asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  const int step = static_cast<int>(gridDim.x >> 1), first = static_cast<int>(blockIdx.x >> 1);
+  Tile t;
+  if (warp < kProducers) {
+    int idx = first, ahead = 0;
+    uint32_t base = 0, n = 0;
+    bool more = get_tile<COLS, LINEAR>(P, idx, rank, t);
+#pragma unroll 1
+    while (more) {
+      const int KB = P.fam[t.fam].K / kBK;
+      produce_any<UP, BF16, LINEAR>(S, P, t, base, ahead, KB, tmem);
+      base += KB;
+      const Tile done = t;
+      idx += step;
+      more = get_tile<COLS, LINEAR>(P, idx, rank, t);
+      ahead = 0;
+      if (more) {
+        ahead = min(kStages, P.fam[t.fam].K / kBK);
+        produce_any<UP, BF16, LINEAR>(S, P, t, base, 0, ahead, tmem);
+      }
+      epilogue<OUT, T>(S, P, done, tmem, n & 1);
+      ++n;
+    }
+  } else if (warp == kProducers) {
+    uint32_t c = 0;
+    const uint32_t full0 = first_cta(&S.full[0]);
+    for (int idx = first; get_tile<COLS, LINEAR>(P, idx, rank, t); idx += step) {
+      const Family& F = P.fam[t.fam];
+      const int KB = F.K / kBK, half = t.n() / 2;
+      // an odd number of 16-row blocks brings the next 16 rows, too
+      const int n128 = half / 128, n64 = (half & 64) / 64, n32 = ((half & 63) + 31) / 32;
+      const uint32_t bytes = (128 * n128 + 64 * n64 + 32 * n32) * kRowBytes;
+      const int row = t.row0 - F.row0 + rank * half;
+      for (int kb = 0; kb < KB; ++kb, ++c) {
+        const uint32_t s = c % kStages;
+        wait_bar(&S.empty[s], ((c / kStages) & 1) ^ 1, P.err, kErrEmpty);
+        if (elect_one()) {
+          if (rank == 0) mbar_arrive_expect_tx(&S.full[s], 2 * bytes);
+          const CUtensorMap* map = P.b_map[t.fam];
+          if (n128) {
+            tma_load_pair(S.b[s], map, kb * kBK, row, full0 + s * 8);
+          } else {
+            if (n64) tma_load_pair(S.b[s], map + 1, kb * kBK, row, full0 + s * 8);
+            for (int b = 0; b < n32; ++b)
+              tma_load_pair(S.b[s] + (64 * n64 + 32 * b) * kRowBytes, map + 2, kb * kBK, row + 64 * n64 + 32 * b, full0 + s * 8);
+          }
+        }
+        __syncwarp();
+      }
+    }
+  } else if (rank == 0) {
+    // The whole warp runs the loop and one elected lane issues: descriptors and addresses stay in uniform
+    // registers.  (In a one-lane branch every tcgen05.mma cost 85 cycles to issue.)
+    uint32_t c = 0, n = 0;
+    const uint64_t desc0 = umma_desc_k_sw128(smem_u32(S.b[0]));
+    for (int idx = first; get_tile<COLS, LINEAR>(P, idx, rank, t); idx += step, ++n) {
+      const int KB = P.fam[t.fam].K / kBK;
+      const uint32_t idesc = umma_idesc_f16(BF16 ? 1 : 0, 2 * kCols, t.n());
+      wait_bar(&S.drained, (n & 1) ^ 1, P.err, kErrDrained);
+      for (int kb = 0; kb < KB; ++kb, ++c) {
+        const uint32_t s = c % kStages;
+        wait_bar(&S.full[s], (c / kStages) & 1, P.err, kErrFull);
+        tc_fence_after_sync();
+        const uint64_t bd = desc0 + s * (kStageBytes >> 4);
+        const uint32_t a = tmem + kTmemA + s * 32;
+        if (elect_one()) {
+#pragma unroll
+          for (int k4 = 0; k4 < kBK / 16; ++k4) umma_ts_f16(tmem, a + k4 * 8, bd + k4 * 2, idesc, k4 != 0 || kb != 0);
+          umma_commit_pair(&S.empty[s]);
+          if (kb == KB - 1) umma_commit_pair(&S.acc_full);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  __syncthreads();
+  pair_sync();  // nobody touches the other's barriers or tensor memory from here on
+  if (warp == kProducers + 1) {
+    tc_fence_after_sync();
+    tmem_dealloc_pair(tmem, kTmemCols);
+  }
+}
+
+// gemm_ts.cu; tiles_bound: most tiles the launch can have
+int launch_up(const Params& P, int tiles_bound, cudaStream_t stream);
+int launch_down(const Params& P, int tiles_bound, cudaStream_t stream);
+int sm_count();
+bool activation_maps(CUtensorMap (&maps)[3], const void* x, int K, long long rows);
+
+}  // namespace ts
+}  // namespace gemq

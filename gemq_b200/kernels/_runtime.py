@@ -76,7 +76,7 @@ def error_word(dev: torch.device) -> torch.Tensor:
 
 def tc_gemm_ok(M: int, N: int, K: int, group_size: int) -> bool:
     """Shapes the tcgen05 GEMM takes; smaller row counts stay on the decode kernel."""
-    return M >= 32 and N % 128 == 0 and K % 64 == 0 and group_size % 64 == 0 and K % group_size == 0
+    return M >= 32 and N % 32 == 0 and K % 64 == 0 and group_size % 64 == 0 and K % group_size == 0
 
 
 def few_rows_ok(w_q, scales, zeros, K: int, N: int, group_size: int) -> bool:

@@ -22,25 +22,33 @@ def _fake_gemm(x, w_q, scales, zeros, nbits, group_size):
     return x.new_empty((M, N), dtype=x.dtype if tc else torch.float16)
 
 
+def _gemm_tc(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int,
+             bias: Optional[Tensor]) -> Tensor:
+    """The tcgen05 GEMM; the arguments have been checked."""
+    x = x.contiguous()
+    M, K = x.shape
+    N = w_q.shape[1]
+    out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    _capi.check("gemq_linear_gemm", _capi.lib.gemq_linear_gemm(
+        x.data_ptr(), None, w_q.data_ptr(), scales.data_ptr(), zeros.data_ptr(), None, None, None, nbits,
+        bias.data_ptr() if bias is not None else None, out.data_ptr(), M, N, K, group_size, int(x.dtype == torch.bfloat16),
+        error_word(x.device).data_ptr(), stream_ptr(x.device)))
+    return out
+
+
 @library_op("dequant_gemm", _fake_gemm)
 def dequant_gemm(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int) -> Tensor:
     """``output[M, N] = x[M, K] @ dequantize(w_q, scales, zeros)``, fp16
     (gemq/triton_kernels/dequant_gemm.py:150-193).  32 rows or more go to the tcgen05 GEMM when
-    N % 128 == 0 and K % 64 == 0; otherwise rows are processed eight at a time by the decode
+    N % 32 == 0 and K % 64 == 0; otherwise rows are processed by the decode
     kernel, in calls of at most 64 rows to bound the split-K workspace."""
     require(x.dim() == 2, "x must be [M, K]")
     M, K = x.shape
     N = w_q.shape[1]
     if tc_gemm_ok(M, N, K, group_size) and x.dtype in (torch.float16, torch.bfloat16):
-        dev = require_cuda(x, w_q, scales, zeros)
+        require_cuda(x, w_q, scales, zeros)
         check_kernel_form(w_q, scales, zeros, K, N, nbits, group_size)
-        x = x.contiguous()
-        out = torch.empty((M, N), dtype=x.dtype, device=dev)
-        _capi.check("gemq_dequant_gemm_tc", _capi.lib.gemq_dequant_gemm_tc(
-            x.data_ptr(), None, w_q.data_ptr(), scales.data_ptr(), zeros.data_ptr(), None, None, None, nbits,
-            out.data_ptr(), M, N, K, group_size, int(x.dtype == torch.bfloat16), error_word(dev).data_ptr(),
-            stream_ptr(dev)))
-        return out
+        return _gemm_tc(x, w_q, scales, zeros, nbits, group_size, None)
     rows = dequant_gemv_rows._init_fn  # the plain function behind the operator
     if M <= _ROW_BLOCK:
         return rows(x, w_q, scales, zeros, nbits, group_size)
@@ -59,10 +67,13 @@ def quant_linear(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: i
     M, K = x.shape
     N = w_q.shape[1]
     half = x.dtype in (torch.float16, torch.bfloat16)
-    if half and not tc_gemm_ok(M, N, K, group_size) and few_rows_ok(w_q, scales, zeros, K, N, group_size):
+    tc = tc_gemm_ok(M, N, K, group_size)
+    if half and (tc or few_rows_ok(w_q, scales, zeros, K, N, group_size)):
         check_kernel_form(w_q, scales, zeros, K, N, nbits, group_size)
         if bias is not None:
             bias = bias.to(device=dev, dtype=x.dtype).contiguous()
+        if tc:
+            return _gemm_tc(x, w_q, scales, zeros, nbits, group_size, bias)
         return linear_rows(x if x.stride(1) == 1 else x.contiguous(), w_q, scales, zeros, nbits, group_size, bias)
     small = M < 32 and x.dtype != torch.float16
     y = dequant_gemm._init_fn(x.to(torch.float16) if small else x, w_q, scales, zeros, nbits, group_size).to(x.dtype)

@@ -195,12 +195,18 @@ int gemq_moe_decode(const gemq_moe_layer_t* layer, const void* x, void* out,
  * y[M, N] = x[M, K] @ deq(W[e]), x and y contiguous fp16 (or bf16 when x_is_bf16; the
  * de-quantised fp16 weights are then rounded to bf16).  `expert` = device pointer to the expert
  * id (NULL: expert 0); nbits / wq_strides / zs_strides may be NULL for a single matrix with
- * fixed_bits.  Needs N % 128 == 0, K % 64 == 0, group_size % 64 == 0.  `err` = one device int32
+ * fixed_bits.  Needs N % 32 == 0, K % 64 == 0, group_size % 64 == 0.  `err` = one device int32
  * that receives a non-zero code if a bounded wait inside the kernel expired. */
 int gemq_dequant_gemm_tc(const void* x, const int64_t* expert, const int32_t* wq, const void* scales,
                          const void* zeros, const int32_t* nbits, const int32_t* wq_strides,
                          const int32_t* zs_strides, int fixed_bits, void* y, int M, int N, int K,
                          int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream);
+
+/* gemq_dequant_gemm_tc with an optional bias [N] of the activation type. */
+int gemq_linear_gemm(const void* x, const int64_t* expert, const int32_t* wq, const void* scales,
+                     const void* zeros, const int32_t* nbits, const int32_t* wq_strides,
+                     const int32_t* zs_strides, int fixed_bits, const void* bias, void* y, int M, int N,
+                     int K, int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream);
 
 /* The same product for a few rows (decode batches; any row count is taken, up to 16 rows per pass
  * over the weights), with an optional bias: y[rows, N] = x @ deq(W) (+ bias), x rows `ldx` elements

@@ -60,3 +60,53 @@ def test_moe_few_rows_edges(bits, D, Fd):
         ref = O.moe_reference_fp32(x, w.float(), sel, w1, w3, w2).numpy()
         assert rel_fro(out.float().cpu().numpy(), ref) < REL_FRO_TOL
         assert torch.equal(out, blk._prefill(x.cuda(), 1, True, routing=(w.cuda(), sel.cuda()))[0])
+
+
+@pytest.mark.parametrize("b", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(32, 128), (288, 640), (576, 1408)])
+def test_gemm_tile_edges(b, N, K):
+    """The tcgen05 GEMM where the last 256-column pair of CTAs is partly or half empty, the k-blocks are fewer
+    than the ring's stages or no multiple of them, and the token count ends inside a 32-row box, fills a tile
+    or goes one past it."""
+    from gemq_b200.kernels import dequant_gemm
+    from gemq_b200.kernels._runtime import error_word
+    from gemq_b200.kernels.dequant_gemm import quant_linear
+    rng = np.random.default_rng(b * 10 + N)
+    lin = MF.draw_linear(rng, N, K, b)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    wq, s, z = t(lin["wq"]), t(lin["s"]), t(lin["z"])
+    W = O.dequantize(lin["wq"], lin["s"], lin["z"], b, 128, K).astype(np.float64)
+    bias = torch.from_numpy(rng.standard_normal(N)).cuda()
+    for M in (32, 33, 255, 256, 257):
+        for dtype in (torch.float16, torch.bfloat16):
+            x = torch.from_numpy(rng.standard_normal((M, K))).to(dtype).cuda()
+            y = dequant_gemm(x, wq, s, z, b, 128)
+            want = x.double().cpu().numpy() @ W
+            # fp16: one rounding of the result.  bf16: the weights are rounded to bf16 as well, errors 2^-9 rms at most
+            # each way
+            tol = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8 + 2.0 ** -9
+            assert rel_fro(y.double().cpu().numpy(), want) < tol, (M, dtype, rel_fro(y.double().cpu().numpy(), want))
+            assert torch.equal(quant_linear(x, wq, s, z, b, 128, bias.to(dtype)), y + bias.to(dtype))
+    assert int(error_word(wq.device).item()) == 0
+
+
+@pytest.mark.parametrize("rows", [[49, 1, 0, 60], [256, 257, 16, 17], [600, 0, 0, 1]])
+@pytest.mark.parametrize("bits", [[1, 2, 3, 4], [3, 4, 1, 2]])
+def test_moe_large_tiles(rows, bits):
+    """Experts with fewer rows than a 32-row box, exactly a tile, one more than a tile, an uneven number of
+    16-row blocks; the second CTA of a pair past the last column (384 = 256 + 128)."""
+    D, Fd = 384, 640
+    layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=4, A=1, bits=bits, seed=5, gate_std=0.02)
+    blk = MF.gpu_block(layer)
+    w1, w3, w2, _ = MF.oracle_parts(layer)
+    g = torch.Generator().manual_seed(sum(rows))
+    sel = torch.cat([torch.full((n,), e, dtype=torch.int64) for e, n in enumerate(rows)])
+    T = sel.numel()
+    sel = sel[torch.randperm(T, generator=g)].view(T, 1)
+    w = (torch.rand(T, 1, generator=g) * 0.5 + 0.5).half()
+    for dtype in (torch.float16, torch.bfloat16):
+        x = torch.randn(T, D, generator=g).to(dtype)
+        out = blk._prefill(x.cuda(), 1, True, routing=(w.to(dtype).cuda(), sel.cuda()))[0]
+        assert blk.prefill_error_code(T) == 0
+        ref = O.moe_reference_fp32(x.float(), w.to(dtype).float(), sel, w1, w3, w2).numpy()
+        assert rel_fro(out.float().cpu().numpy(), ref) < REL_FRO_TOL
