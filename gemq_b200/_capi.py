@@ -62,6 +62,7 @@ _SIGNATURES = {
     "gemq_moe_decode_scratch_bytes": (_Z, [C.POINTER(MoeLayer)]),
     "gemq_dequant_gemm_tc": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _P, _P]),
     "gemq_linear_gemm": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P]),
+    "gemq_linear_takes_gemm": (_I, [_I, _I, _I, _I]),
     "gemq_linear_rows": (_I, [_P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P]),
     "gemq_moe_prefill_scratch_bytes": (_Z, [C.POINTER(MoeLayer), _I]),
     "gemq_moe_prefill": (_I, [C.POINTER(MoeLayer), _P, _P, _P, _P, _P, _I, _I, _I, _I, _P, _Z, _P]),
@@ -95,6 +96,20 @@ def _load() -> C.CDLL:
 
 
 lib = _load()
+
+
+class _NoHost:
+    """Stands in for the native call module when another library was named in the environment (the module is
+    linked to the one next to it): every call goes through ctypes."""
+
+    linear = moe_decode = moe_prefill = staticmethod(lambda *a: None)
+
+
+if os.environ.get("GEMQ_B200_LIB"):
+    host = _NoHost
+else:
+    import torch  # noqa: F401  (its libraries have to be loaded first)
+    from . import _host as host  # noqa: F401
 
 
 def stacked(wq, scales, zeros, nbits, wq_strides, zs_strides=None) -> Stacked:

@@ -1,8 +1,9 @@
-"""Build libgemq_b200.so from the CUDA sources in this directory with nvcc (sm_100a only).
+"""Build libgemq_b200.so from the CUDA sources in this directory with nvcc (sm_100a only), and the
+host-side call module _host.so from host.cpp with g++ against torch's headers.
 
     python -m gemq_b200.csrc.build [--verbose]
 
-The library lands next to the Python package (gemq_b200/libgemq_b200.so).  It is
+Both land next to the Python package (gemq_b200/).  They are
 rebuilt only when a source or header is newer than the library.
 """
 import os
@@ -14,6 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libgemq_b200.so")
+HOST_LIB = os.path.join(PKG, "_host.so")
 SOURCES = ["pack.cu", "tma.cu", "gemv.cu", "gemv_stream.cu", "route.cu", "layer.cu", "decode_fused.cu", "gemm_ts.cu", "prefill.cu", "expert_parallel.cu", "no_alloc.cu",
            "few_linear.cu", "few_moe.cu"]
 HEADERS = ["common.cuh", "gemv.cuh", "few_rows.cuh", "gemm_ts.cuh", "ptx.cuh", os.path.join(ROOT, "include", "gemq_b200.h")]
@@ -27,6 +29,26 @@ def find_nvcc() -> str:
     return nvcc
 
 
+def host_stale() -> bool:
+    if not os.path.exists(HOST_LIB):
+        return True
+    t = os.path.getmtime(HOST_LIB)
+    return any(os.path.getmtime(d) > t for d in (os.path.join(HERE, "host.cpp"), HEADERS[-1], os.path.abspath(__file__)))
+
+
+def build_host() -> None:
+    """g++ host.cpp against the headers of the installed torch; its library is found next to it."""
+    import sysconfig
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    inc = [f"-I{p}" for p in include_paths()] + [f"-I{sysconfig.get_paths()['include']}"]
+    cuda = os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                           *inc, f"-I{cuda}", os.path.join(HERE, "host.cpp"), "-o", HOST_LIB, f"-L{libs}", "-ltorch_python",
+                           "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-L{PKG}", "-l:libgemq_b200.so", "-Wl,-rpath,$ORIGIN"])
+
+
 def is_stale() -> bool:
     if not os.path.exists(LIB):
         return True
@@ -38,6 +60,8 @@ def is_stale() -> bool:
 
 def build(verbose: bool = False, force: bool = False) -> str:
     if not force and not is_stale():
+        if host_stale():
+            build_host()
         return LIB
     nvcc = find_nvcc()
     objdir = os.path.join(HERE, "build")
@@ -62,6 +86,8 @@ def build(verbose: bool = False, force: bool = False) -> str:
     if failed:
         raise RuntimeError("nvcc failed")
     subprocess.check_call([nvcc, "-shared", *ARCH_FLAGS, "-o", LIB, *objs, "-lcudart"])
+    if force or host_stale():
+        build_host()
     return LIB
 
 

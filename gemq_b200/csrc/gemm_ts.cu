@@ -96,6 +96,11 @@ extern "C" int gemq_linear_gemm(const void* x, const int64_t* expert, const int3
   return rc ? rc : launch_status();
 }
 
+extern "C" int gemq_linear_takes_gemm(int rows, int N, int K, int nbits) {
+  (void)N; (void)K; (void)nbits;
+  return rows >= 32;
+}
+
 extern "C" int gemq_dequant_gemm_tc(const void* x, const int64_t* expert, const int32_t* wq, const void* scales,
                                     const void* zeros, const int32_t* nbits, const int32_t* wq_strides,
                                     const int32_t* zs_strides, int fixed_bits, void* y, int M, int N, int K,

@@ -125,12 +125,20 @@ class _QuantFusedMoEBase(nn.Module):
         nbytes = _capi.lib.gemq_moe_decode_scratch_bytes(C.byref(L))
         self._scratch = torch.zeros(nbytes, dtype=torch.uint8, device=dev)
         self._handle = next(_HANDLES)
+        self._layer_ptr = C.addressof(L)
+        self._grouped_ok = self._prefill_ok()
         _BLOCKS[self._handle] = self
 
     # -- forward pieces ----------------------------------------------------------------
     def _decode(self, x: Tensor, route_mode: int):
         """``x [T, D]`` fp16 -> ``out [T, D]``, routing weights and indices, all on the device."""
         return _moe_decode(x, self._handle, route_mode)
+
+    def _host_decode(self, x: Tensor, route_mode: int):
+        """The native call, or None where the wrappers have to go on."""
+        if not plain_call(x):
+            return None
+        return _capi.host.moe_decode(self._layer_ptr, x, self._scratch, self.hidden_dim, self.top_k, route_mode)
 
     def _decode_impl(self, x: Tensor, route_mode: int):
         dev = require_cuda(x)
@@ -289,8 +297,12 @@ class QuantFusedMixtralMoEBlock(_QuantFusedMoEBase):
         """gemq/inference/moe_block.py:165-198."""
         b, s, d = hidden_states.shape
         x = hidden_states.reshape(-1, d)
-        if self._prefill_ok() and x.dtype in (torch.float16, torch.bfloat16):
+        if self._grouped_ok and x.dtype in (torch.float16, torch.bfloat16):
             if plain_call(x):  # the router writes the logits in the activation dtype
+                r = _capi.host.moe_prefill(self._layer_ptr, hidden_states, self._prefill_scratch, self.hidden_dim, self.top_k,
+                                           self.num_experts, ROUTE_FP32_SOFTMAX, True)
+                if r is not None:
+                    return r
                 out, _, _, logits = self._prefill_impl(x, ROUTE_FP32_SOFTMAX, True, logits_dtype=x.dtype)
             else:
                 out, _, _, logits = self._prefill(x, ROUTE_FP32_SOFTMAX, True)
@@ -302,6 +314,9 @@ class QuantFusedMixtralMoEBlock(_QuantFusedMoEBase):
         b, s, d = hidden_states.shape
         x = hidden_states.reshape(-1, self.hidden_dim)
         assert x.shape[0] == 1, f"This function only supports single token forward. But got {x.shape[0]} tokens."
+        y = self._host_decode(hidden_states, ROUTE_FP16)
+        if y is not None:
+            return y, None
         xh = x if x.dtype == torch.float16 else x.to(torch.float16)
         out, _, _ = self._decode(xh.contiguous(), ROUTE_FP16)
         return out.to(hidden_states.dtype).reshape(b, s, d), None
@@ -370,13 +385,20 @@ class QuantFusedDeepseekV2MoEBlock(_QuantFusedMoEBase):
         fused one-token kernels row by row with this path's fp32 routing."""
         b, s, d = hidden_states.shape
         x = hidden_states.reshape(-1, d)
-        grouped = self._prefill_ok() and x.dtype in (torch.float16, torch.bfloat16)
+        grouped = self._grouped_ok and x.dtype in (torch.float16, torch.bfloat16)
         if x.shape[0] <= _MAX_LOOPED_TOKENS or (not grouped and x.shape[0] <= 16):
+            y = self._host_decode(hidden_states, ROUTE_FP32)
+            if y is not None:
+                return y
             xh = x if x.dtype == torch.float16 else x.to(torch.float16)
             out, _, _ = self._decode(xh.contiguous(), ROUTE_FP32)
             return out.to(hidden_states.dtype).reshape(b, s, d)
         if grouped:
             if plain_call(x):
+                r = _capi.host.moe_prefill(self._layer_ptr, hidden_states, self._prefill_scratch, self.hidden_dim, self.top_k,
+                                           self.num_experts, ROUTE_FP32, False)
+                if r is not None:
+                    return r[0]
                 out = self._prefill_impl(x, ROUTE_FP32, bool(self.norm_topk_prob), logits_dtype=None)[0]
             else:
                 out, _, _, _ = self._prefill(x, ROUTE_FP32, bool(self.norm_topk_prob))
@@ -388,6 +410,9 @@ class QuantFusedDeepseekV2MoEBlock(_QuantFusedMoEBase):
         b, s, d = hidden_states.shape
         x = hidden_states.reshape(-1, self.hidden_dim)
         assert x.shape[0] == 1, f"Only supports single token forward. Got {x.shape[0]} tokens."
+        y = self._host_decode(hidden_states, ROUTE_FP32)
+        if y is not None:
+            return y
         xh = x if x.dtype == torch.float16 else x.to(torch.float16)
         out, _, _ = self._decode(xh.contiguous(), ROUTE_FP32)
         return out.to(hidden_states.dtype).reshape(b, s, d)

@@ -11,6 +11,8 @@ import torch
 import torch.nn as nn
 from torch import Tensor
 
+from ..kernels._ops import plain_call
+from ..kernels._runtime import host_linear
 from ..kernels.dequant_gemm import quant_linear
 from .packed_linear import PackedLinear
 
@@ -26,6 +28,10 @@ class QuantLinear(nn.Module):
 
     def forward(self, x: Tensor) -> Tensor:
         """``x [..., in]`` fp16 / bf16 -> ``[..., out]`` in the same dtype."""
+        if plain_call(x):
+            y = host_linear(x, self.W_q, self.scales, self.zeros, self.W_nbits, self.group_size, self.bias, 0)
+            if y is not None:
+                return y
         lead = x.shape[:-1]
         y = quant_linear(x.reshape(-1, self.in_features), self.W_q, self.scales, self.zeros, self.W_nbits, self.group_size,
                          self.bias)

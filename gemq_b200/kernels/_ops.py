@@ -22,12 +22,13 @@ def plain_call(x) -> bool:
             type(x) in (torch.Tensor, torch.nn.Parameter))
 
 
-def library_op(name: str, fake):
+def library_op(name: str, fake, fast=None):
     """``@library_op("name", fake_fn)``: register ``fn`` as ``gemq_b200::name`` (no argument is
     mutated, outputs are fresh tensors) with ``fake_fn`` as its shape/dtype propagation.
 
     A call in eager mode goes straight to ``fn``: the Python dispatch of a custom operator costs
-    20-30 us of host time, more than the kernels of a small call take.  Under ``torch.compile`` and
+    20-30 us of host time, more than the kernels of a small call take.  ``fast`` is tried before it with the
+    positional arguments: native code that returns None for what it does not take.  Under ``torch.compile`` and
     under tracing modes (fake tensors) the call is the operator."""
     def deco(fn):
         op = torch.library.custom_op(f"{NAMESPACE}::{name}", mutates_args=())(fn)
@@ -38,6 +39,10 @@ def library_op(name: str, fake):
         def call(*args, **kwargs):
             if not args or not plain_call(args[0]):
                 return overload(*args, **kwargs)
+            if fast is not None and not kwargs:
+                y = fast(*args)
+                if y is not None:
+                    return y
             return fn(*args, **kwargs)
 
         call._init_fn = fn

@@ -74,6 +74,21 @@ def error_word(dev: torch.device) -> torch.Tensor:
     return t
 
 
+_err_ptrs: dict = {}
+
+
+def host_linear(x, w_q, scales, zeros, nbits, group_size, bias, mode: int):
+    """The native call (csrc/host.cpp) or None.  ``mode``: 0 dense layer, 1 rows operator, 2 one-row operator,
+    3 GEMM operator."""
+    i = x.get_device()
+    p = _err_ptrs.get(i)
+    if p is None:
+        if i < 0:
+            return None
+        p = _err_ptrs[i] = error_word(x.device).data_ptr()
+    return _capi.host.linear(x, w_q, scales, zeros, nbits, group_size, bias, p, mode)
+
+
 def tc_gemm_ok(M: int, N: int, K: int, group_size: int) -> bool:
     """Shapes the tcgen05 GEMM takes; smaller row counts stay on the decode kernel."""
     return M >= 32 and N % 32 == 0 and K % 64 == 0 and group_size % 64 == 0 and K % group_size == 0

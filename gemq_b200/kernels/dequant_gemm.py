@@ -8,7 +8,7 @@ from torch import Tensor
 
 from .. import _capi
 from ._ops import library_op
-from ._runtime import (check_kernel_form, error_word, few_rows_ok, linear_rows, require, require_cuda, stream_ptr,
+from ._runtime import (check_kernel_form, error_word, few_rows_ok, host_linear, linear_rows, require, require_cuda, stream_ptr,
                        tc_gemm_ok)
 from .dequant_gemv import dequant_gemv_rows
 
@@ -36,7 +36,7 @@ def _gemm_tc(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, 
     return out
 
 
-@library_op("dequant_gemm", _fake_gemm)
+@library_op("dequant_gemm", _fake_gemm, lambda *a: host_linear(*a, None, 3) if len(a) == 6 else None)
 def dequant_gemm(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int) -> Tensor:
     """``output[M, N] = x[M, K] @ dequantize(w_q, scales, zeros)``, fp16
     (gemq/triton_kernels/dequant_gemm.py:150-193).  32 rows or more go to the tcgen05 GEMM when
@@ -57,7 +57,8 @@ def dequant_gemm(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: i
 
 
 @library_op("quant_linear",
-            lambda x, w_q, scales, zeros, nbits, group_size, bias: x.new_empty((x.shape[0], w_q.shape[1])))
+            lambda x, w_q, scales, zeros, nbits, group_size, bias: x.new_empty((x.shape[0], w_q.shape[1])),
+            lambda *a: host_linear(*a, 0) if len(a) == 7 else None)
 def quant_linear(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int,
                  bias: Optional[Tensor]) -> Tensor:
     """``x [M, K] @ deq(w_q) + bias`` in x's dtype (fp16 or bf16): what ``QuantLinear`` computes.  Below
@@ -67,7 +68,8 @@ def quant_linear(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: i
     M, K = x.shape
     N = w_q.shape[1]
     half = x.dtype in (torch.float16, torch.bfloat16)
-    tc = tc_gemm_ok(M, N, K, group_size)
+    tc = tc_gemm_ok(M, N, K, group_size) and (
+        not few_rows_ok(w_q, scales, zeros, K, N, group_size) or bool(_capi.lib.gemq_linear_takes_gemm(M, N, K, nbits)))
     if half and (tc or few_rows_ok(w_q, scales, zeros, K, N, group_size)):
         check_kernel_form(w_q, scales, zeros, K, N, nbits, group_size)
         if bias is not None:

@@ -8,7 +8,7 @@ from torch import Tensor
 
 from .. import _capi
 from ._ops import library_op
-from ._runtime import (check_kernel_form, few_rows_ok, gemv_workspace, linear_rows, require, require_cuda,
+from ._runtime import (check_kernel_form, few_rows_ok, gemv_workspace, host_linear, linear_rows, require, require_cuda,
                        stream_ptr)
 
 
@@ -16,7 +16,7 @@ def _fake_rows(x, w_q, scales, zeros, nbits, group_size):
     return x.new_empty((x.shape[0], w_q.shape[1]), dtype=torch.float16)
 
 
-@library_op("dequant_gemv_rows", _fake_rows)
+@library_op("dequant_gemv_rows", _fake_rows, lambda *a: host_linear(*a, None, 1) if len(a) == 6 else None)
 def dequant_gemv_rows(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int) -> Tensor:
     """``x[M, K] @ deq(w_q)`` for a few rows (decode batch); fp16 in, fp16 out."""
     dev = require_cuda(x, w_q, scales, zeros)
@@ -35,7 +35,7 @@ def dequant_gemv_rows(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbi
     return out
 
 
-@library_op("dequant_splitk_gemv", _fake_rows)
+@library_op("dequant_splitk_gemv", _fake_rows, lambda *a: host_linear(*a, None, 2) if len(a) == 6 else None)
 def dequant_splitk_gemv(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int) -> Tensor:
     """``output[1, N] = x[1, K] @ dequantize(w_q, scales, zeros)``
     (gemq/triton_kernels/dequant_gemv.py:118-156).  Unlike the reference's fp16 atomics the

@@ -208,6 +208,9 @@ int gemq_linear_gemm(const void* x, const int64_t* expert, const int32_t* wq, co
                      const int32_t* zs_strides, int fixed_bits, const void* bias, void* y, int M, int N,
                      int K, int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream);
 
+/* Which of the two a dense layer takes: 1 = gemq_linear_gemm, 0 = gemq_linear_rows (a rule on the sizes). */
+int gemq_linear_takes_gemm(int rows, int N, int K, int nbits);
+
 /* The same product for a few rows (decode batches; any row count is taken, up to 16 rows per pass
  * over the weights), with an optional bias: y[rows, N] = x @ deq(W) (+ bias), x rows `ldx` elements
  * apart, x, bias and y fp16 or (x_is_bf16) bf16.  One launch; the packed codes are multiplied in
