@@ -188,7 +188,7 @@ __device__ __forceinline__ void consume_linear(State<NB>& A, LinearShared& S, co
 #pragma unroll 1
   for (int it = 0; it < iters; ++it) {
     const uint32_t st = ring32 + slot * kLinStage;
-    wait_bar(&S.full[slot], par, P.err, kErrFewFull);
+    mbar_sleep_wait(&S.full[slot], par, P.err, kErrFewFull);
     const int sg = lo + it;
     if (sg < hi)
       stage_any<B, NB, kStrip>(A, st + warp * 2 * kStrip, tab32 + it * table_stage_bytes(B, rows), zero, st + kWStage + warp * 1024,
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, NB == 1 ? 3 : 2) few_linear_kernel(c
     int slot = 0;
     uint32_t par = 1;
     for (int it = 0; it < iters; ++it) {
-      wait_bar(&S.empty[slot], par, P.err, kErrFewEmpty);
+      mbar_sleep_wait(&S.empty[slot], par, P.err, kErrFewEmpty);
       unsigned char* st = ring + slot * kLinStage;
       const bool on = box && my_lo + it < my_hi;
       const unsigned boxes = __popc(__ballot_sync(0xffffffffu, on));

@@ -68,7 +68,7 @@ __device__ __forceinline__ void consume_moe(State<NB>& A, MoeShared& S, const Mo
 #pragma unroll 1
   for (int sg = lo; sg < hi; ++sg) {
     const uint32_t st = ring + slot * P.stage_bytes;
-    wait_bar(&S.full[slot], par, P.err, kErrFewFull);
+    mbar_sleep_wait(&S.full[slot], par, P.err, kErrFewFull);
     stage_any<B, NB, kStripStep<MODE>>(A, st + (MODE == kUp ? 1 : 2) * warp * kStrip, st + kWStage + kMetaStage, zero,
                                        st + kWStage + warp * 1024, rows, sg, ngroups, lane);
     __syncwarp();
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 3) few_moe_kernel(const __grid_const
     int slot = 0;
     uint32_t par = 1;
     for (int sg = lo; sg < hi; ++sg) {
-      wait_bar(&S.empty[slot], par, P.err, kErrFewEmpty);
+      mbar_sleep_wait(&S.empty[slot], par, P.err, kErrFewEmpty);
       unsigned char* st = ring + slot * P.stage_bytes;
       if (lane == 0) {
         mbar_arrive_expect_tx(&S.full[slot], kWStage + tb);

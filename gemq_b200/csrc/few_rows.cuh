@@ -365,12 +365,6 @@ __device__ __forceinline__ float4 result4(const State<NB>& S, int st, int nb, in
   return make_float4(S.out[st][0][nb][o], S.out[st][0][nb][2 + o], S.out[st][1][nb][o], S.out[st][1][nb][2 + o]);
 }
 
-// Bounded wait without sleeping: the hardware suspends the warp inside try_wait.
-__device__ __forceinline__ void wait_bar(unsigned long long* bar, uint32_t parity, int* err, int code) {
-  for (int i = 0; i < kSpinLimit; ++i)
-    if (mbar_try_wait(bar, parity)) return;
-  atomicExch(err, code);
-}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }

@@ -47,9 +47,9 @@ static int launch(const Params& P, int tiles_bound, cudaStream_t stream) {
   return cudaLaunchKernelEx(&cfg, gemm_ts_kernel<OUT, BF16>, P) == cudaSuccess ? GEMQ_OK : GEMQ_ERR_LAUNCH;
 }
 
-bool activation_maps(CUtensorMap (&maps)[3], const void* x, int K, long long rows) {
-  for (int i = 0; i < 3; ++i)
-    if (!tensor_map_2d(&maps[i], x, 2, K, rows, kBK, 128 >> i, true)) return false;
+bool activation_maps(CUtensorMap (&maps)[4], const void* x, int K, long long rows) {
+  for (int i = 0; i < 4; ++i)
+    if (!tensor_map_blocks(&maps[i], x, K, rows, 32 * (i + 1))) return false;
   return true;
 }
 

@@ -18,12 +18,14 @@
 // 660 instead of 512 cycles per k-block.)  Tiles of the gate/up pass hold 64 gate and the same 64 up
 // columns per CTA, 16 + 16 per warp, so that a shuffle brings them together.
 //   16 producer warps  four groups that take 64-wide k-blocks in turn: fetch packed words a block of the group
-//                      ahead, de-quantise 64 k x 32 columns per warp, store them to the A ring; they
-//                      also drain the accumulators: first the next tile's first stages are produced,
-//                      so the MMAs go on while the epilogue computes and stores
-//   1 TMA warp         activation boxes of 128, 64 or 32 tokens x 64 k (128B swizzle; an instruction takes about
-//                      100 cycles to issue)
+//                      ahead, de-quantise 64 k x 32 columns per warp, store them to the A ring; they never
+//                      stop between tiles
+//   1 TMA warp         an activation box per stage (32 to 128 tokens x 128 k, 128B swizzle)
 //   1 MMA warp         (first CTA) issues tcgen05.mma and the commits that free the ring stages
+//   4 epilogue warps   round the accumulators to 16 bits into shared memory, which frees them for the next
+//                      tile, then finish and store whole rows while it is computed.  Tiles of up to 128 tokens
+//                      use the two halves of the accumulator columns in turn.  (With the producers doing
+//                      this between tiles, a tile of 128 tokens and 64 k-blocks took 28 us, 9 of them here.)
 // Every wait is bounded.
 #pragma once
 
@@ -33,19 +35,27 @@
 #include "ptx.cuh"
 
 namespace gemq {
+
+// tma.cu
+bool tensor_map_blocks(CUtensorMap* out, const void* base, int K, long long rows, int box_rows);
+
 namespace ts {
 
-constexpr int kBK = 64;            // k-block
+constexpr int kBK = 64;            // k-block of a producer warp
+constexpr int kStageK = 128;       // two of them per ring stage: a stage's waits, fences and branches cost the TMA and
+                                   // the MMA warp about 300 cycles each, 64 k of a half-filled tile only 256 of MMAs
 constexpr int kCols = 128;         // weight columns of a CTA = TMEM lanes
 constexpr int kTokens = 256;       // most tokens of a tile
-constexpr int kStages = 8;
+constexpr int kRowBytes = kBK * 2;
+constexpr int kStages = 4;
 constexpr int kProducers = 16;
 constexpr int kGroups = kProducers / 4;
-constexpr int kThreads = 32 * (kProducers + 2);
-constexpr int kRowBytes = kBK * 2;  // of a k-block
-constexpr int kStageBytes = kTokens / 2 * kBK * 2;  // half of the tokens
+constexpr int kTmaWarp = kProducers, kMmaWarp = kProducers + 1, kEpiWarp = kProducers + 2;
+constexpr int kThreads = 32 * (kEpiWarp + 4);
+constexpr int kOutPitch = kCols * 2 + 16;  // bytes of a staged row: reads of a column of rows hit all banks
+constexpr int kStageBytes = kTokens / 2 * 2 * kRowBytes;  // half of the tokens
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kTmemA = 256;   // A ring behind the accumulators: 32 columns per stage
+constexpr uint32_t kTmemA = 256;   // A ring behind the accumulators: 64 columns per stage
 
 enum { kErrFull = 11, kErrEmpty = 13, kErrAcc = 14, kErrDrained = 15 };
 enum { kOutUp = 0,      // silu(gate) * up, fp16, stored in the order of the down projection's words
@@ -70,7 +80,8 @@ struct Family {
 };
 
 struct alignas(64) Params {
-  CUtensorMap b_map[2][3]; // activations per family, boxes of 128, 64, 32 rows x 64, 128B swizzle
+  // activations per family as (64 k, rows, K / 64): boxes of 32, 64, 96, 128 rows x 128 k, 128B swizzle
+  CUtensorMap b_map[2][4];
   Family fam[2];
   const int4* tiles;       // {expert (-1: shared), first row, rows, 0}, shared tiles first; nullptr: linear
   const int* n_tiles;
@@ -84,8 +95,8 @@ struct alignas(64) Params {
 
 struct Smem {
   alignas(1024) unsigned char b[kStages][kStageBytes];
-  alignas(16) unsigned char out[4][64 * kCols * 2];  // result rows of a quarter of the tokens
-  alignas(8) unsigned long long full[kStages], empty[kStages], acc_full, drained;
+  alignas(16) unsigned char out[kTokens * kOutPitch];  // accumulators rounded to 16 bits
+  alignas(8) unsigned long long full[kStages], empty[kStages], acc_full[2], drained[2];  // [2]: by the tile's parity
   uint32_t tmem_base;
 };
 
@@ -117,13 +128,14 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
       "r"(r[31])
       : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void wait_bar(unsigned long long* bar, uint32_t parity, int* err, int code) {
-  for (int i = 0; i < kSpinLimit; ++i)
-    if (mbar_try_wait(bar, parity)) return;
-  atomicExch(err, code);
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
 }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---- the CTA pair --------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pair_rank() {
@@ -153,12 +165,12 @@ __device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
                "h"(static_cast<unsigned short>(3))
                : "memory");
 }
-// Box into this CTA's shared memory; its bytes count on a barrier of the first CTA (cluster address).
-__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+// Box of rows x two 64-wide k-blocks into this CTA's shared memory; its bytes count on a barrier of the first CTA (cluster address).
+__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, int row, int block, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
           smem_u32(dst)),
-      "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(bar)
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(0), "r"(row), "r"(block), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {
@@ -182,60 +194,75 @@ __device__ __forceinline__ uint32_t act2(__half2 v) {
 __device__ __forceinline__ uint32_t u32(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 __device__ __forceinline__ __half2 h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 
-// W^T[k, n] = fp16(fma(fp16(q), s, z)) (gemq/triton_kernels/utils.py:206-210).  `bits` = one code in each half,
-// POS bits up.  Under the exponent of 2^(10 - POS) the code counts in units of one: the half reads
-// 2^(10 - POS) + q, and one exact subtraction leaves q.
-template <int POS>
-__device__ __forceinline__ __half2 dequant2(uint32_t bits, __half2 s2, __half2 z2) {
-  constexpr uint32_t EXP = (0x6400u - (static_cast<uint32_t>(POS) << 10)) * 0x00010001u;
-  const __half2 q = __hsub2(h2(bits | EXP), __float2half2_rn(static_cast<float>(1 << (10 - POS))));
-  return __hfma2(q, s2, z2);
-}
+// W^T[k, n] = fp16(fma(fp16(q), s, z)) (gemq/triton_kernels/utils.py:206-210), two weights at a time: the
+// masked word holds one code in each half, `pos` bits up; under the exponent of 2^(10 - pos) the code counts in
+// units of one, the half reads 2^(10 - pos) + q and one exact subtraction leaves q.  The exponents are kept in
+// registers, so that masking and setting the exponent is one instruction (as literals they are two): five
+// positions at most, the word is shifted for the others.
+template <int B>
+struct Exps {
+  static constexpr int kPos = B == 1 ? 5 : 10 / B;
+  uint32_t e[kPos];
+  __device__ __forceinline__ Exps() {
+#pragma unroll
+    for (int j = 0; j < kPos; ++j) {
+      e[j] = (0x6400u - (static_cast<uint32_t>(B * j) << 10)) * 0x00010001u;
+      asm volatile("" : "+r"(e[j]));  // not a literal for the compiler
+    }
+  }
+  // code j of the two halves of w
+  template <int J>
+  __device__ __forceinline__ __half2 weights(uint32_t w, __half2 s2, __half2 z2) const {
+    constexpr uint32_t MASK = (((1u << B) - 1u) * 0x00010001u) << (B * J);
+    uint32_t v;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(w), "n"(MASK), "r"(e[J]));  // (w & MASK) | exponent
+    return __hfma2(__hsub2(h2(v), __float2half2_rn(static_cast<float>(1 << (10 - B * J)))), s2, z2);
+  }
+};
 
+// Codes Q and Q + eps / 2 of a packed word.
 template <int B, int Q>
-__device__ __forceinline__ __half2 word_pair(uint32_t w, __half2 s2, __half2 z2) {
-  constexpr int NPOS = 10 / B, JJ = Q % NPOS, SH = (Q / NPOS) * NPOS * B;
-  constexpr uint32_t MASK = ((1u << B) - 1u) * 0x00010001u;
-  return dequant2<B * JJ>((w >> SH) & (MASK << (B * JJ)), s2, z2);
+__device__ __forceinline__ __half2 word_pair(const Exps<B>& X, uint32_t w, __half2 s2, __half2 z2) {
+  constexpr int NPOS = Exps<B>::kPos, JJ = Q % NPOS, SH = (Q / NPOS) * NPOS * B;
+  return X.template weights<JJ>(w >> SH, s2, z2);
 }
 
-// 64 codes of a column as 32 TMEM words.  NAT: neighbouring k share a word; else codes q and q + eps / 2 of a
+// 32 of a column's codes (B words) as 16 TMEM words.  NAT: neighbouring k share a word; else codes q and q + eps / 2 of a
 // packed word do (the activations are stored in that order).
 template <int B, bool BF16, bool NAT, int I, int Q>
-__device__ __forceinline__ void dequant_word(uint32_t (&o)[32], uint32_t w, __half2 s2, __half2 z2) {
+__device__ __forceinline__ void dequant_word(const Exps<B>& X, uint32_t (&o)[16], uint32_t w, __half2 s2, __half2 z2) {
   constexpr int PAIRS = 16 / B;
   if constexpr (Q < PAIRS) {
-    const __half2 a = word_pair<B, Q>(w, s2, z2);
+    const __half2 a = word_pair<B, Q>(X, w, s2, z2);
     if constexpr (!NAT) {
       o[I * PAIRS + Q] = act2<BF16>(a);
-      dequant_word<B, BF16, NAT, I, Q + 1>(o, w, s2, z2);
+      dequant_word<B, BF16, NAT, I, Q + 1>(X, o, w, s2, z2);
     } else {
-      const __half2 b = word_pair<B, Q + 1>(w, s2, z2);
+      const __half2 b = word_pair<B, Q + 1>(X, w, s2, z2);
       o[I * PAIRS + Q / 2] = act2<BF16>(h2(__byte_perm(u32(a), u32(b), 0x5410)));
       o[I * PAIRS + PAIRS / 2 + Q / 2] = act2<BF16>(h2(__byte_perm(u32(a), u32(b), 0x7632)));
-      dequant_word<B, BF16, NAT, I, Q + 2>(o, w, s2, z2);
+      dequant_word<B, BF16, NAT, I, Q + 2>(X, o, w, s2, z2);
     }
   }
 }
 template <int B, bool BF16, bool NAT, int I>
-__device__ __forceinline__ void dequant_words(uint32_t (&o)[32], const uint32_t* w, __half2 s2, __half2 z2) {
-  if constexpr (I < 2 * B) {
-    dequant_word<B, BF16, NAT, I, 0>(o, w[I], s2, z2);
-    dequant_words<B, BF16, NAT, I + 1>(o, w, s2, z2);
+__device__ __forceinline__ void dequant_words(const Exps<B>& X, uint32_t (&o)[16], const uint32_t* w, __half2 s2, __half2 z2) {
+  if constexpr (I < B) {
+    dequant_word<B, BF16, NAT, I, 0>(X, o, w[I], s2, z2);
+    dequant_words<B, BF16, NAT, I + 1>(X, o, w, s2, z2);
   }
 }
 
 // 3-bit: a 64-code window starts at an even code of its first word and spans eight words; always natural
 // order.  All 40 pairs are formed, the window is the 32 from pair (k0 mod 10) / 2 on.
 template <bool BF16>
-__device__ __forceinline__ void dequant_b3(uint32_t (&pr)[40], const uint32_t* w, __half2 s2, __half2 z2) {
+__device__ __forceinline__ void dequant_b3(const Exps<3>& X, uint32_t (&pr)[40], const uint32_t* w, __half2 s2, __half2 z2) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const uint32_t m = (w[i] & 0x00007fffu) | ((w[i] << 1) & 0x7fff0000u);  // codes 0..4 | 5..9
     const uint32_t mh = m >> 9;
-    const uint32_t v0 = u32(dequant2<0>(m & 0x00070007u, s2, z2)), v1 = u32(dequant2<3>(m & 0x00380038u, s2, z2));
-    const uint32_t v2 = u32(dequant2<6>(m & 0x01c001c0u, s2, z2)), v3 = u32(dequant2<0>(mh & 0x00070007u, s2, z2));
-    const uint32_t v4 = u32(dequant2<3>(mh & 0x00380038u, s2, z2));
+    const uint32_t v0 = u32(X.weights<0>(m, s2, z2)), v1 = u32(X.weights<1>(m, s2, z2)), v2 = u32(X.weights<2>(m, s2, z2));
+    const uint32_t v3 = u32(X.weights<0>(mh, s2, z2)), v4 = u32(X.weights<1>(mh, s2, z2));
     pr[5 * i + 0] = act2<BF16>(h2(__byte_perm(v0, v1, 0x5410)));  // codes 0, 1
     pr[5 * i + 1] = act2<BF16>(h2(__byte_perm(v2, v3, 0x5410)));  // 2, 3
     pr[5 * i + 2] = act2<BF16>(h2(__byte_perm(v4, v0, 0x7610)));  // 4, 5
@@ -249,6 +276,8 @@ struct Tile {
   int fam, expert, row0, rows, col0;
   // tokens of the MMA (32, 64, ..), of which each CTA brings half
   __device__ __forceinline__ int n() const { return (rows + 31) & ~31; }
+  // first accumulator column of the CTA's tile number j
+  __device__ __forceinline__ int acc(uint32_t j) const { return rows <= kTokens / 2 ? static_cast<int>(j & 1) * (kTokens / 2) : 0; }
 };
 
 template <int COLS, bool LINEAR>  // COLS: columns of a CTA along N (gate/up: 64)
@@ -280,10 +309,11 @@ __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Til
 }
 
 // ---- producer ------------------------------------------------------------------------------------
-// k-blocks [kb0, kb1) of a tile; `base` = k-blocks this CTA has handled before the tile.
-// (Out of line, like the epilogue: inlined, the 96 registers of 18 warps spill in the k loop.)
+// All k-blocks of a tile; `base` = k-blocks this CTA has handled before the tile (even).  An odd number of
+// blocks is followed by one of zeros: the activations of its stage end in zeros, too.
+// (Out of line: inlined, the 88 registers of 22 warps spill in the k loop.)
 template <bool UP, bool BF16, bool NAT, int B>
-__device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb0, int kb1, uint32_t tmem) {
+__device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb1, uint32_t tmem) {
   constexpr int NW = B == 3 ? 8 : 2 * B;  // words of a 64-code window
   const Family& F = P.fam[T.fam];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -305,13 +335,21 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   const int G = F.G, K = F.K;
   int* const err = P.err;
   const int gshift = (G & (G - 1)) == 0 ? __ffs(G) - 1 : -1;
-  // first k-block of this warp's group at or after kb0
-  int kb = kb0 + static_cast<int>(((warp >> 2) + kGroups - (base + kb0) % kGroups) % kGroups);
+  int kb = static_cast<int>(((warp >> 2) + kGroups - base % kGroups) % kGroups);  // first k-block of this warp's group
+  const int real = kb1;
+  kb1 = (kb1 + 1) & ~1;
   if (kb >= kb1) return;
   struct Set { uint32_t w[NW]; __half s, z; };
-  Set cur, nxt;
+  Set ring[2];
+  const Exps<B> X;
   if (B != 3) wp += static_cast<size_t>(kb) * (2 * B) * N;
   auto fetch = [&](Set& R, int k) {  // blocks in order
+    if (k >= real) {
+#pragma unroll
+      for (int i = 0; i < NW; ++i) R.w[i] = 0u;
+      R.s = R.z = __float2half_rn(0.f);
+      return;
+    }
     const int k0 = k * kBK;
     const int g = gshift >= 0 ? k0 >> gshift : k0 / G;
     if (B == 3) {  // the last window of a matrix may end before its eighth word
@@ -331,20 +369,17 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
     R.s = sp[static_cast<size_t>(g) * N];
     R.z = zp[static_cast<size_t>(g) * N];
   };
-  uint32_t c = base + kb;
+  const uint32_t c = (base + kb) >> 1;  // groups 0 and 1 fill a stage, 2 and 3 the next
   uint32_t s = c % kStages, par = ((c / kStages) & 1) ^ 1;
   const uint32_t full0 = first_cta(&S.full[0]);
-  const uint32_t dst0 = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemA;
-  fetch(cur, kb);
-#pragma unroll 1
-  for (; kb < kb1; kb += kGroups) {
-    if (kb + kGroups < kb1) fetch(nxt, kb + kGroups);
+  const uint32_t dst0 = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemA + ((base + kb) & 1) * 32;
+  auto put = [&](const Set& cur) {
     const __half2 s2 = __half2half2(cur.s), z2 = __half2half2(cur.z);
-    const uint32_t dst = dst0 + s * 32;
-    if (B == 3) {
+    const uint32_t dst = dst0 + s * 64;
+    if constexpr (B == 3) {
       uint32_t pr[40];
-      dequant_b3<BF16>(pr, cur.w, s2, z2);
-      wait_bar(&S.empty[s], par, err, kErrEmpty);
+      dequant_b3<BF16>(X, pr, cur.w, s2, z2);
+      mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
       tc_fence_after_sync();
       switch ((kb * kBK % 10) >> 1) {  // uniform
         case 0: tmem_st32(dst, pr); break;
@@ -354,33 +389,54 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
         default: tmem_st32(dst, pr + 4); break;
       }
     } else {
-      uint32_t o[32];
-      dequant_words<B == 3 ? 2 : B, BF16, NAT, 0>(o, cur.w, s2, z2);
-      wait_bar(&S.empty[s], par, err, kErrEmpty);
+      // in two halves: 16 result registers instead of 32
+      uint32_t o[16];
+      dequant_words<B, BF16, NAT, 0>(X, o, cur.w, s2, z2);
+      mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
       tc_fence_after_sync();
-      tmem_st32(dst, o);
+      tmem_st16(dst, o);
+      dequant_words<B, BF16, NAT, 0>(X, o, cur.w + B, s2, z2);
+      tmem_st16(dst + 16, o);
     }
     tmem_wait_st();
     tc_fence_before_sync();
     __syncwarp();
     if (lane == 0) arrive_at(full0 + s * 8);
-    s += kGroups;
+    s += kGroups / 2;
     if (s >= kStages) { s -= kStages; par ^= 1u; }
-    cur = nxt;
+  };
+  fetch(ring[0], kb);
+#pragma unroll 1
+  for (;;) {
+    if constexpr (B == 3) {  // one copy of the long body, the sets are moved
+      if (kb + kGroups < kb1) fetch(ring[1], kb + kGroups);
+      put(ring[0]);
+      kb += kGroups;
+      if (kb >= kb1) return;
+      ring[0] = ring[1];
+    } else {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (kb + kGroups < kb1) fetch(ring[u ^ 1], kb + kGroups);
+        put(ring[u]);
+        kb += kGroups;
+        if (kb >= kb1) return;
+      }
+    }
   }
 }
 
 template <bool UP, bool BF16, bool NAT>
-__device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb0, int kb1, uint32_t tmem) {
+__device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb1, uint32_t tmem) {
   const Family& F = P.fam[T.fam];
   const int bits = F.nbits && T.expert >= 0 ? F.nbits[T.expert] : F.bits;
-  if (bits == 1) produce<UP, BF16, NAT, 1>(S, P, T, base, kb0, kb1, tmem);
-  else if (bits == 2) produce<UP, BF16, NAT, 2>(S, P, T, base, kb0, kb1, tmem);
-  else if (bits == 3) produce<UP, BF16, NAT, 3>(S, P, T, base, kb0, kb1, tmem);
-  else produce<UP, BF16, NAT, 4>(S, P, T, base, kb0, kb1, tmem);
+  if (bits == 1) produce<UP, BF16, NAT, 1>(S, P, T, base, kb1, tmem);
+  else if (bits == 2) produce<UP, BF16, NAT, 2>(S, P, T, base, kb1, tmem);
+  else if (bits == 3) produce<UP, BF16, NAT, 3>(S, P, T, base, kb1, tmem);
+  else produce<UP, BF16, NAT, 4>(S, P, T, base, kb1, tmem);
 }
 
-// ---- epilogue: warp w owns TMEM lanes (= columns) 32 (w & 3) .. + 31 and tokens 64 (w >> 2) .. + 63 ----
+// ---- epilogue --------------------------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ float as_float(T v);
 template <> __device__ __forceinline__ float as_float<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float as_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
@@ -399,77 +455,93 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// The four warps of a token quarter gather their columns in shared memory and store whole rows, 16 bytes a lane.
-// Short loops on purpose: the code runs once per tile, straight-line it took 7 us of instruction fetches.
 template <int OUT, typename T>
-__device__ __noinline__ void epilogue(Smem& S, const Params& P, const Tile& t, uint32_t tmem, uint32_t parity) {
-  constexpr int ROW = OUT == kOutUp ? kCols / 2 : kCols;  // columns of a staged row
-  const Family& F = P.fam[t.fam];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int lq = warp & 3, tq = warp >> 2;
-  const int rows = min(64, t.rows - 64 * tq);  // valid tokens of this quarter
-  T* st = reinterpret_cast<T*>(S.out[tq]);
-  asm volatile("bar.sync %0, 128;" ::"r"(1 + tq) : "memory");  // the rows of the tile before are out
-  wait_bar(&S.acc_full, parity, P.err, kErrAcc);
-  tc_fence_after_sync();
-  const uint32_t at = tmem + (static_cast<uint32_t>(32 * lq) << 16) + 64 * tq;
-  if (OUT == kOutUp) {
-    // Lanes 0..15 hold x1 of 16 columns, lanes 16..31 x3 of the same: per pair of tokens each half gives the
-    // other one value; the lower half forms h of the even token, the upper half of the odd one.
-    // F.silu(x1) * x3 on fp16 tensors: each step is rounded.
-    const bool up = lane >= 16;
-    const int ob = F.out_nbits && t.expert >= 0 ? F.out_nbits[t.expert] : F.out_bits;
-    const int eps = ob == 3 ? 2 : 32 / ob;  // 3-bit matrices read their rows in natural order
-    const int cc = 16 * lq + (lane & 15), j = cc & (eps - 1);
-    T* dst = st + (cc & ~(eps - 1)) + 2 * (j & (eps / 2 - 1)) + (j >= eps / 2 ? 1 : 0) + (up ? ROW : 0);
+__device__ __forceinline__ void drain(Smem& S, uint32_t at, int rows, int column) {
+  unsigned char* dst = S.out + 2 * column;
 #pragma unroll 1
-    for (int c = 0; c < rows; c += 16) {
-      uint32_t d[16];
-      tmem_ld16(at + c, d);
+  for (int c = 0; c < rows; c += 16) {
+    uint32_t d[16];
+    tmem_ld16(at + c, d);
 #pragma unroll
-      for (int i = 0; i < 16; i += 2) {
-        const float mine = __uint_as_float(up ? d[i + 1] : d[i]), give = __uint_as_float(up ? d[i] : d[i + 1]);
-        const float got = __shfl_xor_sync(0xffffffffu, give, 16);
-        const float x1 = __half2float(__float2half_rn(up ? got : mine)), x3 = __half2float(__float2half_rn(up ? mine : got));
-        dst[(c + i) * ROW] = as_act<T>(__half2float(__float2half_rn(silu_f32(x1))) * x3);
-      }
-    }
-  } else {
-    const int col = t.col0 + 32 * lq + lane;
-    float bias = 0.f, rw0 = 1.f, rw1 = 1.f;
-    const bool has_bias = OUT == kOutLinear && P.bias != nullptr;
-    if (has_bias && col < F.N) bias = as_float<T>(static_cast<const T*>(P.bias)[col]);
-    if (OUT == kOutDown && t.fam == 0 && rows > 0) {
-      const __half* rw = P.row_w + t.row0 + 64 * tq;
-      rw0 = __half2float(rw[min(lane, rows - 1)]);
-      rw1 = __half2float(rw[min(lane + 32, rows - 1)]);
-    }
-    T* dst = st + 32 * lq + lane;
-#pragma unroll 1
-    for (int c = 0; c < rows; c += 16) {
-      uint32_t d[16];
-      tmem_ld16(at + c, d);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        T v = as_act<T>(__uint_as_float(d[i]));
-        if (OUT == kOutDown) v = as_act<T>(as_float<T>(v) * __shfl_sync(0xffffffffu, c < 32 ? rw0 : rw1, (c + i) & 31));
-        if (OUT == kOutLinear && has_bias) v = as_act<T>(as_float<T>(v) + bias);
-        dst[(c + i) * ROW] = v;
-      }
-    }
+    for (int i = 0; i < 16; ++i) *reinterpret_cast<T*>(dst + (c + i) * kOutPitch) = as_act<T>(__uint_as_float(d[i]));
   }
-  tc_fence_before_sync();
-  __syncwarp();
-  if (lane == 0) arrive_at(first_cta(&S.drained));  // the next tile's MMAs may overwrite the accumulators
-  asm volatile("bar.sync %0, 128;" ::"r"(1 + tq) : "memory");
-  constexpr int PIECES = ROW / 8;
+}
+
+// 32 neighbouring h in the order of the words of a matrix with EPS codes per word.
+template <int EPS>
+__device__ __forceinline__ void word_order(const __half (&h)[32], uint32_t (&o)[16]) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const int w = k / (EPS / 2), j = k % (EPS / 2);
+    const __half2 v = __halves2half2(h[w * EPS + j], h[w * EPS + j + EPS / 2]);
+    o[k] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+
+// h = F.silu(x1) * x3 on fp16 tensors, each step rounded: a thread takes 32 columns of a token (x1 and x3 of
+// 16 columns each in two warps' worth of staged columns).
+__device__ __forceinline__ void finish_up(const Smem& S, const Params& P, const Tile& t, int tid) {
+  const Family& F = P.fam[t.fam];
+  const int bits = F.out_nbits && t.expert >= 0 ? F.out_nbits[t.expert] : F.out_bits;
   const size_t pitch = F.N;
-  const int cols = F.N - t.col0;  // N is a multiple of 32
-  T* out = static_cast<T*>(F.out) + static_cast<size_t>(t.row0 - F.row0 + 64 * tq) * pitch + t.col0;
+  __half* const out = static_cast<__half*>(F.out) + static_cast<size_t>(t.row0 - F.row0) * pitch + t.col0;
+  const int rows = t.rows;
+#pragma unroll 1
+  for (int i = tid; i < 2 * rows; i += 128) {
+    const int grp = i >= rows ? 1 : 0, row = i - grp * rows;
+    const unsigned char* src = S.out + row * kOutPitch + 128 * grp;
+    __half h[32];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // eight columns each
+      const unsigned char* p = src + (q >> 1) * 64 + (q & 1) * 16;
+      const uint4 g = *reinterpret_cast<const uint4*>(p), u = *reinterpret_cast<const uint4*>(p + 32);
+      const __half *gh = reinterpret_cast<const __half*>(&g), *uh = reinterpret_cast<const __half*>(&u);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        h[8 * q + k] = __float2half_rn(__half2float(__float2half_rn(silu_f32(__half2float(gh[k])))) * __half2float(uh[k]));
+    }
+    uint32_t o[16];
+    if (bits == 1) word_order<32>(h, o);
+    else if (bits == 2) word_order<16>(h, o);
+    else if (bits == 3) word_order<2>(h, o);  // 3-bit matrices read their rows in natural order
+    else word_order<8>(h, o);
+    uint4* dst = reinterpret_cast<uint4*>(out + row * pitch + 32 * grp);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dst[q] = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+  }
+}
+
+// Eight columns of a row per thread: times the routing weight, or plus the bias.
+template <int OUT, typename T>
+__device__ __forceinline__ void finish_rows(const Smem& S, const Params& P, const Tile& t, int tid) {
+  const Family& F = P.fam[t.fam];
+  const size_t pitch = F.N;
+  const int q = tid & 15, col = t.col0 + 8 * q;
+  if (col >= F.N) return;  // N is a multiple of 32
+  T* const out = static_cast<T*>(F.out) + static_cast<size_t>(t.row0 - F.row0) * pitch + col;
+  const __half* const rw = OUT == kOutDown && t.fam == 0 ? P.row_w + t.row0 : nullptr;
+  const bool has_bias = OUT == kOutLinear && P.bias != nullptr;
+  uint4 bias = make_uint4(0u, 0u, 0u, 0u);
+  if (has_bias) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) reinterpret_cast<T*>(&bias)[k] = static_cast<const T*>(P.bias)[col + k];
+  }
+  const int rows = t.rows;
 #pragma unroll 2
-  for (int p = 32 * lq + lane; p < rows * PIECES; p += 128) {
-    const int r = p / PIECES, q = p % PIECES;
-    if (8 * q < cols) *reinterpret_cast<uint4*>(out + r * pitch + 8 * q) = *reinterpret_cast<const uint4*>(st + r * ROW + 8 * q);
+  for (int row = tid >> 4; row < rows; row += 8) {
+    uint4 v = *reinterpret_cast<const uint4*>(S.out + row * kOutPitch + 16 * q);
+    T* e = reinterpret_cast<T*>(&v);
+    if (OUT == kOutDown) {
+      if (rw) {
+        const float f = __half2float(rw[row]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) e[k] = as_act<T>(as_float<T>(e[k]) * f);
+      }
+    } else if (has_bias) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) e[k] = as_act<T>(as_float<T>(e[k]) + as_float<T>(reinterpret_cast<const T*>(&bias)[k]));
+    }
+    *reinterpret_cast<uint4*>(out + row * pitch) = v;
   }
 }
 
@@ -484,14 +556,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
   const int rank = static_cast<int>(pair_rank());
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(&S.full[s], 9);  // in the first CTA: a group's four warps of either CTA, the activation boxes
+      mbar_init(&S.full[s], 17);  // in the first CTA: two groups' warps of either CTA, the activation boxes
       mbar_init(&S.empty[s], 1);
     }
-    mbar_init(&S.acc_full, 1);
-    mbar_init(&S.drained, 2 * kProducers);
+    for (int j = 0; j < 2; ++j) {
+      mbar_init(&S.acc_full[j], 1);
+      mbar_init(&S.drained[j], 8);  // in the first CTA: the epilogue warps of both
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kProducers + 1) tmem_alloc_pair(&S.tmem_base, kTmemCols);
+  if (warp == kMmaWarp) tmem_alloc_pair(&S.tmem_base, kTmemCols);
   tc_fence_before_sync();
   __syncthreads();
   pair_sync();
@@ -501,85 +575,96 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // The packed words are nobody's result: a linear's producers start on them at once.  Its activations are read,
   // and with that its results written, after the TMA warp's wait.
-  if (!LINEAR || P.expert || warp == kProducers) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!LINEAR || P.expert || warp == kTmaWarp) asm volatile("griddepcontrol.wait;" ::: "memory");
 
+  // Tiles go to the pairs back and forth: the list is sorted by falling time, so who got a long one in a round gets
+  // a short one in the next.
   const int step = static_cast<int>(gridDim.x >> 1), first = static_cast<int>(blockIdx.x >> 1);
+  auto tile_of = [&](int i) { return i * step + ((i & 1) ? step - 1 - first : first); };
   Tile t;
   if (warp < kProducers) {
-    int idx = first, ahead = 0;
-    uint32_t base = 0, n = 0;
-    bool more = get_tile<COLS, LINEAR>(P, idx, rank, t);
+    uint32_t base = 0;
 #pragma unroll 1
-    while (more) {
+    for (int i = 0; get_tile<COLS, LINEAR>(P, tile_of(i), rank, t); ++i) {
       const int KB = P.fam[t.fam].K / kBK;
-      produce_any<UP, BF16, LINEAR>(S, P, t, base, ahead, KB, tmem);
-      base += KB;
-      const Tile done = t;
-      idx += step;
-      more = get_tile<COLS, LINEAR>(P, idx, rank, t);
-      ahead = 0;
-      if (more) {
-        ahead = min(kStages, P.fam[t.fam].K / kBK);
-        produce_any<UP, BF16, LINEAR>(S, P, t, base, 0, ahead, tmem);
-      }
-      epilogue<OUT, T>(S, P, done, tmem, n & 1);
-      ++n;
+      produce_any<UP, BF16, LINEAR>(S, P, t, base, KB, tmem);
+      base += (KB + 1) & ~1;
     }
-  } else if (warp == kProducers) {
+  } else if (warp == kTmaWarp) {
     uint32_t c = 0;
     const uint32_t full0 = first_cta(&S.full[0]);
-    for (int idx = first; get_tile<COLS, LINEAR>(P, idx, rank, t); idx += step) {
+    int* const err = P.err;
+    for (int i = 0; get_tile<COLS, LINEAR>(P, tile_of(i), rank, t); ++i) {
       const Family& F = P.fam[t.fam];
-      const int KB = F.K / kBK, half = t.n() / 2;
-      // an odd number of 16-row blocks brings the next 16 rows, too
-      const int n128 = half / 128, n64 = (half & 64) / 64, n32 = ((half & 63) + 31) / 32;
-      const uint32_t bytes = (128 * n128 + 64 * n64 + 32 * n32) * kRowBytes;
+      const int SB = (F.K + kStageK - 1) / kStageK, half = t.n() / 2;
+      const int box = (half + 31) / 32;  // in 32 rows: an odd number of 16-row blocks brings the next 16 rows, too
+      const uint32_t bytes = 2 * 32 * box * kRowBytes;
       const int row = t.row0 - F.row0 + rank * half;
-      for (int kb = 0; kb < KB; ++kb, ++c) {
+      const CUtensorMap* const map = &P.b_map[t.fam][box - 1];
+      for (int sb = 0; sb < SB; ++sb, ++c) {
         const uint32_t s = c % kStages;
-        wait_bar(&S.empty[s], ((c / kStages) & 1) ^ 1, P.err, kErrEmpty);
+        mbar_sleep_wait(&S.empty[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&S.full[s], 2 * bytes);
-          const CUtensorMap* map = P.b_map[t.fam];
-          if (n128) {
-            tma_load_pair(S.b[s], map, kb * kBK, row, full0 + s * 8);
-          } else {
-            if (n64) tma_load_pair(S.b[s], map + 1, kb * kBK, row, full0 + s * 8);
-            for (int b = 0; b < n32; ++b)
-              tma_load_pair(S.b[s] + (64 * n64 + 32 * b) * kRowBytes, map + 2, kb * kBK, row + 64 * n64 + 32 * b, full0 + s * 8);
-          }
+          tma_load_pair(S.b[s], map, row, 2 * sb, full0 + s * 8);
         }
         __syncwarp();
       }
     }
-  } else if (rank == 0) {
+  } else if (warp == kMmaWarp && rank == 0) {
     // The whole warp runs the loop and one elected lane issues: descriptors and addresses stay in uniform
     // registers.  (In a one-lane branch every tcgen05.mma cost 85 cycles to issue.)
-    uint32_t c = 0, n = 0;
+    uint32_t s = 0, par = 0, j = 0;
+    bool small = true;  // the tile before fits one half of the accumulators
     const uint64_t desc0 = umma_desc_k_sw128(smem_u32(S.b[0]));
-    for (int idx = first; get_tile<COLS, LINEAR>(P, idx, rank, t); idx += step, ++n) {
-      const int KB = P.fam[t.fam].K / kBK;
+    int* const err = P.err;
+    for (; get_tile<COLS, LINEAR>(P, tile_of(j), rank, t); ++j) {
+      const int SB = (P.fam[t.fam].K + kStageK - 1) / kStageK;
       const uint32_t idesc = umma_idesc_f16(BF16 ? 1 : 0, 2 * kCols, t.n());
-      wait_bar(&S.drained, (n & 1) ^ 1, P.err, kErrDrained);
-      for (int kb = 0; kb < KB; ++kb, ++c) {
-        const uint32_t s = c % kStages;
-        wait_bar(&S.full[s], (c / kStages) & 1, P.err, kErrFull);
+      const uint32_t second = ((t.n() / 2 + 31) / 32 * 32 * kRowBytes) >> 4;  // distance of a stage's second k-block
+      // The accumulators of the tile two back are out; with a tile over 128 tokens also those of the last.
+      mbar_sleep_wait(&S.drained[j & 1], ((j >> 1) & 1) ^ 1, err, kErrDrained);
+      const bool now_small = t.rows <= kTokens / 2;
+      if (j > 0 && !(small && now_small)) mbar_sleep_wait(&S.drained[(j - 1) & 1], ((j - 1) >> 1) & 1, err, kErrDrained);
+      small = now_small;
+      const uint32_t acc = tmem + t.acc(j);
+      for (int sb = 0; sb < SB; ++sb) {
+        mbar_sleep_wait(&S.full[s], par, err, kErrFull);
         tc_fence_after_sync();
         const uint64_t bd = desc0 + s * (kStageBytes >> 4);
-        const uint32_t a = tmem + kTmemA + s * 32;
+        const uint32_t a = tmem + kTmemA + s * 64;
         if (elect_one()) {
 #pragma unroll
-          for (int k4 = 0; k4 < kBK / 16; ++k4) umma_ts_f16(tmem, a + k4 * 8, bd + k4 * 2, idesc, k4 != 0 || kb != 0);
+          for (int k = 0; k < kStageK / 16; ++k)
+            umma_ts_f16(acc, a + k * 8, bd + (k & 3) * 2 + (k < 4 ? 0u : second), idesc, k != 0 || sb != 0);
           umma_commit_pair(&S.empty[s]);
-          if (kb == KB - 1) umma_commit_pair(&S.acc_full);
+          if (sb == SB - 1) umma_commit_pair(&S.acc_full[j & 1]);
         }
         __syncwarp();
+        if (++s == kStages) { s = 0; par ^= 1u; }
       }
+    }
+  }
+  if (warp >= kEpiWarp) {
+    const int lq = warp & 3, tid = static_cast<int>(threadIdx.x) - 32 * kEpiWarp;
+    uint32_t j = 0;
+#pragma unroll 1
+    for (; get_tile<COLS, LINEAR>(P, tile_of(j), rank, t); ++j) {
+      mbar_sleep_wait(&S.acc_full[j & 1], (j >> 1) & 1, P.err, kErrAcc);
+      tc_fence_after_sync();
+      drain<OUT, T>(S, tmem + (static_cast<uint32_t>(32 * lq) << 16) + t.acc(j), t.rows, 32 * lq + (threadIdx.x & 31));
+      tc_fence_before_sync();
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) arrive_at(first_cta(&S.drained[j & 1]));  // a later tile's MMAs may overwrite them
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (UP) finish_up(S, P, t, tid);
+      else finish_rows<OUT, T>(S, P, t, tid);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
     }
   }
   __syncthreads();
   pair_sync();  // nobody touches the other's barriers or tensor memory from here on
-  if (warp == kProducers + 1) {
+  if (warp == kMmaWarp) {
     tc_fence_after_sync();
     tmem_dealloc_pair(tmem, kTmemCols);
   }
@@ -589,7 +674,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream);
 int launch_down(const Params& P, int tiles_bound, cudaStream_t stream);
 int sm_count();
-bool activation_maps(CUtensorMap (&maps)[3], const void* x, int K, long long rows);
+bool activation_maps(CUtensorMap (&maps)[4], const void* x, int K, long long rows);
 
 }  // namespace ts
 }  // namespace gemq

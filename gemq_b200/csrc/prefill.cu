@@ -46,13 +46,24 @@ template <typename T>
 __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, const long long* __restrict__ idx, const T* __restrict__ w,
                                                                     const int* __restrict__ nbits, int R, int A, int E, int tokens,
                                                                     int shared_bits, int* err) {
-  __shared__ int count[256], start[256], first_tile[256], taken;
+  __shared__ int count[256], start[256], first_tile[256], cost[256], order[256], taken;
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int e = tid; e < E; e += kPlanThreads) count[e] = 0;
+  // Time of a tile by bit width: 3 bits 1.8, 4 bits 1.2 times the 1- and 2-bit ones (measured with 128 rows).
+  for (int e = tid; e < E; e += kPlanThreads) {
+    count[e] = 0;
+    const int b = nbits[e];
+    cost[e] = b == 3 ? 4 : (b == 4 ? 3 : b);
+  }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (tid == 0) *err = 0;
   __syncthreads();
+  // experts with the longest tiles first
+  for (int e = tid; e < E; e += kPlanThreads) {
+    int r = 0;
+    for (int o = 0; o < E; ++o) r += cost[o] > cost[e] || (cost[o] == cost[e] && o < e) ? 1 : 0;
+    order[r] = e;
+  }
   const int trips = (R + kPlanThreads - 1) / kPlanThreads;
   for (int i = 0; i < trips; ++i) {
     const int p = i * kPlanThreads + tid;
@@ -74,16 +85,17 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
   if (tid < 32) {  // scan of rows and tiles over the experts
     int row = 0, tile = sh_tiles;
     for (int e0 = 0; e0 < E; e0 += 32) {
-      const int n = e0 + lane < E ? count[e0 + lane] : 0, nt = (n + kTile - 1) / kTile;
+      const int e = e0 + lane < E ? order[e0 + lane] : -1;
+      const int n = e >= 0 ? count[e] : 0, nt = (n + kTile - 1) / kTile;
       int sr = n, stl = nt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int a = __shfl_up_sync(0xffffffffu, sr, o), b = __shfl_up_sync(0xffffffffu, stl, o);
         if (lane >= o) { sr += a; stl += b; }
       }
-      if (e0 + lane < E) {
-        start[e0 + lane] = row + sr - n;
-        first_tile[e0 + lane] = tile + stl - nt;
+      if (e >= 0) {
+        start[e] = row + sr - n;
+        first_tile[e] = tile + stl - nt;
       }
       row += __shfl_sync(0xffffffffu, sr, 31);
       tile += __shfl_sync(0xffffffffu, stl, 31);

@@ -40,6 +40,23 @@ __device__ __forceinline__ void mbar_wait(unsigned long long* bar, uint32_t pari
   }
   atomicExch(err, code);
 }
+// Bounded wait of a warp that sleeps in hardware until the phase ends (at most 20 us a time, about a second in
+// all).  Without the time hint try_wait comes back after some tens of cycles, and warps that wait long -- for
+// the end of a tile, say -- spend the issue slots of the others.
+__device__ __forceinline__ void mbar_sleep_wait(unsigned long long* bar, uint32_t parity, int* err, int code) {
+  for (int i = 0; i < (1 << 16); ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(20000)
+        : "memory");
+    if (ok) return;
+  }
+  atomicExch(err, code);
+}
 // Tiled TMA load of one box at element coordinates (x = column, y = row); x * element size
 // must be a multiple of 16 bytes (it is: columns come in multiples of 32).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {

@@ -98,4 +98,33 @@ bool tensor_map_strips(CUtensorMap* out, const void* base, int N, long long rows
   return true;
 }
 
+// 16-bit activations [rows, K] as (64, rows, K / 64): one box brings `box_rows` rows of two neighbouring 64-wide
+// k-blocks, each as swizzled rows of 128 bytes; a block past the end is zero-filled.
+bool tensor_map_blocks(CUtensorMap* out, const void* base, int K, long long rows, int box_rows) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const MapKey key{base, rows, K, 2, 64, box_rows, 2, dev};
+  std::lock_guard<std::mutex> lock(g_mu);
+  auto it = g_cache.find(key);
+  if (it != g_cache.end()) {
+    *out = it->second;
+    return true;
+  }
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (!enc) return false;
+  const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(K / 64)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K) * 2, 128};
+  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 2};
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  CUtensorMap m;
+  if (enc(&m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return false;
+  if (g_cache.size() > 4096) g_cache.clear();
+  g_cache[key] = m;
+  *out = m;
+  return true;
+}
+
 }  // namespace gemq
