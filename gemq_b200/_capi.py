@@ -76,6 +76,9 @@ _SIGNATURES = {
     "gemq_static_scratch_bytes": (_Z, []),
     "gemq_workspace_error_word": (_P, [_P]),
     "gemq_workspace_wait_limit_word": (_P, [_P]),
+    "gemq_step_gemv": (_I, [_P, _P, _I, _P, C.c_float, _P, _P, _I, _P, _I, _P, _I, _P, _I, _I, _P]),
+    "gemq_step_norm": (_I, [_P, _P, _I, _P, C.c_float, _P, _P, _I, _I, _P]),
+    "gemq_step_attention": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P]),
     "gemq_moe_decode": (_I, [C.POINTER(MoeLayer), _P, _P, _P, _P, _I, _I, _I, _P, _Z, _P]),
 }
 

@@ -19,6 +19,9 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch import Tensor
 
+from .. import _capi
+from ..kernels._ops import plain_call
+from ..kernels._runtime import stream_ptr
 from .kv_cache import StaticCache
 
 MIXTRAL_8X7B_CONFIG = dict(hidden_size=4096, intermediate_size=14336, num_local_experts=8, num_experts_per_tok=2,
@@ -37,10 +40,14 @@ class RMSNorm(nn.Module):
         return (v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)).to(x.dtype) * self.weight
 
 
+def inverse_frequencies(hd: int, theta: float, device) -> Tensor:
+    return 1.0 / (theta ** (torch.arange(0, hd, 2, device=device, dtype=torch.float32) / hd))
+
+
 def rotary(x: Tensor, pos: Tensor, theta: float) -> Tensor:
     """x [B, H, S, hd], pos [S] -> rotated (half-split convention)."""
     hd = x.shape[-1]
-    inv = 1.0 / (theta ** (torch.arange(0, hd, 2, device=x.device, dtype=torch.float32) / hd))
+    inv = inverse_frequencies(hd, theta, x.device)
     ang = pos.float()[:, None] * inv[None, :]
     cos, sin = torch.cat([ang.cos(), ang.cos()], -1), torch.cat([ang.sin(), ang.sin()], -1)
     x1, x2 = x[..., : hd // 2], x[..., hd // 2:]
@@ -125,14 +132,89 @@ class MixtralDecoder(nn.Module):
         for m in self.modules():
             if isinstance(m, RMSNorm):
                 m.to(device=device, dtype=dtype)
+        self.register_buffer("_inv_freq", inverse_frequencies(cfg.head_dim, cfg.rope_theta, device), persistent=False)
 
     @torch.no_grad()
     def forward(self, input_ids: Tensor, past_key_values: StaticCache, cache_position: Tensor) -> Tensor:
         """input_ids [B, S], cache_position [S] -> logits of the last position [B, vocab]."""
         x = self.embed_tokens(input_ids)
+        if input_ids.shape == (1, 1) and plain_call(x) and self._step_ok(x, past_key_values, cache_position):
+            return self._step(x.view(-1), past_key_values, cache_position)
         for layer in self.layers:
             x = layer(x, past_key_values, cache_position)
         return self.lm_head(self.norm(x[:, -1]))
+
+    def _step_ok(self, x: Tensor, cache: StaticCache, pos: Tensor) -> bool:
+        """Whether the step kernels take one token of one sequence: an unquantised attention of the standard
+        modules, head sizes and widths the kernels are written for, an initialised cache of x's type."""
+        c, D = self.config, self.config.hidden_size
+        H, Hkv, hd = c.num_attention_heads, c.num_key_value_heads, c.head_dim
+        if x.dtype not in (torch.float16, torch.bfloat16) or pos.dtype != torch.int64 or pos.numel() != 1:
+            return False
+        if hd not in (64, 128) or H % Hkv or H // Hkv > 8 or D % 256 or (H * hd) % 256 or max(D, H * hd) > 16384:
+            return False
+
+        def plain(t, shape):
+            return t is not None and t.shape == shape and t.dtype == x.dtype and t.device == x.device and t.is_contiguous() \
+                and t.data_ptr() % 16 == 0
+
+        def linear(m, n, k):
+            return type(m) is nn.Linear and m.bias is None and plain(m.weight, (n, k))
+
+        def norm(m):
+            return type(m) is RMSNorm and plain(m.weight, (D,))
+
+        inv = self._inv_freq
+        if inv.dtype != torch.float32 or inv.device != x.device or pos.device != x.device:
+            return False
+        if not (norm(self.norm) and linear(self.lm_head, c.vocab_size, D)):
+            return False
+        for layer, kv in zip(self.layers, cache.layers):
+            a = layer.self_attn
+            if not (linear(a.q_proj, H * hd, D) and linear(a.k_proj, Hkv * hd, D) and linear(a.v_proj, Hkv * hd, D)
+                    and linear(a.o_proj, D, H * hd) and norm(layer.input_layernorm) and norm(layer.post_attention_layernorm)):
+                return False
+            shape = (1, Hkv, cache.max_cache_len, hd)
+            if not (kv.is_initialized and plain(kv.keys, shape) and plain(kv.values, shape)):
+                return False
+        return True
+
+    def _step(self, x: Tensor, cache: StaticCache, pos: Tensor) -> Tensor:
+        """One token of one sequence, ``x [D]``: per layer two matrix kernels, the attention and the normalisation
+        around the MoE block's one-token call.  As separate tensor operations a layer's ninety launches took 260 us
+        in a captured step, 50 of them the MoE block (hidden 4096, 600 positions)."""
+        c, lib, st = self.config, _capi.lib, stream_ptr(x.device)
+        H, Hkv, hd, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.hidden_size
+        bf = int(x.dtype == torch.bfloat16)
+        ptr = Tensor.data_ptr
+        y, y_half = None, 0  # what the running sum still lacks
+
+        def gemv(norm, mats, K, keep_sum):
+            out = x.new_empty(sum(m.weight.shape[0] for m in mats))
+            total = torch.empty_like(x) if keep_sum and y is not None else None
+            w = [v for m in mats for v in (ptr(m.weight), m.weight.shape[0])] + [None, 0] * (3 - len(mats))
+            _capi.check("gemq_step_gemv", lib.gemq_step_gemv(
+                ptr(x), None if y is None else ptr(y), y_half, None if norm is None else ptr(norm.weight),
+                0.0 if norm is None else norm.eps, None if total is None else ptr(total), *w, ptr(out), K, bf, st))
+            return out, x if total is None else total
+
+        for layer, kv in zip(self.layers, cache.layers):
+            a = layer.self_attn
+            qkv, x = gemv(layer.input_layernorm, (a.q_proj, a.k_proj, a.v_proj), D, True)
+            att = x.new_empty(H * hd)
+            _capi.check("gemq_step_attention", lib.gemq_step_attention(
+                ptr(qkv), ptr(self._inv_freq), ptr(pos), ptr(kv.keys), ptr(kv.values), ptr(att), H, Hkv, hd,
+                kv.keys.shape[2], bf, st))
+            o = x.new_empty(D)
+            _capi.check("gemq_step_gemv", lib.gemq_step_gemv(
+                ptr(att), None, 0, None, 0.0, None, ptr(a.o_proj.weight), D, None, 0, None, 0, ptr(o), H * hd, bf, st))
+            post, total = layer.post_attention_layernorm, torch.empty_like(x)
+            h = torch.empty((1, 1, D), dtype=torch.float16, device=x.device)
+            _capi.check("gemq_step_norm", lib.gemq_step_norm(
+                ptr(x), ptr(o), 0, ptr(post.weight), post.eps, ptr(total), ptr(h), D, bf, st))
+            x, y_half = total, 1
+            y, _ = layer.block_sparse_moe(h)
+        return gemv(self.norm, (self.lm_head,), D, False)[0].view(1, -1)
 
     def expert_bytes_per_token(self) -> float:
         """Algorithmic bytes of the expert weights one decoded token streams (two experts per layer

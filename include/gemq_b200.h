@@ -275,6 +275,29 @@ int gemq_ep_unpack_rows(const void* payload, int rows, int D, void* x, int64_t* 
 int gemq_ep_combine(const void* back, const int64_t* where, const int64_t* sel, int tokens, int top_k, int D,
                     int is_bf16, void* out, gemq_stream_t stream);
 
+/* ---- one decode step of one sequence, around the MoE blocks ----------------------------------- */
+
+/* No counterpart in the reference, which runs these as the host model's own torch modules.  16-bit type T is
+ * fp16, or bf16 with is_bf16; every pointer 16-byte aligned.
+ * h = x + T(res) (res nullable; fp16 with res_is_half, else T), written to sum_out if that is given (another buffer
+ * than x and res); n = RMSNorm(h) * norm_weight, or h itself without norm_weight;
+ * out [rows0 + rows1 + rows2] = the matrices [rows, K] of T, one after the other, times n.  rows1 and rows2 may be 0.
+ * K % 256 == 0, K <= 16384. */
+int gemq_step_gemv(const void* x, const void* res, int res_is_half, const void* norm_weight, float eps, void* sum_out,
+                   const void* w0, int rows0, const void* w1, int rows1, const void* w2, int rows2, void* out, int K,
+                   int is_bf16, gemq_stream_t stream);
+
+/* The same sum and normalisation alone; the normalised vector is written as fp16.  K % 8 == 0, K <= 16384. */
+int gemq_step_norm(const void* x, const void* res, int res_is_half, const void* weight, float eps, void* sum_out,
+                   void* out_half, int K, int is_bf16, gemq_stream_t stream);
+
+/* qkv [(heads + 2 * kv_heads) * head_dim]: rotary embedding (half-split, inv_freq fp32 [head_dim / 2]) of queries and
+ * key at position pos[0] (device memory, taken as 0 .. cache_len - 1), key and value stored there in keys / values
+ * [kv_heads, cache_len, head_dim], then softmax attention over positions 0 .. pos: out [heads * head_dim].
+ * head_dim 64 or 128, heads a multiple of kv_heads, at most 8 times as many. */
+int gemq_step_attention(const void* qkv, const float* inv_freq, const int64_t* pos, void* keys, void* values, void* out,
+                        int heads, int kv_heads, int head_dim, int cache_len, int is_bf16, gemq_stream_t stream);
+
 /* ---- for callers that cannot allocate --------------------------------------------------------- */
 
 /* No counterpart in the reference.  y[1, N] = x[1, K] @ deq(wq), the same result as
