@@ -121,56 +121,79 @@ __device__ __forceinline__ void build_pow2(const LinearParams& P, unsigned char*
   }
 }
 
-// 3-bit: groups are not word aligned.  Group statistics first (half a warp per group), then the pieces.
+// 3-bit: groups are not word aligned.  Group statistics first (half a warp per group and row), then the pieces,
+// a lane's two words at a time.
 template <typename T>
 __device__ __forceinline__ void build_b3(const LinearParams& P, unsigned char* tab, const T* x, int rows, int lo, int hi, int lane) {
   const int goff = stage_pieces(3) * 64 * rows, tb = table_stage_bytes(3, rows), re = (rows + 1) & ~1;
   const bool vec = P.vec != 0;
   const int g0 = 5 * (lo >> 2), ng = min(P.K / kGroup, 5 * ((hi + 3) >> 2)) - g0;
   const int h = lane >> 4, l16 = lane & 15;
+  // four loads in flight: one after the other they cost a trip to L2 each, 40 us for 16 rows of 4096
+  constexpr int kAhead = 4;
 #pragma unroll 1
-  for (int t = 0; t < rows; ++t) {
-#pragma unroll 4
-    for (int i = 0; i < ng; i += 2) {
-      const int gl = i + h;
-      float mx = 0.f, sm = 0.f;
-      if (gl < ng) {
-        const uint4 v = load8(x + static_cast<size_t>(t) * P.ldx + (g0 + gl) * kGroup + 8 * l16, vec);
-        const T* e = reinterpret_cast<const T*>(&v);
+  for (int i0 = h; i0 < rows * ng + h; i0 += 2 * kAhead) {
+    uint4 v[kAhead];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float f = to_f<T>(e[k]);
-          mx = fmaxf(mx, fabsf(f));
-          sm += f;
-        }
+    for (int u = 0; u < kAhead; ++u) {
+      const int i = i0 + 2 * u, t = i / ng;
+      v[u] = i < rows * ng ? load8(x + static_cast<size_t>(t) * P.ldx + (g0 + i - t * ng) * kGroup + 8 * l16, vec)
+                           : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int i = i0 + 2 * u, t = i / ng;
+      const T* e = reinterpret_cast<const T*>(&v[u]);
+      float mx = 0.f, sm = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float f = to_f<T>(e[k]);
+        mx = fmaxf(mx, fabsf(f));
+        sm += f;
       }
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) {
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         sm += __shfl_xor_sync(0xffffffffu, sm, o);
       }
-      if (l16 == 0 && gl < ng) {
+      if (l16 == 0 && i < rows * ng) {
         int sg, slot;
-        group_place(3, g0 + gl, sg, slot);
+        group_place(3, g0 + i - t * ng, sg, slot);
         *reinterpret_cast<float2*>(tab + (sg - lo) * tb + goff + (slot * re + t) * 8) = group_pair(group_exponent(mx), sm);
       }
     }
   }
   __syncwarp();
 #pragma unroll 1
-  for (int t = 0; t < rows; ++t) {
-    const T* xr = x + static_cast<size_t>(t) * P.ldx;  // out of L1 now
+  for (int i = lane; i < (hi - lo) * 12; i += 32) {
+    const int sg = i / 12, r = i - 12 * sg, pass = r >> 2, c = r & 3;
+    const PassB3 p = pass_of_b3(lo + sg, pass, c);
+    const bool on = p.grp - g0 < ng;  // past the last group: zeros
+    int gs, slot;
+    group_place(3, p.grp, gs, slot);
+    const unsigned char* un = tab + (gs - lo) * tb + goff + slot * re * 8;
+    unsigned char* dst = tab + sg * tb + 3 * pass * rows * 64 + c * 16;
 #pragma unroll 2
-    for (int i = lane; i < (hi - lo) * 36; i += 32) {
-      const int sg = i / 36, r = i - 36 * sg, q = r >> 2, c = r & 3;
-      const uint4 v = piece_b3(lo + sg, q, c, [&](int k) { return k < P.K ? to_f<T>(xr[k]) : 0.f; }, [&](int grp) {
-        if (grp - g0 >= ng) return 0.f;
-        int gs, slot;
-        group_place(3, grp, gs, slot);
-        const float un = *reinterpret_cast<const float*>(tab + (gs - lo) * tb + goff + (slot * re + t) * 8);
-        return pow2i(24 - (static_cast<int>(__float_as_uint(un) >> 23) - 127));  // un = 2^(24 - ce)
-      });
-      *reinterpret_cast<uint4*>(tab + sg * tb + (q * rows + t) * 64 + c * 16) = v;
+    for (int t = 0; t < rows; ++t) {
+      const T* xr = x + static_cast<size_t>(t) * P.ldx + p.k0;  // out of L1 now
+      float v[20];
+#pragma unroll
+      for (int j = 0; j < 20; j += 4) {
+        uint2 q = make_uint2(0u, 0u);
+        T* e = reinterpret_cast<T*>(&q);
+        if (on && p.k0 + j < P.K) {
+          if (vec) q = *reinterpret_cast<const uint2*>(xr + j);
+          else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) e[k] = xr[j + k];
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[j + k] = to_f<T>(e[k]);
+      }
+      // un = 2^(24 - ce)
+      const float f = on ? pow2i(24 - (static_cast<int>(__float_as_uint(*reinterpret_cast<const float*>(un + t * 8)) >> 23) - 127)) : 0.f;
+      put_pass_b3(v, f, p, dst + t * 64, 64 * rows);
     }
   }
 }

@@ -429,26 +429,43 @@ __device__ __forceinline__ void word_pieces(const float (&x)[32 / B], float f, u
   }
 }
 
-// 3-bit: piece q (0..8) of stage sg for lane column c.  x(k) = activation k, 0 past the end; f(group) = factor.
-template <typename X, typename G>
-__device__ __forceinline__ uint4 piece_b3(int sg, int q, int c, X x, G factor) {
-  const int pass = q / 3, s4 = sg & 3;
+// 3-bit: the three pieces that pass `pass` (0..2) of stage sg has for lane column c.  They hold the lane's twenty
+// activations k0 .. k0 + 19 (two packed words); the ones outside the pass's group are masked out, two per operand.
+struct PassB3 {
+  int k0, grp;
+  uint32_t mask[10];
+};
+__device__ __forceinline__ PassB3 pass_of_b3(int sg, int pass, int c) {
+  const int s4 = sg & 3;
   // pass -> block of the stage, and which of its two groups (0: it has one, 1: the first, 2: the second)
   const int blk = 2 * sg + (s4 < 2 ? (pass > 0) : (pass == 2));
   const int part = s4 < 2 ? pass : (pass == 2 ? 0 : pass + 1);
   const int end = 5 * (sg >> 2) + s4;  // the group that ends in this stage
-  const int grp = part == 0 ? (s4 < 2 ? end : end + 1) : end + part - 1;
-  const float f = factor(grp);
-  __half v[8];
+  PassB3 p;
+  p.grp = part == 0 ? (s4 < 2 ? end : end + 1) : end + part - 1;
+  p.k0 = 80 * blk + 20 * c;
+  const int first = max(p.grp * kGroup - p.k0, 0), last = min(max((p.grp + 1) * kGroup - p.k0, 0), 20);
+  const uint32_t on = first < 20 ? (1u << last) - (1u << first) : 0u;
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int slot = 4 * (q % 3) + (e >> 1);  // operand slot 0..9, above: padding
-    const int pr = slot % 5;
-    const int k = (8 * blk + 2 * c + (slot >= 5)) * 10 + pr + 5 * (e & 1);
-    const float xv = slot < 10 && (k >> 7) == grp ? x(k) : 0.f;
-    v[e] = __float2half_rn(xv * (f * pow2i(-Fmt<3>::pos(pr))));
+  for (int s = 0; s < 10; ++s) {
+    const int j = 10 * (s / 5) + s % 5;
+    p.mask[s] = ((on >> j) & 1u ? 0x0000ffffu : 0u) | ((on >> (j + 5)) & 1u ? 0xffff0000u : 0u);
   }
-  return *reinterpret_cast<const uint4*>(v);
+  return p;
+}
+// x = the twenty activations, f = the group's factor, step = bytes from a piece to the next.
+__device__ __forceinline__ void put_pass_b3(const float (&x)[20], float f, const PassB3& p, unsigned char* dst, int step) {
+  uint32_t h[12];
+#pragma unroll
+  for (int s = 0; s < 10; ++s) {
+    const int j = 10 * (s / 5) + s % 5;
+    const float m = f * pow2i(-Fmt<3>::pos(s % 5));
+    const __half2 v = __floats2half2_rn(x[j] * m, x[j + 5] * m);
+    h[s] = *reinterpret_cast<const uint32_t*>(&v) & p.mask[s];
+  }
+  h[10] = h[11] = 0u;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(dst + q * step) = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
 }
 
 // Stage and slot of a group.
@@ -491,11 +508,16 @@ __device__ __forceinline__ void group_to_table(const T* v, int bits, int grp, un
     // the group's passes, counted from the run's first: 0, 1 | 2, 3, 4 | 5, 6 | 7, 8, 9 | 10, 11
     const int first = i5 == 0 ? 0 : (i5 == 1 ? 2 : (i5 == 2 ? 5 : (i5 == 3 ? 7 : 10)));
     const int count = (i5 == 1 || i5 == 3) ? 3 : 2;
-    for (int i = l16; i < count * 12; i += 16) {
-      const int ps = first + i / 12, q3 = (i % 12) >> 2, c = i & 3;
-      const int s3 = 4 * run + ps / 3, q = 3 * (ps % 3) + q3;
-      const uint4 o = piece_b3(s3, q, c, [&](int k) { return to_f<T>(v[k - grp * kGroup]); }, [&](int) { return f; });
-      *reinterpret_cast<uint4*>(tab + s3 * tb + (q * rows + t) * 64 + c * 16) = o;
+    if (l16 < 4 * count) {
+      const int ps = first + (l16 >> 2), c = l16 & 3, s3 = 4 * run + ps / 3, pass = ps % 3;
+      const PassB3 p = pass_of_b3(s3, pass, c);
+      float x[20];
+#pragma unroll
+      for (int j = 0; j < 20; ++j) {
+        const int k = p.k0 + j - grp * kGroup;
+        x[j] = k >= 0 && k < kGroup ? to_f<T>(v[k]) : 0.f;
+      }
+      put_pass_b3(x, f, p, tab + s3 * tb + (3 * pass * rows + t) * 64 + c * 16, 64 * rows);
     }
     return;
   }
