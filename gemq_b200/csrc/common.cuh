@@ -20,6 +20,19 @@ inline int launch_status() {
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Multiprocessors of the current device, 0 on failure.
+inline int sm_count() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (!cached[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
 // Streaming 128-bit load: weights are read once per step, so they should not
 // displace the activation tables or metadata in L1.
 __device__ __forceinline__ uint4 ld_stream_v4(const uint32_t* p) {

@@ -1573,18 +1573,6 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
 }  // namespace fused
 
 // ---- host ----------------------------------------------------------------------------------------
-static int fused_sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
 static fused::Mat3 mat_of(const gemq_stacked_t& W) {
   return {reinterpret_cast<const uint32_t*>(W.wq), static_cast<const __half*>(W.scales), static_cast<const __half*>(W.zeros)};
 }
@@ -1612,7 +1600,7 @@ bool decode_fused_ok(const gemq_moe_layer_t* L, size_t partial_floats) {
   const size_t slices = static_cast<size_t>(cdiv(cdiv(D > maxf ? D : maxf, kGroup), 4));
   if (slices * c_total > partial_floats) return false;
   // parts per CTA (a part is a run of quanta of one matrix and column chunk): bound for any bit widths
-  int sms = fused_sm_count();
+  int sms = sm_count();
   if (sms <= 0) return false;
   const int u0 = pairs * 2 * cdiv(D / kGroup, 4), u1 = nch1 * (A * cdiv(F / kGroup, 4) + cdiv(SF / kGroup, 4));
   const int grid = (u0 > u1 ? u0 : u1) < sms ? (u0 > u1 ? u0 : u1) : sms;
@@ -1637,7 +1625,7 @@ int launch_decode_fused(const gemq_moe_layer_t* L, const __half* x, __half* out,
       return GEMQ_ERR_LAUNCH;
     attr_set[dev] = true;
   }
-  const int sms = fused_sm_count();
+  const int sms = sm_count();
   if (sms <= 0) return GEMQ_ERR_LAUNCH;
   FusedParams P = {};
   P.x = x; P.gate = static_cast<const __half*>(L->gate); P.out = out;

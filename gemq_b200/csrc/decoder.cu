@@ -422,14 +422,6 @@ cudaLaunchConfig_t config(dim3 grid, int threads, size_t smem, gemq_stream_t st,
   return cfg;
 }
 
-int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (!cached[dev] && cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  return cached[dev];
-}
-
 }  // namespace
 }  // namespace gemq
 

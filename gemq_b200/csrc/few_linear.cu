@@ -47,6 +47,73 @@ __device__ __forceinline__ uint4 load8(const T* p, bool vec) {
   return v;
 }
 
+// The raw activations of `items` (stage, row) pairs become pieces in place.
+template <typename T, int B, int kAhead>
+__device__ __forceinline__ void convert_pow2(unsigned char* tab, int rows, int items, int lane) {
+  using F = Fmt<B>;
+  constexpr int EPS = F::kEps, QW = EPS / 8;
+  const int goff = stage_pieces(B) * 64 * rows, tb = table_stage_bytes(B, rows), re = (rows + 1) & ~1;
+  const int wr = (lane >> 2) & 3, c = lane & 3, h = lane >> 4;
+  const int slot = B == 1 ? wr : (B == 2 ? wr >> 1 : 0);  // the group of the lane's word
+  auto advance = [&](int& sg, int& t) {
+    for (t += 2; t >= rows; t -= rows) ++sg;
+  };
+  int sg = 0, t = h;
+  if (t >= rows) { t = 0; sg = 1; }
+#pragma unroll 1
+  for (int i0 = h; i0 < items + h; i0 += 2 * kAhead) {
+    uint4 raw[kAhead][QW];
+    unsigned char* st[kAhead];
+    int row[kAhead];
+    float mx[kAhead], sm[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const bool on = i0 + 2 * u < items;
+      st[u] = tab + (on ? sg : 0) * tb;
+      row[u] = on ? t : 0;
+#pragma unroll
+      for (int j = 0; j < QW; ++j)
+        raw[u][j] = *reinterpret_cast<const uint4*>(st[u] + ((wr * QW + j) * rows + row[u]) * 64 + c * 16);
+      advance(sg, t);
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      mx[u] = sm[u] = 0.f;
+#pragma unroll
+      for (int j = 0; j < QW; ++j) {
+        const T* e = reinterpret_cast<const T*>(&raw[u][j]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float f = to_f<T>(e[k]);
+          mx[u] = fmaxf(mx[u], fabsf(f));
+          sm[u] += f;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 4 * B; o <<= 1)
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        mx[u] = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], o));
+        sm[u] += __shfl_xor_sync(0xffffffffu, sm[u], o);
+      }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i0 + 2 * u < items) {
+        const int ce = group_exponent(mx[u]);
+        if ((lane & (4 * B - 1)) == 0) *reinterpret_cast<float2*>(st[u] + goff + (slot * re + row[u]) * 8) = group_pair(ce, sm[u]);
+        float xv[EPS];
+#pragma unroll
+        for (int j = 0; j < QW; ++j) {
+          const T* e = reinterpret_cast<const T*>(&raw[u][j]);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) xv[8 * j + k] = to_f<T>(e[k]);
+        }
+        word_pieces<B>(xv, pow2i(ce), st[u] + (wr * QW * rows + row[u]) * 64 + c * 16, 64 * rows);
+      }
+  }
+}
+
 // One warp: table of the k range of stages [lo, hi) for `rows` rows, 1/2/4-bit.  A lane takes one packed
 // word's activations (32 / B neighbours), a half-warp a stage, 4 * B lanes a group.  The activations are
 // first copied raw to where their pieces will stand (same size, same lane), all copies in flight at once,
@@ -56,20 +123,23 @@ template <typename T, int B>
 __device__ __forceinline__ void build_pow2(const LinearParams& P, unsigned char* tab, const T* x, int rows, int lo, int hi, int lane) {
   using F = Fmt<B>;
   constexpr int EPS = F::kEps, QW = EPS / 8;
-  const int goff = stage_pieces(B) * 64 * rows, tb = table_stage_bytes(B, rows), re = (rows + 1) & ~1;
+  const int tb = table_stage_bytes(B, rows);
   const bool vec = P.vec != 0;
   const int wr = (lane >> 2) & 3, c = lane & 3, h = lane >> 4;
-  const int ns = hi - lo;
+  const int items = (hi - lo) * rows;  // (stage, row), half a warp each
   const int kl = (lo * kStageRows + 8 * (wr >> 1) + F::row(c, wr & 1)) * EPS;  // first activation of the word in stage lo
-  const int slot = B == 1 ? wr : (B == 2 ? wr >> 1 : 0);                      // its group
   unsigned char* mine = tab + wr * QW * rows * 64 + c * 16;
-#pragma unroll 1
-  for (int sg = h; sg < ns; sg += 2) {
-    const int k0 = kl + sg * kStageRows * EPS;
-    const T* src = x + (k0 < P.K ? k0 : 0);
-    unsigned char* dst = mine + sg * tb;
+  auto advance = [&](int& sg, int& t) {  // two items on
+    for (t += 2; t >= rows; t -= rows) ++sg;
+  };
+  {
+    int sg = 0, t = h;
+    if (t >= rows) { t = 0; sg = 1; }
 #pragma unroll 2
-    for (int t = 0; t < rows; ++t) {
+    for (int i = h; i < items; i += 2) {
+      const int k0 = kl + sg * kStageRows * EPS;
+      const T* src = x + static_cast<size_t>(t) * P.ldx + (k0 < P.K ? k0 : 0);
+      unsigned char* dst = mine + sg * tb + t * 64;
 #pragma unroll
       for (int j = 0; j < QW; ++j) {
         if (vec) {
@@ -80,45 +150,14 @@ __device__ __forceinline__ void build_pow2(const LinearParams& P, unsigned char*
           *reinterpret_cast<uint4*>(dst + j * 64 * rows) = k0 < P.K ? load8(src + 8 * j, false) : make_uint4(0u, 0u, 0u, 0u);
         }
       }
-      src += P.ldx;
-      dst += 64;
+      advance(sg, t);
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
-#pragma unroll 1
-  for (int s0 = 0; s0 < ns; s0 += 2) {
-    const int sg = s0 + h;
-    const bool on = sg < ns;
-    unsigned char* st = tab + (on ? sg : s0) * tb;
-#pragma unroll 1
-    for (int t = 0; t < rows; ++t) {
-      unsigned char* dst = st + (wr * QW * rows + t) * 64 + c * 16;
-      float xv[EPS];
-      float mx = 0.f, sm = 0.f;
-#pragma unroll
-      for (int j = 0; j < QW; ++j) {
-        const uint4 v = *reinterpret_cast<const uint4*>(dst + j * 64 * rows);
-        const T* e = reinterpret_cast<const T*>(&v);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float f = to_f<T>(e[k]);
-          xv[8 * j + k] = f;
-          mx = fmaxf(mx, fabsf(f));
-          sm += f;
-        }
-      }
-#pragma unroll
-      for (int o = 1; o < 4 * B; o <<= 1) {
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        sm += __shfl_xor_sync(0xffffffffu, sm, o);
-      }
-      if (on) {
-        const int ce = group_exponent(mx);
-        if ((lane & (4 * B - 1)) == 0) *reinterpret_cast<float2*>(st + goff + (slot * re + t) * 8) = group_pair(ce, sm);
-        word_pieces<B>(xv, pow2i(ce), dst, 64 * rows);
-      }
-    }
-  }
+  // One row: an item at a time, there are few and the instructions are cold.  More: kAhead items of a half-warp
+  // side by side, the shuffles of a group's maximum and sum are a chain of 500 cycles.
+  if (rows == 1) convert_pow2<T, B, 1>(tab, 1, items, lane);
+  else convert_pow2<T, B, B == 1 ? 2 : 4>(tab, rows, items, lane);
 }
 
 // 3-bit: groups are not word aligned.  Group statistics first (half a warp per group and row), then the pieces,
@@ -127,7 +166,8 @@ template <typename T>
 __device__ __forceinline__ void build_b3(const LinearParams& P, unsigned char* tab, const T* x, int rows, int lo, int hi, int lane) {
   const int goff = stage_pieces(3) * 64 * rows, tb = table_stage_bytes(3, rows), re = (rows + 1) & ~1;
   const bool vec = P.vec != 0;
-  const int g0 = 5 * (lo >> 2), ng = min(P.K / kGroup, 5 * ((hi + 3) >> 2)) - g0;
+  // the groups that its stages meet
+  const int g0 = 5 * (lo >> 2) + (lo & 3), ng = hi > lo ? min(P.K / kGroup, 5 * ((hi - 1) >> 2) + ((hi - 1) & 3) + 2) - g0 : 0;
   const int h = lane >> 4, l16 = lane & 15;
   // four loads in flight: one after the other they cost a trip to L2 each, 40 us for 16 rows of 4096
   constexpr int kAhead = 4;
@@ -157,24 +197,26 @@ __device__ __forceinline__ void build_b3(const LinearParams& P, unsigned char* t
         sm += __shfl_xor_sync(0xffffffffu, sm, o);
       }
       if (l16 == 0 && i < rows * ng) {
+        const int grp = g0 + i - t * ng, i5 = grp % 5;
         int sg, slot;
-        group_place(3, g0 + i - t * ng, sg, slot);
-        *reinterpret_cast<float2*>(tab + (sg - lo) * tb + goff + (slot * re + t) * 8) = group_pair(group_exponent(mx), sm);
+        group_place(3, grp, sg, slot);
+        const float2 fs = group_pair(group_exponent(mx), sm);
+        if (sg >= lo && sg < hi) *reinterpret_cast<float2*>(tab + (sg - lo) * tb + goff + (slot * re + t) * 8) = fs;
+        if (i5 >= 1 && i5 <= 3 && sg > lo) *reinterpret_cast<float2*>(tab + (sg - 1 - lo) * tb + goff + (re + t) * 8) = fs;
       }
     }
   }
   __syncwarp();
+  const int halves = (hi - lo) * 12 <= 16 ? 2 : 1;  // one stage: half the lanes take the odd rows
 #pragma unroll 1
-  for (int i = lane; i < (hi - lo) * 12; i += 32) {
+  for (int i = lane & (32 / halves - 1); i < (hi - lo) * 12; i += 32 / halves) {
     const int sg = i / 12, r = i - 12 * sg, pass = r >> 2, c = r & 3;
     const PassB3 p = pass_of_b3(lo + sg, pass, c);
-    const bool on = p.grp - g0 < ng;  // past the last group: zeros
-    int gs, slot;
-    group_place(3, p.grp, gs, slot);
-    const unsigned char* un = tab + (gs - lo) * tb + goff + slot * re * 8;
+    const bool on = p.grp < P.K / kGroup;  // past the last group: zeros
+    const unsigned char* un = tab + sg * tb + goff + p.slot * re * 8;
     unsigned char* dst = tab + sg * tb + 3 * pass * rows * 64 + c * 16;
 #pragma unroll 2
-    for (int t = 0; t < rows; ++t) {
+    for (int t = halves == 2 ? lane >> 4 : 0; t < rows; t += halves) {
       const T* xr = x + static_cast<size_t>(t) * P.ldx + p.k0;  // out of L1 now
       float v[20];
 #pragma unroll
@@ -325,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, NB == 1 ? 3 : 2) few_linear_kernel(c
   // ---- add the warps' and the cluster's parts of k, in order ----------------------------------------
   __syncthreads();
   if (P.splits > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-  float* mine = reinterpret_cast<float*>(ring + P.ring * kLinStage + kCons * P.tab_bytes);  // [splits][16][64] in rank 0
+  float* mine = reinterpret_cast<float*>(ring + P.ring * kLinStage + kCons * P.tab_bytes);  // [splits][tile_rows][64] in rank 0
   const uint32_t rank = P.splits > 1 ? cluster_rank() : 0u;
   for (int i = tid; i < rows * 16; i += kThreads) {
     const int t = i >> 4, n4 = (i & 15) * 4;
@@ -335,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, NB == 1 ? 3 : 2) few_linear_kernel(c
       const float4 u = *reinterpret_cast<const float4*>(red + (q * kTileRows + t) * 64 + n4);
       v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
     }
-    float* dst = mine + (rank * kTileRows + t) * 64 + n4;
+    float* dst = mine + (rank * P.tile_rows + t) * 64 + n4;
     if (rank == 0) *reinterpret_cast<float4*>(dst) = v;
     else st_cluster_f4(smem_u32(dst), 0u, v);
   }
@@ -350,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, NB == 1 ? 3 : 2) few_linear_kernel(c
     if (n >= P.N) continue;
     float4 v = *reinterpret_cast<const float4*>(mine + t * 64 + n4);
     for (int q = 1; q < P.splits; ++q) {
-      const float4 u = *reinterpret_cast<const float4*>(mine + (q * kTileRows + t) * 64 + n4);
+      const float4 u = *reinterpret_cast<const float4*>(mine + (q * P.tile_rows + t) * 64 + n4);
       v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
     }
     const float f[4] = {v.x, v.y, v.z, v.w};
@@ -397,6 +439,48 @@ static int launch_linear(const LinearParams& P, dim3 grid, size_t smem, cudaStre
 using namespace gemq;
 using namespace gemq::few;
 
+// A warp's part of k is whole stages.  The cluster grows while the CTAs run at once (three per SM) and every warp
+// keeps a stage, and as long as the warps' tables do not fit twice per SM.  448 CTAs on 444 places: 12.4 us
+// instead of 9.3 (4 rows, 2816 x 14336, 2 bits).
+static bool linear_split(int rows, int N, int K, int nbits, int* tile_rows, int* splits_out, int* tab_bytes, size_t* smem) {
+  const int cols = cdiv(N, 64), units = n_stages(K, nbits), sms = sm_count();
+  if (sms <= 0) return false;
+  for (int tr = rows < kTileRows ? rows : kTileRows; tr > 0; tr = tr > 1 ? (tr + 1) / 2 : 0) {
+    const int tiles = cdiv(rows, tr);
+    int splits = 1;
+    while (splits < 8 && cols * tiles * splits * 2 <= 3 * sms && units >= kCons * splits * 2) splits *= 2;
+    for (;; splits *= 2) {
+      *tab_bytes = (cdiv(units, kCons * splits) * table_stage_bytes(nbits, tr) + 127) / 128 * 128;
+      *smem = 1024 + static_cast<size_t>(kMaxRing) * kLinStage + static_cast<size_t>(kCons) * *tab_bytes +
+              static_cast<size_t>(splits) * tr * 64 * sizeof(float);
+      if (*smem <= kMaxDyn / 2 || splits == 8 || units < kCons * splits * 2) break;
+    }
+    *tile_rows = tr;
+    *splits_out = splits;
+    if (*smem <= kMaxDyn) return true;
+  }
+  return false;
+}
+
+// Estimates in us of what the two kernels were measured to take (1 to 64 rows of 14 shapes, 512 to 14336 wide).  The
+// GEMM: a fixed 3 and its de-quantisation, which grows with K and the bits and not with the rows; the few-row kernel:
+// rounds of the chip, each with a start and a table of the k of a warp.  Where the lines cross the two differ by less
+// than the estimates are off; the 3-bit table costs 2.5 times the others'.
+extern "C" int gemq_linear_takes_gemm(int rows, int N, int K, int nbits) {
+  int tr, splits, tab;
+  size_t smem;
+  const int sms = sm_count();
+  if (rows <= 0 || N <= 0 || K <= 0 || nbits < 1 || nbits > 4 || sms <= 0) return rows >= 32;
+  if (!linear_split(rows, N, K, nbits, &tr, &splits, &tab, &smem)) return 1;
+  static const float per_k[4] = {0.40f, 0.40f, 0.78f, 0.50f};
+  const float gemm = 3.f + cdiv(cdiv(N, 256) * cdiv(rows, 256), sms / 2) * (K / 128) * per_k[nbits - 1];
+  const int per_sm = tr > 8 || 3 * (smem + 2048) > kMaxDyn ? (2 * (smem + 2048) > kMaxDyn ? 1 : 2) : 3;
+  const int rounds = cdiv(cdiv(N, 64) * splits * cdiv(rows, tr), per_sm * sms);
+  const float warp_k = static_cast<float>(K) / static_cast<float>(kCons * splits);
+  const float few = rounds * (tr > 8 ? 3.5f + 0.033f * warp_k : 3.f + warp_k * (0.006f + 0.0008f * tr)) * (nbits == 3 ? 2.5f : 1.f);
+  return gemm < few;
+}
+
 extern "C" int gemq_linear_rows(const void* x, int ldx, int x_is_bf16, const int32_t* wq, const void* scales, const void* zeros,
                                 const void* bias, void* y, int rows, int N, int K, int nbits, int group_size, int32_t* err,
                                 gemq_stream_t stream) {
@@ -412,31 +496,12 @@ extern "C" int gemq_linear_rows(const void* x, int ldx, int x_is_bf16, const int
   P.ldx = ldx;
   P.vec = aligned16(x) && (ldx % 8 == 0 || rows == 1);
   P.rows = rows; P.N = N; P.K = K; P.bits = nbits;
-  // A warp's part of k is whole stages (3-bit: whole runs of four).  The cluster grows while the CTAs do not
-  // fill the chip and every warp keeps a unit, and as long as the warps' tables do not fit twice per SM.
-  const int cols = cdiv(N, 64);
-  const int unit = nbits == 3 ? 4 : 1, units = cdiv(n_stages(K, nbits), unit);
-  P.tile_rows = rows < kTileRows ? rows : kTileRows;
-  size_t smem = 0;
-  for (;;) {
-    const int tiles = cdiv(rows, P.tile_rows);
-    int splits = 1;
-    while (splits < 8 && cols * tiles * splits * 2 <= 480 && units >= kCons * splits * 2) splits *= 2;
-    for (;; splits *= 2) {
-      P.splits = splits;
-      P.tab_bytes = (cdiv(units, kCons * splits) * unit * table_stage_bytes(nbits, P.tile_rows) + 127) / 128 * 128;
-      P.ring = kMaxRing;
-      smem = 1024 + static_cast<size_t>(P.ring) * kLinStage + static_cast<size_t>(kCons) * P.tab_bytes +
-             static_cast<size_t>(splits) * kTileRows * 64 * sizeof(float);
-      if (smem <= kMaxDyn / 2 || splits == 8 || units < kCons * splits * 2) break;
-    }
-    if (smem <= kMaxDyn) break;
-    if (P.tile_rows == 1) return GEMQ_ERR_BAD_SHAPE;
-    P.tile_rows = (P.tile_rows + 1) / 2;
-  }
+  size_t smem;
+  if (!linear_split(rows, N, K, nbits, &P.tile_rows, &P.splits, &P.tab_bytes, &smem)) return GEMQ_ERR_BAD_SHAPE;
+  P.ring = kMaxRing;
   const int tiles = cdiv(rows, P.tile_rows);
   if (tiles > 65535) return GEMQ_ERR_BAD_SHAPE;
-  const dim3 grid(cols * P.splits, 1, tiles);
+  const dim3 grid(cdiv(N, 64) * P.splits, 1, tiles);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (P.tile_rows > 8)
     return x_is_bf16 ? launch_linear<__nv_bfloat16, 2>(P, grid, smem, st) : launch_linear<__half, 2>(P, grid, smem, st);

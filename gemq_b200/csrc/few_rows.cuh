@@ -45,8 +45,7 @@ __host__ __device__ constexpr int n_stages(int K, int bits) { return cdiv(packed
 // Table pieces of a stage: 16 bytes per row and lane column = the B registers of two k-steps.
 // 3-bit: three passes of five k-steps, padded to six.
 __host__ __device__ constexpr int stage_pieces(int bits) { return bits == 3 ? 9 : 16 / bits; }
-// Group slots of a stage.  3-bit: the group that ends in stage s of a run of four, and behind the run's last
-// stage the fifth group.
+// Group slots of a stage.  3-bit: the two groups that a stage (160 k) meets; the one that ends in it is the first.
 __host__ __device__ constexpr int stage_slots(int bits) { return bits == 3 ? 2 : 4 / bits; }
 // Bytes of a stage of the table: pieces [piece][row][lane column], then per group slot and row (row count
 // rounded up to even) what undoes the row's scaling of the group, and the sum of its activations.
@@ -335,7 +334,9 @@ __device__ __forceinline__ void pass_b3(State<NB>& S, uint32_t W, TablePtr<NB>& 
 
 // A stage of a 3-bit matrix.  64 packed rows = 640 k = five groups = four stages; a group ends inside
 // blocks 1, 3, 4, 6 of the run and at its end.  A block with two groups takes two passes whose table
-// entries hold only the one or the other.  `s4` = stage of the run, `left` = groups from the run's first on.
+// entries hold only the one or the other.  Both groups of a stage are folded in it, so that a reduction can be
+// split at any stage: 4096 k are 26 of them, but only 7 runs.  `s4` = stage of the run, `left` = groups from the
+// run's first on.
 template <int NB, int STEP>
 __device__ __forceinline__ void stage_b3(State<NB>& S, uint32_t W, uint32_t T, uint32_t zero, uint32_t meta, int rows, int s4, int left,
                                          int lane) {
@@ -345,11 +346,12 @@ __device__ __forceinline__ void stage_b3(State<NB>& S, uint32_t W, uint32_t T, u
 #pragma unroll 1
   for (int p = 0; p < 3; ++p) {
     pass_b3<NB, STEP>(S, W, t, late ? p >> 1 : (p + 1) >> 1, lane);
-    if (p == (late ? 0 : 1) && s4 < left) fold<NB, true>(S, meta, ft, rows, lane);
+    const bool first = p == (late ? 0 : 1);
+    if (first || (p == 2 && s4 + 1 < left))
+      fold<NB, true>(S, meta + (first ? 0 : 256), ft + (first ? 0 : 16 * ((rows + 1) >> 1)), rows, lane);
   }
-  if (s4 == 3 && left > 4) fold<NB, true>(S, meta + 256, ft + 16 * ((rows + 1) >> 1), rows, lane);
   const int c = lane & 3;
-  add_offsets<NB>(S, meta, ft, rows, (c == 0 && s4 < left) || (c == 1 && s4 == 3 && left > 4), lane);
+  add_offsets<NB>(S, meta, ft, rows, c == 0 || (c == 1 && s4 == 3 && left > 4), lane);
 }
 
 template <int B, int NB, int STEP>
@@ -387,13 +389,11 @@ __device__ __forceinline__ void tma_load_strips(void* dst, const CUtensorMap* ma
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Part p of n of a matrix's stages: whole stages, for 3-bit whole runs of four.
+// Part p of n of a matrix's stages.
 __device__ __forceinline__ void stage_range(int bits, int K, int p, int n, int& lo, int& hi) {
   const int st = n_stages(K, bits);
-  const int unit = bits == 3 ? 4 : 1;
-  const int u = cdiv(st, unit);
-  lo = min(st, (u * p / n) * unit);
-  hi = min(st, (u * (p + 1) / n) * unit);
+  lo = st * p / n;
+  hi = st * (p + 1) / n;
 }
 
 template <typename T> __device__ __forceinline__ float to_f(T v);
@@ -432,7 +432,7 @@ __device__ __forceinline__ void word_pieces(const float (&x)[32 / B], float f, u
 // 3-bit: the three pieces that pass `pass` (0..2) of stage sg has for lane column c.  They hold the lane's twenty
 // activations k0 .. k0 + 19 (two packed words); the ones outside the pass's group are masked out, two per operand.
 struct PassB3 {
-  int k0, grp;
+  int k0, grp, slot;
   uint32_t mask[10];
 };
 __device__ __forceinline__ PassB3 pass_of_b3(int sg, int pass, int c) {
@@ -442,7 +442,8 @@ __device__ __forceinline__ PassB3 pass_of_b3(int sg, int pass, int c) {
   const int part = s4 < 2 ? pass : (pass == 2 ? 0 : pass + 1);
   const int end = 5 * (sg >> 2) + s4;  // the group that ends in this stage
   PassB3 p;
-  p.grp = part == 0 ? (s4 < 2 ? end : end + 1) : end + part - 1;
+  p.slot = part == 0 ? (s4 < 2 ? 0 : 1) : part - 1;
+  p.grp = end + p.slot;
   p.k0 = 80 * blk + 20 * c;
   const int first = max(p.grp * kGroup - p.k0, 0), last = min(max((p.grp + 1) * kGroup - p.k0, 0), 20);
   const uint32_t on = first < 20 ? (1u << last) - (1u << first) : 0u;
@@ -468,7 +469,8 @@ __device__ __forceinline__ void put_pass_b3(const float (&x)[20], float f, const
   for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(dst + q * step) = make_uint4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
 }
 
-// Stage and slot of a group.
+// Stage and slot of a group; 3-bit: the ones in which it ends.  What undoes its scaling also goes to slot 1 of the
+// stage before, where groups 1 to 3 of a run begin.
 __device__ __forceinline__ void group_place(int bits, int grp, int& sg, int& slot) {
   if (bits == 3) { sg = 4 * (grp / 5) + min(grp % 5, 3); slot = grp % 5 == 4 ? 1 : 0; }
   else { const int n = 4 / bits; sg = grp / n; slot = grp - sg * n; }
@@ -505,6 +507,8 @@ __device__ __forceinline__ void group_to_table(const T* v, int bits, int grp, un
     *reinterpret_cast<float2*>(tab + sg * tb + stage_pieces(bits) * 64 * rows + (slot * re + t) * 8) = group_pair(ce, sm);
   if (bits == 3) {
     const int i5 = grp % 5, run = grp / 5;
+    if (l16 == 0 && i5 >= 1 && i5 <= 3)
+      *reinterpret_cast<float2*>(tab + (sg - 1) * tb + stage_pieces(3) * 64 * rows + (re + t) * 8) = group_pair(ce, sm);
     // the group's passes, counted from the run's first: 0, 1 | 2, 3, 4 | 5, 6 | 7, 8, 9 | 10, 11
     const int first = i5 == 0 ? 0 : (i5 == 1 ? 2 : (i5 == 2 ? 5 : (i5 == 3 ? 7 : 10)));
     const int count = (i5 == 1 || i5 == 3) ? 3 : 2;

@@ -4,18 +4,6 @@
 namespace gemq {
 namespace ts {
 
-int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
 template <int OUT, bool BF16>
 static int launch(const Params& P, int tiles_bound, cudaStream_t stream) {
   static bool done[64] = {false};
@@ -94,11 +82,6 @@ extern "C" int gemq_linear_gemm(const void* x, const int64_t* expert, const int3
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int rc = x_is_bf16 ? launch<kOutLinear, true>(P, tiles, st) : launch<kOutLinear, false>(P, tiles, st);
   return rc ? rc : launch_status();
-}
-
-extern "C" int gemq_linear_takes_gemm(int rows, int N, int K, int nbits) {
-  (void)N; (void)K; (void)nbits;
-  return rows >= 32;
 }
 
 extern "C" int gemq_dequant_gemm_tc(const void* x, const int64_t* expert, const int32_t* wq, const void* scales,

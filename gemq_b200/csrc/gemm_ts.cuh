@@ -673,7 +673,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
 // gemm_ts.cu; tiles_bound: most tiles the launch can have
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream);
 int launch_down(const Params& P, int tiles_bound, cudaStream_t stream);
-int sm_count();
 bool activation_maps(CUtensorMap (&maps)[4], const void* x, int K, long long rows);
 
 }  // namespace ts

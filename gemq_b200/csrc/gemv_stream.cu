@@ -921,18 +921,6 @@ static bool tensor_map(CUtensorMap* out, const void* base, int N, long long rows
                  : tensor_map_2d(out, base, 2, N, rows, 128, 4, false);
 }
 
-static int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
 static int launch_stream_t(GemvParams& P, cudaStream_t stream, int units_bound) {
   static bool attr_set[64] = {false};
   int dev = 0;

@@ -61,16 +61,16 @@ def dequant_gemm(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: i
             lambda *a: host_linear(*a, 0) if len(a) == 7 else None)
 def quant_linear(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, group_size: int,
                  bias: Optional[Tensor]) -> Tensor:
-    """``x [M, K] @ deq(w_q) + bias`` in x's dtype (fp16 or bf16): what ``QuantLinear`` computes.  Below
-    the row count of the tcgen05 GEMM, and for widths it does not take, one call of the few-row kernel
-    reads x and writes y in their own dtype; before, bf16 rows went through fp16 copies either side."""
+    """``x [M, K] @ deq(w_q) + bias`` in x's dtype (fp16 or bf16): what ``QuantLinear`` computes, in one call
+    of the tcgen05 GEMM or of the few-row kernel, whichever is estimated the faster; either reads x and writes
+    y in their own dtype."""
     dev = require_cuda(x, w_q, scales, zeros)
     M, K = x.shape
     N = w_q.shape[1]
     half = x.dtype in (torch.float16, torch.bfloat16)
-    tc = tc_gemm_ok(M, N, K, group_size) and (
-        not few_rows_ok(w_q, scales, zeros, K, N, group_size) or bool(_capi.lib.gemq_linear_takes_gemm(M, N, K, nbits)))
-    if half and (tc or few_rows_ok(w_q, scales, zeros, K, N, group_size)):
+    few = few_rows_ok(w_q, scales, zeros, K, N, group_size)
+    tc = bool(_capi.lib.gemq_linear_takes_gemm(M, N, K, nbits)) if few else tc_gemm_ok(M, N, K, group_size)
+    if half and (tc or few):
         check_kernel_form(w_q, scales, zeros, K, N, nbits, group_size)
         if bias is not None:
             bias = bias.to(device=dev, dtype=x.dtype).contiguous()
