@@ -467,9 +467,10 @@ static bool init_attrs() {
 }
 
 // Layers and batches this path takes: group 128, extents in whole groups, and on average at most
-// kFewAverage rows per expert (above, the tensor cores' de-quantised tiles cost less than two passes
-// over the packed words).
-constexpr int kFewAverage = 12;
+// kFewAverage rows per expert (above, the tensor cores' de-quantised tiles, whose cost does not grow with the rows,
+// win): 24 rows per expert take 323 against 452 us (8 experts of 4096 x 14336), 214 against 239 (64 of
+// 2048 x 1408), 135 against 129 (32 of them); 32 rows 393 against 454, 266 against 259, 153 against 133.
+constexpr int kFewAverage = 24;
 bool moe_few_rows_ok(const gemq_moe_layer_t* L, int tokens) {
   const int D = L->hidden, F = L->ffn, SF = L->shared_ffn;
   if (L->group_size != kGroup || D % kGroup || F % kGroup || SF % kGroup || D > 32768) return false;

@@ -717,16 +717,24 @@ extern "C" size_t gemq_gemv_workspace_bytes(int total_cols, int max_k, int token
   return gemv_workspace_bytes(total_cols, max_k, tokens);
 }
 
-// One matrix goes to the one-launch few-row kernel (few_linear.cu) for every shape that takes: 8.9 us
-// against 12.2 us for a 14336 x 4096 2-bit matrix and one row, 9.2 against 32.6 us for 13 rows of a 4-bit
-// 4096 x 4096 one (which took a pass over the weights per eight rows here).
+// One matrix goes to the one-launch few-row kernel (few_linear.cu): 8.9 us against 12.2 us for a 14336 x 4096
+// 2-bit matrix and one row, 9.2 against 32.6 us for 13 rows of a 4-bit 4096 x 4096 one (which took a pass over the
+// weights per eight rows here).  Except one row of a matrix that is both wide and deep: there its 64-column tiles
+// load some SMs twice as much as others for the whole product, where the quanta of the streaming kernel are dealt
+// evenly: 14336 x 14336 takes 22.7 / 43.4 / 26.6 us here against 24.3 / 59 / 30.5 (2, 3, 4 bits).  4096 x 14336
+// still is faster there (10.5 against 12.4, 2 bits); the line is between the two.
 extern "C" int gemq_linear_rows(const void* x, int ldx, int x_is_bf16, const int32_t* wq, const void* scales, const void* zeros,
                                 const void* bias, void* y, int rows, int N, int K, int nbits, int group_size, int32_t* err,
                                 gemq_stream_t stream);
 
+extern "C" int gemq_one_row_streams(int N, int K) {
+  const int sms = sm_count();
+  return sms > 0 && N > 64 * sms && K >= 8192;
+}
+
 namespace gemq {
-bool few_linear_takes(const void* wq, const void* scales, const void* zeros, const void* y, int N, int K, int G) {
-  return G == kGroup && K % kGroup == 0 && K <= 32768 && N % 32 == 0 && aligned16(wq) && aligned16(scales) && aligned16(zeros) &&
+bool few_linear_takes(const void* wq, const void* scales, const void* zeros, const void* y, int rows, int N, int K, int G) {
+  return !(rows == 1 && gemq_one_row_streams(N, K)) && G == kGroup && K % kGroup == 0 && K <= 32768 && N % 32 == 0 && aligned16(wq) && aligned16(scales) && aligned16(zeros) &&
          aligned16(y);
 }
 }  // namespace gemq
@@ -757,7 +765,7 @@ extern "C" int gemq_dequant_gemv(const void* x, int ldx, const int32_t* wq, cons
                                  void* workspace, size_t workspace_bytes, gemq_stream_t stream) {
   if (!x || !wq || !scales || !zeros || !y || tokens <= 0 || N <= 0 || K <= 0 || group_size <= 0 || !bits_ok(nbits))
     return GEMQ_ERR_BAD_ARG;
-  if (ldy == N && few_linear_takes(wq, scales, zeros, y, N, K, group_size)) {
+  if (ldy == N && few_linear_takes(wq, scales, zeros, y, tokens, N, K, group_size)) {
     if (!workspace || workspace_bytes < kMaxCounters * sizeof(int) || !aligned16(workspace)) return GEMQ_ERR_WORKSPACE;
     return gemq_linear_rows(x, ldx, 0, wq, scales, zeros, nullptr, y, tokens, N, K, nbits, group_size,
                             static_cast<int*>(workspace) + kErrWord, stream);

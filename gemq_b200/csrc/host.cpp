@@ -52,6 +52,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (K <= 0 || K % 128 || K > 32768 || N <= 0 || N % 32 || x->numel() == 0) return none();
   const int64_t M = x->numel() / K;
   if (M > (1 << 30) || (mode == kOneRowOp && M != 1)) return none();
+  if (M == 1 && x->scalar_type() == at::kHalf && gemq_one_row_streams(static_cast<int>(N), static_cast<int>(K))) return none();
   const bool gemm = mode == kLayer ? gemq_linear_takes_gemm(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(nbits))
                                    : mode == kGemmOp && M >= 32;
   if (mode != kLayer && !gemm && x->scalar_type() != at::kHalf) return none();

@@ -13,7 +13,7 @@
 
 namespace gemq {
 
-bool few_linear_takes(const void* wq, const void* scales, const void* zeros, const void* y, int N, int K, int G);  // gemv.cu
+bool few_linear_takes(const void* wq, const void* scales, const void* zeros, const void* y, int rows, int N, int K, int G);  // gemv.cu
 
 constexpr size_t kStaticScratchBytes = 2u << 20;  // 32 KB of arrival counters + fp32 split-K partial slots
 
@@ -58,7 +58,7 @@ extern "C" int gemq_dequant_gemv_static(const void* x, const int32_t* wq, const 
   void* ws = nullptr;
   if (int rc = static_scratch_ptr(&ws)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (few_linear_takes(wq, scales, zeros, y, N, K, group_size))  // needs no scratch: only the error word is used
+  if (few_linear_takes(wq, scales, zeros, y, 1, N, K, group_size))  // needs no scratch: only the error word is used
     return gemq_linear_rows(x, K, 0, wq, scales, zeros, nullptr, y, 1, N, K, nbits, group_size, static_cast<int*>(ws) + kErrWord,
                             stream);
   // The array keeps whatever the previous call left.  Kernels leave counters and partial slots

@@ -26,9 +26,9 @@ from .packed_linear import is_packed_linear
 
 ROUTE_FP16, ROUTE_FP32_SOFTMAX, ROUTE_FP32 = 0, 1, 2
 # Decode batches up to this many rows run the one-launch layer kernel row by row; larger ones go through the
-# expert-sorted grouped GEMM, which reads every distinct expert (and the shared experts) once per call and is
-# faster from about six rows on (measured on the DeepSeek-V2-Lite shape: 360 vs 275 us at 8 rows, 779 vs 333 at 16).
-_MAX_LOOPED_TOKENS = 4
+# expert-sorted kernels, which read every distinct expert (and the shared experts) once per call: two rows of the
+# DeepSeek-V2-Lite shape take 61 us there, 84 in the loop.
+_MAX_LOOPED_TOKENS = 1
 
 
 def _excl_cumsum(vals, device):

@@ -94,6 +94,11 @@ def tc_gemm_ok(M: int, N: int, K: int, group_size: int) -> bool:
     return M >= 32 and N % 32 == 0 and K % 64 == 0 and group_size % 64 == 0 and K % group_size == 0
 
 
+def one_row_streams(M: int, N: int, K: int) -> bool:
+    """One row of a matrix that the split-K streaming kernel takes in less time than the few-row kernel."""
+    return M == 1 and bool(_capi.lib.gemq_one_row_streams(N, K))
+
+
 def few_rows_ok(w_q, scales, zeros, K: int, N: int, group_size: int) -> bool:
     """Matrices the few-row kernel takes (``gemq_linear_rows``)."""
     return (group_size == 128 and K % 128 == 0 and K <= 32768 and N % 32 == 0 and

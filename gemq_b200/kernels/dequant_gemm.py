@@ -8,7 +8,7 @@ from torch import Tensor
 
 from .. import _capi
 from ._ops import library_op
-from ._runtime import (check_kernel_form, error_word, few_rows_ok, host_linear, linear_rows, require, require_cuda, stream_ptr,
+from ._runtime import (check_kernel_form, error_word, few_rows_ok, host_linear, linear_rows, one_row_streams, require, require_cuda, stream_ptr,
                        tc_gemm_ok)
 from .dequant_gemv import dequant_gemv_rows
 
@@ -68,7 +68,7 @@ def quant_linear(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: i
     M, K = x.shape
     N = w_q.shape[1]
     half = x.dtype in (torch.float16, torch.bfloat16)
-    few = few_rows_ok(w_q, scales, zeros, K, N, group_size)
+    few = few_rows_ok(w_q, scales, zeros, K, N, group_size) and not (x.dtype == torch.float16 and one_row_streams(M, N, K))
     tc = bool(_capi.lib.gemq_linear_takes_gemm(M, N, K, nbits)) if few else tc_gemm_ok(M, N, K, group_size)
     if half and (tc or few):
         check_kernel_form(w_q, scales, zeros, K, N, nbits, group_size)

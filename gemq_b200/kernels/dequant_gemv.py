@@ -8,7 +8,7 @@ from torch import Tensor
 
 from .. import _capi
 from ._ops import library_op
-from ._runtime import (check_kernel_form, few_rows_ok, gemv_workspace, host_linear, linear_rows, require, require_cuda,
+from ._runtime import (check_kernel_form, few_rows_ok, gemv_workspace, host_linear, linear_rows, one_row_streams, require, require_cuda,
                        stream_ptr)
 
 
@@ -25,7 +25,7 @@ def dequant_gemv_rows(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbi
     N = w_q.shape[1]
     check_kernel_form(w_q, scales, zeros, K, N, nbits, group_size)
     x = x if x.stride(1) == 1 else x.contiguous()
-    if few_rows_ok(w_q, scales, zeros, K, N, group_size):
+    if few_rows_ok(w_q, scales, zeros, K, N, group_size) and not one_row_streams(M, N, K):
         return linear_rows(x, w_q, scales, zeros, nbits, group_size)
     out = torch.empty((M, N), dtype=torch.float16, device=dev)
     ws = gemv_workspace(dev, N, K, M)

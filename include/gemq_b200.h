@@ -208,6 +208,9 @@ int gemq_linear_gemm(const void* x, const int64_t* expert, const int32_t* wq, co
                      const int32_t* zs_strides, int fixed_bits, const void* bias, void* y, int M, int N,
                      int K, int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream);
 
+/* 1: gemq_dequant_gemv takes one row of such a matrix to the split-K streaming kernel, not to gemq_linear_rows. */
+int gemq_one_row_streams(int N, int K);
+
 /* Which of the two a dense layer takes: 1 = gemq_linear_gemm, 0 = gemq_linear_rows (a rule on the sizes). */
 int gemq_linear_takes_gemm(int rows, int N, int K, int nbits);
 
