@@ -568,9 +568,11 @@ __device__ void route_cta(Smem& S, const FusedParams& P) {
   }
 }
 
-// ---- plan (warp 0) ----------------------------------------------------------------------------
+// ---- plan -------------------------------------------------------------------------------------
+// Warp 0 makes the parts of phase 0, warp 1 those of phase 1, a lane a part.  By one warp and one lane per slot it
+// took 9 us of a Mixtral token's 52 and of a DeepSeek-V2-Lite token's 27.
 // a / b for a < 2^24, b > 0: one approximate reciprocal and a correction instead of the integer
-// division sequence (the plan is a single warp's chain of dependent instructions).
+// division sequence (the plan is a chain of dependent instructions).
 __device__ __forceinline__ unsigned small_div(unsigned a, unsigned b) {
   unsigned q = __float2uint_rz(__fdividef(__uint2float_rz(a), __uint2float_rz(b)));
   if (q * b > a) --q;
@@ -580,9 +582,9 @@ __device__ __forceinline__ unsigned small_div(unsigned a, unsigned b) {
 __device__ __forceinline__ int quanta_of(int groups, int bits) { return bits == 3 ? (groups + 4) / 5 : (groups + 3) >> 2; }
 
 __device__ void make_plan(Smem& S, const FusedParams& P) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, ph = threadIdx.x >> 5;
   const int Sn = P.S;
-  // slots
+  // slots (by both warps alike)
   int Fs = 0, b1 = 1, b2 = 1;
   if (lane < Sn) {
     SlotInfo I;
@@ -629,13 +631,13 @@ __device__ void make_plan(Smem& S, const FusedParams& P) {
   int nq1 = lane < Sn ? quanta_of(Fs / kGroup, b2) : 0;
   int in_nch = nch0, in_fs = fs, in_nq1 = nq1;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
+  for (int o = 1; o < 16; o <<= 1) {
     const int a = __shfl_up_sync(0xffffffffu, in_nch, o), b = __shfl_up_sync(0xffffffffu, in_fs, o),
               c = __shfl_up_sync(0xffffffffu, in_nq1, o);
     if (lane >= o) { in_nch += a; in_fs += b; in_nq1 += c; }
   }
-  const int pairs_total = __shfl_sync(0xffffffffu, in_nch, 31);
-  const int expected1 = __shfl_sync(0xffffffffu, in_nq1, 31);
+  const int pairs_total = __shfl_sync(0xffffffffu, in_nch, kMaxS - 1);
+  const int expected1 = __shfl_sync(0xffffffffu, in_nq1, kMaxS - 1);
   const int nch1 = cdiv(P.D, 128);
   const int base1 = 3 * pairs_total;
   if (lane < Sn) {
@@ -647,32 +649,33 @@ __device__ void make_plan(Smem& S, const FusedParams& P) {
     I.maskb[0] = pairs_total + 2 * (in_nch - nch0);
     I.maskb[1] = base1 + nch1 + lane * nch1;
   }
-  if (lane == 0) {
+  if (lane == 0) {  // both warps: the same values
     S.pairs_total = pairs_total;
     S.expected1 = expected1;
-    S.overflow = 0;
   }
   __syncwarp();
-  // ranges and parts of the two phases
-  int pbase = 0;
+  // range of the phase: units [ulo, uhi) of each slot (lane), and the parts they make
+  unsigned ulo = 0, uhi = 0, cm_lo = 0;
+  int nq = 1, first = 0, np_total = 0, pbase = 0;
 #pragma unroll 1
-  for (int ph = 0; ph < 2; ++ph) {
+  for (int q = 0; q <= ph; ++q) {
+    pbase += np_total;
     unsigned n_units = 0, cost = 1;
-    int nq = 1;
+    nq = 1;
     if (lane < Sn) {
       const SlotInfo& I = S.slot[lane];
-      nq = I.nq[ph];
-      n_units = static_cast<unsigned>(I.nch[ph]) * (ph ? 1u : 2u) * nq;
-      cost = quantum_cost(I.bits[ph]);
+      nq = I.nq[q];
+      n_units = static_cast<unsigned>(I.nch[q]) * (q ? 1u : 2u) * nq;
+      cost = quantum_cost(I.bits[q]);
     }
     const unsigned wgt = n_units * cost;
     unsigned incl = wgt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < 16; o <<= 1) {  // at most kMaxS lanes
       const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
-    const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+    const unsigned total = __shfl_sync(0xffffffffu, incl, kMaxS - 1);
     const unsigned prefix = incl - wgt;
     // cut points: any monotone function of the CTA index evaluated the same way by both neighbours
     const float per_cta = static_cast<float>(total) / static_cast<float>(gridDim.x);
@@ -680,72 +683,82 @@ __device__ void make_plan(Smem& S, const FusedParams& P) {
     const unsigned hi = blockIdx.x + 1 == gridDim.x ? total
                                                     : min(total, static_cast<unsigned>(per_cta * static_cast<float>(blockIdx.x + 1)));
     const bool small = total < (1u << 23);  // always, for the layers this kernel takes; the exact form stays as the guard
-    unsigned ulo = lo <= prefix ? 0u : (small ? small_div(lo - prefix + cost - 1, cost) : (lo - prefix + cost - 1) / cost);
-    unsigned uhi = hi <= prefix ? 0u : (small ? small_div(hi - prefix + cost - 1, cost) : (hi - prefix + cost - 1) / cost);
+    ulo = lo <= prefix ? 0u : (small ? small_div(lo - prefix + cost - 1, cost) : (lo - prefix + cost - 1) / cost);
+    uhi = hi <= prefix ? 0u : (small ? small_div(hi - prefix + cost - 1, cost) : (hi - prefix + cost - 1) / cost);
     ulo = min(ulo, n_units);
     uhi = min(uhi, n_units);
-    const unsigned cm_lo = small ? small_div(ulo, nq) : ulo / nq;
+    cm_lo = small ? small_div(ulo, nq) : ulo / nq;
     const int np = uhi > ulo ? static_cast<int>((small ? small_div(uhi - 1, nq) : (uhi - 1) / nq) - cm_lo + 1) : 0;
     int inp = np;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < 16; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, inp, o);
       if (lane >= o) inp += t;
     }
-    const int np_total = __shfl_sync(0xffffffffu, inp, 31);
-    int pi = pbase + inp - np;
-    if (pbase + np_total > kMaxParts) {
-      if (lane == 0) S.overflow = 1;
-    } else if (np > 0) {
-      const SlotInfo& I = S.slot[lane];
-      const int B = I.bits[ph];
-      const int K = ph ? I.F : P.D, N = ph ? P.D : I.F;
-      const int ngroups = K / kGroup;
-      const int first_cm = static_cast<int>(cm_lo);
+    np_total = __shfl_sync(0xffffffffu, inp, kMaxS - 1);
+    first = inp - np;
+  }
+  const bool fits = pbase + np_total <= kMaxParts;
+  if (ph == 1 && lane == 0) {
+    S.overflow = fits ? 0 : 1;
+    S.n_parts = fits ? pbase + np_total : 0;
+  }
+  if (!fits) return;
+  // a lane per part; the run lanes of a phase's parts go round in one sequence
+  int runs = 0;
 #pragma unroll 1
-      for (int k = 0; k < np; ++k, ++pi) {
-        const int cm = first_cm + k;
-        const int c = ph ? cm : (cm >> 1), m = ph ? 0 : (cm & 1), mi = ph ? 2 : m;
-        const int qa = max(static_cast<int>(ulo), cm * nq) - cm * nq;
-        const int qb = min(static_cast<int>(uhi), (cm + 1) * nq) - cm * nq;
-        PartDesc d;
-        const int n0 = c * 128;
-        d.w = I.wq[mi] + n0;
-        d.sc = I.sc[mi] + n0;
-        d.zr = I.zr[mi] + n0;
-        d.N = N; d.B = B; d.ngroups = ngroups;
-        d.kw = B == 3 ? b3_rows(K) : (K * B) >> 5;
-        if (B == 3) { d.run_lo = qa; d.run_hi = min(qb, nq); }
-        else { d.run_lo = 2 * qa; d.run_hi = min(2 * qb, cdiv(ngroups, 2)); }
-        d.ncols = min(128, N - n0);
-        d.tab = ph ? 8 + lane : B;
-        d.phase = ph; d.s = lane; d.c = c;
-        d.qa = qa; d.qb = qb;
-        if (ph) {
-          d.ctr = base1 + c;
-          d.expected = expected1;
-          d.mask = I.maskb[1] + c;
-          d.colp = I.colb[1] + n0;
-        } else {
-          d.ctr = I.ctrb + c;  // index of a 64-bit word
-          d.expected = 2 * nq;
-          d.mask = m;          // phase 0: which half of the slot set this part's bit goes to
-          d.colp = I.colb[0] + m * I.F + n0;
-        }
-        S.parts[pi] = d;
+  for (int k0 = 0; k0 < np_total; k0 += 32) {
+    const int k = k0 + lane;
+    int s = 0;
+#pragma unroll 1
+    for (int q = 1; q < Sn; ++q)
+      if (k >= __shfl_sync(0xffffffffu, first, q)) s = q;  // the last such slot: the ones before it with as many have none
+    const int cm = static_cast<int>(__shfl_sync(0xffffffffu, cm_lo, s)) + k - __shfl_sync(0xffffffffu, first, s);
+    const int lo = static_cast<int>(__shfl_sync(0xffffffffu, ulo, s)), hi = static_cast<int>(__shfl_sync(0xffffffffu, uhi, s));
+    const int sq = __shfl_sync(0xffffffffu, nq, s);
+    const SlotInfo& I = S.slot[s];
+    const int B = I.bits[ph];
+    const int K = ph ? I.F : P.D, N = ph ? P.D : I.F;
+    const int ngroups = K / kGroup;
+    const int c = ph ? cm : (cm >> 1), m = ph ? 0 : (cm & 1), mi = ph ? 2 : m;
+    const int qa = max(lo, cm * sq) - cm * sq;
+    const int qb = min(hi, (cm + 1) * sq) - cm * sq;
+    const int run_lo = B == 3 ? qa : 2 * qa, run_hi = B == 3 ? min(qb, sq) : min(2 * qb, cdiv(ngroups, 2));
+    const int n = k < np_total ? run_hi - run_lo : 0;
+    int before = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += t;
+    }
+    const int all = __shfl_sync(0xffffffffu, before, 31);
+    if (k < np_total) {
+      PartDesc& d = S.parts[pbase + k];
+      const int n0 = c * 128;
+      d.w = I.wq[mi] + n0;
+      d.sc = I.sc[mi] + n0;
+      d.zr = I.zr[mi] + n0;
+      d.N = N; d.B = B; d.ngroups = ngroups;
+      d.kw = B == 3 ? b3_rows(K) : (K * B) >> 5;
+      d.run_lo = run_lo; d.run_hi = run_hi;
+      d.roff = (runs + before - n) % kLanes;
+      d.ncols = min(128, N - n0);
+      d.tab = ph ? 8 + s : B;
+      d.phase = ph; d.s = s; d.c = c;
+      d.qa = qa; d.qb = qb;
+      if (ph) {
+        d.ctr = base1 + c;
+        d.expected = expected1;
+        d.mask = I.maskb[1] + c;
+        d.colp = I.colb[1] + n0;
+      } else {
+        d.ctr = I.ctrb + c;  // index of a 64-bit word
+        d.expected = 2 * sq;
+        d.mask = m;          // phase 0: which half of the slot set this part's bit goes to
+        d.colp = I.colb[0] + m * I.F + n0;
       }
     }
-    pbase += np_total;
-  }
-  __syncwarp();
-  if (lane == 0) {
-    const int n = S.overflow ? 0 : pbase;
-    int runs = 0;
-    for (int p = 0; p < n; ++p) {
-      S.parts[p].roff = runs % kLanes;
-      runs += S.parts[p].run_hi - S.parts[p].run_lo;
-    }
-    S.n_parts = n;
+    runs += all;
   }
 }
 
@@ -1552,7 +1565,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
     S.sel_w[threadIdx.x] = P.w[threadIdx.x];
   }
   __syncthreads();
-  if (warp == 0) make_plan(S, P);
+  if (warp < 2) make_plan(S, P);
   __syncthreads();
   if (S.overflow && threadIdx.x == 0) atomicExch(err, 14);
   if (warp < kCons) consumer_role(S, P, err);
