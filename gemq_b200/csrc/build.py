@@ -17,8 +17,8 @@ ROOT = os.path.dirname(PKG)
 LIB = os.path.join(PKG, "libgemq_b200.so")
 HOST_LIB = os.path.join(PKG, "_host.so")
 SOURCES = ["pack.cu", "tma.cu", "gemv.cu", "gemv_stream.cu", "route.cu", "layer.cu", "decode_fused.cu", "gemm_ts.cu", "prefill.cu", "expert_parallel.cu", "no_alloc.cu",
-           "few_linear.cu", "few_moe.cu", "decoder.cu"]
-HEADERS = ["common.cuh", "gemv.cuh", "few_rows.cuh", "gemm_ts.cuh", "ptx.cuh", os.path.join(ROOT, "include", "gemq_b200.h")]
+           "few_linear.cu", "few_moe.cu", "few_one.cu", "decoder.cu"]
+HEADERS = ["common.cuh", "gemv.cuh", "few_rows.cuh", "few_table.cuh", "gemm_ts.cuh", "ptx.cuh", os.path.join(ROOT, "include", "gemq_b200.h")]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -67,6 +67,11 @@ int launch_decode_fused(const gemq_moe_layer_t* L, const __half* x, __half* out,
                         int route_in_kernel, int route_mode, float* partial, int* counters, float* h,
                         cudaStream_t stream);
 
+// few_one.cu
+bool moe_one_ok(const gemq_moe_layer_t* L);
+int moe_one(const gemq_moe_layer_t* L, const __half* x, __half* out, const int64_t* idx, const __half* w, int* counters, float* h,
+            cudaStream_t st);
+
 // GEMQ_B200_DECODE=stream selects the three-launch path (router, gate/up GEMV, down GEMV) for
 // layers the single-launch kernel would take; read once.
 static bool fused_enabled() {
@@ -108,7 +113,18 @@ extern "C" int gemq_moe_decode(const gemq_moe_layer_t* L, const void* x, void* o
   if (!carve(L, scratch, scratch_bytes, &S)) return GEMQ_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-  // Single-launch path: router, both projections and the combine in one persistent kernel per token.
+  if (fused_enabled() && aligned16(x) && aligned16(out) && aligned16(L->gate) && moe_one_ok(L)) {
+    if (do_route)
+      if (const int rc = gemq_moe_route(x, L->gate, tokens, D, L->n_experts, A, route_mode, L->renorm, 0, idx, w, nullptr, stream)) return rc;
+    for (int t = 0; t < tokens; ++t)
+      if (const int rc = moe_one(L, static_cast<const __half*>(x) + static_cast<size_t>(t) * D, static_cast<__half*>(out) + static_cast<size_t>(t) * D,
+                                 idx + static_cast<size_t>(t) * A, static_cast<const __half*>(w) + static_cast<size_t>(t) * A,
+                                 static_cast<int*>(S.gemv_ws), S.h, st))
+        return rc;
+    return GEMQ_OK;
+  }
+
+  // Large experts, single-launch path: router, both projections and the combine in one persistent kernel per token.
   {
     int* counters = static_cast<int*>(S.gemv_ws);
     float* partial = reinterpret_cast<float*>(static_cast<char*>(S.gemv_ws) + kMaxCounters * sizeof(int));
