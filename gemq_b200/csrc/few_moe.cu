@@ -264,29 +264,56 @@ template <typename T>
 __global__ void __launch_bounds__(kPlanThreads) few_plan_kernel(Plan pl, const long long* __restrict__ idx, const T* __restrict__ w,
                                                                 const int* __restrict__ nbits, int R, int A, int E, int tokens,
                                                                 int tile_rows, int shared, int* err) {
-  __shared__ int count[256], start[256], cursor[256], key[256];
+  __shared__ int count[256], start[256], n_tile[256], key[256];
   const int tid = threadIdx.x;
-  for (int e = tid; e < E; e += kPlanThreads) { count[e] = 0; cursor[e] = 0; key[e] = nbits[e]; }
+  for (int e = tid; e < E; e += kPlanThreads) { count[e] = 0; key[e] = nbits[e]; }
   pdl_launch();
   pdl_wait();
   if (tid == 0) *err = 0;
   __syncthreads();
-  for (int i = tid; i < R; i += kPlanThreads) {
+  // A thread's first kHeld pairs stay in registers, loads in flight together; longer lists go through pl.inv.
+  constexpr int kHeld = 2;
+  int ex[kHeld], at[kHeld];
+  T wt[kHeld];
+  long long id[kHeld];
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const int i = tid + u * kPlanThreads;
+    id[u] = i < R ? idx[i] : 0;
+    if (i < R) wt[u] = w[i];
+  }
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    ex[u] = -1;
+    if (tid + u * kPlanThreads < R) {
+      if (id[u] < 0 || id[u] >= E) atomicExch(err, kErrBadExpertId);
+      else {
+        ex[u] = static_cast<int>(id[u]);
+        at[u] = atomicAdd(&count[ex[u]], 1);
+      }
+    }
+  }
+  for (int i = tid + kHeld * kPlanThreads; i < R; i += kPlanThreads) {
     const long long e = idx[i];
     if (e < 0 || e >= E) atomicExch(err, kErrBadExpertId);
-    else atomicAdd(&count[static_cast<int>(e)], 1);
+    pl.inv[i] = e < 0 || e >= E ? -1 : atomicAdd(&count[static_cast<int>(e)], 1);
   }
   __syncthreads();
   // longest first: two blocks of eight rows take twice the MMAs of one, more bits more copying
-  for (int e = tid; e < E; e += kPlanThreads) key[e] += count[e] > 8 ? 8 : 0;
+  for (int e = tid; e < E; e += kPlanThreads) {
+    key[e] += count[e] > 8 ? 8 : 0;
+    n_tile[e] = cdiv(count[e], tile_rows);
+  }
   __syncthreads();
   const int sh_tiles = shared ? cdiv(tokens, tile_rows) : 0;
   for (int e = tid; e < E; e += kPlanThreads) {
     int row = 0, tile = sh_tiles, total = sh_tiles;
+    const int mine = key[e];
+#pragma unroll 4
     for (int o = 0; o < E; ++o) {
-      const int n = count[o], nt = cdiv(n, tile_rows);
+      const int n = count[o], nt = n_tile[o], k = key[o];
       total += nt;
-      if (key[o] > key[e] || (key[o] == key[e] && o < e)) { row += n; tile += nt; }
+      if (k > mine || (k == mine && o < e)) { row += n; tile += nt; }
     }
     start[e] = row;
     for (int r = 0; r < count[e]; r += tile_rows) pl.tiles[tile++] = make_int4(e, row + r, min(tile_rows, count[e] - r), 0);
@@ -297,14 +324,23 @@ __global__ void __launch_bounds__(kPlanThreads) few_plan_kernel(Plan pl, const l
   if (shared)
     for (int i = tid; i < tokens; i += kPlanThreads) pl.src[R + i] = i;
   __syncthreads();
-  for (int i = tid; i < R; i += kPlanThreads) {
-    const long long e = idx[i];
-    int pos = -1;
-    if (e >= 0 && e < E) {
-      pos = start[e] + atomicAdd(&cursor[static_cast<int>(e)], 1);
+#pragma unroll
+  for (int u = 0; u < kHeld; ++u) {
+    const int i = tid + u * kPlanThreads;
+    if (i >= R) continue;
+    const int pos = ex[u] < 0 ? -1 : start[ex[u]] + at[u];
+    if (pos >= 0) {
       pl.src[pos] = i / A;
-      pl.row_w[pos] = __float2half_rn(to_f<T>(w[i]));
+      pl.row_w[pos] = __float2half_rn(to_f<T>(wt[u]));
     }
+    pl.inv[i] = pos;
+  }
+  for (int i = tid + kHeld * kPlanThreads; i < R; i += kPlanThreads) {
+    const int p = pl.inv[i];
+    if (p < 0) continue;
+    const int pos = start[static_cast<int>(idx[i])] + p;
+    pl.src[pos] = i / A;
+    pl.row_w[pos] = __float2half_rn(to_f<T>(w[i]));
     pl.inv[i] = pos;
   }
 }

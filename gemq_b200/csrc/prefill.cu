@@ -33,20 +33,21 @@ constexpr int kErrBadExpert = 21;
 struct Plan {
   int4* tiles;     // {expert (-1: shared), first row, rows, 0}: the shared expert's tiles first
   int* n_tiles;
-  int* src;        // sorted row -> token, -1: nobody's row
-  int* row_bits;   // sorted row -> bit width of the matrices that read it
-  int* inv;        // (token, slot) -> sorted row, -1: expert id out of range
-  __half* row_w;   // sorted row -> routing weight
+  int* start;      // expert -> its first sorted row
+  int* at;         // (token, slot) -> place among its expert's rows, -1: expert id out of range
+  int* inv;        // (token, slot) -> sorted row, -1: expert id out of range (from the gather on)
+  __half* row_w;   // sorted row -> routing weight (from the gather on)
 };
 
 constexpr int kPlanThreads = 1024;
 
-// One CTA.  Lanes with the same expert claim their rows together: one shared-memory atomic per warp and expert.
-template <typename T>
-__global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, const long long* __restrict__ idx, const T* __restrict__ w,
-                                                                    const int* __restrict__ nbits, int R, int A, int E, int tokens,
-                                                                    int shared_bits, int* err) {
-  __shared__ int count[256], start[256], first_tile[256], cost[256], order[256], taken;
+// One CTA; it reads the expert ids once, four trips of loads in flight, and leaves everything per row to the gather
+// (with that here, 12000 rows took 28 us).  Lanes with the same expert claim their rows together: one shared-memory
+// atomic per warp and expert.
+__global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, const long long* __restrict__ idx,
+                                                                    const int* __restrict__ nbits, int R, int E, int tokens,
+                                                                    bool shared, int* err) {
+  __shared__ int count[256], start[256], first_tile[256], cost[256], order[256];
   const int tid = threadIdx.x, lane = tid & 31;
   // Time of a tile by bit width: 3 bits 1.8, 4 bits 1.2 times the 1- and 2-bit ones (measured with 128 rows).
   for (int e = tid; e < E; e += kPlanThreads) {
@@ -64,24 +65,29 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
     for (int o = 0; o < E; ++o) r += cost[o] > cost[e] || (cost[o] == cost[e] && o < e) ? 1 : 0;
     order[r] = e;
   }
-  const int trips = (R + kPlanThreads - 1) / kPlanThreads;
-  for (int i = 0; i < trips; ++i) {
-    const int p = i * kPlanThreads + tid;
-    int e = -1;
-    if (p < R) {
-      const long long v = idx[p];
-      if (v >= 0 && v < E) e = static_cast<int>(v);
-      else atomicExch(err, kErrBadExpert);
+  constexpr int kAhead = 4;
+#pragma unroll 1
+  for (int p0 = tid; p0 < R + tid; p0 += kAhead * kPlanThreads) {
+    long long id[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) id[u] = p0 + u * kPlanThreads < R ? idx[p0 + u * kPlanThreads] : 0;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int p = p0 + u * kPlanThreads;
+      int e = -1;
+      if (p < R) {
+        if (id[u] >= 0 && id[u] < E) e = static_cast<int>(id[u]);
+        else atomicExch(err, kErrBadExpert);
+      }
+      const unsigned peers = __match_any_sync(0xffffffffu, e);
+      int at = 0;
+      if (e >= 0 && lane == __ffs(peers) - 1) at = atomicAdd(&count[e], __popc(peers));
+      at = __shfl_sync(0xffffffffu, at, __ffs(peers) - 1);
+      if (p < R) pl.at[p] = e >= 0 ? at + __popc(peers & ((1u << lane) - 1u)) : -1;
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, e);
-    int at = 0;
-    if (e >= 0 && lane == __ffs(peers) - 1) at = atomicAdd(&count[e], __popc(peers));
-    at = __shfl_sync(0xffffffffu, at, __ffs(peers) - 1);
-    // place among the expert's rows; the expert's first row is added below
-    if (p < R) pl.inv[p] = e >= 0 ? at + __popc(peers & ((1u << lane) - 1u)) : -1;
   }
   __syncthreads();
-  const int sh_tiles = shared_bits ? (tokens + kTile - 1) / kTile : 0;
+  const int sh_tiles = shared ? (tokens + kTile - 1) / kTile : 0;
   if (tid < 32) {  // scan of rows and tiles over the experts
     int row = 0, tile = sh_tiles;
     for (int e0 = 0; e0 < E; e0 += 32) {
@@ -95,15 +101,13 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
       }
       if (e >= 0) {
         start[e] = row + sr - n;
+        pl.start[e] = start[e];
         first_tile[e] = tile + stl - nt;
       }
       row += __shfl_sync(0xffffffffu, sr, 31);
       tile += __shfl_sync(0xffffffffu, stl, 31);
     }
-    if (lane == 0) {
-      *pl.n_tiles = tile;
-      taken = row;
-    }
+    if (lane == 0) *pl.n_tiles = tile;
   }
   __syncthreads();
   // an expert's tiles are of even size, in whole blocks of 16 rows
@@ -114,39 +118,23 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
       pl.tiles[first_tile[e] + t] = make_int4(e, start[e] + lo, hi - lo, 0);
     }
   }
-  for (int i = taken + tid; i < R; i += kPlanThreads) pl.src[i] = -1;  // ids out of range leave rows over
   for (int i = tid; i < sh_tiles; i += kPlanThreads)
     pl.tiles[i] = make_int4(-1, R + i * kTile, min(kTile, tokens - i * kTile), 0);
-  if (shared_bits)
-    for (int i = tid; i < tokens; i += kPlanThreads) {
-      pl.src[R + i] = i;
-      pl.row_bits[R + i] = shared_bits;
-    }
-  for (int p = tid; p < R; p += kPlanThreads) {
-    const int at = pl.inv[p];
-    if (at < 0) continue;
-    const int e = static_cast<int>(idx[p]);
-    const int row = start[e] + at;
-    pl.inv[p] = row;
-    pl.src[row] = p / A;
-    pl.row_bits[row] = nbits[e];
-    pl.row_w[row] = __float2half_rn(ts::as_float<T>(w[p]));
-  }
 }
 
-// Sorted row <- its token's activation in fp16 (bf16 activations are converted here), k in the order in which a
-// packed word's codes become MMA operands: code q next to code q + eps / 2; 3-bit words keep the natural order.
-// A thread handles 32 k.
+// The sorted rows of a token's experts, and its row of the shared expert, <- its activation in fp16 (bf16 activations
+// are converted here), k in the order in which a packed word's codes become MMA operands: code q next to code
+// q + eps / 2; 3-bit words keep the natural order.  A thread handles 32 k of a token for all of them.
 template <typename T>
-__global__ void __launch_bounds__(256) prefill_gather_kernel(Plan pl, const T* __restrict__ x, __half* __restrict__ xs, int rows, int D) {
+__global__ void __launch_bounds__(128) prefill_gather_kernel(Plan pl, const T* __restrict__ x, const long long* __restrict__ idx,
+                                                             const T* __restrict__ w, const int* __restrict__ nbits,
+                                                             __half* __restrict__ xs, int tokens, int A, int D, int shared_bits) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int per_row = D / 32;
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  const int row = i / per_row, c = i - row * per_row;
-  if (row >= rows) return;
-  const int tok = pl.src[row], bits = pl.row_bits[row];
-  if (tok < 0) return;
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  const int tok = i / per_row, c = i - tok * per_row;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tok >= tokens) return;
   const uint4* s = reinterpret_cast<const uint4*>(x + static_cast<size_t>(tok) * D + 32 * c);
   __half h[32];
 #pragma unroll
@@ -156,22 +144,45 @@ __global__ void __launch_bounds__(256) prefill_gather_kernel(Plan pl, const T* _
 #pragma unroll
     for (int k = 0; k < 8; ++k) h[8 * j + k] = __float2half_rn(ts::as_float<T>(e[k]));
   }
-  __half o[32];
-  auto order = [&](auto EPS) {
+  auto put = [&](int row, auto EPS) {
     constexpr int E = decltype(EPS)::value;
+    __half o[32];
 #pragma unroll
     for (int k = 0; k < 32; ++k) {
-      const int w = k / E, j = k % E;
-      o[w * E + 2 * (j % (E / 2)) + j / (E / 2)] = h[k];
+      const int q = k / E, j = k % E;
+      o[q * E + 2 * (j % (E / 2)) + j / (E / 2)] = h[k];
     }
-  };
-  if (bits == 1) order(std::integral_constant<int, 32>{});
-  else if (bits == 2) order(std::integral_constant<int, 16>{});
-  else if (bits == 4) order(std::integral_constant<int, 8>{});
-  else order(std::integral_constant<int, 2>{});
-  uint4* d = reinterpret_cast<uint4*>(xs + static_cast<size_t>(row) * D + 32 * c);
+    uint4* d = reinterpret_cast<uint4*>(xs + static_cast<size_t>(row) * D + 32 * c);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) d[j] = reinterpret_cast<const uint4*>(o)[j];
+    for (int j = 0; j < 4; ++j) d[j] = reinterpret_cast<const uint4*>(o)[j];
+  };
+  const int R = tokens * A;
+  int rows[kMaxSlots], bits[kMaxSlots];
+#pragma unroll
+  for (int a = 0; a < kMaxSlots; ++a) {  // all of a token's loads in flight
+    rows[a] = -1;
+    if (a < A) {
+      const int at = pl.at[tok * A + a];
+      const int e = at < 0 ? 0 : static_cast<int>(idx[tok * A + a]);
+      if (at >= 0) rows[a] = pl.start[e] + at;
+      bits[a] = nbits[e];
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < kMaxSlots; ++a) {
+    if (a >= A) break;
+    if (c == 0) pl.inv[tok * A + a] = rows[a];
+    if (rows[a] < 0) continue;
+    if (c == 0) pl.row_w[rows[a]] = __float2half_rn(ts::as_float<T>(w[tok * A + a]));
+    if (bits[a] == 1) put(rows[a], std::integral_constant<int, 32>{});
+    else if (bits[a] == 2) put(rows[a], std::integral_constant<int, 16>{});
+    else if (bits[a] == 4) put(rows[a], std::integral_constant<int, 8>{});
+    else put(rows[a], std::integral_constant<int, 2>{});
+  }
+  if (shared_bits == 1) put(R + tok, std::integral_constant<int, 32>{});
+  else if (shared_bits == 2) put(R + tok, std::integral_constant<int, 16>{});
+  else if (shared_bits == 4) put(R + tok, std::integral_constant<int, 8>{});
+  else if (shared_bits) put(R + tok, std::integral_constant<int, 2>{});
 }
 
 // out[t] = contributions of the token's experts added in increasing expert id, each addition
@@ -234,7 +245,7 @@ struct Scratch {
   __half* hs;   // [T, SF]
   __half* ys;   // [R + T, D]
   char* few;    // scratch of the few-row path (shares the bytes behind the error word)
-  int rows, max_tiles;
+  int max_tiles;
 };
 
 size_t layout(const gemq_moe_layer_t* L, int tokens, Scratch* S, char* base) {
@@ -246,8 +257,8 @@ size_t layout(const gemq_moe_layer_t* L, int tokens, Scratch* S, char* base) {
   char* er = take(2 * sizeof(int));
   const size_t few_at = off;
   char* tl = take(sizeof(int4) * tiles);
-  char* src = take(sizeof(int) * rows);
-  char* rb = take(sizeof(int) * rows);
+  char* starts = take(sizeof(int) * L->n_experts);
+  char* at = take(sizeof(int) * R);
   char* inv = take(sizeof(int) * R);
   char* rw = take(sizeof(__half) * R);
   char* xs = take(2 * rows * L->hidden);
@@ -258,8 +269,8 @@ size_t layout(const gemq_moe_layer_t* L, int tokens, Scratch* S, char* base) {
     S->err = reinterpret_cast<int*>(er);
     S->plan.n_tiles = S->err + 1;
     S->plan.tiles = reinterpret_cast<int4*>(tl);
-    S->plan.src = reinterpret_cast<int*>(src);
-    S->plan.row_bits = reinterpret_cast<int*>(rb);
+    S->plan.start = reinterpret_cast<int*>(starts);
+    S->plan.at = reinterpret_cast<int*>(at);
     S->plan.inv = reinterpret_cast<int*>(inv);
     S->plan.row_w = reinterpret_cast<__half*>(rw);
     S->xs = reinterpret_cast<__half*>(xs);
@@ -267,7 +278,6 @@ size_t layout(const gemq_moe_layer_t* L, int tokens, Scratch* S, char* base) {
     S->hs = reinterpret_cast<__half*>(hs);
     S->ys = reinterpret_cast<__half*>(ys);
     S->few = base ? base + few_at : nullptr;
-    S->rows = static_cast<int>(rows);
     S->max_tiles = static_cast<int>(tiles);
   }
   if (few::moe_few_rows_ok(L, tokens)) {
@@ -310,11 +320,11 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
         cudaStream_t st) {
   const int D = L->hidden, F = L->ffn, A = L->top_k, E = L->n_experts, SF = L->shared_ffn, R = tokens * A;
   const int sh_tiles = SF ? cdiv(tokens, kTile) : 0;
-  bool ok = launch_pdl(prefill_plan_kernel<T>, dim3(1), kPlanThreads, st, S.plan, idx, static_cast<const T*>(w),
-                       static_cast<const int*>(L->w1.nbits), R, A, E, tokens, SF ? L->s1.nbits : 0, S.err);
-  const size_t items = static_cast<size_t>(S.rows) * (D / 32);
-  ok = ok && launch_pdl(prefill_gather_kernel<T>, dim3(static_cast<unsigned>((items + 255) / 256)), 256, st, S.plan,
-                        static_cast<const T*>(x), S.xs, S.rows, D);
+  const int* nbits = static_cast<const int*>(L->w1.nbits);
+  bool ok = launch_pdl(prefill_plan_kernel, dim3(1), kPlanThreads, st, S.plan, idx, nbits, R, E, tokens, SF > 0, S.err);
+  const size_t items = static_cast<size_t>(tokens) * (D / 32);
+  ok = ok && launch_pdl(prefill_gather_kernel<T>, dim3(static_cast<unsigned>((items + 127) / 128)), 128, st, S.plan,
+                        static_cast<const T*>(x), idx, static_cast<const T*>(w), nbits, S.xs, tokens, A, D, SF ? L->s1.nbits : 0);
   if (!ok) return GEMQ_ERR_LAUNCH;
 
   ts::Params U = {};
