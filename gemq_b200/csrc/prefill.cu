@@ -152,9 +152,13 @@ __global__ void __launch_bounds__(128) prefill_gather_kernel(Plan pl, const T* _
       const int q = k / E, j = k % E;
       o[q * E + 2 * (j % (E / 2)) + j / (E / 2)] = h[k];
     }
-    uint4* d = reinterpret_cast<uint4*>(xs + static_cast<size_t>(row) * D + 32 * c);
+    __half* d = xs + static_cast<size_t>(row) * D + 32 * c;
+    const uint32_t* v = reinterpret_cast<const uint32_t*>(o);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) d[j] = reinterpret_cast<const uint4*>(o)[j];
+    for (int j = 0; j < 2; ++j)  // whole 32-byte sectors
+      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(d + 16 * j), "r"(v[8 * j]), "r"(v[8 * j + 1]),
+                   "r"(v[8 * j + 2]), "r"(v[8 * j + 3]), "r"(v[8 * j + 4]), "r"(v[8 * j + 5]), "r"(v[8 * j + 6]), "r"(v[8 * j + 7])
+                   : "memory");
   };
   const int R = tokens * A;
   int rows[kMaxSlots], bits[kMaxSlots];
