@@ -61,7 +61,8 @@ _SIGNATURES = {
     "gemq_moe_route": (_I, [_P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P]),
     "gemq_moe_decode_scratch_bytes": (_Z, [C.POINTER(MoeLayer)]),
     "gemq_dequant_gemm_tc": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _P, _P]),
-    "gemq_linear_gemm": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P]),
+    "gemq_linear_gemm": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P, _Z, _P]),
+    "gemq_linear_gemm_scratch_bytes": (_Z, [_I, _I, _I, _I]),
     "gemq_one_row_streams": (_I, [_I, _I]),
     "gemq_linear_takes_gemm": (_I, [_I, _I, _I, _I]),
     "gemq_linear_rows": (_I, [_P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P]),

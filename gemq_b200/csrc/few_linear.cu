@@ -7,6 +7,7 @@
 // shared memory, and are added in a fixed order.  A table built by a launch of its own cost 3 us and a
 // dependent launch per call, as much as the product itself.
 #include "few_table.cuh"
+#include "gemm_ts.cuh"
 
 namespace gemq {
 namespace few {
@@ -258,21 +259,20 @@ static bool linear_split(int rows, int N, int K, int nbits, int* tile_rows, int*
 }
 
 // Estimates in us of what the two kernels were measured to take (1 to 64 rows of 14 shapes, 512 to 14336 wide).  The
-// GEMM: a fixed 3 and its de-quantisation, which grows with K and the bits and not with the rows; the few-row kernel:
-// rounds of the chip, each with a start and a table of the k of a warp.  Where the lines cross the two differ by less
-// than the estimates are off; the 3-bit table costs 2.5 times the others'.
+// GEMM: linear_plan; the few-row kernel: rounds of the chip, each with a start and a table of the k of a warp.  Where the lines cross the two differ by less
+// than the estimates are off; the 3-bit table costs up to 2.5 times the others'.
 extern "C" int gemq_linear_takes_gemm(int rows, int N, int K, int nbits) {
   int tr, splits, tab;
   size_t smem;
   const int sms = sm_count();
   if (rows <= 0 || N <= 0 || K <= 0 || nbits < 1 || nbits > 4 || sms <= 0) return rows >= 32;
   if (!linear_split(rows, N, K, nbits, &tr, &splits, &tab, &smem)) return 1;
-  static const float per_k[4] = {0.40f, 0.40f, 0.78f, 0.50f};
-  const float gemm = 3.f + cdiv(cdiv(N, 256) * cdiv(rows, 256), sms / 2) * (K / 128) * per_k[nbits - 1];
+  const float gemm = ts::linear_plan(rows, N, K, nbits, true).us;
   const int per_sm = tr > 8 || 3 * (smem + 2048) > kMaxDyn ? (2 * (smem + 2048) > kMaxDyn ? 1 : 2) : 3;
   const int rounds = cdiv(cdiv(N, 64) * splits * cdiv(rows, tr), per_sm * sms);
   const float warp_k = static_cast<float>(K) / static_cast<float>(kCons * splits);
-  const float few = rounds * (tr > 8 ? 3.5f + 0.033f * warp_k : 3.f + warp_k * (0.006f + 0.0008f * tr)) * (nbits == 3 ? 2.5f : 1.f);
+  const float few = rounds * (rounds > 2 ? 1.5f : 1.f) * (tr > 8 ? 3.f + 0.024f * warp_k : 3.f + warp_k * (0.003f + 0.0011f * tr)) *
+                    (nbits == 3 ? 1.2f + 0.17f * (tr > 8 ? 8 : tr) : 1.f);
   return gemm < few;
 }
 

@@ -44,16 +44,86 @@ bool activation_maps(CUtensorMap (&maps)[4], const void* x, int K, long long row
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream) { return launch<kOutUp, false>(P, tiles_bound, stream); }
 int launch_down(const Params& P, int tiles_bound, cudaStream_t stream) { return launch<kOutDown, false>(P, tiles_bound, stream); }
 
+// A tile's time is its k-blocks': the de-quantisation of 256 columns (by bit width, whatever the tokens), or the MMAs of
+// many tokens.  Few tokens and few columns leave most of the 74 pairs without a tile, so the tokens go to smaller tiles
+// (more of them, each with its own de-quantisation) or k is split (fp32 parts through memory and a second launch),
+// whichever is estimated to end first.  4096 x 4096, 2 bits, 32 rows: 16.0 us unsplit, on 16 pairs; 14336 x 1024: 48, on 4.
+LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split) {
+  static const float block_us[4] = {0.20f, 0.20f, 0.39f, 0.25f};
+  const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, KB = K / kBK, ct = cdiv(N, 2 * kCols);
+  const float dequant = block_us[bits >= 1 && bits <= 4 ? bits - 1 : 1];
+  LinearPlan best = {kTokens, 1, (KB + 1) & ~1, 1e30f};
+  for (int tr = kTokens; tr >= 32; tr /= 2) {
+    const long long tiles = static_cast<long long>(ct) * cdiv(M, tr);
+    const float mma = 0.37f * static_cast<float>(M < tr ? M : tr) / kTokens;
+    for (int sp = 1; sp == 1 || (may_split && sp <= 16 && tiles * sp <= pairs && KB / sp >= 8); ++sp) {
+      const int kb = (cdiv(KB, sp) + 1) & ~1;
+      if (sp > 1 && cdiv(KB, kb) != sp) continue;
+      const float rounds = static_cast<float>((tiles * sp + pairs - 1) / pairs);
+      float us = 3.f + rounds * static_cast<float>(kb) * (mma > dequant ? mma : dequant);
+      if (sp > 1) us += 2.5f + 8e-6f / 4.f * static_cast<float>(sp) * static_cast<float>(M) * static_cast<float>(N);
+      if (us < 0.97f * best.us) best = {tr, sp, kb, us};
+    }
+  }
+  return best;
+}
+
+// The parts of k, in order, rounded and biased like the one launch does.  A thread takes four columns.
+template <typename T>
+__global__ void __launch_bounds__(256) linear_sum_kernel(const float* __restrict__ partial, const T* __restrict__ bias, T* __restrict__ y,
+                                                         int splits, long long total, int N) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 4;
+  if (i >= total) return;
+  float4 v = *reinterpret_cast<const float4*>(partial + i);
+#pragma unroll 4
+  for (int s = 1; s < splits; ++s) {
+    const float4 u = *reinterpret_cast<const float4*>(partial + s * total + i);
+    v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+  }
+  const float f[4] = {v.x, v.y, v.z, v.w};
+  T o[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    o[k] = as_act<T>(f[k]);
+    if (bias) o[k] = as_act<T>(as_float<T>(o[k]) + as_float<T>(bias[i % N + k]));
+  }
+  *reinterpret_cast<uint2*>(y + i) = *reinterpret_cast<const uint2*>(o);
+}
+
+template <typename T>
+static int launch_sum(const Params& P, void* y, cudaStream_t st) {
+  const long long total = static_cast<long long>(P.rows) * P.fam[0].N;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((total / 4 + 255) / 256));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, linear_sum_kernel<T>, static_cast<const float*>(P.partial), static_cast<const T*>(P.bias),
+                            static_cast<T*>(y), P.splits, total, P.fam[0].N) == cudaSuccess ? GEMQ_OK : GEMQ_ERR_LAUNCH;
+}
+
 }  // namespace ts
 }  // namespace gemq
 
 using namespace gemq;
 using namespace gemq::ts;
 
+extern "C" size_t gemq_linear_gemm_scratch_bytes(int M, int N, int K, int nbits) {
+  if (M <= 0 || N <= 0 || K <= 0 || N % 32 || K % kBK) return 0;
+  const LinearPlan L = linear_plan(M, N, K, nbits, true);
+  return L.splits > 1 ? static_cast<size_t>(L.splits) * M * N * sizeof(float) : 0;
+}
+
 extern "C" int gemq_linear_gemm(const void* x, const int64_t* expert, const int32_t* wq, const void* scales, const void* zeros,
                                 const int32_t* nbits, const int32_t* wq_strides, const int32_t* zs_strides, int fixed_bits,
                                 const void* bias, void* y, int M, int N, int K, int group_size, int x_is_bf16, int32_t* err,
-                                gemq_stream_t stream) {
+                                void* scratch, size_t scratch_bytes, gemq_stream_t stream) {
   if (!x || !wq || !scales || !zeros || !y || !err || M <= 0 || N <= 0 || K <= 0 || group_size <= 0) return GEMQ_ERR_BAD_ARG;
   if (!nbits && (fixed_bits < 1 || fixed_bits > 4)) return GEMQ_ERR_BAD_ARG;
   if (N % 32 || K % kBK || group_size % kBK || K % group_size) return GEMQ_ERR_BAD_SHAPE;
@@ -72,15 +142,22 @@ extern "C" int gemq_linear_gemm(const void* x, const int64_t* expert, const int3
   P.rows = M;
   P.bias = bias;
   P.err = err;
-  // Fewer tokens per tile (which then costs its de-quantisation; that does not shrink with the tokens) as
-  // long as there are CTA pairs to take the tiles.
-  const int pairs = sm_count() / 2;
   F.col_tiles = cdiv(N, 2 * kCols);
-  P.tile_rows = kTokens;
-  while (P.tile_rows > 32 && F.col_tiles * cdiv(M, P.tile_rows / 2) <= pairs) P.tile_rows /= 2;
-  const int tiles = F.col_tiles * cdiv(M, P.tile_rows);
+  const size_t need = scratch && aligned16(scratch) && !nbits ? gemq_linear_gemm_scratch_bytes(M, N, K, fixed_bits) : 0;
+  const LinearPlan L = linear_plan(M, N, K, nbits ? 2 : fixed_bits, need > 0 && scratch_bytes >= need);
+  P.tile_rows = L.tile_rows;
+  P.splits = L.splits;
+  P.split_kb = L.split_kb;
+  P.partial = static_cast<float*>(scratch);
+  const int tiles = F.col_tiles * cdiv(M, P.tile_rows) * P.splits;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int rc = x_is_bf16 ? launch<kOutLinear, true>(P, tiles, st) : launch<kOutLinear, false>(P, tiles, st);
+  int rc;
+  if (P.splits > 1) {
+    rc = x_is_bf16 ? launch<kOutPartial, true>(P, tiles, st) : launch<kOutPartial, false>(P, tiles, st);
+    if (!rc) rc = x_is_bf16 ? launch_sum<__nv_bfloat16>(P, y, st) : launch_sum<__half>(P, y, st);
+  } else {
+    rc = x_is_bf16 ? launch<kOutLinear, true>(P, tiles, st) : launch<kOutLinear, false>(P, tiles, st);
+  }
   return rc ? rc : launch_status();
 }
 
@@ -89,5 +166,5 @@ extern "C" int gemq_dequant_gemm_tc(const void* x, const int64_t* expert, const 
                                     const int32_t* zs_strides, int fixed_bits, void* y, int M, int N, int K,
                                     int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream) {
   return gemq_linear_gemm(x, expert, wq, scales, zeros, nbits, wq_strides, zs_strides, fixed_bits, nullptr, y, M, N, K, group_size,
-                          x_is_bf16, err, stream);
+                          x_is_bf16, err, nullptr, 0, stream);
 }

@@ -60,7 +60,8 @@ constexpr uint32_t kTmemA = 256;   // A ring behind the accumulators: 64 columns
 enum { kErrFull = 11, kErrEmpty = 13, kErrAcc = 14, kErrDrained = 15 };
 enum { kOutUp = 0,      // silu(gate) * up, fp16, stored in the order of the down projection's words
        kOutDown = 1,    // times the row's routing weight, fp16
-       kOutLinear = 2   // activation type
+       kOutLinear = 2,  // activation type
+       kOutPartial = 3  // linear, a part of k: fp32 sums, added by linear_sum_kernel
 };
 
 // One matrix family of a launch: routed experts, or the shared expert.
@@ -88,6 +89,8 @@ struct alignas(64) Params {
   int shared_tiles;
   const long long* expert; // linear: expert id read on the device, or nullptr -> 0
   int rows, tile_rows;     // linear: rows, tokens per tile
+  int splits, split_kb;    // linear: parts of k, k-blocks of a part (even)
+  float* partial;          // [splits][rows][N]
   const __half* row_w;     // down: routing weight per sorted row
   const void* bias;        // linear
   int* err;
@@ -274,6 +277,7 @@ __device__ __forceinline__ void dequant_b3(const Exps<3>& X, uint32_t (&pr)[40],
 // A tile of the launch, as one CTA of the pair sees it.
 struct Tile {
   int fam, expert, row0, rows, col0;
+  int kb0, kbn, part;  // its k-blocks, its part of k
   // tokens of the MMA (32, 64, ..), of which each CTA brings half
   __device__ __forceinline__ int n() const { return (rows + 31) & ~31; }
   // first accumulator column of the CTA's tile number j
@@ -284,6 +288,15 @@ template <int COLS, bool LINEAR>  // COLS: columns of a CTA along N (gate/up: 64
 __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Tile& t) {
   if (LINEAR) {
     const Family& F = P.fam[0];
+    t.part = 0;
+    t.kb0 = 0;
+    t.kbn = F.K / kBK;
+    if (P.splits > 1) {
+      t.part = idx % P.splits;
+      idx /= P.splits;
+      t.kb0 = t.part * P.split_kb;
+      t.kbn = min(P.split_kb, t.kbn - t.kb0);
+    }
     const int mt = idx / F.col_tiles;
     if (mt * P.tile_rows >= P.rows) return false;
     t.fam = 0;
@@ -301,6 +314,8 @@ __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Til
   if (mt >= *P.n_tiles) return false;
   const int4 d = P.tiles[mt];
   t.fam = fam;
+  t.part = t.kb0 = 0;
+  t.kbn = P.fam[fam].K / kBK;
   t.expert = d.x;
   t.row0 = d.y;
   t.rows = d.z;
@@ -313,7 +328,7 @@ __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Til
 // blocks is followed by one of zeros: the activations of its stage end in zeros, too.
 // (Out of line: inlined, the 88 registers of 22 warps spill in the k loop.)
 template <bool UP, bool BF16, bool NAT, int B>
-__device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb1, uint32_t tmem) {
+__device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
   constexpr int NW = B == 3 ? 8 : 2 * B;  // words of a 64-code window
   const Family& F = P.fam[T.fam];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -336,8 +351,9 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   int* const err = P.err;
   const int gshift = (G & (G - 1)) == 0 ? __ffs(G) - 1 : -1;
   int kb = static_cast<int>(((warp >> 2) + kGroups - base % kGroups) % kGroups);  // first k-block of this warp's group
-  const int real = kb1;
-  kb1 = (kb1 + 1) & ~1;
+  const int real = T.kb0 + T.kbn, kb1 = T.kb0 + ((T.kbn + 1) & ~1);
+  base -= T.kb0;  // base + kb counts the blocks this CTA has handled
+  kb += T.kb0;
   if (kb >= kb1) return;
   struct Set { uint32_t w[NW]; __half s, z; };
   Set ring[2];
@@ -427,13 +443,13 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
 }
 
 template <bool UP, bool BF16, bool NAT>
-__device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, int kb1, uint32_t tmem) {
+__device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
   const Family& F = P.fam[T.fam];
   const int bits = F.nbits && T.expert >= 0 ? F.nbits[T.expert] : F.bits;
-  if (bits == 1) produce<UP, BF16, NAT, 1>(S, P, T, base, kb1, tmem);
-  else if (bits == 2) produce<UP, BF16, NAT, 2>(S, P, T, base, kb1, tmem);
-  else if (bits == 3) produce<UP, BF16, NAT, 3>(S, P, T, base, kb1, tmem);
-  else produce<UP, BF16, NAT, 4>(S, P, T, base, kb1, tmem);
+  if (bits == 1) produce<UP, BF16, NAT, 1>(S, P, T, base, tmem);
+  else if (bits == 2) produce<UP, BF16, NAT, 2>(S, P, T, base, tmem);
+  else if (bits == 3) produce<UP, BF16, NAT, 3>(S, P, T, base, tmem);
+  else produce<UP, BF16, NAT, 4>(S, P, T, base, tmem);
 }
 
 // ---- epilogue --------------------------------------------------------------------------------------
@@ -464,6 +480,22 @@ __device__ __forceinline__ void drain(Smem& S, uint32_t at, int rows, int column
     tmem_ld16(at + c, d);
 #pragma unroll
     for (int i = 0; i < 16; ++i) *reinterpret_cast<T*>(dst + (c + i) * kOutPitch) = as_act<T>(__uint_as_float(d[i]));
+  }
+}
+
+// A part of k: the fp32 sums of a column, a warp's 32 columns next to each other.
+__device__ __forceinline__ void drain_partial(const Params& P, const Tile& t, uint32_t at, int col) {
+  const size_t pitch = P.fam[0].N;
+  float* dst = P.partial + (static_cast<size_t>(t.part) * P.rows + t.row0) * pitch + col;
+  const int rows = t.rows;
+  const bool on = col < P.fam[0].N;
+#pragma unroll 1
+  for (int c = 0; c < rows; c += 16) {
+    uint32_t d[16];
+    tmem_ld16(at + c, d);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (on && c + i < rows) dst[static_cast<size_t>(c + i) * pitch] = __uint_as_float(d[i]);
   }
 }
 
@@ -547,7 +579,7 @@ __device__ __forceinline__ void finish_rows(const Smem& S, const Params& P, cons
 
 template <int OUT, bool BF16>
 __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_constant__ Params P) {
-  constexpr bool UP = OUT == kOutUp, LINEAR = OUT == kOutLinear;
+  constexpr bool UP = OUT == kOutUp, LINEAR = OUT == kOutLinear || OUT == kOutPartial;
   constexpr int COLS = UP ? kCols / 2 : kCols;
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -586,9 +618,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     uint32_t base = 0;
 #pragma unroll 1
     for (int i = 0; get_tile<COLS, LINEAR>(P, tile_of(i), rank, t); ++i) {
-      const int KB = P.fam[t.fam].K / kBK;
-      produce_any<UP, BF16, LINEAR>(S, P, t, base, KB, tmem);
-      base += (KB + 1) & ~1;
+      produce_any<UP, BF16, LINEAR>(S, P, t, base, tmem);
+      base += (t.kbn + 1) & ~1;
     }
   } else if (warp == kTmaWarp) {
     uint32_t c = 0;
@@ -596,7 +627,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     int* const err = P.err;
     for (int i = 0; get_tile<COLS, LINEAR>(P, tile_of(i), rank, t); ++i) {
       const Family& F = P.fam[t.fam];
-      const int SB = (F.K + kStageK - 1) / kStageK, half = t.n() / 2;
+      const int SB = (t.kbn + 1) / 2, half = t.n() / 2;
       const int box = (half + 31) / 32;  // in 32 rows: an odd number of 16-row blocks brings the next 16 rows, too
       const uint32_t bytes = 2 * 32 * box * kRowBytes;
       const int row = t.row0 - F.row0 + rank * half;
@@ -606,7 +637,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
         mbar_sleep_wait(&S.empty[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&S.full[s], 2 * bytes);
-          tma_load_pair(S.b[s], map, row, 2 * sb, full0 + s * 8);
+          tma_load_pair(S.b[s], map, row, t.kb0 + 2 * sb, full0 + s * 8);
         }
         __syncwarp();
       }
@@ -619,7 +650,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     const uint64_t desc0 = umma_desc_k_sw128(smem_u32(S.b[0]));
     int* const err = P.err;
     for (; get_tile<COLS, LINEAR>(P, tile_of(j), rank, t); ++j) {
-      const int SB = (P.fam[t.fam].K + kStageK - 1) / kStageK;
+      const int SB = (t.kbn + 1) / 2;
       const uint32_t idesc = umma_idesc_f16(BF16 ? 1 : 0, 2 * kCols, t.n());
       const uint32_t second = ((t.n() / 2 + 31) / 32 * 32 * kRowBytes) >> 4;  // distance of a stage's second k-block
       // The accumulators of the tile two back are out; with a tile over 128 tokens also those of the last.
@@ -652,10 +683,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     for (; get_tile<COLS, LINEAR>(P, tile_of(j), rank, t); ++j) {
       mbar_sleep_wait(&S.acc_full[j & 1], (j >> 1) & 1, P.err, kErrAcc);
       tc_fence_after_sync();
-      drain<OUT, T>(S, tmem + (static_cast<uint32_t>(32 * lq) << 16) + t.acc(j), t.rows, 32 * lq + (threadIdx.x & 31));
+      const uint32_t at = tmem + (static_cast<uint32_t>(32 * lq) << 16) + t.acc(j);
+      const int column = 32 * lq + static_cast<int>(threadIdx.x & 31);
+      if (OUT == kOutPartial) drain_partial(P, t, at, t.col0 + column);
+      else drain<OUT, T>(S, at, t.rows, column);
       tc_fence_before_sync();
       __syncwarp();
       if ((threadIdx.x & 31) == 0) arrive_at(first_cta(&S.drained[j & 1]));  // a later tile's MMAs may overwrite them
+      if (OUT == kOutPartial) continue;
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (UP) finish_up(S, P, t, tid);
       else finish_rows<OUT, T>(S, P, t, tid);
@@ -669,6 +704,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     tmem_dealloc_pair(tmem, kTmemCols);
   }
 }
+
+// gemm_ts.cu: tokens of a tile and parts of k of a linear, and the time they are estimated to take
+struct LinearPlan {
+  int tile_rows, splits, split_kb;
+  float us;
+};
+LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split);
 
 // gemm_ts.cu; tiles_bound: most tiles the launch can have
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream);

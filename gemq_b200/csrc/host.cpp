@@ -87,9 +87,12 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int rc;
   if (gemm) {
     if (ldx != K || !aligned16(x->data_ptr())) return none();
+    const size_t parts = gemq_linear_gemm_scratch_bytes(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), static_cast<int>(nbits));
+    Tensor scratch;
+    if (parts) scratch = empty_cuda({static_cast<int64_t>(parts / 4)}, at::kFloat, *x);
     rc = gemq_linear_gemm(x->data_ptr(), nullptr, static_cast<const int32_t*>(wp), s->data_ptr(), z->data_ptr(), nullptr, nullptr,
                           nullptr, static_cast<int>(nbits), bp, y.data_ptr(), static_cast<int>(M), static_cast<int>(N),
-                          static_cast<int>(K), 128, bf, err, stream_of(*x));
+                          static_cast<int>(K), 128, bf, err, parts ? scratch.data_ptr() : nullptr, parts, stream_of(*x));
     if (rc) return none();
   } else {
     rc = gemq_linear_rows(x->data_ptr(), static_cast<int>(ldx), bf, static_cast<const int32_t*>(wp), s->data_ptr(), z->data_ptr(),

@@ -29,10 +29,12 @@ def _gemm_tc(x: Tensor, w_q: Tensor, scales: Tensor, zeros: Tensor, nbits: int, 
     M, K = x.shape
     N = w_q.shape[1]
     out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    parts = _capi.lib.gemq_linear_gemm_scratch_bytes(M, N, K, nbits)
+    scratch = torch.empty(parts, dtype=torch.uint8, device=x.device) if parts else None
     _capi.check("gemq_linear_gemm", _capi.lib.gemq_linear_gemm(
         x.data_ptr(), None, w_q.data_ptr(), scales.data_ptr(), zeros.data_ptr(), None, None, None, nbits,
         bias.data_ptr() if bias is not None else None, out.data_ptr(), M, N, K, group_size, int(x.dtype == torch.bfloat16),
-        error_word(x.device).data_ptr(), stream_ptr(x.device)))
+        error_word(x.device).data_ptr(), scratch.data_ptr() if parts else None, parts, stream_ptr(x.device)))
     return out
 
 

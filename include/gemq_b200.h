@@ -202,11 +202,15 @@ int gemq_dequant_gemm_tc(const void* x, const int64_t* expert, const int32_t* wq
                          const int32_t* zs_strides, int fixed_bits, void* y, int M, int N, int K,
                          int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream);
 
-/* gemq_dequant_gemm_tc with an optional bias [N] of the activation type. */
+/* gemq_dequant_gemm_tc with an optional bias [N] of the activation type, and optional scratch (16-byte aligned):
+ * with gemq_linear_gemm_scratch_bytes of it a matrix of known bit width may be split along K, which fills the chip
+ * where there are few rows and columns.  The size is 0 where that would not pay. */
+size_t gemq_linear_gemm_scratch_bytes(int M, int N, int K, int nbits);
 int gemq_linear_gemm(const void* x, const int64_t* expert, const int32_t* wq, const void* scales,
                      const void* zeros, const int32_t* nbits, const int32_t* wq_strides,
                      const int32_t* zs_strides, int fixed_bits, const void* bias, void* y, int M, int N,
-                     int K, int group_size, int x_is_bf16, int32_t* err, gemq_stream_t stream);
+                     int K, int group_size, int x_is_bf16, int32_t* err, void* scratch, size_t scratch_bytes,
+                     gemq_stream_t stream);
 
 /* 1: gemq_dequant_gemv takes one row of such a matrix to the split-K streaming kernel, not to gemq_linear_rows. */
 int gemq_one_row_streams(int N, int K);

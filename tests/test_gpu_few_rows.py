@@ -70,7 +70,7 @@ def test_gemm_tile_edges(b, N, K):
     or goes one past it."""
     from gemq_b200.kernels import dequant_gemm
     from gemq_b200.kernels._runtime import error_word
-    from gemq_b200.kernels.dequant_gemm import quant_linear
+    from gemq_b200.kernels.dequant_gemm import _gemm_tc
     rng = np.random.default_rng(b * 10 + N)
     lin = MF.draw_linear(rng, N, K, b)
     t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
@@ -86,7 +86,32 @@ def test_gemm_tile_edges(b, N, K):
             # each way
             tol = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8 + 2.0 ** -9
             assert rel_fro(y.double().cpu().numpy(), want) < tol, (M, dtype, rel_fro(y.double().cpu().numpy(), want))
-            assert torch.equal(quant_linear(x, wq, s, z, b, 128, bias.to(dtype)), y + bias.to(dtype))
+            assert torch.equal(_gemm_tc(x, wq, s, z, b, 128, bias.to(dtype)), y + bias.to(dtype))
+    assert int(error_word(wq.device).item()) == 0
+
+
+@pytest.mark.parametrize("b", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K,M", [(288, 2176, 1), (96, 4096, 33), (1024, 5376, 100)])
+def test_gemm_split_k(b, N, K, M):
+    """The tcgen05 GEMM with k in parts: an odd number of k-blocks, a last part shorter than the others, 3-bit parts that
+    begin at every place of a packed word, fewer rows than a tile."""
+    from gemq_b200 import _capi
+    from gemq_b200.kernels._runtime import error_word
+    from gemq_b200.kernels.dequant_gemm import _gemm_tc
+    assert _capi.lib.gemq_linear_gemm_scratch_bytes(M, N, K, b) >= 2 * 4 * M * N
+    rng = np.random.default_rng(b * 10 + N)
+    lin = MF.draw_linear(rng, N, K, b)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    wq, s, z = t(lin["wq"]), t(lin["s"]), t(lin["z"])
+    W = O.dequantize(lin["wq"], lin["s"], lin["z"], b, 128, K).astype(np.float64)
+    bias = torch.from_numpy(rng.standard_normal(N)).cuda()
+    for dtype in (torch.float16, torch.bfloat16):
+        x = torch.from_numpy(rng.standard_normal((M, K))).to(dtype).cuda()
+        y = _gemm_tc(x, wq, s, z, b, 128, None)
+        want = x.double().cpu().numpy() @ W
+        tol = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8 + 2.0 ** -9  # as in the test above
+        assert rel_fro(y.double().cpu().numpy(), want) < tol, (dtype, rel_fro(y.double().cpu().numpy(), want))
+        assert torch.equal(_gemm_tc(x, wq, s, z, b, 128, bias.to(dtype)), y + bias.to(dtype))
     assert int(error_word(wq.device).item()) == 0
 
 
