@@ -131,10 +131,11 @@ __device__ __forceinline__ void build_pow2(const Rows& P, unsigned char* tab, co
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
-  // One row: an item at a time, there are few and the instructions are cold.  More: kAhead items of a half-warp
-  // side by side, the shuffles of a group's maximum and sum are a chain of 500 cycles.
-  if (rows == 1) convert_pow2<T, B, 1>(tab, 1, items, lane);
-  else convert_pow2<T, B, B == 1 ? 2 : 4>(tab, rows, items, lane);
+  // One row: an item at a time.  More: two items of a half-warp side by side, the shuffles of a group's maximum and sum
+  // are a chain.  Not more: the instructions come from a cold cache, the largest stall of a kernel this small (8 rows,
+  // 4096 x 4096, 2 bits: 6.2, 6.1, 6.3 us with one, two, four; 4 rows: 5.7, 5.8, 6.4).
+  if (rows == 1 || B == 1) convert_pow2<T, B, 1>(tab, rows, items, lane);
+  else convert_pow2<T, B, 2>(tab, rows, items, lane);
 }
 
 // 3-bit: groups are not word aligned.  Group statistics first (half a warp per group and row), then the pieces,
