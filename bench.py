@@ -320,7 +320,7 @@ def run_cfg2(dev):
         s = e0.elapsed_time(e1) * 1e-3 / n
         out[f"bs{B}"] = {"tokens_per_s": B / s, "us_per_step": s * 1e6, "algorithmic_bytes_per_step": sum(byts) / len(byts),
                          "hbm_frac": sum(byts) / len(byts) / s / 1e9 / hbm_peak,
-                         "path": "one-launch layer kernel per row" if B <= 4 else "expert-sorted grouped GEMM"}
+                         "path": "router, up and down launches" if B == 1 else "expert-sorted few-row kernels"}
     return out
 
 
@@ -407,7 +407,7 @@ def run_prefill(args, rank, local_rank, world, dev):
                       "l2": "inputs larger than L2: ~0.4 GB of packed weights per step"},
            "e2e": {"value": T * steps / e2e_s, "unit": "tokens/s", "h2d_bytes_per_step": 2 * T * D // world,
                    "d2h_bytes_per_step": 2 * T * D // world},
-           "roofline": {"bound": "tensor", "kernel": "grouped_gemm_kernel (gate/up + down; whole prefill call timed)",
+           "roofline": {"bound": "tensor", "kernel": "gemm_ts_kernel (gate/up + down; whole prefill call timed)",
                         "achieved": ach / world, "peak": peak_tf, "peak_kind": kind, "unit": "TFLOP/s",
                         "frac": ach / world / peak_tf, "frac_sustained": ach / world / peak_sus if peak_sus else None,
                         "traffic": PREFILL_TRAFFIC_BYTES if world == 1 and T == 4096 else None}}
