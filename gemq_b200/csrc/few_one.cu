@@ -229,12 +229,12 @@ __global__ void __launch_bounds__(kThreads, 3) few_one_kernel(const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int members = MODE == 0 ? 1 : P.S * P.splits;  // of the cluster
   const int rank = MODE == 0 ? 0 : static_cast<int>(blockIdx.x % members);
-  const int s = MODE == 0 ? static_cast<int>(blockIdx.y) : rank / P.splits;  // slot
+  const int per_slot = P.N[0] / 32, tile = static_cast<int>(blockIdx.x) / members;
+  const int s = MODE == 0 ? min(tile / per_slot, P.A) : rank / P.splits;  // slot; up: the shared expert's tiles come last
   const int part = MODE == 0 ? 0 : rank % P.splits;
-  const int n0 = MODE == 0 ? 32 * static_cast<int>(blockIdx.x) : 64 * static_cast<int>(blockIdx.x / members);
+  const int n0 = MODE == 0 ? 32 * (tile - s * per_slot) : 64 * tile;
   const int fam = s >= P.A ? 1 : 0;
   const int N = P.N[fam], K = P.K[fam], ngroups = K / kGroup;
-  if (MODE == 0 && n0 >= N) return;  // the launch covers the wider of the two families
   // what does not depend on the kernel before: barriers, the experts' bit widths and offsets
   if (tid == 0) {
     for (int i = 0; i < kMaxRing; ++i) {
@@ -485,7 +485,7 @@ int moe_one(const gemq_moe_layer_t* L, const __half* x, __half* out, const int64
   U.N[0] = F; U.N[1] = SF;
   U.tab_bytes = one_table_bytes(D, kCons, 1);
   const int most = F > SF ? F : SF;
-  if (const int rc = launch_one<0>(U, dim3(cdiv(most, 32), S), 1, st)) return rc;
+  if (const int rc = launch_one<0>(U, dim3(A * (F / 32) + SF / 32), 1, st)) return rc;
   Q.x = h;
   Q.out = out;
   Q.K[0] = F; Q.K[1] = SF;
