@@ -237,3 +237,26 @@ def test_expert_parallel_two_gpus_matches_single_gpu():
     results = mgr.dict()
     mp.spawn(_ep_worker, args=(2, 29611, results), nprocs=2, join=True)
     assert max(results.values()) == 0.0, dict(results)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,E,D,A", [(296, 64, 256, 6), (297, 64, 2048, 6), (593, 7, 256, 2), (597, 8, 4096, 2), (607, 9, 512, 3),
+                                     (608, 16, 768, 2), (609, 17, 2048, 4), (601, 32, 1280, 6), (305, 33, 256, 16), (311, 61, 2048, 6)])
+def test_router_many_tokens(T, E, D, A, dtype):
+    """Edges of 16-token CTAs, of eight-expert tiles and of the line to one token per CTA, against fp64 products."""
+    from gemq_b200.inference.moe_block import ROUTE_FP32, route_tokens
+    gen = torch.Generator().manual_seed(T * 64 + E)
+    x, g = torch.randn(T, D, generator=gen).to(dtype).cuda(), (0.05 * torch.randn(E, D, generator=gen)).to(dtype).cuda()
+    w, idx, logits = route_tokens(x, g, A, ROUTE_FP32, True)
+    # Products are exact; a sum passes at most D / 128 + 8 additions and the 16 places of one tensor-core step, each off
+    # by at most one fp32 ulp of the running sum (bounded by the sum of magnitudes).
+    bound = (D / 128 + 8 + 16) * 2.0 ** -23 * (x.double().abs() @ g.double().abs().T)
+    assert ((logits.double() - x.double() @ g.double().T).abs() <= bound).all()
+    # Selection and weights from the kernel's own logits; neighbours closer than 1e-5 may change places.
+    p = logits.double().softmax(1)
+    top, _ = p.topk(A, dim=1)
+    got = p.gather(1, idx)
+    assert (idx.sort(1).values.diff(dim=1) > 0).all()
+    assert (got - top).abs().max() < 1e-5
+    want = got / got.sum(1, keepdim=True)
+    assert ((w.double() - want).abs() <= want * torch.finfo(dtype).eps).all()
