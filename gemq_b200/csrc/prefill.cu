@@ -252,7 +252,11 @@ struct Scratch {
   int max_tiles;
 };
 
+// The gather stores 32 bytes at a time, callers align their scratch to 16: the pieces start at the next multiple of 32.
+constexpr size_t kAlign = 32, kSlack = kAlign - 16;
+
 size_t layout(const gemq_moe_layer_t* L, int tokens, Scratch* S, char* base) {
+  if (base) base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + kAlign - 1) / kAlign * kAlign);
   const size_t R = static_cast<size_t>(tokens) * L->top_k, SF = L->shared_ffn;
   const size_t rows = R + (SF ? tokens : 0);
   const size_t tiles = R / kTile + (R < static_cast<size_t>(L->n_experts) ? R : L->n_experts) + (SF ? cdiv(tokens, kTile) : 0);
@@ -288,7 +292,7 @@ size_t layout(const gemq_moe_layer_t* L, int tokens, Scratch* S, char* base) {
     const size_t n = few_at + few::moe_few_rows_bytes(L, tokens);
     off = n > off ? n : off;
   }
-  return off;
+  return off + kSlack;
 }
 
 void fill(ts::Family& F, int m, const gemq_stacked_t& W) {

@@ -47,3 +47,19 @@ def test_expert_bit_draw_respects_mean():
         bits = draw_expert_bits(8, seed)
         assert set(bits) <= {1, 2, 3, 4} and 1.5 <= sum(bits) / 8 <= 2.5
     assert draw_expert_bits(64, 3) == draw_expert_bits(64, 3)
+
+
+@pytest.mark.parametrize("tokens", [3, 300])
+def test_prefill_scratch_may_be_aligned_to_16_bytes_only(tokens):
+    """The n-token layer stores 32 bytes at a time into scratch that callers align to 16: wherever the scratch begins,
+    its pieces begin at a multiple of 32 and lie inside the size that was asked for."""
+    import ctypes as C
+    from gemq_b200 import _capi
+    layer = _capi.MoeLayer()
+    layer.hidden, layer.ffn, layer.n_experts, layer.top_k, layer.group_size = 256, 512, 4, 2, 128
+    size = _capi.lib.gemq_moe_prefill_scratch_bytes(C.byref(layer), tokens)
+    bases = [(1 << 20) + 16 * k for k in range(4)]
+    first = [_capi.lib.gemq_moe_prefill_error_word(C.byref(layer), tokens, b) for b in bases]  # the first piece
+    assert all(f % 32 == 0 and f >= b for f, b in zip(first, bases))
+    used = size - max(f - b for f, b in zip(first, bases))
+    assert used % 32 == 0  # whole pieces: the rest of the size is room for the shift

@@ -260,3 +260,23 @@ def test_router_many_tokens(T, E, D, A, dtype):
     assert (got - top).abs().max() < 1e-5
     want = got / got.sum(1, keepdim=True)
     assert ((w.double() - want).abs() <= want * torch.finfo(dtype).eps).all()
+
+
+@pytest.mark.parametrize("T", [3, 300])
+def test_prefill_scratch_at_an_odd_multiple_of_16(T):
+    """The same bits from a scratch that is 16- but not 32-byte aligned (few-row path and large path)."""
+    import ctypes as C
+    from gemq_b200 import _capi
+    from gemq_b200.kernels._runtime import stream_ptr
+    blk = MF.gpu_block(MF.make_layer("mixtral", D=256, Fd=512, E=4, A=2, bits=[4, 1, 3, 2], seed=6, gate_std=0.02))
+    x = torch.randn(T, 256, generator=torch.Generator().manual_seed(3)).half().cuda()
+    size = _capi.lib.gemq_moe_prefill_scratch_bytes(C.byref(blk._layer), T)
+    outs = []
+    for shift in (0, 16):
+        scratch = torch.empty(size + 32, dtype=torch.uint8, device="cuda")[shift:shift + size]
+        assert scratch.data_ptr() % 32 == shift
+        out, idx, w = torch.empty_like(x), torch.empty(T, 2, dtype=torch.int64, device="cuda"), torch.empty_like(x[:, :2]).contiguous()
+        assert _capi.lib.gemq_moe_prefill(C.byref(blk._layer), x.data_ptr(), out.data_ptr(), idx.data_ptr(), w.data_ptr(), None, T, 1, 1,
+                                          0, scratch.data_ptr(), size, stream_ptr(x.device)) == 0
+        outs.append(out)
+    assert torch.equal(*outs) and torch.isfinite(outs[0]).all()
