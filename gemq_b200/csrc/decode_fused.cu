@@ -569,7 +569,7 @@ __device__ void route_cta(Smem& S, const FusedParams& P) {
 }
 
 // ---- plan -------------------------------------------------------------------------------------
-// Warp 0 makes the parts of phase 0, warp 1 those of phase 1, a lane a part.  By one warp and one lane per slot it
+// Warp 0 fills the slots; then it makes the parts of phase 0 and warp 1 those of phase 1, a lane a part.  By one warp and one lane per slot it
 // took 9 us of a Mixtral token's 52 and of a DeepSeek-V2-Lite token's 27.
 // a / b for a < 2^24, b > 0: one approximate reciprocal and a correction instead of the integer
 // division sequence (the plan is a chain of dependent instructions).
@@ -584,14 +584,14 @@ __device__ __forceinline__ int quanta_of(int groups, int bits) { return bits == 
 __device__ void make_plan(Smem& S, const FusedParams& P) {
   const int lane = threadIdx.x & 31, ph = threadIdx.x >> 5;
   const int Sn = P.S;
-  // slots (by both warps alike)
+  // slots: both warps go through them for the sums below, only warp 0 stores
   int Fs = 0, b1 = 1, b2 = 1;
+  SlotInfo I = {};
   if (lane < Sn) {
-    SlotInfo I;
     if (lane < P.A) {
       int e = S.sel_e[lane];
       if (e < 0 || e >= P.E) {  // caller-supplied routing with an id out of range: never index with it
-        atomicExch(P.counters + kErrSlot, kErrBadExpert);
+        if (ph == 0) atomicExch(P.counters + kErrSlot, kErrBadExpert);
         e = e < 0 ? 0 : P.E - 1;
       }
       const bool pre = P.E <= kMetaE;  // tables staged in shared memory ahead of the dependency wait
@@ -623,7 +623,6 @@ __device__ void make_plan(Smem& S, const FusedParams& P) {
     I.nq[1] = quanta_of(Fs / kGroup, b2);
     I.nch[0] = cdiv(Fs, 128);
     I.nch[1] = cdiv(P.D, 128);
-    S.slot[lane] = I;
   }
   // exclusive prefix sums over the slots: h / partial offsets, pair counters, down quanta
   int nch0 = lane < Sn ? cdiv(Fs, 128) : 0;
@@ -640,20 +639,20 @@ __device__ void make_plan(Smem& S, const FusedParams& P) {
   const int expected1 = __shfl_sync(0xffffffffu, in_nq1, kMaxS - 1);
   const int nch1 = cdiv(P.D, 128);
   const int base1 = 3 * pairs_total;
-  if (lane < Sn) {
-    SlotInfo& I = S.slot[lane];
+  if (ph == 0 && lane < Sn) {
     I.hoff = in_fs - fs;
     I.ctrb = in_nch - nch0;
     I.colb[0] = 2 * (in_fs - fs);
     I.colb[1] = P.up_cols + lane * P.D;  // the phases overlap in time: their partial columns must not
     I.maskb[0] = pairs_total + 2 * (in_nch - nch0);
     I.maskb[1] = base1 + nch1 + lane * nch1;
+    S.slot[lane] = I;
   }
-  if (lane == 0) {  // both warps: the same values
+  if (ph == 0 && lane == 0) {
     S.pairs_total = pairs_total;
     S.expected1 = expected1;
   }
-  __syncwarp();
+  asm volatile("bar.sync 2, 64;" ::: "memory");  // the two warps
   // range of the phase: units [ulo, uhi) of each slot (lane), and the parts they make
   unsigned ulo = 0, uhi = 0, cm_lo = 0;
   int nq = 1, first = 0, np_total = 0, pbase = 0;

@@ -72,14 +72,15 @@ bool moe_one_ok(const gemq_moe_layer_t* L);
 int moe_one(const gemq_moe_layer_t* L, const __half* x, __half* out, const int64_t* idx, const __half* w, int* counters, float* h,
             cudaStream_t st);
 
-// GEMQ_B200_DECODE=stream selects the three-launch path (router, gate/up GEMV, down GEMV) for
-// layers the single-launch kernel would take; read once.
-static bool fused_enabled() {
-  static const bool on = [] {
+// GEMQ_B200_DECODE pins the one-token path, read once: "stream" the three launches (router, gate/up GEMV, down GEMV),
+// "persistent" the one launch of decode_fused.cu (GEMQ_ERR_BAD_SHAPE for layers it does not take).
+enum class OneToken { kBest, kStream, kPersistent };
+static OneToken one_token_path() {
+  static const OneToken path = [] {
     const char* v = getenv("GEMQ_B200_DECODE");
-    return !(v && v[0] == 's');
+    return !v ? OneToken::kBest : v[0] == 's' ? OneToken::kStream : v[0] == 'p' ? OneToken::kPersistent : OneToken::kBest;
   }();
-  return on;
+  return path;
 }
 
 }  // namespace gemq
@@ -113,7 +114,7 @@ extern "C" int gemq_moe_decode(const gemq_moe_layer_t* L, const void* x, void* o
   if (!carve(L, scratch, scratch_bytes, &S)) return GEMQ_ERR_WORKSPACE;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-  if (fused_enabled() && aligned16(x) && aligned16(out) && aligned16(L->gate) && moe_one_ok(L)) {
+  if (one_token_path() == OneToken::kBest && aligned16(x) && aligned16(out) && aligned16(L->gate) && moe_one_ok(L)) {
     if (do_route)
       if (const int rc = gemq_moe_route(x, L->gate, tokens, D, L->n_experts, A, route_mode, L->renorm, 0, idx, w, nullptr, stream)) return rc;
     for (int t = 0; t < tokens; ++t)
@@ -129,7 +130,7 @@ extern "C" int gemq_moe_decode(const gemq_moe_layer_t* L, const void* x, void* o
     int* counters = static_cast<int*>(S.gemv_ws);
     float* partial = reinterpret_cast<float*>(static_cast<char*>(S.gemv_ws) + kMaxCounters * sizeof(int));
     const size_t partial_floats = (S.gemv_ws_bytes - kMaxCounters * sizeof(int)) / sizeof(float);
-    if (fused_enabled() && aligned16(x) && aligned16(out) && aligned16(L->gate) && decode_fused_ok(L, partial_floats)) {
+    if (one_token_path() != OneToken::kStream && aligned16(x) && aligned16(out) && aligned16(L->gate) && decode_fused_ok(L, partial_floats)) {
       const bool in_kernel = do_route && L->n_experts <= 32 && A <= L->n_experts && D % 256 == 0;
       if (do_route && !in_kernel) {
         const int rc = gemq_moe_route(x, L->gate, tokens, D, L->n_experts, A, route_mode, L->renorm, 0, idx, w, nullptr,
@@ -146,6 +147,7 @@ extern "C" int gemq_moe_decode(const gemq_moe_layer_t* L, const void* x, void* o
       }
       return GEMQ_OK;
     }
+    if (one_token_path() == OneToken::kPersistent) return GEMQ_ERR_BAD_SHAPE;
   }
 
   if (do_route) {
