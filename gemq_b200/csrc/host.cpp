@@ -7,6 +7,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -128,7 +129,8 @@ PyObject* moe_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // moe_prefill(layer_ptr, x, scratch | None, hidden, top_k, n_experts, route_mode, want_logits)
-// -> (out, logits | None), logits [T, E] of x's type; None also when the scratch is too small.
+// -> (out, logits | None), logits [T, E] of x's type; None also when the scratch is too small, and under capture
+// (the block then keeps the scratch for the graph).
 PyObject* moe_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 8) { PyErr_SetString(PyExc_TypeError, "moe_prefill takes 8 arguments"); return nullptr; }
   const auto* L = static_cast<const gemq_moe_layer_t*>(PyLong_AsVoidPtr(a[0]));
@@ -141,6 +143,7 @@ PyObject* moe_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t T = x->numel() / D;
   if (T > (1 << 24) || gemq_moe_prefill_scratch_bytes(L, static_cast<int>(T)) > static_cast<size_t>(sc->numel())) return none();
   c10::cuda::CUDAGuard guard(x->device());
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return none();
   Tensor out = empty_cuda(x->sizes(), x->scalar_type(), *x);
   Tensor logits;
   if (want) logits = empty_cuda({T, E}, x->scalar_type(), *x);

@@ -79,6 +79,7 @@ class _QuantFusedMoEBase(nn.Module):
         self._layer = None       # ctypes struct handed to the library
         self._scratch = None
         self._prefill_scratch = None
+        self._graph_scratch = []  # prefill scratch that a captured graph uses: replays go on with its address
         self._nbits_host = None
 
     # -- construction ---------------------------------------------------------------
@@ -186,15 +187,26 @@ class _QuantFusedMoEBase(nn.Module):
         out = _moe_prefill_routed(x, routing[0], routing[1], self._handle, route_mode, renorm)
         return out, routing[0], routing[1], None
 
+    def _prefill_buffer(self, nbytes: int, dev) -> Tensor:
+        """Scratch of an n-token call.  It grows with the largest call; a buffer that was used under capture is kept
+        when it is replaced.  From then on sizes at least double, so that graphs captured for growing batches
+        do not add up to more than twice the largest."""
+        sc = self._prefill_scratch
+        if sc is None or sc.numel() < nbytes:
+            if self._graph_scratch:
+                nbytes = max(nbytes, 2 * self._graph_scratch[-1].numel())
+            sc = self._prefill_scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        if torch.cuda.is_current_stream_capturing() and not (self._graph_scratch and self._graph_scratch[-1] is sc):
+            self._graph_scratch.append(sc)
+        return sc
+
     def _prefill_impl(self, x: Tensor, route_mode: int, renorm: bool, routing=None, logits_dtype=torch.float32):
         """``logits_dtype``: fp32, x's dtype, or None (no logits are wanted)."""
         dev = require_cuda(x)
         x = x.contiguous()
         T = x.shape[0]
         bf = x.dtype == torch.bfloat16
-        nbytes = _capi.lib.gemq_moe_prefill_scratch_bytes(C.byref(self._layer), T)
-        if self._prefill_scratch is None or self._prefill_scratch.numel() < nbytes:
-            self._prefill_scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        sc = self._prefill_buffer(_capi.lib.gemq_moe_prefill_scratch_bytes(C.byref(self._layer), T), dev)
         out = torch.empty_like(x)
         if routing is not None:
             w, idx = routing[0].contiguous(), routing[1].contiguous()
@@ -204,7 +216,6 @@ class _QuantFusedMoEBase(nn.Module):
             w = torch.empty((T, self.top_k), dtype=x.dtype, device=dev)
             logits = torch.empty((T, self.num_experts), dtype=logits_dtype, device=dev) if logits_dtype is not None else None
             do_route = 1 if logits_dtype == torch.float32 else 2
-        sc = self._prefill_scratch
         _capi.check("gemq_moe_prefill", _capi.lib.gemq_moe_prefill(
             C.byref(self._layer), x.data_ptr(), out.data_ptr(), idx.data_ptr(), w.data_ptr(),
             logits.data_ptr() if logits is not None else None, T, do_route, route_mode, int(bf), sc.data_ptr(), sc.numel(), stream_ptr(dev)))

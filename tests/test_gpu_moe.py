@@ -280,3 +280,33 @@ def test_prefill_scratch_at_an_odd_multiple_of_16(T):
                                           0, scratch.data_ptr(), size, stream_ptr(x.device)) == 0
         outs.append(out)
     assert torch.equal(*outs) and torch.isfinite(outs[0]).all()
+
+
+@pytest.mark.parametrize("T", [3, 40])
+def test_graph_of_a_batch_survives_a_larger_call(T):
+    """A captured decode batch, then a call that needs more scratch, other tensors where the old scratch might have
+    gone, and a replay: the graph's result and the other tensors are what they were."""
+    layer = MF.make_layer("deepseek", D=256, Fd=384, E=16, A=6, bits=[1, 2, 3, 4] * 4, seed=4, gate_std=1 / 16.0, n_shared=2)
+    blk = MF.gpu_block(layer)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, 1, 256, device="cuda", generator=gen).half()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        want = blk(x).clone()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            out = blk(x)
+        torch.cuda.synchronize()
+        small = blk._prefill_scratch
+        size = small.numel()
+        assert small is blk._graph_scratch[-1]
+        del small
+        blk(torch.randn(1, 900, 256, device="cuda", generator=gen).half())
+        assert blk._prefill_scratch.numel() > size
+        others = [torch.full((size,), 7, dtype=torch.uint8, device="cuda") for _ in range(4)]
+        for _ in range(3):
+            g.replay()
+        torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert all(bool((o == 7).all()) for o in others)
