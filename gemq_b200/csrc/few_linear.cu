@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kThreads, NB == 1 ? 3 : 2) few_linear_kernel(c
   float* red = reinterpret_cast<float*>(ring);  // the warps' sums, over the drained ring
 
   if (warp == kCons) {
-    // ---- producer: nothing it reads is written by a kernel of this stream -----------------------
+    // ---- producer ------------------------------------------------------------------------------
     const int gshift = P.bits == 3 ? 1 : (P.bits == 4 ? 0 : (P.bits == 2 ? 1 : 2));  // log2 of the groups per stage
     const int ngroups = P.K / kGroup;
     const int piece = lane & 3, mst = (lane >> 2) & 1, kind = (lane >> 3) & 1;
@@ -113,6 +113,17 @@ __global__ void __launch_bounds__(kThreads, NB == 1 ? 3 : 2) few_linear_kernel(c
     const uint32_t mdst = kWStage + kind * 128 + mst * 64 + piece * 16;
     const bool box = lane < kCons;
     const int my_lo = S.lo[lane & 3], my_hi = S.hi[lane & 3];
+    // The matrix may be a result of the launch before (a layer packed and called at once): up to the wait its first
+    // stages come into L2 only, where such a result goes, too.
+    for (int it = 0; it < min(iters, P.ring); ++it)
+      if (box && my_lo + it < my_hi) tma_prefetch_strips(&P.wmap, (my_lo + it) * kStageRows, n0 >> 5);
+    if ((lane & 7) == 0 && col < P.N)
+      for (int i = lane >> 4; i < (kCons << gshift); i += 2) {
+        const int cw = i >> gshift, gi = i & ((1 << gshift) - 1), sg = S.lo[cw];
+        const int grp = P.bits == 3 ? 5 * (sg >> 2) + (sg & 3) + gi : (sg << gshift) + gi;
+        if (sg < S.hi[cw] && grp < ngroups) prefetch_l2(mbase + static_cast<size_t>(grp) * P.N);
+      }
+    pdl_wait();
     int slot = 0;
     uint32_t par = 1;
     for (int it = 0; it < iters; ++it) {

@@ -386,6 +386,12 @@ __device__ __forceinline__ void tma_load_strips(void* dst, const CUtensorMap* ma
       "l"(reinterpret_cast<unsigned long long>(map)), "r"(0), "r"(row), "r"(strip), "r"(smem_u32(bar))
       : "memory");
 }
+// The same box into L2.
+__device__ __forceinline__ void tma_prefetch_strips(const CUtensorMap* map, int row, int strip) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<unsigned long long>(map)),
+               "r"(0), "r"(row), "r"(strip)
+               : "memory");
+}
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

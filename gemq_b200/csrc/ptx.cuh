@@ -57,6 +57,7 @@ __device__ __forceinline__ void mbar_sleep_wait(unsigned long long* bar, uint32_
   }
   atomicExch(err, code);
 }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 // Tiled TMA load of one box at element coordinates (x = column, y = row); x * element size
 // must be a multiple of 16 bytes (it is: columns come in multiples of 32).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {

@@ -159,6 +159,8 @@ typedef struct {
   int group_size;
 } gemq_single_t;
 
+/* The integer tables of the stacked matrices (nbits, strides) are read ahead of the wait for the launch before a
+ * layer call, which must not write them.  Everything else may be a result of that launch. */
 typedef struct {
   int hidden;        /* D */
   int ffn;           /* F */
@@ -289,6 +291,7 @@ int gemq_ep_combine(const void* back, const int64_t* where, const int64_t* sel, 
  * h = x + T(res) (res nullable; fp16 with res_is_half, else T), written to sum_out if that is given (another buffer
  * than x and res); n = RMSNorm(h) * norm_weight, or h itself without norm_weight;
  * out [rows0 + rows1 + rows2] = the matrices [rows, K] of T, one after the other, times n.  rows1 and rows2 may be 0.
+ * The matrices are read ahead of the wait for the launch before this one, which must not write them.
  * K % 256 == 0, K <= 16384. */
 int gemq_step_gemv(const void* x, const void* res, int res_is_half, const void* norm_weight, float eps, void* sum_out,
                    const void* w0, int rows0, const void* w1, int rows1, const void* w2, int rows2, void* out, int K,

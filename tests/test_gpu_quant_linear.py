@@ -42,3 +42,27 @@ def test_hqq_layer_as_quant_linear(nbits, rows):
     assert y.shape == (rows, out_f)
     assert rel_fro(y, ref) < REL_FRO_TOL, rel_fro(y, ref)
     assert max_abs(y, ref) < MAX_ABS_TOL, max_abs(y, ref)
+
+
+@pytest.mark.parametrize("rows", [1, 13, 200])
+@pytest.mark.parametrize("nbits", [2, 3])
+def test_weights_written_by_the_launch_before(rows, nbits):
+    """The matrix, its scales and its offsets are results of the launches right before the call, whose kernels start
+    before those have ended: the call waits for them (few-row kernel and tcgen05 GEMM)."""
+    from gemq_b200 import synth
+    from gemq_b200.inference import PackedLinear, QuantLinear
+    gen = synth.generator(rows + nbits, "cuda")
+    srcs = [synth.make_linear(4096, 2048, nbits, 128, gen, "cuda") for _ in range(2)]
+    x = torch.randn(rows, 2048, device="cuda", generator=gen).to(torch.bfloat16)
+    want = [QuantLinear(s)(x) for s in srcs]
+    own = PackedLinear(srcs[0].W_q.clone(), srcs[0].scales.clone(), srcs[0].zeros.clone(), nbits, 128, 2048, 4096)
+    layer = QuantLinear(own)
+    torch.cuda.synchronize()
+    got = []
+    for i in range(40):
+        s = srcs[i % 2]
+        for dst, src in (((own.scales, s.scales), (own.zeros, s.zeros), (own.W_q, s.W_q)) if i % 4 < 2 else
+                         ((own.W_q, s.W_q), (own.zeros, s.zeros), (own.scales, s.scales))):
+            torch.add(src, 0, out=dst)  # a kernel, not a copy
+        got.append(layer(x))
+    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
