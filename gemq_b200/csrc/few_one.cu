@@ -398,21 +398,52 @@ static size_t one_smem(int tab_bytes, int cluster, int ring) {
   return 1024 + static_cast<size_t>(kCons) * tab_bytes + static_cast<size_t>(cluster) * 64 * 4 + ring * static_cast<size_t>(kWStage + kMetaStage);
 }
 
+// Dynamic shared memory of a launch: 227 KB less the static part.
+constexpr size_t kOneDyn = kMaxDyn - 8192;
+
+// Ring stages: a third one where it costs no CTA of the three an SM can hold; 0: not even two fit.
+static int one_ring(int tab_bytes, int cluster) {
+  auto per_sm = [&](int ring) { return 227 * 1024 / (one_smem(tab_bytes, cluster, ring) + sizeof(OneShared) + 1024); };
+  const bool third = per_sm(kMaxRing) >= 3 || per_sm(kMaxRing) == per_sm(2);
+  if (third && one_smem(tab_bytes, cluster, kMaxRing) <= kOneDyn) return kMaxRing;
+  return one_smem(tab_bytes, cluster, 2) <= kOneDyn ? 2 : 0;
+}
+
+// Shape of the two launches of a layer; `ok`: both fit.
+struct OnePlan {
+  int tab[2], ring[2];  // up, down
+  int splits;           // of the down launch: parts of a slot
+  bool ok;
+};
+static OnePlan one_plan(const gemq_moe_layer_t* L) {
+  OnePlan p = {};
+  const int D = L->hidden, F = L->ffn, SF = L->shared_ffn, S = L->top_k + (SF > 0 ? 1 : 0);
+  const int most = F > SF ? F : SF, shorter = SF && SF < F ? SF : F, tiles = cdiv(D, 64), sms = sm_count();
+  // as many parts as run at once (their tables decide how many CTAs an SM holds), a group a warp at least
+  for (p.splits = 8 / S; p.splits > 1; --p.splits) {
+    const size_t smem = one_smem(one_table_bytes(most, kCons * p.splits, 2), S * p.splits, 2) + sizeof(OneShared) + 1024;
+    const int per_sm = static_cast<int>(227 * 1024 / smem);
+    if (shorter >= kGroup * kCons * p.splits && tiles * S * p.splits <= (per_sm > 3 ? 3 : per_sm) * sms) break;
+  }
+  p.tab[0] = one_table_bytes(D, kCons, 1);
+  p.tab[1] = one_table_bytes(most, kCons * p.splits, 2);
+  p.ring[0] = one_ring(p.tab[0], 1);
+  p.ring[1] = one_ring(p.tab[1], S * p.splits);
+  p.ok = sms > 0 && p.ring[0] && p.ring[1];
+  return p;
+}
+
 template <int MODE>
-static int launch_one(OneParams& P, dim3 grid, int cluster, cudaStream_t st) {
+static int launch_one(const OneParams& P, dim3 grid, int cluster, cudaStream_t st) {
   static bool done[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GEMQ_ERR_LAUNCH;
   if (!done[dev]) {
-    if (cudaFuncSetAttribute(few_one_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDyn - 8192) != cudaSuccess)
+    if (cudaFuncSetAttribute(few_one_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneDyn) != cudaSuccess)
       return GEMQ_ERR_LAUNCH;
     done[dev] = true;
   }
-  // a third stage where it costs no CTA of the three an SM can hold
-  auto per_sm = [&](int ring) { return 227 * 1024 / (one_smem(P.tab_bytes, cluster, ring) + sizeof(OneShared) + 1024); };
-  P.ring = per_sm(kMaxRing) >= 3 || per_sm(kMaxRing) == per_sm(2) ? kMaxRing : 2;
   const size_t smem = one_smem(P.tab_bytes, cluster, P.ring);
-  if (smem > static_cast<size_t>(kMaxDyn - 8192)) return GEMQ_ERR_BAD_SHAPE;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
@@ -434,8 +465,8 @@ static int launch_one(OneParams& P, dim3 grid, int cluster, cudaStream_t st) {
 
 using namespace few;
 
-// Layers this path takes: extents in whole groups, eight slots at most (the cluster), tables that leave room for a ring,
-// and fewer weights than where the persistent kernel is the faster.
+// Layers this path takes: extents in whole groups, eight slots at most (the cluster), tables that leave room for a ring
+// in either launch, and fewer weights than where the persistent kernel is the faster.
 bool moe_one_ok(const gemq_moe_layer_t* L) {
   const int D = L->hidden, F = L->ffn, SF = L->shared_ffn, A = L->top_k, S = A + (SF > 0 ? 1 : 0);
   if (L->group_size != kGroup || D % kGroup || F % kGroup || SF % kGroup || S > 8 || L->n_experts > kOneMaxE) return false;
@@ -449,13 +480,15 @@ bool moe_one_ok(const gemq_moe_layer_t* L) {
   if (SF)
     for (const void* p : shared)
       if (!p || !aligned16(p)) return false;
-  return L->w1.wq_rows > 0 && L->w3.wq_rows > 0 && L->w2.wq_rows > 0;
+  return L->w1.wq_rows > 0 && L->w3.wq_rows > 0 && L->w2.wq_rows > 0 && one_plan(L).ok;
 }
 
 // One token; idx / w hold its routing (written by the launch before or older), h [S slots] fp32 scratch.
 int moe_one(const gemq_moe_layer_t* L, const __half* x, __half* out, const int64_t* idx, const __half* w, int* counters, float* h,
             cudaStream_t st) {
   const int D = L->hidden, F = L->ffn, SF = L->shared_ffn, A = L->top_k, S = A + (SF > 0 ? 1 : 0);
+  const OnePlan plan = one_plan(L);
+  if (!plan.ok) return GEMQ_ERR_BAD_SHAPE;
   OneParams U = {};
   U.idx = reinterpret_cast<const long long*>(idx);
   U.w = w; U.counters = counters; U.h = h;
@@ -483,24 +516,17 @@ int moe_one(const gemq_moe_layer_t* L, const __half* x, __half* out, const int64
   U.x = x;
   U.K[0] = U.K[1] = D;
   U.N[0] = F; U.N[1] = SF;
-  U.tab_bytes = one_table_bytes(D, kCons, 1);
-  const int most = F > SF ? F : SF;
+  U.tab_bytes = plan.tab[0];
+  U.ring = plan.ring[0];
   if (const int rc = launch_one<0>(U, dim3(A * (F / 32) + SF / 32), 1, st)) return rc;
   Q.x = h;
   Q.out = out;
   Q.K[0] = F; Q.K[1] = SF;
   Q.N[0] = Q.N[1] = D;
-  // as many parts as run at once (their tables decide how many CTAs an SM holds), a group a warp at least
-  const int tiles = cdiv(D, 64), sms = sm_count(), shorter = SF && SF < F ? SF : F;
-  int splits = 8 / S;
-  for (; splits > 1; --splits) {
-    const size_t smem = one_smem(one_table_bytes(most, kCons * splits, 2), S * splits, 2) + sizeof(OneShared) + 1024;
-    const int per_sm = static_cast<int>(227 * 1024 / smem);
-    if (shorter >= kGroup * kCons * splits && tiles * S * splits <= (per_sm > 3 ? 3 : per_sm) * sms) break;
-  }
-  Q.splits = splits;
-  Q.tab_bytes = one_table_bytes(most, kCons * splits, 2);
-  return launch_one<1>(Q, dim3(tiles * S * splits), S * splits, st);
+  Q.splits = plan.splits;
+  Q.tab_bytes = plan.tab[1];
+  Q.ring = plan.ring[1];
+  return launch_one<1>(Q, dim3(cdiv(D, 64) * S * plan.splits), S * plan.splits, st);
 }
 
 }  // namespace gemq
