@@ -107,7 +107,7 @@ class _NoHost:
     """Stands in for the native call module when another library was named in the environment (the module is
     linked to the one next to it): every call goes through ctypes."""
 
-    linear = moe_decode = moe_prefill = staticmethod(lambda *a: None)
+    plain = linear = moe_decode = moe_prefill = staticmethod(lambda *a: None)
 
 
 if os.environ.get("GEMQ_B200_LIB"):

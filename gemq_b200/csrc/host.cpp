@@ -7,11 +7,15 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include "../../include/gemq_b200.h"
 
@@ -29,6 +33,22 @@ void* stream_of(const Tensor& x) { return c10::cuda::getCurrentCUDAStream(x.get_
 
 Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType t, const Tensor& like) {
   return at::empty(sizes, at::TensorOptions().dtype(t).device(like.device()));
+}
+
+// plain(*args) -> whether the call is one that nobody but its caller looks at: kernels/_ops.py, plain_call, which asks
+// here first.  A default device is a function mode: False, the Python form tells it from others.
+PyObject* plain(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  const auto& tls = c10::impl::tls_local_dispatch_key_set().included_;
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled() ||
+      tls.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) || torch::jit::tracer::isTracing())
+    Py_RETURN_FALSE;
+  const bool grad = c10::GradMode::is_enabled();
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    if (!THPVariable_Check(a[i])) continue;
+    const Tensor* t = tensor(a[i]);
+    if (!t || (grad && t->requires_grad()) || t->_fw_grad(0).defined()) Py_RETURN_FALSE;
+  }
+  Py_RETURN_TRUE;
 }
 
 // linear(x, w_q, scales, zeros, nbits, group_size, bias | None, err_word_ptr, mode)
@@ -170,6 +190,7 @@ PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
 }
 
 PyMethodDef methods[] = {
+    {"plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<plain>)), METH_FASTCALL, nullptr},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<linear>)), METH_FASTCALL, nullptr},
     {"moe_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<moe_decode>)), METH_FASTCALL, nullptr},
     {"moe_prefill", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<moe_prefill>)), METH_FASTCALL, nullptr},

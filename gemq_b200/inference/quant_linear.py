@@ -28,11 +28,14 @@ class QuantLinear(nn.Module):
 
     def forward(self, x: Tensor) -> Tensor:
         """``x [..., in]`` fp16 / bf16 -> ``[..., out]`` in the same dtype."""
-        if plain_call(x):
-            y = host_linear(x, self.W_q, self.scales, self.zeros, self.W_nbits, self.group_size, self.bias, 0)
+        w_q, scales, zeros, bias = self.W_q, self.scales, self.zeros, self.bias
+        plain = plain_call(x, w_q, scales, zeros, bias)
+        if plain:
+            y = host_linear(x, w_q, scales, zeros, self.W_nbits, self.group_size, bias, 0)
             if y is not None:
                 return y
         lead = x.shape[:-1]
-        y = quant_linear(x.reshape(-1, self.in_features), self.W_q, self.scales, self.zeros, self.W_nbits, self.group_size,
-                         self.bias)
+        y = quant_linear(x.reshape(-1, self.in_features), w_q, scales, zeros, self.W_nbits, self.group_size, bias if plain else None)
+        if bias is not None and not plain:  # the same value; the addition has a gradient, the operator has none
+            y = y + bias.to(y.dtype)
         return y.reshape(*lead, self.out_features)
