@@ -131,24 +131,41 @@ class _QuantFusedMoEBase(nn.Module):
         _BLOCKS[self._handle] = self
 
     # -- forward pieces ----------------------------------------------------------------
+    def _gate_in_place(self) -> bool:
+        """The router's matrix is where and what the library was given: not so after ``.to(dtype)`` and the like, which put
+        another tensor into the parameter.  The call then routes with that one (``_route``)."""
+        w = self.gate.weight
+        return w.data_ptr() == self._layer.gate and w.dtype == torch.float16 and w.is_contiguous()
+
     def _decode(self, x: Tensor, route_mode: int):
         """``x [T, D]`` fp16 -> ``out [T, D]``, routing weights and indices, all on the device."""
         return _moe_decode(x, self._handle, route_mode)
 
     def _host_decode(self, x: Tensor, route_mode: int):
         """The native call, or None where the wrappers have to go on."""
-        if not plain_call(x):
+        if not (plain_call(x) and self._gate_in_place()):
             return None
         return _capi.host.moe_decode(self._layer_ptr, x, self._scratch, self.hidden_dim, self.top_k, route_mode)
+
+    def _host_prefill(self, x: Tensor, route_mode: int, want_logits: bool):
+        """The same for n tokens, ``x`` a plain one: ``(out, logits)`` or None."""
+        if not self._gate_in_place():
+            return None
+        return _capi.host.moe_prefill(self._layer_ptr, x, self._prefill_scratch, self.hidden_dim, self.top_k, self.num_experts,
+                                      route_mode, want_logits)
 
     def _decode_impl(self, x: Tensor, route_mode: int):
         dev = require_cuda(x)
         T = x.shape[0]
         out = torch.empty_like(x)
-        idx = torch.empty((T, self.top_k), dtype=torch.int64, device=dev)
-        w = torch.empty((T, self.top_k), dtype=torch.float16, device=dev)
+        do_route = self._gate_in_place()
+        if do_route:
+            idx = torch.empty((T, self.top_k), dtype=torch.int64, device=dev)
+            w = torch.empty((T, self.top_k), dtype=torch.float16, device=dev)
+        else:
+            w, idx, _ = self._route(x, route_mode, bool(self._layer.renorm))
         _capi.check("gemq_moe_decode", _capi.lib.gemq_moe_decode(
-            C.byref(self._layer), x.data_ptr(), out.data_ptr(), idx.data_ptr(), w.data_ptr(), T, 1, route_mode,
+            C.byref(self._layer), x.data_ptr(), out.data_ptr(), idx.data_ptr(), w.data_ptr(), T, int(do_route), route_mode,
             self._scratch.data_ptr(), self._scratch.numel(), stream_ptr(dev)))
         return out, w, idx
 
@@ -211,6 +228,9 @@ class _QuantFusedMoEBase(nn.Module):
         if routing is not None:
             w, idx = routing[0].contiguous(), routing[1].contiguous()
             logits, do_route = None, 0
+        elif not self._gate_in_place():
+            w, idx, logits = self._route(x, route_mode, renorm)
+            logits, do_route = logits.to(logits_dtype) if logits_dtype is not None else None, 0
         else:
             idx = torch.empty((T, self.top_k), dtype=torch.int64, device=dev)
             w = torch.empty((T, self.top_k), dtype=x.dtype, device=dev)
@@ -310,8 +330,7 @@ class QuantFusedMixtralMoEBlock(_QuantFusedMoEBase):
         x = hidden_states.reshape(-1, d)
         if self._grouped_ok and x.dtype in (torch.float16, torch.bfloat16):
             if plain_call(x):  # the router writes the logits in the activation dtype
-                r = _capi.host.moe_prefill(self._layer_ptr, hidden_states, self._prefill_scratch, self.hidden_dim, self.top_k,
-                                           self.num_experts, ROUTE_FP32_SOFTMAX, True)
+                r = self._host_prefill(hidden_states, ROUTE_FP32_SOFTMAX, True)
                 if r is not None:
                     return r
                 out, _, _, logits = self._prefill_impl(x, ROUTE_FP32_SOFTMAX, True, logits_dtype=x.dtype)
@@ -406,8 +425,7 @@ class QuantFusedDeepseekV2MoEBlock(_QuantFusedMoEBase):
             return out.to(hidden_states.dtype).reshape(b, s, d)
         if grouped:
             if plain_call(x):
-                r = _capi.host.moe_prefill(self._layer_ptr, hidden_states, self._prefill_scratch, self.hidden_dim, self.top_k,
-                                           self.num_experts, ROUTE_FP32, False)
+                r = self._host_prefill(hidden_states, ROUTE_FP32, False)
                 if r is not None:
                     return r[0]
                 out = self._prefill_impl(x, ROUTE_FP32, bool(self.norm_topk_prob), logits_dtype=None)[0]

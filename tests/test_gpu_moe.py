@@ -310,3 +310,29 @@ def test_graph_of_a_batch_survives_a_larger_call(T):
         torch.cuda.synchronize()
     assert torch.equal(out, want)
     assert all(bool((o == 7).all()) for o in others)
+
+
+@pytest.mark.parametrize("family", ["mixtral", "deepseek"])
+@pytest.mark.parametrize("convert", ["bfloat16", "float", "replace"])
+def test_gate_that_was_converted_after_construction(family, convert):
+    """``.to(dtype)`` and the like put another tensor into the gate's parameter: the calls use that one, not the memory
+    the first one had.  Values of the gate are kept by bf16 and fp16 alike, so the results are the same bits."""
+    kw = dict(D=256, Fd=384, E=16, A=6, bits=[1, 2, 3, 4] * 4, seed=4, gate_std=1 / 16.0)
+    layer = MF.make_layer(family, **kw, **({"n_shared": 2} if family == "deepseek" else {}))
+    g = torch.from_numpy(layer["gate"]).to(torch.bfloat16).to(torch.float16)
+    layer["gate"] = torch.where(g.abs() < 2.0 ** -14, torch.zeros_like(g), g).numpy()
+    want, blk = MF.gpu_block(layer), MF.gpu_block(layer)
+    if convert == "replace":
+        blk.gate.weight.data = blk.gate.weight.data.clone()
+    else:
+        getattr(blk, convert)()
+    junk = [torch.full_like(want.gate.weight, 9.0) for _ in range(8)]  # where the first gate may have been
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    for shape in ((1, 1, 256), (4, 1, 256), (1, 300, 256)):
+        for dtype in (torch.float16, torch.bfloat16):
+            x = torch.randn(*shape, device="cuda", generator=gen).to(dtype)
+            with torch.no_grad():
+                a, b = want(x), blk(x)
+            for u, v in zip(*((t if isinstance(t, tuple) else (t,)) for t in (a, b))):
+                assert (u is None and v is None) or (u.dtype == v.dtype and torch.equal(u, v)), (shape, dtype)
+    assert len(junk) == 8 and blk.decode_error_code() == 0
