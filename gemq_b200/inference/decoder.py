@@ -132,7 +132,11 @@ class MixtralDecoder(nn.Module):
         for m in self.modules():
             if isinstance(m, RMSNorm):
                 m.to(device=device, dtype=dtype)
-        self.register_buffer("_inv_freq", inverse_frequencies(cfg.head_dim, cfg.rope_theta, device), persistent=False)
+        self._init_rotary(device)
+
+    def _init_rotary(self, device) -> None:
+        c = self.config
+        self.register_buffer("_inv_freq", inverse_frequencies(c.head_dim, c.rope_theta, device), persistent=False)
 
     @torch.no_grad()
     def forward(self, input_ids: Tensor, past_key_values: StaticCache, cache_position: Tensor) -> Tensor:
@@ -169,8 +173,11 @@ class MixtralDecoder(nn.Module):
             return False
         if not (norm(self.norm) and linear(self.lm_head, c.vocab_size, D)):
             return False
-        for layer, kv in zip(self.layers, cache.layers):
+        for layer in self.layers:
             a = layer.self_attn
+            if not 0 <= a.layer_idx < len(cache.layers):
+                return False
+            kv = cache.layers[a.layer_idx]
             if not (linear(a.q_proj, H * hd, D) and linear(a.k_proj, Hkv * hd, D) and linear(a.v_proj, Hkv * hd, D)
                     and linear(a.o_proj, D, H * hd) and norm(layer.input_layernorm) and norm(layer.post_attention_layernorm)):
                 return False
@@ -198,8 +205,9 @@ class MixtralDecoder(nn.Module):
                 0.0 if norm is None else norm.eps, None if total is None else ptr(total), *w, ptr(out), K, bf, st))
             return out, x if total is None else total
 
-        for layer, kv in zip(self.layers, cache.layers):
+        for layer in self.layers:
             a = layer.self_attn
+            kv = cache.layers[a.layer_idx]
             qkv, x = gemv(layer.input_layernorm, (a.q_proj, a.k_proj, a.v_proj), D, True)
             att = x.new_empty(H * hd)
             _capi.check("gemq_step_attention", lib.gemq_step_attention(

@@ -44,3 +44,30 @@ def test_step_kernels_equal_tensor_operations(hidden, heads, kv_heads, hd, cache
                 assert float((x.double() - y.double()).norm() / y.double().norm()) < 2 * 9 * eps
                 rest = [i for i in range(cache_len) if i != p]
                 assert torch.equal(x[:, :, rest], y[:, :, rest])
+
+
+def test_step_writes_the_cache_of_the_layers_own_index():
+    """A decoder whose first layer was dropped: prefill and step agree on the cache layers, and one layer short of
+    cache is an error in both."""
+    from gemq_b200.inference import MixtralDecoder, StaticCache
+    model = MixtralDecoder(seed=5, hidden_size=256, intermediate_size=512, num_local_experts=4, num_experts_per_tok=2,
+                           num_hidden_layers=3, num_attention_heads=4, num_key_value_heads=2, head_dim=64, vocab_size=96)
+    model.layers = model.layers[1:]
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    prompt, tok, pos = torch.randint(0, 96, (1, 9), device="cuda", generator=gen), torch.tensor([[3]], device="cuda"), \
+        torch.tensor([9], device="cuda")
+    caches = [StaticCache(model.config, 40) for _ in range(2)]
+    for c in caches:
+        model(prompt, c, torch.arange(9, device="cuda"))
+        c.layers[0].lazy_initialization(*(torch.zeros(1, 2, 1, 64, dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+    assert model._step_ok(model.embed_tokens(tok), caches[0], pos)
+    got = model(tok, caches[0], pos).double()
+    model._step_ok = lambda *a: False
+    want = model(tok, caches[1], pos).double()
+    del model._step_ok
+    assert not caches[0].layers[0].keys.any()
+    assert float((got - want).norm() / want.norm()) < 2 * 9 * torch.finfo(torch.bfloat16).eps
+    assert not torch.equal(caches[0].layers[2].keys[:, :, 9], torch.zeros_like(caches[0].layers[2].keys[:, :, 9]))
+    caches[0].layers = caches[0].layers[:2]
+    with pytest.raises(IndexError):
+        model(tok, caches[0], pos)
