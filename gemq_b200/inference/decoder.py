@@ -22,7 +22,8 @@ from torch import Tensor
 from .. import _capi
 from ..kernels._ops import plain_call
 from ..kernels._runtime import stream_ptr
-from .kv_cache import StaticCache
+from .kv_cache import StaticCache, StaticLayer
+from .moe_block import QuantFusedMixtralMoEBlock
 
 MIXTRAL_8X7B_CONFIG = dict(hidden_size=4096, intermediate_size=14336, num_local_experts=8, num_experts_per_tok=2,
                            num_hidden_layers=32, num_attention_heads=32, num_key_value_heads=8, head_dim=128,
@@ -95,6 +96,16 @@ class DecoderLayer(nn.Module):
         return x + y.reshape(B, S, D).to(x.dtype)
 
 
+def _untouched(m: nn.Module, cls) -> bool:
+    """A module of exactly this class whose call is the class's ``forward``: no hooks, no ``forward`` of its own."""
+    return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__
+
+
+def _global_hooks() -> bool:
+    mod = torch.nn.modules.module
+    return bool(mod._global_forward_hooks or mod._global_forward_pre_hooks)
+
+
 class MixtralDecoder(nn.Module):
     """Random-initialised Mixtral-architecture decoder; every MoE block is quantised with mixed
     bits (mean ``mean_bits`` per layer), attention stays in bf16 unless ``attn_bits`` is given
@@ -136,6 +147,7 @@ class MixtralDecoder(nn.Module):
 
     def _init_rotary(self, device) -> None:
         c = self.config
+        self._inv_of = (c.head_dim, c.rope_theta)
         self.register_buffer("_inv_freq", inverse_frequencies(c.head_dim, c.rope_theta, device), persistent=False)
 
     @torch.no_grad()
@@ -150,7 +162,7 @@ class MixtralDecoder(nn.Module):
 
     def _step_ok(self, x: Tensor, cache: StaticCache, pos: Tensor) -> bool:
         """Whether the step kernels take one token of one sequence: an unquantised attention of the standard
-        modules, head sizes and widths the kernels are written for, an initialised cache of x's type."""
+        modules as they come (no hooks, no replaced ``forward``, no autocast), head sizes and widths the kernels are written for, an initialised cache of x's type."""
         c, D = self.config, self.config.hidden_size
         H, Hkv, hd = c.num_attention_heads, c.num_key_value_heads, c.head_dim
         if x.dtype not in (torch.float16, torch.bfloat16) or pos.dtype != torch.int64 or pos.numel() != 1:
@@ -163,19 +175,25 @@ class MixtralDecoder(nn.Module):
                 and t.data_ptr() % 16 == 0
 
         def linear(m, n, k):
-            return type(m) is nn.Linear and m.bias is None and plain(m.weight, (n, k))
+            return _untouched(m, nn.Linear) and m.bias is None and plain(m.weight, (n, k))
 
         def norm(m):
-            return type(m) is RMSNorm and plain(m.weight, (D,))
+            return _untouched(m, RMSNorm) and plain(m.weight, (D,))
 
+        # what is computed without a call of the module must be what the call would compute
+        if _global_hooks() or torch.is_autocast_enabled("cuda") or type(cache) is not StaticCache:
+            return False
         inv = self._inv_freq
-        if inv.dtype != torch.float32 or inv.device != x.device or pos.device != x.device:
+        if inv.dtype != torch.float32 or inv.device != x.device or pos.device != x.device or self._inv_of != (hd, c.rope_theta):
             return False
         if not (norm(self.norm) and linear(self.lm_head, c.vocab_size, D)):
             return False
         for layer in self.layers:
+            if not (_untouched(layer, DecoderLayer) and _untouched(layer.self_attn, Attention) and layer.self_attn.cfg is c
+                    and _untouched(layer.block_sparse_moe, QuantFusedMixtralMoEBlock)):
+                return False
             a = layer.self_attn
-            if not 0 <= a.layer_idx < len(cache.layers):
+            if not 0 <= a.layer_idx < len(cache.layers) or type(cache.layers[a.layer_idx]) is not StaticLayer:
                 return False
             kv = cache.layers[a.layer_idx]
             if not (linear(a.q_proj, H * hd, D) and linear(a.k_proj, Hkv * hd, D) and linear(a.v_proj, Hkv * hd, D)

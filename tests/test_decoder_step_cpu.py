@@ -48,3 +48,56 @@ def test_cache_layers_are_found_by_the_layers_own_index():
     assert ok(m, c)
     c.layers[2].is_initialized = False
     assert not ok(m, c)
+
+
+MODULES = [lambda m: m.layers[1], lambda m: m.layers[1].self_attn, lambda m: m.layers[1].self_attn.q_proj,
+           lambda m: m.layers[1].self_attn.o_proj, lambda m: m.layers[1].input_layernorm,
+           lambda m: m.layers[1].post_attention_layernorm, lambda m: m.layers[1].block_sparse_moe, lambda m: m.norm,
+           lambda m: m.lm_head]
+
+
+@pytest.mark.parametrize("pick", MODULES)
+def test_modules_that_somebody_hooked_are_called(pick):
+    m, c = model(), cache()
+    sub = pick(m)
+    for register in (sub.register_forward_hook, sub.register_forward_pre_hook):
+        handle = register(lambda *a: None)
+        assert not ok(m, c)
+        handle.remove()
+    assert ok(m, c)
+    sub.forward = lambda *a: None  # an instance's own
+    assert not ok(m, c)
+    del sub.forward
+    assert ok(m, c)
+
+
+def test_replaced_modules_settings_and_caches_are_not_the_kernels():
+    m, c = model(), cache()
+
+    class Other(D.Attention):
+        pass
+
+    m.layers[1].self_attn.__class__ = Other
+    assert not ok(m, c)
+    m.layers[1].self_attn.__class__ = D.Attention
+    moe, m.layers[0].block_sparse_moe = m.layers[0].block_sparse_moe, nn.Identity()
+    assert not ok(m, c)
+    m.layers[0].block_sparse_moe = moe
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    assert not ok(m, c)
+    handle.remove()
+    with torch.autocast("cuda", dtype=torch.float16, enabled=True):
+        auto = torch.is_autocast_enabled("cuda")  # not without a device
+        assert ok(m, c) != auto
+    m.config.rope_theta = 1e4  # the tensor operations follow the configuration
+    assert not ok(m, c)
+    m.config.rope_theta = 1e6
+
+    class OtherCache(StaticCache):
+        def update(self, *a):
+            raise NotImplementedError
+
+    c.__class__ = OtherCache
+    assert not ok(m, c)
+    c.__class__ = StaticCache
+    assert ok(m, c) and not ok(m, c, torch.tensor([5, 6])) and not ok(m, c, torch.tensor([5], dtype=torch.int32))

@@ -71,3 +71,24 @@ def test_step_writes_the_cache_of_the_layers_own_index():
     caches[0].layers = caches[0].layers[:2]
     with pytest.raises(IndexError):
         model(tok, caches[0], pos)
+
+
+def test_hooks_see_the_modules_of_a_step():
+    """A hook that changes what a projection returns changes the step, as it does with the tensor operations."""
+    from gemq_b200.inference import MixtralDecoder, StaticCache
+    model = MixtralDecoder(seed=5, hidden_size=256, intermediate_size=512, num_local_experts=4, num_experts_per_tok=2,
+                           num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=64, vocab_size=96)
+    tok, pos = torch.tensor([[3]], device="cuda"), torch.tensor([4], device="cuda")
+    outs = []
+    for hooked, own in ((False, True), (True, True), (True, False)):
+        c = StaticCache(model.config, 40)
+        for layer in c.layers:
+            layer.lazy_initialization(*(torch.zeros(1, 2, 1, 64, dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+        handle = model.layers[1].self_attn.v_proj.register_forward_hook(lambda m, a, y: -y) if hooked else None
+        if not own:
+            model._step_ok = lambda *a: False
+        outs.append(model(tok, c, pos))
+        if hooked:
+            handle.remove()
+    del model._step_ok
+    assert not torch.equal(outs[0], outs[1]) and torch.equal(outs[1], outs[2])
