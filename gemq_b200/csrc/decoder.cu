@@ -225,7 +225,9 @@ __global__ void __launch_bounds__(kAttnThreads) step_attn_kernel(const __grid_co
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   // The position and the cache below it are older than the launch before this one: the first keys and values are
   // on their way, and the angles made, before the wait for the projections.
-  const int pos = static_cast<int>(max(0ll, min(*P.pos, static_cast<long long>(P.L - 1))));
+  const long long at = *P.pos;
+  const int pos = static_cast<int>(max(0ll, min(at, static_cast<long long>(P.L - 1))));
+  const bool inside = at == pos;  // a position outside the cache: nothing is stored, the result is not a number
   const int chunks = pos / kChunk + 1;
   const T* qkv = static_cast<const T*>(P.qkv);
   T* kc = static_cast<T*>(P.keys) + static_cast<size_t>(h) * P.L * HD;
@@ -271,10 +273,15 @@ __global__ void __launch_bounds__(kAttnThreads) step_attn_kernel(const __grid_co
       rotate(k, i, a, b);
       new_k[i] = Num<T>::r(a);
       new_k[i + HD / 2] = Num<T>::r(b);
-      kc[static_cast<size_t>(pos) * HD + i] = Num<T>::r(a);
-      kc[static_cast<size_t>(pos) * HD + i + HD / 2] = Num<T>::r(b);
+      if (inside) {
+        kc[static_cast<size_t>(pos) * HD + i] = Num<T>::r(a);
+        kc[static_cast<size_t>(pos) * HD + i + HD / 2] = Num<T>::r(b);
+      }
     }
-    for (int i = tid; i < HD; i += kAttnThreads) vc[static_cast<size_t>(pos) * HD + i] = new_v[i] = v[i];
+    for (int i = tid; i < HD; i += kAttnThreads) {
+      new_v[i] = v[i];
+      if (inside) vc[static_cast<size_t>(pos) * HD + i] = v[i];
+    }
   }
   float o[kMaxG][4];
 #pragma unroll
@@ -401,7 +408,7 @@ __global__ void __launch_bounds__(kAttnThreads) step_attn_kernel(const __grid_co
       l = fmaf(part_l[r][g], f, l);
       a = fmaf(part_o[r][g][d], f, a);
     }
-    static_cast<T*>(P.out)[static_cast<size_t>(h * G) * HD + i] = Num<T>::r(a / l);
+    static_cast<T*>(P.out)[static_cast<size_t>(h * G) * HD + i] = Num<T>::r(inside ? a / l : __int_as_float(0x7fc00000));
   }
 }
 

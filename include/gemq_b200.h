@@ -302,7 +302,8 @@ int gemq_step_norm(const void* x, const void* res, int res_is_half, const void* 
                    void* out_half, int K, int is_bf16, gemq_stream_t stream);
 
 /* qkv [(heads + 2 * kv_heads) * head_dim]: rotary embedding (half-split, inv_freq fp32 [head_dim / 2]) of queries and
- * key at position pos[0] (device memory, taken as 0 .. cache_len - 1), key and value stored there in keys / values
+ * key at position pos[0] (device memory; outside 0 .. cache_len - 1 nothing is stored and out is NaN), key and value
+ * stored there in keys / values
  * [kv_heads, cache_len, head_dim], then softmax attention over positions 0 .. pos: out [heads * head_dim].
  * pos and the cached positions are read ahead of the wait for the launch before this one, which must not write them.
  * head_dim 64 or 128, heads a multiple of kv_heads, at most 8 times as many. */

@@ -92,3 +92,19 @@ def test_hooks_see_the_modules_of_a_step():
             handle.remove()
     del model._step_ok
     assert not torch.equal(outs[0], outs[1]) and torch.equal(outs[1], outs[2])
+
+
+@pytest.mark.parametrize("position", [-1, 40, 2 ** 40])
+def test_position_outside_the_cache_is_visible(position):
+    """The tensor operations refuse such a position; the step's kernels store nothing and give no numbers."""
+    from gemq_b200.inference import MixtralDecoder, StaticCache
+    model = MixtralDecoder(seed=5, hidden_size=256, intermediate_size=512, num_local_experts=4, num_experts_per_tok=2,
+                           num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=64, vocab_size=96)
+    c = StaticCache(model.config, 40)
+    for layer in c.layers:
+        layer.lazy_initialization(*(torch.zeros(1, 2, 1, 64, dtype=torch.bfloat16, device="cuda") for _ in range(2)))
+    out = model(torch.tensor([[3]], device="cuda"), c, torch.tensor([position], device="cuda"))
+    assert torch.isnan(out).all()
+    assert not any(t.any() for layer in c.layers for t in (layer.keys, layer.values))
+    assert all(layer.block_sparse_moe.decode_error_code() == 0 for layer in model.layers)
+    assert torch.isfinite(model(torch.tensor([[3]], device="cuda"), c, torch.tensor([39], device="cuda"))).all()
