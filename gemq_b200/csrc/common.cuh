@@ -33,6 +33,12 @@ inline int sm_count() {
   return cached[dev];
 }
 
+// For rules that also size buffers: without a device those of a whole B200.
+inline int sm_count_or_default() {
+  const int n = sm_count();
+  return n > 0 ? n : 148;
+}
+
 // Streaming 128-bit load: weights are read once per step, so they should not
 // displace the activation tables or metadata in L1.
 __device__ __forceinline__ uint4 ld_stream_v4(const uint32_t* p) {

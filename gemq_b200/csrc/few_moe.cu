@@ -225,7 +225,6 @@ struct TableParams {
   const int* src;
   const int* nbits;
   int sbits;
-  int tile_rows;
   unsigned char* table;
   size_t tile_stride;
 };
@@ -422,7 +421,7 @@ static int down_splits(const gemq_moe_layer_t* L, int tokens, int tile_rows) {
   const int R = tokens * L->top_k, E = L->n_experts;
   const int tiles = (R < E ? R : E) + (L->shared_ffn ? cdiv(tokens, tile_rows) : 0);
   const int kmax = L->ffn > L->shared_ffn ? L->ffn : L->shared_ffn;
-  const int want = 6 * 148 / (cdiv(L->hidden, 64 * kCons) * tiles);
+  const int want = 6 * sm_count_or_default() / (cdiv(L->hidden, 64 * kCons) * tiles);
   const int most = kmax / 512;  // a part keeps at least 512 of the reduction
   int s = want < 1 ? 1 : want;
   s = s > most ? most : s;
@@ -547,7 +546,6 @@ int moe_few_rows(const gemq_moe_layer_t* L, const void* x, void* out, const long
   T.x = x; T.K = D;
   T.tiles = Y.plan.tiles; T.n_tiles = Y.plan.n_tiles; T.src = Y.plan.src;
   T.nbits = L->w1.nbits; T.sbits = L->s1.nbits;
-  T.tile_rows = Y.tile_rows;
   T.table = Y.tabx; T.tile_stride = Y.stride_x;
   const dim3 tgrid(Y.tile_rows, Y.max_tiles);
   ok = bf16 ? launch(few_table_kernel<__nv_bfloat16>, tgrid, kTabThreads, static_cast<size_t>(D) * 2, st, T)

@@ -328,10 +328,10 @@ static cudaError_t launch_many(const RouteArgs& R) {
 
 template <typename T, typename G>
 static cudaError_t launch_route_any(const RouteArgs& R) {
-  // The many-token kernel is flat up to 148 * 16 tokens (7 to 9 us); one token per CTA is faster while its CTAs are one
+  // The many-token kernel is flat up to 16 tokens per SM (7 to 9 us); one token per CTA is faster while its CTAs are one
   // round: two per SM for 16 warps (64 experts: 301 tokens 11.6 against 8.5 us, 200 tokens 8.3 against 8.4), four below
   // (8 experts: 509 tokens 6.3 against 7.0, 767 tokens 8.3 against 7.2).
-  const int round = 148 * (R.E > 32 ? 2 : 4);
+  const int round = sm_count_or_default() * (R.E > 32 ? 2 : 4);
   const bool many = R.tokens > round && R.E <= 64 && R.D % (32 * kRouteWarps) == 0 &&
                     ((reinterpret_cast<uintptr_t>(R.x) | reinterpret_cast<uintptr_t>(R.gate)) & 15u) == 0;
   if (many)
