@@ -114,7 +114,11 @@ if os.environ.get("GEMQ_B200_LIB"):
     host = _NoHost
 else:
     import torch  # noqa: F401  (its libraries have to be loaded first)
-    from . import _host as host  # noqa: F401
+    try:
+        from . import _host as host  # noqa: F401
+    except ImportError as e:
+        raise ImportError(f"gemq_b200/_host.so is missing or was built against another torch than {torch.__version__} ({e}).  "
+                          "Build it with `python -m gemq_b200.csrc.build`.") from e
 
 
 def stacked(wq, scales, zeros, nbits, wq_strides, zs_strides=None) -> Stacked:

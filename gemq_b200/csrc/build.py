@@ -4,7 +4,7 @@ host-side call module _host.so from host.cpp with g++ against torch's headers.
     python -m gemq_b200.csrc.build [--verbose]
 
 Both land next to the Python package (gemq_b200/).  They are
-rebuilt only when a source or header is newer than the library.
+rebuilt only when a source or header is newer than the library, _host.so also when torch is another one.
 """
 import os
 import shutil
@@ -29,9 +29,21 @@ def find_nvcc() -> str:
     return nvcc
 
 
+# the torch that _host.so was built against: its C++ interface changes with the version
+HOST_STAMP = os.path.join(HERE, "build", "host.torch")
+
+
+def torch_build() -> str:
+    import torch
+    return f"{torch.__version__} {torch.version.git_version} {sys.version_info[:2]}"
+
+
 def host_stale() -> bool:
-    if not os.path.exists(HOST_LIB):
+    if not os.path.exists(HOST_LIB) or not os.path.exists(HOST_STAMP):
         return True
+    with open(HOST_STAMP) as f:
+        if f.read() != torch_build():
+            return True
     t = os.path.getmtime(HOST_LIB)
     return any(os.path.getmtime(d) > t for d in (os.path.join(HERE, "host.cpp"), HEADERS[-1], os.path.abspath(__file__)))
 
@@ -47,6 +59,9 @@ def build_host() -> None:
     subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
                            *inc, f"-I{cuda}", os.path.join(HERE, "host.cpp"), "-o", HOST_LIB, f"-L{libs}", "-ltorch_python",
                            "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-L{PKG}", "-l:libgemq_b200.so", "-Wl,-rpath,$ORIGIN"])
+    os.makedirs(os.path.dirname(HOST_STAMP), exist_ok=True)
+    with open(HOST_STAMP, "w") as f:
+        f.write(torch_build())
 
 
 def is_stale() -> bool:
