@@ -108,3 +108,45 @@ def test_position_outside_the_cache_is_visible(position):
     assert not any(t.any() for layer in c.layers for t in (layer.keys, layer.values))
     assert all(layer.block_sparse_moe.decode_error_code() == 0 for layer in model.layers)
     assert torch.isfinite(model(torch.tensor([[3]], device="cuda"), c, torch.tensor([39], device="cuda"))).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,kv_heads,hd,cache_len,positions", [
+    (4, 2, 64, 40, (0, 1, 31, 39)),                   # shorter than one piece of the attention
+    (4, 4, 128, 1100, (63, 64, 511, 512, 1099)),      # one query head a key head; edges of a piece and of a round
+    (6, 2, 128, 600, (0, 65, 448, 599)),              # three of four query heads
+    (16, 2, 64, 600, (64, 599)),                      # eight query heads a key head
+    (32, 8, 128, 700, (575, 576, 640)),
+])
+def test_step_attention_against_fp64(heads, kv_heads, hd, cache_len, positions, dtype):
+    """The attention by itself: one position left out of 600 changes it by 4 %, the bound is one rounding."""
+    from gemq_b200 import _capi
+    from gemq_b200.inference.decoder import inverse_frequencies
+    from gemq_b200.kernels._runtime import stream_ptr
+    gen = torch.Generator(device="cuda").manual_seed(heads * cache_len)
+    inv, G = inverse_frequencies(hd, 1e6, "cuda"), heads // kv_heads
+    eps = torch.finfo(dtype).eps
+    for p in positions:
+        qkv = torch.randn((heads + 2 * kv_heads) * hd, device="cuda", generator=gen).to(dtype)
+        keys, values = (torch.randn(kv_heads, cache_len, hd, device="cuda", generator=gen).to(dtype) for _ in range(2))
+        k2, v2, out = keys.clone(), values.clone(), qkv.new_empty(heads * hd)
+        pos = torch.tensor([p], device="cuda")
+        assert _capi.lib.gemq_step_attention(qkv.data_ptr(), inv.data_ptr(), pos.data_ptr(), k2.data_ptr(), v2.data_ptr(), out.data_ptr(),
+                                             heads, kv_heads, hd, cache_len, int(dtype == torch.bfloat16), stream_ptr(out.device)) == 0
+        q, k, v = qkv.double().view(-1, hd).split([heads, kv_heads, kv_heads])
+        ang = (float(p) * inv).double()  # an fp32 product, like the kernel's
+        cos, sin = torch.cat([ang.cos()] * 2), torch.cat([ang.sin()] * 2)
+        rot = lambda t: (t * cos + torch.cat([-t[:, hd // 2:], t[:, :hd // 2]], 1) * sin).to(dtype).double()
+        q, k = rot(q), rot(k)
+        # stored: the value itself, the rotated key up to a rounding that falls to the other side
+        assert torch.equal(v2[:, p].double(), v) and ((k2[:, p].double() - k).abs() <= eps * k.abs() + 2.0 ** -20).all()
+        rest = [i for i in range(cache_len) if i != p]
+        assert torch.equal(k2[:, rest], keys[:, rest]) and torch.equal(v2[:, rest], values[:, rest])
+        K, V = k2[:, :p + 1].double().repeat_interleave(G, 0), v2[:, :p + 1].double().repeat_interleave(G, 0)
+        s = (K @ q[:, :, None])[:, :, 0] * hd ** -0.5
+        want = (s.softmax(1)[:, None] @ V)[:, 0]
+        # the output's rounding is at most eps / 2 of each value.  A rotated query element that was rounded to the other
+        # side (one in some thousands) moves its head's scores by eps / sqrt(hd) of a product of order one; fp32 sums and
+        # the fast exponential are below 2^-12.
+        err = (out.double().view(heads, hd) - want).norm(dim=1) / want.norm(dim=1)
+        assert float(err.max()) < 0.5 * eps + 2.0 ** -12 + eps * hd ** -0.5, (p, err.max())

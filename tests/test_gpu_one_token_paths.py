@@ -55,3 +55,43 @@ def test_layer_at_the_limit_of_shared_memory(hidden, ffn, top_k, n_shared):
     got = out.view(1, -1).float().cpu().numpy()
     assert rel_fro(got, ref) < REL_FRO_TOL, rel_fro(got, ref)
     assert max_abs(got, ref) < f16_abs_bound(ref)
+
+
+@pytest.mark.parametrize("D,Fd,SF,A,E", [
+    (128, 128, 0, 1, 2),       # one slot; fewer stages than warps
+    (256, 384, 0, 2, 4),
+    (640, 256, 128, 1, 3),     # the shared expert is the shorter one; 3-bit runs that end inside a stage
+    (384, 256, 896, 2, 5),     # ... the longer one
+    (256, 1408, 512, 6, 40),   # seven slots: one part each
+    (512, 384, 384, 7, 9),     # eight slots
+    (256, 2048, 0, 8, 8),
+    (2048, 1024, 0, 2, 44),
+])
+@pytest.mark.parametrize("shared_bits", [3, 4])
+def test_few_row_launches_at_their_edges(D, Fd, SF, A, E, shared_bits):
+    """Slots, cluster sizes and reduction lengths of the one-token few-row launches, routed and shared."""
+    import numpy as np
+    import moe_fixtures as MF
+    from oracle import gemq_oracle as O
+    if not SF and shared_bits == 4:
+        pytest.skip("no shared expert")
+    bits = [(3, 1, 4, 2)[e % 4] for e in range(E)]
+    layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=E, A=A, bits=bits, seed=D + Fd + A, gate_std=0.1)
+    mode = 0
+    if SF:
+        rng = np.random.default_rng(SF)
+        layer["shared"] = (MF.draw_linear(rng, SF, D, shared_bits), MF.draw_linear(rng, D, SF, shared_bits),
+                           MF.draw_linear(rng, SF, D, shared_bits))
+        c = layer["cfg"]
+        c.moe_intermediate_size, c.n_routed_experts, c.n_shared_experts, c.norm_topk_prob = Fd, E, 1, False
+        layer["family"], mode = "deepseek", 2
+    blk = MF.gpu_block(layer)
+    w1, w3, w2, sh = MF.oracle_parts(layer)
+    x = torch.randn(3, D, generator=torch.Generator().manual_seed(A)).half()
+    for t in range(3):
+        out = blk(x[t].cuda().view(1, 1, -1))
+        out = (out[0] if isinstance(out, tuple) else out).view(1, -1)
+        assert blk.decode_error_code() == 0
+        _, gw, gi = blk._decode(x[t:t + 1].cuda(), mode)
+        ref = np.asarray(O.moe_reference_fp32(x[t:t + 1], gw.float().cpu(), gi.cpu(), w1, w3, w2, *([sh] if sh else [])), dtype=np.float32)
+        assert rel_fro(out.float().cpu().numpy(), ref) < REL_FRO_TOL
