@@ -5,8 +5,8 @@
 // Here it is four launches:
 //   step_gemv   [x + residual -> RMSNorm ->] one or more unquantised matrices times the vector.  Bound by the
 //               weights' bytes: a warp takes a row, all its loads in flight at once; the first row is on its way
-//               before the wait for the previous kernel, so the normalisation (which every CTA repeats: 8 KB out
-//               of L2) hides behind it
+//               before the wait for the previous kernel (which must not write it), so the normalisation (which every
+//               CTA repeats: 8 KB out of L2) hides behind it
 //   step_attn   rotary embedding, cache update and attention over the cached positions; a cluster of eight CTAs
 //               per key / value head splits the positions and merges in the first CTA's shared memory
 //   step_norm   x + residual -> RMSNorm, as the fp16 vector the MoE block takes
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) step_gemv_kernel(const __grid
     }
   };
   At cur = {first, 0}, ahead = {first, 0};
-  fill(va, ahead);  // weights are nobody's result
+  fill(va, ahead);  // the matrices are older than the launch before (in the decoder: than the embedding)
   next(ahead);
   fill(vb, ahead);
   next(ahead);

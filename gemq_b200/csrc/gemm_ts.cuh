@@ -605,8 +605,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
   const uint32_t tmem = S.tmem_base;
   // Only now: a CTA of the next kernel must not take this SM's tensor memory first.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // Everything may be a result of the launch before, a linear's packed words, too (a layer packed and called at once).
-  // Bringing its first words into L2 ahead of this wait gains nothing (1000 rows, 4096 x 4096, 4 bits: 36.6 and 36.7 us).
+  // Everything may be a result of the launch before, a linear's packed words, too (a layer packed and called at once): no
+  // early look at them.  It would gain where linears follow one another with nothing in between (4096 x 1024, 2 bits,
+  // 64 rows: 7.9 instead of 9.9 us; 1000 rows of 4096 x 4096, 4 bits: 30.5 instead of 31.6), behind any other kernel nothing.
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // Tiles go to the pairs back and forth: the list is sorted by falling time, so who got a long one in a round gets

@@ -25,7 +25,7 @@ from ..kernels._runtime import require_cuda, stream_ptr
 from .packed_linear import is_packed_linear
 
 ROUTE_FP16, ROUTE_FP32_SOFTMAX, ROUTE_FP32 = 0, 1, 2
-# Decode batches up to this many rows run the one-launch layer kernel row by row; larger ones go through the
+# Decode batches up to this many rows run the one-token kernels row by row; larger ones go through the
 # expert-sorted kernels, which read every distinct expert (and the shared experts) once per call: two rows of the
 # DeepSeek-V2-Lite shape take 61 us there, 84 in the loop.
 _MAX_LOOPED_TOKENS = 1
@@ -411,8 +411,8 @@ class QuantFusedDeepseekV2MoEBlock(_QuantFusedMoEBase):
         return dequant_gemm(F.silu(x1) * x3, self.shared_w2_wq, self.shared_w2_scales, self.shared_w2_zeros, b, g)
 
     def forward_n_tokens(self, hidden_states: Tensor) -> Tensor:
-        """gemq/inference/moe_block.py:448-486.  A handful of rows (decode batches) run the
-        fused one-token kernels row by row with this path's fp32 routing."""
+        """gemq/inference/moe_block.py:448-486.  One row, and up to 16 of a layer the expert-sorted kernels do not take,
+        run the one-token kernels row by row with this path's fp32 routing."""
         b, s, d = hidden_states.shape
         x = hidden_states.reshape(-1, d)
         grouped = self._grouped_ok and x.dtype in (torch.float16, torch.bfloat16)

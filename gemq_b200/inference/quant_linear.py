@@ -2,8 +2,8 @@
 
 The reference quantises attention and dense-MLP linears to 4 bits (``--attn_wbits 4
 --dense_wbits 4``, gemq/quantize.py:333-343) and runs them with gemlite's kernels
-(gemq/inference/patch.py:71-79).  The same packed format goes through this library's GEMV
-(a few rows) and tcgen05 GEMM (32 rows or more) entry points, any bit width from 1 to 4.
+(gemq/inference/patch.py:71-79).  The same packed format goes through this library's few-row
+kernel or its tcgen05 GEMM, whichever is estimated the faster for the rows, any bit width from 1 to 4.
 """
 from __future__ import annotations
 

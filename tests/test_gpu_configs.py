@@ -154,8 +154,9 @@ def test_mixtral_prefill_bf16_small():
 def test_decode_three_bit_run_remainders(D, Fd, bits):
     """One-token layer with 3-bit experts whose reduction lengths leave every remainder of groups
     in the last 5-group run (10 and 5 groups: none; 6 and 15: one and none; 4 and 3), and packed rows that
-    end inside a 16-row quad: the integer 3-bit path masks rows that straddle two groups and zero-fills
-    rows past the end of the matrix."""
+    end inside 16 rows (a stage of the few-row launches, a quad of the one launch, which
+    test_gpu_one_token_paths.py runs this on, too): words that straddle two groups are masked, rows past the end of the
+    matrix come as zeros."""
     layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=4, A=2, bits=bits, seed=21, gate_std=0.02)
     blk = MF.gpu_block(layer)
     w1, w3, w2, _ = MF.oracle_parts(layer)
@@ -174,8 +175,8 @@ def test_decode_three_bit_run_remainders(D, Fd, bits):
 
 
 def test_decode_layer_is_bit_reproducible_over_many_graph_replays():
-    """The cross-CTA sums of the one-launch decode layer are formed in a fixed order whichever
-    CTA completes a chunk: 60 replays of each of six captured layer calls (Mixtral config-1 shape
+    """The cross-CTA sums of a decode layer are formed in a fixed order, in the one launch whichever
+    CTA completes a chunk (the DeepSeek layers: clusters of the few-row launches): 60 replays of each of six captured layer calls (Mixtral config-1 shape
     and DeepSeek config-2 shape) give bit-identical outputs, and no wait runs out."""
     from gemq_b200 import synth
     dev = torch.device("cuda")
@@ -241,8 +242,8 @@ def _set_word(blk, fn, value):
 
 
 def test_decode_wait_limit_expires_and_is_reported():
-    """A wait limit of one poll makes the bounded waits of the layer kernel run out: the launch
-    still returns, the error word says so, and after the scratch is reset the layer is correct again."""
+    """A wait limit of one poll makes the bounded waits of a layer's launches run out: they
+    still return, the error word says so, and after the scratch is reset the layer is correct again."""
     from gemq_b200 import _capi
     layer = MF.make_layer("mixtral", D=512, Fd=1024, E=4, A=2, bits=[1, 2, 3, 4], seed=31, gate_std=0.02)
     blk = MF.gpu_block(layer)
