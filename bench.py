@@ -33,8 +33,8 @@ LAYER_SEED0 = 100
 # DRAM bytes (read + write) of one launch of the decode layer kernel over its algorithmic bytes,
 # from an ncu capture of three launches (1.038, 1.035, 1.012); applied to the bench's own average bytes per launch.
 DECODE_TRAFFIC_RATIO = 1.03
-# DRAM bytes of one prefill call at N = 1 (gate/up launch + down launch), from an ncu capture.
-PREFILL_TRAFFIC_BYTES = 497.4e6 + 218.5e6 + 464.7e6 + 55.2e6
+# DRAM bytes of one prefill call at N = 1 (gate/up launch + down launch, read and written), from an ncu capture.
+PREFILL_TRAFFIC_BYTES = 628.8e6 + 220.3e6 + 603.1e6 + 95.4e6
 MIN_TIMED_SECONDS = 0.5
 
 
