@@ -471,15 +471,37 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-template <int OUT, typename T>
-__device__ __forceinline__ void drain(Smem& S, uint32_t at, int rows, int column) {
-  unsigned char* dst = S.out + 2 * column;
+// 16 tokens of 16 lanes: two mma fragments (a thread has two neighbouring tokens of lanes l / 4 and l / 4 + 8) of 8 tokens each.
+__device__ __forceinline__ void tmem_ld_fragments(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+template <typename T>
+__device__ __forceinline__ uint32_t pack_act(uint32_t lo, uint32_t hi) {
+  const T v[2] = {as_act<T>(__uint_as_float(lo)), as_act<T>(__uint_as_float(hi))};
+  return *reinterpret_cast<const uint32_t*>(v);
+}
+
+// The accumulators of a warp's 32 weight columns, rounded, to rows of tokens in shared memory.  What the MMAs of the next
+// tile wait for, so few instructions: fragments whose 8 x 8 blocks stmatrix transposes, per 16 tokens two loads, eight
+// conversions, two stores (a column's values one by one took 16 stores of two bytes).
+template <typename T>
+__device__ __forceinline__ void drain(Smem& S, uint32_t at, int rows, int lq, int lane) {
+  uint32_t dst = smem_u32(S.out) + (8 * (lane >> 4) + (lane & 7)) * kOutPitch + 2 * (32 * lq + 8 * ((lane >> 3) & 1));
 #pragma unroll 1
-  for (int c = 0; c < rows; c += 16) {
-    uint32_t d[16];
-    tmem_ld16(at + c, d);
+  for (int c = 0; c < rows; c += 16, dst += 16 * kOutPitch) {
+    uint32_t d[2][8];
+    tmem_ld_fragments(at + c, d[0]);
+    tmem_ld_fragments(at + (16u << 16) + c, d[1]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 16; ++i) *reinterpret_cast<T*>(dst + (c + i) * kOutPitch) = as_act<T>(__uint_as_float(d[i]));
+    for (int h = 0; h < 2; ++h)
+      asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst + 32 * h),
+                   "r"(pack_act<T>(d[h][0], d[h][1])), "r"(pack_act<T>(d[h][2], d[h][3])), "r"(pack_act<T>(d[h][4], d[h][5])),
+                   "r"(pack_act<T>(d[h][6], d[h][7]))
+                   : "memory");
   }
 }
 
@@ -687,7 +709,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const uint32_t at = tmem + (static_cast<uint32_t>(32 * lq) << 16) + t.acc(j);
       const int column = 32 * lq + static_cast<int>(threadIdx.x & 31);
       if (OUT == kOutPartial) drain_partial(P, t, at, t.col0 + column);
-      else drain<OUT, T>(S, at, t.rows, column);
+      else drain<T>(S, at, t.rows, lq, static_cast<int>(threadIdx.x & 31));
       tc_fence_before_sync();
       __syncwarp();
       if ((threadIdx.x & 31) == 0) arrive_at(first_cta(&S.drained[j & 1]));  // a later tile's MMAs may overwrite them
