@@ -41,6 +41,14 @@ bool activation_maps(CUtensorMap (&maps)[4], const void* x, int K, long long row
   return true;
 }
 
+bool word_maps(CUtensorMap (&maps)[4], const void* wq, const void* scales, const void* zeros, int N, long long rows, int G, int bits,
+               int columns) {
+  if (!aligned16(wq) || !aligned16(scales) || !aligned16(zeros) || rows <= 0 || G % kStageK) return false;
+  for (int b = 1; b <= 4; ++b)
+    if ((!bits || b == bits) && !tensor_map_2d(&maps[b - 1], wq, 4, N, rows, columns, stage_rows(b), false)) return false;
+  return true;
+}
+
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream) { return launch<kOutUp, false>(P, tiles_bound, stream); }
 int launch_down(const Params& P, int tiles_bound, cudaStream_t stream) { return launch<kOutDown, false>(P, tiles_bound, stream); }
 
@@ -139,6 +147,8 @@ extern "C" int gemq_linear_gemm(const void* x, const int64_t* expert, const int3
   F.N = N; F.K = K; F.G = group_size;
   F.out = y;
   P.expert = reinterpret_cast<const long long*>(expert);
+  P.staged = !expert && !nbits && !wq_strides && !zs_strides &&
+             word_maps(P.w_map[0][0], wq, scales, zeros, N, fixed_bits == 3 ? cdiv(K, 10) : K * fixed_bits / 32, group_size, fixed_bits, kCols);
   P.rows = M;
   P.bias = bias;
   P.err = err;

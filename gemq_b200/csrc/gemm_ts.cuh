@@ -81,6 +81,8 @@ struct Family {
 };
 
 struct alignas(64) Params {
+  // packed words per family, matrix and bit width (linear: [0][0][0]): boxes of a CTA's columns x the rows of 128 k
+  CUtensorMap w_map[2][2][4];
   // activations per family as (64 k, rows, K / 64): boxes of 32, 64, 96, 128 rows x 128 k, 128B swizzle
   CUtensorMap b_map[2][4];
   Family fam[2];
@@ -94,12 +96,21 @@ struct alignas(64) Params {
   const __half* row_w;     // down: routing weight per sorted row
   const void* bias;        // linear
   int* err;
+  int staged;              // tiles of up to kStagedTokens: the words come through shared memory
 };
+
+// A stage of a tile of up to 192 tokens leaves a quarter of its shared memory free: there the TMA warp puts the stage's
+// packed words, up to three stages ahead of the producers.
+constexpr int kStagedTokens = 192, kWordsAt = kStagedTokens / 2 * 2 * kRowBytes;
+static_assert(kWordsAt + 16 * kCols * 4 <= kStageBytes, "128 k of 4 bits");
+// Packed rows of 128 k; 3-bit rows from the one in which the first code lies.
+__host__ __device__ constexpr int stage_rows(int bits) { return bits == 3 ? 14 : 4 * bits; }
 
 struct Smem {
   alignas(1024) unsigned char b[kStages][kStageBytes];
   alignas(16) unsigned char out[kTokens * kOutPitch];  // accumulators rounded to 16 bits
-  alignas(8) unsigned long long full[kStages], empty[kStages], acc_full[2], drained[2];  // [2]: by the tile's parity
+  alignas(16) unsigned char scales[kStages][kCols * 4];  // of the stage's group: [matrix][scales, offsets][columns]
+  alignas(8) unsigned long long full[kStages], empty[kStages], words[kStages], acc_full[2], drained[2];  // [2]: by the tile's parity
   uint32_t tmem_base;
 };
 
@@ -323,11 +334,64 @@ __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Til
   return true;
 }
 
+__device__ __forceinline__ int tile_bits(const Params& P, const Tile& t) {
+  const Family& F = P.fam[t.fam];
+  return F.nbits && t.expert >= 0 ? F.nbits[t.expert] : F.bits;
+}
+
+// Words, scales and offsets of a tile, as its CTA's TMA warp brings them into the stages.
+template <bool UP>
+struct TileWords {
+  const CUtensorMap* map[2];
+  const __half* scales[4];  // of the CTA's first column: [matrix][scales, offsets]
+  int bits, row0, col, bytes;
+  uint32_t all, parts;      // bytes of a stage; of a row of scales
+  size_t N;
+  int G;
+  __device__ __forceinline__ void init(const Params& P, const Tile& t) {
+    const Family& F = P.fam[t.fam];
+    bits = tile_bits(P, t);
+    N = F.N;
+    G = F.G;
+    col = t.col0;
+    const bool stacked = t.expert >= 0 && F.wq_strides;
+    row0 = stacked ? static_cast<int>(static_cast<unsigned>(F.wq_strides[t.expert]) / static_cast<unsigned>(F.N)) : 0;
+    const int columns = UP ? kCols / 2 : kCols;
+    const int valid = min(max(F.N - col, 0), columns);
+    parts = 2 * valid;
+#pragma unroll
+    for (int m = 0; m < (UP ? 2 : 1); ++m) {
+      map[m] = &P.w_map[t.fam][m][bits - 1];
+      size_t off = col;
+      if (t.expert >= 0) off += F.zs_strides[m] ? static_cast<size_t>(F.zs_strides[m][t.expert]) : static_cast<size_t>(t.expert) * (F.K / F.G) * N;
+      scales[2 * m] = F.scales[m] + off;
+      scales[2 * m + 1] = F.zeros[m] + off;
+    }
+    all = (UP ? 2 : 1) * (stage_rows(bits) * columns * 4 + 2 * parts);
+  }
+  __device__ __forceinline__ void load(unsigned char* stage, unsigned char* sc, unsigned long long* bar, int kb) const {
+    const int k0 = kb * kBK, row = row0 + (bits == 3 ? k0 / 10 : k0 * bits / 32), g = k0 / G;
+    mbar_arrive_expect_tx(bar, all);
+#pragma unroll
+    for (int m = 0; m < (UP ? 2 : 1); ++m) {
+      tma_load_2d(stage + kWordsAt + m * stage_rows(bits) * kCols * 2, map[m], col, row, bar);
+#pragma unroll
+      for (int z = 0; z < 2; ++z)
+        if (parts)
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           smem_u32(sc + m * 256 + z * (UP ? kCols : 2 * kCols))),
+                       "l"(scales[2 * m + z] + static_cast<size_t>(g) * N), "r"(parts), "r"(smem_u32(bar))
+                       : "memory");
+    }
+  }
+};
+
 // ---- producer ------------------------------------------------------------------------------------
 // All k-blocks of a tile; `base` = k-blocks this CTA has handled before the tile (even).  An odd number of
 // blocks is followed by one of zeros: the activations of its stage end in zeros, too.
 // (Out of line: inlined, the 88 registers of 22 warps spill in the k loop.)
-template <bool UP, bool BF16, bool NAT, int B>
+// STAGED: packed words, scales and offsets lie in the stage.
+template <bool UP, bool BF16, bool NAT, int B, bool STAGED>
 __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
   constexpr int NW = B == 3 ? 8 : 2 * B;  // words of a 64-code window
   const Family& F = P.fam[T.fam];
@@ -356,7 +420,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   kb += T.kb0;
   if (kb >= kb1) return;
   struct Set { uint32_t w[NW]; __half s, z; };
-  Set ring[2];
+  Set ring[STAGED ? 1 : 2];
   const Exps<B> X;
   if (B != 3) wp += static_cast<size_t>(kb) * (2 * B) * N;
   auto fetch = [&](Set& R, int k) {  // blocks in order
@@ -389,6 +453,29 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   uint32_t s = c % kStages, par = ((c / kStages) & 1) ^ 1;
   const uint32_t full0 = first_cta(&S.full[0]);
   const uint32_t dst0 = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemA + ((base + kb) & 1) * 32;
+  // STAGED
+  constexpr uint32_t kPitch = UP ? kCols * 2 : kCols * 4;
+  const int in_row = UP ? 16 * (warp & 3) + (lane & 15) : 32 * (warp & 3) + lane;
+  const uint32_t words0 = smem_u32(S.b[0]) + kWordsAt + mi * stage_rows(B) * kPitch + 4 * in_row;
+  const uint32_t scales0 = smem_u32(S.scales[0]) + mi * 256 + 2 * in_row;
+  auto take = [&](Set& R) {
+    if (kb >= real) {
+#pragma unroll
+      for (int i = 0; i < NW; ++i) R.w[i] = 0u;
+      R.s = R.z = __float2half_rn(0.f);
+      return;
+    }
+    mbar_sleep_wait(&S.words[s], par ^ 1u, err, kErrFull);
+    const int row = B == 3 ? kb * kBK / 10 - (kb & ~1) * kBK / 10 : (kb & 1) * 2 * B;
+    const uint32_t w = words0 + s * kStageBytes + row * kPitch, sc = scales0 + s * (kCols * 4);
+#pragma unroll
+    for (int i = 0; i < NW; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(R.w[i]) : "r"(w + i * kPitch) : "memory");
+    unsigned short a, b;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(a) : "r"(sc) : "memory");
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(sc + kPitch / 2) : "memory");
+    R.s = __ushort_as_half(a);
+    R.z = __ushort_as_half(b);
+  };
   auto put = [&](const Set& cur) {
     const __half2 s2 = __half2half2(cur.s), z2 = __half2half2(cur.z);
     const uint32_t dst = dst0 + s * 64;
@@ -421,10 +508,19 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
     s += kGroups / 2;
     if (s >= kStages) { s -= kStages; par ^= 1u; }
   };
+  if constexpr (STAGED) {
+#pragma unroll 1
+    for (; kb < kb1; kb += kGroups) {
+      take(ring[0]);
+      put(ring[0]);
+    }
+    return;
+  }
   fetch(ring[0], kb);
 #pragma unroll 1
   for (;;) {
-    if constexpr (B == 3) {  // one copy of the long body, the sets are moved
+    if constexpr (STAGED) {
+    } else if constexpr (B == 3) {  // one copy of the long body, the sets are moved
       if (kb + kGroups < kb1) fetch(ring[1], kb + kGroups);
       put(ring[0]);
       kb += kGroups;
@@ -442,14 +538,18 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   }
 }
 
+template <bool UP, bool BF16, bool NAT, bool STAGED>
+__device__ __forceinline__ void produce_bits(Smem& S, const Params& P, const Tile& T, int bits, uint32_t base, uint32_t tmem) {
+  if (bits == 1) produce<UP, BF16, NAT, 1, STAGED>(S, P, T, base, tmem);
+  else if (bits == 2) produce<UP, BF16, NAT, 2, STAGED>(S, P, T, base, tmem);
+  else if (bits == 3) produce<UP, BF16, NAT, 3, STAGED>(S, P, T, base, tmem);
+  else produce<UP, BF16, NAT, 4, STAGED>(S, P, T, base, tmem);
+}
 template <bool UP, bool BF16, bool NAT>
 __device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
-  const Family& F = P.fam[T.fam];
-  const int bits = F.nbits && T.expert >= 0 ? F.nbits[T.expert] : F.bits;
-  if (bits == 1) produce<UP, BF16, NAT, 1>(S, P, T, base, tmem);
-  else if (bits == 2) produce<UP, BF16, NAT, 2>(S, P, T, base, tmem);
-  else if (bits == 3) produce<UP, BF16, NAT, 3>(S, P, T, base, tmem);
-  else produce<UP, BF16, NAT, 4>(S, P, T, base, tmem);
+  const int bits = tile_bits(P, T);
+  if (P.staged && T.rows <= kStagedTokens) produce_bits<UP, BF16, NAT, true>(S, P, T, bits, base, tmem);
+  else produce_bits<UP, BF16, NAT, false>(S, P, T, bits, base, tmem);
 }
 
 // ---- epilogue --------------------------------------------------------------------------------------
@@ -612,6 +712,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&S.full[s], 17);  // in the first CTA: two groups' warps of either CTA, the activation boxes
       mbar_init(&S.empty[s], 1);
+      mbar_init(&S.words[s], 1);
     }
     for (int j = 0; j < 2; ++j) {
       mbar_init(&S.acc_full[j], 1);
@@ -655,11 +756,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const uint32_t bytes = 2 * 32 * box * kRowBytes;
       const int row = t.row0 - F.row0 + rank * half;
       const CUtensorMap* const map = &P.b_map[t.fam][box - 1];
+      const bool staged = P.staged && t.rows <= kStagedTokens;
+      TileWords<UP> words;
+      if (staged) words.init(P, t);
       for (int sb = 0; sb < SB; ++sb, ++c) {
         const uint32_t s = c % kStages;
         mbar_sleep_wait(&S.empty[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&S.full[s], 2 * bytes);
+          if (staged) words.load(S.b[s], S.scales[s], &S.words[s], t.kb0 + 2 * sb);
+          else mbar_arrive(&S.words[s]);  // the barrier's phases follow the stages
           tma_load_pair(S.b[s], map, row, t.kb0 + 2 * sb, full0 + s * 8);
         }
         __syncwarp();
@@ -739,6 +845,10 @@ LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split);
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream);
 int launch_down(const Params& P, int tiles_bound, cudaStream_t stream);
 bool activation_maps(CUtensorMap (&maps)[4], const void* x, int K, long long rows);
+// Maps of a matrix's packed words (rows of N; all widths, or one) and whether words, scales and offsets can be staged: bulk copies
+// want 16-byte boundaries, a stage one group.
+bool word_maps(CUtensorMap (&maps)[4], const void* wq, const void* scales, const void* zeros, int N, long long rows, int G, int bits,
+               int columns);
 
 }  // namespace ts
 }  // namespace gemq

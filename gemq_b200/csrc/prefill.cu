@@ -321,6 +321,8 @@ bool launch_pdl(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st, A
   return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
 }
 
+int rows_of(int K, int bits) { return bits == 3 ? cdiv(K, 10) : K * bits / 32; }
+
 bool shape_ok(int N, int K, int G) { return N % 128 == 0 && K % ts::kBK == 0 && G % ts::kBK == 0 && K % G == 0; }
 
 template <typename T>
@@ -351,6 +353,13 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
     U.fam[1].N = SF; U.fam[1].K = D; U.fam[1].G = L->s1.group_size; U.fam[1].col_tiles = cdiv(SF, kUpCols);
     U.fam[1].out = S.hs; U.fam[1].row0 = R;
   }
+  const gemq_stacked_t* const up[2] = {&L->w1, &L->w3};
+  const gemq_single_t* const sup[2] = {&L->s1, &L->s3};
+  U.staged = 1;
+  for (int m = 0; m < 2 && U.staged; ++m)
+    U.staged = ts::word_maps(U.w_map[0][m], up[m]->wq, up[m]->scales, up[m]->zeros, F, up[m]->wq_rows, L->group_size, 0, kUpCols / 2) &&
+               (!SF || ts::word_maps(U.w_map[1][m], sup[m]->wq, sup[m]->scales, sup[m]->zeros, SF, rows_of(D, sup[m]->nbits),
+                                     L->s1.group_size, sup[m]->nbits, kUpCols / 2));
   const int routed_tiles = S.max_tiles - sh_tiles;
   if (int rc = ts::launch_up(U, routed_tiles * cdiv(F, kUpCols) + sh_tiles * cdiv(SF, kUpCols), st)) return rc;
 
@@ -368,6 +377,9 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
     Q.fam[1].N = D; Q.fam[1].K = SF; Q.fam[1].G = L->s2.group_size; Q.fam[1].col_tiles = ct;
     Q.fam[1].out = S.ys + static_cast<size_t>(R) * D; Q.fam[1].row0 = R;
   }
+  Q.staged = ts::word_maps(Q.w_map[0][0], L->w2.wq, L->w2.scales, L->w2.zeros, D, L->w2.wq_rows, L->group_size, 0, ts::kCols) &&
+             (!SF || ts::word_maps(Q.w_map[1][0], L->s2.wq, L->s2.scales, L->s2.zeros, D, rows_of(SF, L->s2.nbits), L->s2.group_size,
+                                   L->s2.nbits, ts::kCols));
   if (int rc = ts::launch_down(Q, S.max_tiles * ct, st)) return rc;
   ok = launch_pdl(prefill_combine_kernel<T>, dim3(tokens), 128, st, static_cast<const int*>(S.plan.inv), idx,
                   static_cast<const __half*>(S.ys), SF ? R : -1, static_cast<T*>(out), A, D);
