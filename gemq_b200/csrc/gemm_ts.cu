@@ -9,7 +9,8 @@ static int launch(const Params& P, int tiles_bound, cudaStream_t stream) {
   static bool done[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GEMQ_ERR_LAUNCH;
-  const size_t smem = sizeof(Smem) + 1024;
+  const size_t smem = sizeof(Smem);
+  static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of a CTA");
   if (!done[dev]) {
     if (cudaFuncSetAttribute(gemm_ts_kernel<OUT, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
         cudaSuccess)

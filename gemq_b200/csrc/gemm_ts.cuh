@@ -96,12 +96,13 @@ struct alignas(64) Params {
   const __half* row_w;     // down: routing weight per sorted row
   const void* bias;        // linear
   int* err;
-  int staged;              // tiles of up to kStagedTokens: the words come through shared memory
+  int staged;              // the words come through shared memory
 };
 
-// A stage of a tile of up to 192 tokens leaves a quarter of its shared memory free: there the TMA warp puts the stage's
-// packed words, up to three stages ahead of the producers.
-constexpr int kStagedTokens = 192, kWordsAt = kStagedTokens / 2 * 2 * kRowBytes;
+// The TMA warp brings a stage's packed words, scales and offsets, too, up to three stages ahead of the producers.  The words
+// of 128 k have a place of their own up to 3 bits; at 4 bits they take the quarter of the stage that tiles of up to 192
+// tokens leave free (above, the MMAs take longer anyway).
+constexpr int kStagedTokens = 192, kWordsAt = kStagedTokens / 2 * 2 * kRowBytes, kWordBytes = 14 * kCols * 4;
 static_assert(kWordsAt + 16 * kCols * 4 <= kStageBytes, "128 k of 4 bits");
 // Packed rows of 128 k; 3-bit rows from the one in which the first code lies.
 __host__ __device__ constexpr int stage_rows(int bits) { return bits == 3 ? 14 : 4 * bits; }
@@ -109,6 +110,7 @@ __host__ __device__ constexpr int stage_rows(int bits) { return bits == 3 ? 14 :
 struct Smem {
   alignas(1024) unsigned char b[kStages][kStageBytes];
   alignas(16) unsigned char out[kTokens * kOutPitch];  // accumulators rounded to 16 bits
+  alignas(128) unsigned char packed[kStages][kWordBytes];
   alignas(16) unsigned char scales[kStages][kCols * 4];  // of the stage's group: [matrix][scales, offsets][columns]
   alignas(8) unsigned long long full[kStages], empty[kStages], words[kStages], acc_full[2], drained[2];  // [2]: by the tile's parity
   uint32_t tmem_base;
@@ -339,6 +341,8 @@ __device__ __forceinline__ int tile_bits(const Params& P, const Tile& t) {
   return F.nbits && t.expert >= 0 ? F.nbits[t.expert] : F.bits;
 }
 
+__device__ __forceinline__ bool staged(const Params& P, int rows, int bits) { return P.staged && (bits <= 3 || rows <= kStagedTokens); }
+
 // Words, scales and offsets of a tile, as its CTA's TMA warp brings them into the stages.
 template <bool UP>
 struct TileWords {
@@ -369,12 +373,12 @@ struct TileWords {
     }
     all = (UP ? 2 : 1) * (stage_rows(bits) * columns * 4 + 2 * parts);
   }
-  __device__ __forceinline__ void load(unsigned char* stage, unsigned char* sc, unsigned long long* bar, int kb) const {
+  __device__ __forceinline__ void load(unsigned char* at, unsigned char* sc, unsigned long long* bar, int kb) const {
     const int k0 = kb * kBK, row = row0 + (bits == 3 ? k0 / 10 : k0 * bits / 32), g = k0 / G;
     mbar_arrive_expect_tx(bar, all);
 #pragma unroll
     for (int m = 0; m < (UP ? 2 : 1); ++m) {
-      tma_load_2d(stage + kWordsAt + m * stage_rows(bits) * kCols * 2, map[m], col, row, bar);
+      tma_load_2d(at + m * stage_rows(bits) * kCols * 2, map[m], col, row, bar);
 #pragma unroll
       for (int z = 0; z < 2; ++z)
         if (parts)
@@ -456,7 +460,8 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   // STAGED
   constexpr uint32_t kPitch = UP ? kCols * 2 : kCols * 4;
   const int in_row = UP ? 16 * (warp & 3) + (lane & 15) : 32 * (warp & 3) + lane;
-  const uint32_t words0 = smem_u32(S.b[0]) + kWordsAt + mi * stage_rows(B) * kPitch + 4 * in_row;
+  constexpr uint32_t kWordStep = B == 4 ? kStageBytes : kWordBytes;
+  const uint32_t words0 = (B == 4 ? smem_u32(S.b[0]) + kWordsAt : smem_u32(S.packed[0])) + mi * stage_rows(B) * kPitch + 4 * in_row;
   const uint32_t scales0 = smem_u32(S.scales[0]) + mi * 256 + 2 * in_row;
   auto take = [&](Set& R) {
     if (kb >= real) {
@@ -467,7 +472,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
     }
     mbar_sleep_wait(&S.words[s], par ^ 1u, err, kErrFull);
     const int row = B == 3 ? kb * kBK / 10 - (kb & ~1) * kBK / 10 : (kb & 1) * 2 * B;
-    const uint32_t w = words0 + s * kStageBytes + row * kPitch, sc = scales0 + s * (kCols * 4);
+    const uint32_t w = words0 + s * kWordStep + row * kPitch, sc = scales0 + s * (kCols * 4);
 #pragma unroll
     for (int i = 0; i < NW; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(R.w[i]) : "r"(w + i * kPitch) : "memory");
     unsigned short a, b;
@@ -548,7 +553,7 @@ __device__ __forceinline__ void produce_bits(Smem& S, const Params& P, const Til
 template <bool UP, bool BF16, bool NAT>
 __device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
   const int bits = tile_bits(P, T);
-  if (P.staged && T.rows <= kStagedTokens) produce_bits<UP, BF16, NAT, true>(S, P, T, bits, base, tmem);
+  if (staged(P, T.rows, bits)) produce_bits<UP, BF16, NAT, true>(S, P, T, bits, base, tmem);
   else produce_bits<UP, BF16, NAT, false>(S, P, T, bits, base, tmem);
 }
 
@@ -705,7 +710,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
   constexpr int COLS = UP ? kCols / 2 : kCols;
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  Smem& S = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  Smem& S = *reinterpret_cast<Smem*>(smem_raw);  // no other shared memory: aligned like the array
   const int warp = threadIdx.x >> 5;
   const int rank = static_cast<int>(pair_rank());
   if (threadIdx.x == 0) {
@@ -756,15 +761,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const uint32_t bytes = 2 * 32 * box * kRowBytes;
       const int row = t.row0 - F.row0 + rank * half;
       const CUtensorMap* const map = &P.b_map[t.fam][box - 1];
-      const bool staged = P.staged && t.rows <= kStagedTokens;
+      const bool with_words = staged(P, t.rows, tile_bits(P, t));
       TileWords<UP> words;
-      if (staged) words.init(P, t);
+      if (with_words) words.init(P, t);
       for (int sb = 0; sb < SB; ++sb, ++c) {
         const uint32_t s = c % kStages;
         mbar_sleep_wait(&S.empty[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&S.full[s], 2 * bytes);
-          if (staged) words.load(S.b[s], S.scales[s], &S.words[s], t.kb0 + 2 * sb);
+          if (with_words) words.load(words.bits == 4 ? S.b[s] + kWordsAt : S.packed[s], S.scales[s], &S.words[s], t.kb0 + 2 * sb);
           else mbar_arrive(&S.words[s]);  // the barrier's phases follow the stages
           tma_load_pair(S.b[s], map, row, t.kb0 + 2 * sb, full0 + s * 8);
         }

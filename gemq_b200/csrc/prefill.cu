@@ -49,22 +49,15 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
                                                                     bool shared, int* err) {
   __shared__ int count[256], start[256], first_tile[256], cost[256], order[256];
   const int tid = threadIdx.x, lane = tid & 31;
-  // Time of a tile by bit width: 3 bits 1.8, 4 bits 1.2 times the 1- and 2-bit ones (measured with 128 rows).
+  int width = 0;
   for (int e = tid; e < E; e += kPlanThreads) {
     count[e] = 0;
-    const int b = nbits[e];
-    cost[e] = b == 3 ? 4 : (b == 4 ? 3 : b);
+    width = nbits[e];
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (tid == 0) *err = 0;
   __syncthreads();
-  // experts with the longest tiles first
-  for (int e = tid; e < E; e += kPlanThreads) {
-    int r = 0;
-    for (int o = 0; o < E; ++o) r += cost[o] > cost[e] || (cost[o] == cost[e] && o < e) ? 1 : 0;
-    order[r] = e;
-  }
   constexpr int kAhead = 4;
 #pragma unroll 1
   for (int p0 = tid; p0 < R + tid; p0 += kAhead * kPlanThreads) {
@@ -85,6 +78,22 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
       at = __shfl_sync(0xffffffffu, at, __ffs(peers) - 1);
       if (p < R) pl.at[p] = e >= 0 ? at + __popc(peers & ((1u << lane) - 1u)) : -1;
     }
+  }
+  __syncthreads();
+  // Experts with the longest tiles first: cycles of 128 k by the tile's MMAs, or by the de-quantisation.  (By bit width alone
+  // the pairs' shares differed by a quarter where 400 tokens meet 32 experts unevenly.)  E <= 256: one expert a thread.
+  if (tid < E) {
+    const int n = count[tid], nt = (n + kTile - 1) / kTile, rows = nt ? (n + nt - 1) / nt : 0;
+    const int mma = 4 * rows + 76, words = width == 3 ? 1700 : (width == 4 ? 1050 : (width == 2 ? 900 : 850));
+    cost[tid] = n ? (mma > words ? mma : words) : 0;
+  }
+  __syncthreads();
+  if (tid < E) {
+    int r = 0;
+    const int mine = cost[tid];
+#pragma unroll 8
+    for (int o = 0; o < E; ++o) r += cost[o] > mine || (cost[o] == mine && o < tid) ? 1 : 0;
+    order[r] = tid;
   }
   __syncthreads();
   const int sh_tiles = shared ? (tokens + kTile - 1) / kTile : 0;
