@@ -17,10 +17,11 @@
 // activations out of shared memory and has to bring in as many: 128 bytes a cycle, all shared memory can do;
 // 660 instead of 512 cycles per k-block.)  Tiles of the gate/up pass hold 64 gate and the same 64 up
 // columns per CTA, 16 + 16 per warp, so that a shuffle brings them together.
-//   16 producer warps  four groups that take 64-wide k-blocks in turn: fetch packed words a block of the group
-//                      ahead, de-quantise 64 k x 32 columns per warp, store them to the A ring; they never
-//                      stop between tiles
-//   1 TMA warp         an activation box per stage (32 to 128 tokens x 128 k, 128B swizzle)
+//   16 producer warps  four groups that take 64-wide k-blocks in turn: packed words from shared memory (or loaded a
+//                      block of the group ahead), de-quantise 64 k x 32 columns per warp, store them to the A ring;
+//                      they never stop between tiles
+//   1 TMA warp         per stage an activation box (32 to 128 tokens x 128 k, 128B swizzle), and the packed words,
+//                      scales and offsets of its 128 k (509 Mixtral tokens 531 -> 455 us, 4096 2650 -> 2490)
 //   1 MMA warp         (first CTA) issues tcgen05.mma and the commits that free the ring stages
 //   4 epilogue warps   round the accumulators to 16 bits into shared memory, which frees them for the next
 //                      tile, then finish and store whole rows while it is computed.  Tiles of up to 128 tokens
@@ -86,7 +87,7 @@ struct alignas(64) Params {
   // activations per family as (64 k, rows, K / 64): boxes of 32, 64, 96, 128 rows x 128 k, 128B swizzle
   CUtensorMap b_map[2][4];
   Family fam[2];
-  const int4* tiles;       // {expert (-1: shared), first row, rows, 0}, shared tiles first; nullptr: linear
+  const int4* tiles;       // {expert (-1: shared), first row, rows, 1: offsets not staged}, shared tiles first; nullptr: linear
   const int* n_tiles;
   int shared_tiles;
   const long long* expert; // linear: expert id read on the device, or nullptr -> 0
@@ -290,6 +291,7 @@ __device__ __forceinline__ void dequant_b3(const Exps<3>& X, uint32_t (&pr)[40],
 // A tile of the launch, as one CTA of the pair sees it.
 struct Tile {
   int fam, expert, row0, rows, col0;
+  int odd;             // its matrices do not begin at whole rows and 16-byte boundaries
   int kb0, kbn, part;  // its k-blocks, its part of k
   // tokens of the MMA (32, 64, ..), of which each CTA brings half
   __device__ __forceinline__ int n() const { return (rows + 31) & ~31; }
@@ -312,7 +314,7 @@ __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Til
     }
     const int mt = idx / F.col_tiles;
     if (mt * P.tile_rows >= P.rows) return false;
-    t.fam = 0;
+    t.fam = t.odd = 0;
     t.expert = P.expert ? static_cast<int>(*P.expert) : 0;
     t.row0 = mt * P.tile_rows;
     t.rows = min(P.tile_rows, P.rows - t.row0);
@@ -332,6 +334,7 @@ __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Til
   t.expert = d.x;
   t.row0 = d.y;
   t.rows = d.z;
+  t.odd = d.w;
   t.col0 = (2 * (i % ct) + rank) * COLS;
   return true;
 }
@@ -341,7 +344,9 @@ __device__ __forceinline__ int tile_bits(const Params& P, const Tile& t) {
   return F.nbits && t.expert >= 0 ? F.nbits[t.expert] : F.bits;
 }
 
-__device__ __forceinline__ bool staged(const Params& P, int rows, int bits) { return P.staged && (bits <= 3 || rows <= kStagedTokens); }
+__device__ __forceinline__ bool staged(const Params& P, const Tile& t, int bits) {
+  return P.staged && !t.odd && (bits <= 3 || t.rows <= kStagedTokens);
+}
 
 // Words, scales and offsets of a tile, as its CTA's TMA warp brings them into the stages.
 template <bool UP>
@@ -553,7 +558,7 @@ __device__ __forceinline__ void produce_bits(Smem& S, const Params& P, const Til
 template <bool UP, bool BF16, bool NAT>
 __device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
   const int bits = tile_bits(P, T);
-  if (staged(P, T.rows, bits)) produce_bits<UP, BF16, NAT, true>(S, P, T, bits, base, tmem);
+  if (staged(P, T, bits)) produce_bits<UP, BF16, NAT, true>(S, P, T, bits, base, tmem);
   else produce_bits<UP, BF16, NAT, false>(S, P, T, bits, base, tmem);
 }
 
@@ -761,7 +766,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const uint32_t bytes = 2 * 32 * box * kRowBytes;
       const int row = t.row0 - F.row0 + rank * half;
       const CUtensorMap* const map = &P.b_map[t.fam][box - 1];
-      const bool with_words = staged(P, t.rows, tile_bits(P, t));
+      const bool with_words = staged(P, t, tile_bits(P, t));
       TileWords<UP> words;
       if (with_words) words.init(P, t);
       for (int sb = 0; sb < SB; ++sb, ++c) {

@@ -31,7 +31,7 @@ constexpr int kDownCols = 2 * ts::kCols;
 constexpr int kErrBadExpert = 21;
 
 struct Plan {
-  int4* tiles;     // {expert (-1: shared), first row, rows, 0}: the shared expert's tiles first
+  int4* tiles;     // {expert (-1: shared), first row, rows, 1: matrices off whole rows}: the shared expert's tiles first
   int* n_tiles;
   int* start;      // expert -> its first sorted row
   int* at;         // (token, slot) -> place among its expert's rows, -1: expert id out of range
@@ -41,18 +41,31 @@ struct Plan {
 
 constexpr int kPlanThreads = 1024;
 
+// Where an expert's matrices begin: words, and scales and offsets (nullptr: whole matrices one after the other).
+struct Offsets {
+  const int* words[2];   // of gate and up, of down
+  int pitch[2];
+  const int* scales[3];
+};
+
 // One CTA; it reads the expert ids once, four trips of loads in flight, and leaves everything per row to the gather
 // (with that here, 12000 rows took 28 us).  Lanes with the same expert claim their rows together: one shared-memory
 // atomic per warp and expert.
 __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, const long long* __restrict__ idx,
-                                                                    const int* __restrict__ nbits, int R, int E, int tokens,
+                                                                    const int* __restrict__ nbits, Offsets off, int R, int E, int tokens,
                                                                     bool shared, int* err) {
-  __shared__ int count[256], start[256], first_tile[256], cost[256], order[256];
+  __shared__ int odd[256], count[256], start[256], first_tile[256], cost[256], order[256];
   const int tid = threadIdx.x, lane = tid & 31;
   int width = 0;
   for (int e = tid; e < E; e += kPlanThreads) {
     count[e] = 0;
     width = nbits[e];
+    int o = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) o |= off.words[i] ? off.words[i][e] % off.pitch[i] : 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o |= off.scales[i] ? off.scales[i][e] & 7 : 0;
+    odd[e] = o ? 1 : 0;
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -124,7 +137,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
     const int n = count[e], nt = (n + kTile - 1) / kTile, blocks = (n + 15) / 16;
     for (int t = lane; t < nt; t += 32) {
       const int lo = 16 * (blocks * t / nt), hi = min(n, 16 * (blocks * (t + 1) / nt));
-      pl.tiles[first_tile[e] + t] = make_int4(e, start[e] + lo, hi - lo, 0);
+      pl.tiles[first_tile[e] + t] = make_int4(e, start[e] + lo, hi - lo, odd[e]);
     }
   }
   for (int i = tid; i < sh_tiles; i += kPlanThreads)
@@ -340,7 +353,8 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
   const int D = L->hidden, F = L->ffn, A = L->top_k, E = L->n_experts, SF = L->shared_ffn, R = tokens * A;
   const int sh_tiles = SF ? cdiv(tokens, kTile) : 0;
   const int* nbits = static_cast<const int*>(L->w1.nbits);
-  bool ok = launch_pdl(prefill_plan_kernel, dim3(1), kPlanThreads, st, S.plan, idx, nbits, R, E, tokens, SF > 0, S.err);
+  const Offsets off = {{L->w1.wq_strides, L->w2.wq_strides}, {F, D}, {L->w1.zs_strides, L->w3.zs_strides, L->w2.zs_strides}};
+  bool ok = launch_pdl(prefill_plan_kernel, dim3(1), kPlanThreads, st, S.plan, idx, nbits, off, R, E, tokens, SF > 0, S.err);
   const size_t items = static_cast<size_t>(tokens) * (D / 32);
   ok = ok && launch_pdl(prefill_gather_kernel<T>, dim3(static_cast<unsigned>((items + 127) / 128)), 128, st, S.plan,
                         static_cast<const T*>(x), idx, static_cast<const T*>(w), nbits, S.xs, tokens, A, D, SF ? L->s1.nbits : 0);
