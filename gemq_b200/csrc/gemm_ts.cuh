@@ -475,6 +475,11 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
       R.s = R.z = __float2half_rn(0.f);
       return;
     }
+    // The stage's release first.  The TMA warp flips words[s] in every use of the stage, these warps look at it in staged tiles only;
+    // before the MMAs of its last use are complete, that use's own phase may be open, and the parity of the one before lets
+    // the wait pass (a staged tile behind one that was not: words of another tile, or none).  They are complete only after the
+    // TMA warp had arrived for that use.  It asks for the words of this one behind the same release: nothing is lost.
+    mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
     mbar_sleep_wait(&S.words[s], par ^ 1u, err, kErrFull);
     const int row = B == 3 ? kb * kBK / 10 - (kb & ~1) * kBK / 10 : (kb & 1) * 2 * B;
     const uint32_t w = words0 + s * kWordStep + row * kPitch, sc = scales0 + s * (kCols * 4);
@@ -492,7 +497,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
     if constexpr (B == 3) {
       uint32_t pr[40];
       dequant_b3<BF16>(X, pr, cur.w, s2, z2);
-      mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
+      if (!STAGED) mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
       tc_fence_after_sync();
       switch ((kb * kBK % 10) >> 1) {  // uniform
         case 0: tmem_st32(dst, pr); break;
@@ -505,7 +510,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
       // in two halves: 16 result registers instead of 32
       uint32_t o[16];
       dequant_words<B, BF16, NAT, 0>(X, o, cur.w, s2, z2);
-      mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
+      if (!STAGED) mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
       tc_fence_after_sync();
       tmem_st16(dst, o);
       dequant_words<B, BF16, NAT, 0>(X, o, cur.w + B, s2, z2);

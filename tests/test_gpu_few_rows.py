@@ -176,3 +176,44 @@ def test_moe_staged_words(rows, bits):
         assert blk.prefill_error_code(T) == 0
         ref = O.moe_reference_fp32(x, w.float(), sel, w1, w3, w2).numpy()
         assert rel_fro(out.float().cpu().numpy(), ref) < REL_FRO_TOL
+
+
+def _reference(layer, x, w, sel):
+    """Layer output in fp32 for one expert per token, an expert's rows at a time."""
+    deq = lambda l: torch.from_numpy(O.dequantize(l["wq"], l["s"], l["z"], l["b"], 128, l["i"]).astype(np.float32))
+    ffn = lambda x, w1, w3, w2: (torch.nn.functional.silu(x @ deq(w1)) * (x @ deq(w3))) @ deq(w2)
+    x, out = x.float(), torch.zeros(x.shape)
+    for e, mats in enumerate(zip(layer["w1"], layer["w3"], layer["w2"])):
+        rows = sel[:, 0] == e
+        out[rows] = w.float()[rows] * ffn(x[rows], *mats)
+    if layer["shared"]:
+        s1, s2, s3 = layer["shared"]
+        out += ffn(x, s1, s3, s2)
+    return out.numpy()
+
+
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("D,Fd", [(1280, 1024), (2560, 256)])
+def test_moe_staged_behind_unstaged_tiles(D, Fd, shared):
+    """Every pair of CTAs gets 4-bit tiles of 256 rows, whose packed words do not come through the stages, and then tiles whose
+    words do: routed experts of 2 and 1 bits behind a 4-bit one, or 3 bits behind the shared expert, whose tiles lead the list.
+    Reduction lengths of two stages (a use of every second stage) to twenty."""
+    g = torch.Generator().manual_seed(D)
+    if shared:
+        T = 5120
+        layer = MF.make_layer("deepseek", D=D, Fd=Fd, E=2, A=1, bits=[3, 1], seed=3, gate_std=0.02, n_shared=1)
+        sel = (torch.arange(T) >= 2560).long()
+    else:
+        layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=3, A=1, bits=[4, 2, 1], seed=3, gate_std=0.02)
+        sel = torch.tensor([0] * 5120 + [1] * 2560 + [2] * 2560)
+        T = sel.numel()
+    blk = MF.gpu_block(layer)
+    sel = sel[torch.randperm(T, generator=g)].view(T, 1)
+    w = (torch.rand(T, 1, generator=g) * 0.5 + 0.5).half()
+    x = torch.randn(T, D, generator=g).half()
+    args = (x.cuda(), 1, True)
+    out = blk._prefill(*args, routing=(w.cuda(), sel.cuda()))[0]
+    assert blk.prefill_error_code(T) == 0
+    assert rel_fro(out.float().cpu().numpy(), _reference(layer, x, w, sel)) < REL_FRO_TOL
+    for _ in range(20):
+        assert torch.equal(out, blk._prefill(*args, routing=(w.cuda(), sel.cuda()))[0])
