@@ -135,6 +135,15 @@ __global__ void __launch_bounds__(kThreads, 3) few_moe_kernel(const __grid_const
   MoeShared& S = *reinterpret_cast<MoeShared*>(smem_raw);
   unsigned char* ring = smem_raw + 1024;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // Tiles and weights are read ahead of the wait, the table after it: the first stages travel under the tail of the launch
+  // before (16 DeepSeek-V2-Lite tokens 87.4 -> 82.5 us).  What makes this sound is the table launch: each of its CTAs waits
+  // before it lets up start, so the plan, and what came before the call, is complete before a CTA of up runs, and those of down start
+  // after some of up's.  (That the producer warps release ahead of their wait does not matter then; released by the other warps
+  // alone, after theirs: 83.1 -> 83.9 us.)  The plan of the call before may lie at the same place, and this kernel has not
+  // waited yet: it is read from L2.
+  const int tile = blockIdx.y;
+  const int n_tiles = __ldcg(P.n_tiles);
+  const int4 d = __ldcg(P.tiles + tile);  // the list is as long as the grid
   if (tid == 0) {
     for (int s = 0; s < kMaxRing; ++s) {
       mbar_init(&S.full[s], 1 + 32);
@@ -143,12 +152,10 @@ __global__ void __launch_bounds__(kThreads, 3) few_moe_kernel(const __grid_const
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (tid >= 64 && tid < 68) reinterpret_cast<uint32_t*>(S.zero)[tid - 64] = 0u;
-  // The launch before lets this one start once its own wait is over: the plan two or more launches back is complete, and all that
-  // was before it.  Tiles and weights are read ahead of the wait, the table after it: the first stages travel under the tail of
-  // the launch before (16 DeepSeek-V2-Lite tokens 87.4 -> 82.5 us, 32 Mixtral tokens 172.1 -> 167.1).
-  const int tile = blockIdx.y;
-  if (tile >= *P.n_tiles) return;
-  const int4 d = P.tiles[tile];
+  if (tile >= n_tiles) {
+    if (tile == 0) pdl_wait();  // a grid without a tile does not end before the launch ahead of it, either
+    return;
+  }
   const int fam = d.x < 0 ? 1 : 0, row0 = d.y, rows = d.z;
   const int N = P.N[fam], K = P.K[fam], ngroups = K / kGroup;
   constexpr int kCols = MODE == kUp ? 32 * kCons : 64 * kCons;
@@ -159,7 +166,7 @@ __global__ void __launch_bounds__(kThreads, 3) few_moe_kernel(const __grid_const
   int lo, hi;
   stage_range(bits, K, part, P.splits, lo, hi);
   __syncthreads();
-  if (warp != kCons) pdl_wait();
+  if (warp != kCons) pdl_wait();  // the producer: behind its first loads
   pdl_launch();
 
   if (warp == kCons) {
@@ -249,7 +256,7 @@ __global__ void __launch_bounds__(kTabThreads) few_table_kernel(const __grid_con
   T* xs = reinterpret_cast<T*>(smem_raw);
   const int tile = blockIdx.y, t = blockIdx.x, tid = threadIdx.x;
   pdl_wait();
-  pdl_launch();  // after the wait: the products read the plan ahead of theirs
+  pdl_launch();  // after the wait, in every CTA: the products read the plan and the weights ahead of theirs
   if (tile >= *P.n_tiles) return;
   const int4 d = P.tiles[tile];
   if (t >= d.z) return;

@@ -217,3 +217,48 @@ def test_moe_staged_behind_unstaged_tiles(D, Fd, shared):
     assert rel_fro(out.float().cpu().numpy(), _reference(layer, x, w, sel)) < REL_FRO_TOL
     for _ in range(20):
         assert torch.equal(out, blk._prefill(*args, routing=(w.cuda(), sel.cuda()))[0])
+
+
+@pytest.mark.parametrize("shared", [0, 2])
+def test_moe_few_rows_one_behind_the_other(shared):
+    """Decode batches on one scratch with nothing in between but kernels that write their weights: the products read the plan, which
+    replaces that of the call before at the same place, and their first weights ahead of their waits.  Routings with one tile, with
+    a tile for every expert, with tiles of many rows and (ids out of range) with none."""
+    E, A, D, Fd = 16, 2, 512, 384
+    make = lambda seed: MF.make_layer("deepseek" if shared else "mixtral", D=D, Fd=Fd, E=E, A=A, bits=[1, 2, 3, 4] * 4, seed=seed,
+                                      gate_std=0.02, n_shared=shared)
+    blk, other = MF.gpu_block(make(1)), MF.gpu_block(make(2))
+    names = [n for n in vars(blk) if n.endswith(("_wq", "_scales", "_zeros")) and getattr(blk, n) is not None]
+    weights = [{n: getattr(b, n).clone() for n in names} for b in (blk, other)]
+    g = torch.Generator().manual_seed(shared)
+    calls = []
+    for i in range(24):
+        T = (24, 24, 24, 9, 40, 24)[i % 6]
+        sel = (torch.full((T, A), i % E), torch.randint(0, E, (T, A), generator=g), torch.arange(T * A).view(T, A) % E,
+               torch.randint(0, 3, (T, A), generator=g), torch.full((T, A), E + 1), torch.randint(8, E, (T, A), generator=g))[i % 6]
+        w = torch.softmax(torch.randn(T, A, generator=g), -1).half().cuda()
+        calls.append((torch.randn(T, D, generator=g).half().cuda(), w, sel.cuda(), (i // 6 + i) % 2))
+
+    def write(which):
+        for n in names:  # kernels, not copies
+            torch.add(weights[which][n], 0, out=getattr(blk, n))
+
+    for rewritten in (True, False):
+        want = []
+        for x, w, sel, which in calls:
+            write(which if rewritten else 0)
+            torch.cuda.synchronize()
+            want.append(blk._prefill(x, 1, True, routing=(w, sel))[0].clone())
+            torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = []
+            for x, w, sel, which in calls:
+                if rewritten:
+                    write(which)
+                got.append(blk._prefill(x, 1, True, routing=(w, sel))[0])
+        for _ in range(10):
+            for y in got:
+                y.fill_(float("nan"))
+            graph.replay()
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
