@@ -18,6 +18,9 @@ inline int launch_status() {
   return e == cudaSuccess ? GEMQ_OK : GEMQ_ERR_LAUNCH;
 }
 
+// A bit width as the kernels read it: tables on the device may hold anything.
+__host__ __device__ constexpr int clamp_bits(int b) { return b < 1 ? 1 : (b > 4 ? 4 : b); }
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Multiprocessors of the current device, 0 on failure.

@@ -169,7 +169,6 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
   return v;
 }
 
-__device__ __forceinline__ int clamp_bits(int b) { return b < 1 ? 1 : (b > 4 ? 4 : b); }
 __device__ __forceinline__ int quantum_groups(int bits) { return bits == 3 ? 5 : 4; }
 // relative cost of a quantum, for the byte/issue balanced deal of the quanta to the CTAs
 // (relative time of a quantum measured in place: the low bit widths are bound by the MMA and

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 3) few_moe_kernel(const __grid_const
   const int part = static_cast<int>(blockIdx.x % P.splits), n0 = kCols * static_cast<int>(blockIdx.x / P.splits);
   if (n0 >= N) return;  // the launch covers the wider of the two families
   int bits = fam ? P.sbits : P.nbits[d.x];
-  bits = bits < 1 ? 1 : (bits > 4 ? 4 : bits);
+  bits = clamp_bits(bits);
   int lo, hi;
   stage_range(bits, K, part, P.splits, lo, hi);
   __syncthreads();
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kThreads, 3) few_moe_kernel(const __grid_const
   int nbits2 = 0;
   if (MODE == kUp) {
     nbits2 = fam ? P.next_sbits : P.next_nbits[d.x];
-    nbits2 = nbits2 < 1 ? 1 : (nbits2 > 4 ? 4 : nbits2);
+    nbits2 = clamp_bits(nbits2);
   }
   if (MAXNB == 1 || rows <= 8)
     run_tile<MODE, 1>(S, P, ring, bits, lo, hi, rows, row0, N, ngroups, n0, next, nbits2, warp, lane);
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kTabThreads) few_table_kernel(const __grid_con
   const int4 d = P.tiles[tile];
   if (t >= d.z) return;
   int bits = d.x < 0 ? P.sbits : P.nbits[d.x];
-  bits = bits < 1 ? 1 : (bits > 4 ? 4 : bits);
+  bits = clamp_bits(bits);
   const T* src = static_cast<const T*>(P.x) + static_cast<size_t>(P.src[d.y + t]) * P.K;
   for (int i = tid; i < P.K / 8; i += kTabThreads) reinterpret_cast<uint4*>(xs)[i] = reinterpret_cast<const uint4*>(src)[i];
   __syncthreads();
@@ -587,7 +587,7 @@ int moe_few_rows(const gemq_moe_layer_t* L, const void* x, void* out, const long
     U.zr[m] = static_cast<const __half*>(up[m]->zeros);
     U.zss[m] = up[m]->zs_strides;
     if (SF) {
-      if (!tensor_map_strips(&U.wmap[2 + m], sup[m]->wq, SF, packed_rows(D, sup[m]->nbits), kCons)) return GEMQ_ERR_LAUNCH;
+      if (!tensor_map_strips(&U.wmap[2 + m], sup[m]->wq, SF, packed_rows(D, L->s1.nbits), kCons)) return GEMQ_ERR_LAUNCH;
       U.sc[2 + m] = static_cast<const __half*>(sup[m]->scales);
       U.zr[2 + m] = static_cast<const __half*>(sup[m]->zeros);
     }

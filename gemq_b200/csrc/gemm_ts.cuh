@@ -341,7 +341,7 @@ __device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Til
 
 __device__ __forceinline__ int tile_bits(const Params& P, const Tile& t) {
   const Family& F = P.fam[t.fam];
-  return F.nbits && t.expert >= 0 ? F.nbits[t.expert] : F.bits;
+  return clamp_bits(F.nbits && t.expert >= 0 ? F.nbits[t.expert] : F.bits);  // indexes the maps of packed words
 }
 
 __device__ __forceinline__ bool staged(const Params& P, const Tile& t, int bits) {
@@ -651,7 +651,7 @@ __device__ __forceinline__ void word_order(const __half (&h)[32], uint32_t (&o)[
 // 16 columns each in two warps' worth of staged columns).
 __device__ __forceinline__ void finish_up(const Smem& S, const Params& P, const Tile& t, int tid) {
   const Family& F = P.fam[t.fam];
-  const int bits = F.out_nbits && t.expert >= 0 ? F.out_nbits[t.expert] : F.out_bits;
+  const int bits = clamp_bits(F.out_nbits && t.expert >= 0 ? F.out_nbits[t.expert] : F.out_bits);
   const size_t pitch = F.N;
   __half* const out = static_cast<__half*>(F.out) + static_cast<size_t>(t.row0 - F.row0) * pitch + t.col0;
   const int rows = t.rows;

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(128) prefill_gather_kernel(Plan pl, const T* _
       const int at = pl.at[tok * A + a];
       const int e = at < 0 ? 0 : static_cast<int>(idx[tok * A + a]);
       if (at >= 0) rows[a] = pl.start[e] + at;
-      bits[a] = nbits[e];
+      bits[a] = clamp_bits(nbits[e]);
     }
   }
 #pragma unroll
@@ -357,7 +357,8 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
   bool ok = launch_pdl(prefill_plan_kernel, dim3(1), kPlanThreads, st, S.plan, idx, nbits, off, R, E, tokens, SF > 0, S.err);
   const size_t items = static_cast<size_t>(tokens) * (D / 32);
   ok = ok && launch_pdl(prefill_gather_kernel<T>, dim3(static_cast<unsigned>((items + 127) / 128)), 128, st, S.plan,
-                        static_cast<const T*>(x), idx, static_cast<const T*>(w), nbits, S.xs, tokens, A, D, SF ? L->s1.nbits : 0);
+                        static_cast<const T*>(x), idx, static_cast<const T*>(w), nbits, S.xs, tokens, A, D,
+                        SF ? clamp_bits(L->s1.nbits) : 0);
   if (!ok) return GEMQ_ERR_LAUNCH;
 
   ts::Params U = {};
@@ -378,11 +379,12 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
   }
   const gemq_stacked_t* const up[2] = {&L->w1, &L->w3};
   const gemq_single_t* const sup[2] = {&L->s1, &L->s3};
+  const int sb = clamp_bits(L->s1.nbits), sb2 = clamp_bits(L->s2.nbits);  // as the tiles look the maps up
   U.staged = 1;
   for (int m = 0; m < 2 && U.staged; ++m)
     U.staged = ts::word_maps(U.w_map[0][m], up[m]->wq, up[m]->scales, up[m]->zeros, F, up[m]->wq_rows, L->group_size, 0, kUpCols / 2) &&
-               (!SF || ts::word_maps(U.w_map[1][m], sup[m]->wq, sup[m]->scales, sup[m]->zeros, SF, rows_of(D, sup[m]->nbits),
-                                     L->s1.group_size, sup[m]->nbits, kUpCols / 2));
+               (!SF || ts::word_maps(U.w_map[1][m], sup[m]->wq, sup[m]->scales, sup[m]->zeros, SF, rows_of(D, sb), L->s1.group_size,
+                                     sb, kUpCols / 2));
   const int routed_tiles = S.max_tiles - sh_tiles;
   if (int rc = ts::launch_up(U, routed_tiles * cdiv(F, kUpCols) + sh_tiles * cdiv(SF, kUpCols), st)) return rc;
 
@@ -401,8 +403,8 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
     Q.fam[1].out = S.ys + static_cast<size_t>(R) * D; Q.fam[1].row0 = R;
   }
   Q.staged = ts::word_maps(Q.w_map[0][0], L->w2.wq, L->w2.scales, L->w2.zeros, D, L->w2.wq_rows, L->group_size, 0, ts::kCols) &&
-             (!SF || ts::word_maps(Q.w_map[1][0], L->s2.wq, L->s2.scales, L->s2.zeros, D, rows_of(SF, L->s2.nbits), L->s2.group_size,
-                                   L->s2.nbits, ts::kCols));
+             (!SF || ts::word_maps(Q.w_map[1][0], L->s2.wq, L->s2.scales, L->s2.zeros, D, rows_of(SF, sb2), L->s2.group_size, sb2,
+                                   ts::kCols));
   if (int rc = ts::launch_down(Q, S.max_tiles * ct, st)) return rc;
   ok = launch_pdl(prefill_combine_kernel<T>, dim3(tokens), 128, st, static_cast<const int*>(S.plan.inv), idx,
                   static_cast<const __half*>(S.ys), SF ? R : -1, static_cast<T*>(out), A, D);

@@ -172,7 +172,8 @@ typedef struct {
   int shared_ffn;    /* 0, or n_shared * F (moe_block.py:400-412) */
   const void* gate;  /* fp16 [E, D] */
   gemq_stacked_t w1, w3, w2;
-  gemq_single_t s1, s3, s2; /* used when shared_ffn > 0 */
+  gemq_single_t s1, s3, s2; /* used when shared_ffn > 0; s1's nbits and group_size hold for s3, too, and for one token for
+                               s2 (gemq/inference/moe_block.py:410-412) */
 } gemq_moe_layer_t;
 
 /* Device scratch of one decode step; sizes from gemq_moe_decode_scratch_bytes. */

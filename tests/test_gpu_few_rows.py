@@ -262,3 +262,18 @@ def test_moe_few_rows_one_behind_the_other(shared):
                 y.fill_(float("nan"))
             graph.replay()
             assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("T", [40, 400])  # few-row launches and the GEMM
+def test_moe_bit_width_tables(T):
+    """Widths on the device are clamped before they choose a map of packed words, and the shared expert's third matrix is read with
+    the first one's width."""
+    layer = MF.make_layer("deepseek", D=256, Fd=384, E=4, A=2, bits=[4, 4, 1, 4], seed=1, gate_std=0.02, n_shared=1)
+    blk = MF.gpu_block(layer)
+    x = torch.randn(T, 256, generator=torch.Generator().manual_seed(T)).half().cuda()
+    want = blk._prefill(x, 2, False)[0].clone()
+    for name in ("w1", "w2", "w3"):
+        getattr(blk, f"{name}_nbits").copy_(torch.tensor([4, 7, -3, 33]))
+    blk._layer.s3.nbits = 3
+    assert torch.equal(blk._prefill(x, 2, False)[0], want)
+    assert blk.prefill_error_code(T) == 0
