@@ -69,4 +69,23 @@ __device__ __forceinline__ float pow2i(int e) {  // 2^e for e in [-126, 127]
 
 __device__ __forceinline__ float silu_f32(float v) { return v / (1.0f + __expf(-v)); }
 
+// Where the experts of a layer begin: words (w3 lies like w1), and scales and offsets (nullptr: whole matrices one after the other).
+struct Offsets {
+  const int* words[2];   // of gate and up, of down
+  int pitch[2];
+  const int* scales[3];
+};
+inline Offsets expert_offsets(const gemq_moe_layer_t* L) {
+  return {{L->w1.wq_strides, L->w2.wq_strides}, {L->ffn, L->hidden}, {L->w1.zs_strides, L->w3.zs_strides, L->w2.zs_strides}};
+}
+// An expert whose words do not begin at a whole row, or its scales not at a 16-byte boundary: tiled and bulk copies cannot take it.
+__device__ __forceinline__ bool off_boundary(const Offsets& off, int e) {
+  int o = 0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) o |= off.words[i] ? off.words[i][e] % off.pitch[i] : 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) o |= off.scales[i] ? off.scales[i][e] & 7 : 0;
+  return o != 0;
+}
+
 }  // namespace gemq

@@ -17,7 +17,7 @@ namespace gemq {
 namespace few {
 
 enum { kUp = 0, kDown = 1 };
-constexpr int kErrBadExpertId = 21;
+constexpr int kErrBadExpertId = 21, kErrOffBoundary = 22;
 
 // Tile of an expert: {expert (-1: the shared expert), first sorted row, rows, 0}.
 struct Plan {
@@ -276,15 +276,17 @@ __global__ void __launch_bounds__(kTabThreads) few_table_kernel(const __grid_con
 // ---- permutation of the batch: one CTA -----------------------------------------------------------
 constexpr int kPlanThreads = 512;
 
+// Experts that begin off a whole row of words or a 16-byte boundary of scales cannot be copied by these launches: their rows are
+// left out like those of an id out of range, and reported.  (The GEMM, which larger batches take, loads them.)
 // Sorted rows: the experts whose tiles take longest first (the CTAs start in this order); the shared
 // expert's tokens come behind the routed rows, its tiles lead the tile list.
 template <typename T>
 __global__ void __launch_bounds__(kPlanThreads) few_plan_kernel(Plan pl, const long long* __restrict__ idx, const T* __restrict__ w,
-                                                                const int* __restrict__ nbits, int R, int A, int E, int tokens,
-                                                                int tile_rows, int shared, int* err) {
+                                                                const int* __restrict__ nbits, Offsets off, int R, int A, int E,
+                                                                int tokens, int tile_rows, int shared, int* err) {
   __shared__ int count[256], start[256], n_tile[256], key[256];
   const int tid = threadIdx.x;
-  for (int e = tid; e < E; e += kPlanThreads) { count[e] = 0; key[e] = nbits[e]; }
+  for (int e = tid; e < E; e += kPlanThreads) { count[e] = 0; key[e] = off_boundary(off, e) ? -1 : clamp_bits(nbits[e]); }
   pdl_launch();
   pdl_wait();
   if (tid == 0) *err = 0;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(kPlanThreads) few_plan_kernel(Plan pl, const l
     ex[u] = -1;
     if (tid + u * kPlanThreads < R) {
       if (id[u] < 0 || id[u] >= E) atomicExch(err, kErrBadExpertId);
+      else if (key[static_cast<int>(id[u])] < 0) atomicExch(err, kErrOffBoundary);
       else {
         ex[u] = static_cast<int>(id[u]);
         at[u] = atomicAdd(&count[ex[u]], 1);
@@ -313,8 +316,9 @@ __global__ void __launch_bounds__(kPlanThreads) few_plan_kernel(Plan pl, const l
   }
   for (int i = tid + kHeld * kPlanThreads; i < R; i += kPlanThreads) {
     const long long e = idx[i];
-    if (e < 0 || e >= E) atomicExch(err, kErrBadExpertId);
-    pl.inv[i] = e < 0 || e >= E ? -1 : atomicAdd(&count[static_cast<int>(e)], 1);
+    const int bad = e < 0 || e >= E ? kErrBadExpertId : (key[static_cast<int>(e)] < 0 ? kErrOffBoundary : 0);
+    if (bad) atomicExch(err, bad);
+    pl.inv[i] = bad ? -1 : atomicAdd(&count[static_cast<int>(e)], 1);
   }
   __syncthreads();
   // longest first: two blocks of eight rows take twice the MMAs of one, more bits more copying
@@ -555,10 +559,10 @@ int moe_few_rows(const gemq_moe_layer_t* L, const void* x, void* out, const long
   bool ok;
   if (bf16)
     ok = launch(few_plan_kernel<__nv_bfloat16>, dim3(1), kPlanThreads, 0, st, Y.plan, idx, static_cast<const __nv_bfloat16*>(w),
-                static_cast<const int*>(L->w1.nbits), R, A, E, tokens, Y.tile_rows, SF > 0 ? 1 : 0, err);
+                static_cast<const int*>(L->w1.nbits), expert_offsets(L), R, A, E, tokens, Y.tile_rows, SF > 0 ? 1 : 0, err);
   else
     ok = launch(few_plan_kernel<__half>, dim3(1), kPlanThreads, 0, st, Y.plan, idx, static_cast<const __half*>(w),
-                static_cast<const int*>(L->w1.nbits), R, A, E, tokens, Y.tile_rows, SF > 0 ? 1 : 0, err);
+                static_cast<const int*>(L->w1.nbits), expert_offsets(L), R, A, E, tokens, Y.tile_rows, SF > 0 ? 1 : 0, err);
   if (!ok) return GEMQ_ERR_LAUNCH;
 
   TableParams T = {};

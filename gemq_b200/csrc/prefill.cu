@@ -41,13 +41,6 @@ struct Plan {
 
 constexpr int kPlanThreads = 1024;
 
-// Where an expert's matrices begin: words, and scales and offsets (nullptr: whole matrices one after the other).
-struct Offsets {
-  const int* words[2];   // of gate and up, of down
-  int pitch[2];
-  const int* scales[3];
-};
-
 // One CTA; it reads the expert ids once, four trips of loads in flight, and leaves everything per row to the gather
 // (with that here, 12000 rows took 28 us).  Lanes with the same expert claim their rows together: one shared-memory
 // atomic per warp and expert.
@@ -60,12 +53,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
   for (int e = tid; e < E; e += kPlanThreads) {
     count[e] = 0;
     width = nbits[e];
-    int o = 0;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) o |= off.words[i] ? off.words[i][e] % off.pitch[i] : 0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) o |= off.scales[i] ? off.scales[i][e] & 7 : 0;
-    odd[e] = o ? 1 : 0;
+    odd[e] = off_boundary(off, e) ? 1 : 0;
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -353,7 +341,7 @@ int run(const gemq_moe_layer_t* L, const Scratch& S, const void* x, void* out, c
   const int D = L->hidden, F = L->ffn, A = L->top_k, E = L->n_experts, SF = L->shared_ffn, R = tokens * A;
   const int sh_tiles = SF ? cdiv(tokens, kTile) : 0;
   const int* nbits = static_cast<const int*>(L->w1.nbits);
-  const Offsets off = {{L->w1.wq_strides, L->w2.wq_strides}, {F, D}, {L->w1.zs_strides, L->w3.zs_strides, L->w2.zs_strides}};
+  const Offsets off = expert_offsets(L);
   bool ok = launch_pdl(prefill_plan_kernel, dim3(1), kPlanThreads, st, S.plan, idx, nbits, off, R, E, tokens, SF > 0, S.err);
   const size_t items = static_cast<size_t>(tokens) * (D / 32);
   ok = ok && launch_pdl(prefill_gather_kernel<T>, dim3(static_cast<unsigned>((items + 127) / 128)), 128, st, S.plan,

@@ -83,7 +83,7 @@ typedef struct {
   const void* scales;
   const void* zeros;
   const int32_t* nbits;      /* [E] */
-  const int32_t* wq_strides; /* [E] int32 element offsets into wq */
+  const int32_t* wq_strides; /* [E] int32 element offsets into wq: whole rows, experts are concatenated along dim 0 */
   const int32_t* zs_strides; /* [E] element offsets into scales/zeros, or NULL: expert e starts at row e*(K/G) */
   int64_t wq_rows;           /* rows (dim 0) of the stacked wq tensor */
   int64_t zs_rows;           /* rows (dim 0) of the stacked scales / zeros tensors */
@@ -239,7 +239,9 @@ size_t gemq_moe_prefill_scratch_bytes(const gemq_moe_layer_t* layer, int tokens)
  * GEMM scaled by the routing weight, per-token combine in expert order, shared experts.
  * x, out: [tokens, D] fp16 or bf16; idx int64 [tokens, A]; w [tokens, A] in the activation dtype;
  * logits [tokens, E] or NULL: fp32 with do_route = 1, the activation type with do_route = 2.  The
- * router uses the fp16 gate of `layer`, rounded to bf16 for bf16 activations. */
+ * router uses the fp16 gate of `layer`, rounded to bf16 for bf16 activations.
+ * An expert whose words begin off a whole row, or its scales at an offset that is no multiple of 8: batches of few rows per
+ * expert leave it out and report it (error word 22), larger ones compute it. */
 int gemq_moe_prefill(const gemq_moe_layer_t* layer, const void* x, void* out, int64_t* idx, void* w,
                      void* logits, int tokens, int do_route, int route_mode, int x_is_bf16,
                      void* scratch, size_t scratch_bytes, gemq_stream_t stream);

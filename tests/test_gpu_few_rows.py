@@ -277,3 +277,60 @@ def test_moe_bit_width_tables(T):
     blk._layer.s3.nbits = 3
     assert torch.equal(blk._prefill(x, 2, False)[0], want)
     assert blk.prefill_error_code(T) == 0
+
+
+def _shift(blk, words, scales):
+    """The block's experts with `words` int32 and `scales` fp16 elements ahead of each."""
+    for name in ("w1", "w2", "w3"):
+        for suffix, table, gap in (("wq", "wq_strides", words), ("scales", "zs_strides", scales), ("zeros", "zs_strides", scales)):
+            old = getattr(blk, f"{name}_{suffix}")
+            at = getattr(blk, f"{name}_{table}").tolist() + [old.numel()]
+            new = torch.zeros(-(-(old.numel() + gap * len(at)) // old.shape[1]), old.shape[1], dtype=old.dtype, device=old.device)
+            for e in range(len(at) - 1):
+                new.view(-1)[at[e] + gap * (e + 1):at[e + 1] + gap * (e + 1)] = old.reshape(-1)[at[e]:at[e + 1]]
+            setattr(blk, f"{name}_{suffix}", new)
+        for table, gap in (("wq_strides", words), ("zs_strides", scales)):
+            t = getattr(blk, f"{name}_{table}")
+            setattr(blk, f"{name}_{table}", t + gap * torch.arange(1, t.numel() + 1, dtype=torch.int32, device=t.device))
+    blk._build_layer(blk._layer.route_mode, bool(blk._layer.renorm), blk._layer.shared_ffn)
+
+
+@pytest.mark.parametrize("words,scales", [(0, 8), (5, 0), (32, 0), (0, 3), (9, 1)])
+def test_moe_experts_off_whole_rows(words, scales):
+    """Experts that begin off a whole row of words or a 16-byte boundary of scales: the GEMM's producers load them, few-row launches
+    leave them out and say so.  Eight scales more are a boundary."""
+    layer = MF.make_layer("mixtral", D=384, Fd=256, E=4, A=1, bits=[1, 2, 3, 4], seed=7, gate_std=0.02)
+    blk, moved = MF.gpu_block(layer), MF.gpu_block(layer)
+    _shift(moved, words, scales)
+    g = torch.Generator().manual_seed(words + scales)
+    for T in (16, 300, 1200):
+        x, w = torch.randn(T, 384, generator=g).half().cuda(), torch.rand(T, 1, generator=g).half().cuda()
+        sel = torch.randint(0, 4, (T, 1), generator=g).cuda()
+        want = blk._prefill(x, 1, True, routing=(w, sel))[0]
+        got = moved._prefill(x, 1, True, routing=(w, sel))[0]
+        if T == 16 and (words or scales % 8):
+            assert moved.prefill_error_code(T) == 22 and not got.any()
+        else:
+            assert moved.prefill_error_code(T) == 0 and torch.equal(got, want)
+        assert blk.prefill_error_code(T) == 0
+
+
+@pytest.mark.parametrize("b", [1, 2, 3, 4])
+def test_gemm_of_unaligned_views(b):
+    """A dense matrix whose words, scales or offsets begin off a 16-byte boundary is loaded by the GEMM's producers: the same sums."""
+    from gemq_b200.kernels import dequant_gemm
+    from gemq_b200.kernels._runtime import error_word
+    N, K, M = 288, 1408, 200
+    lin = MF.draw_linear(np.random.default_rng(b), N, K, b)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    mats = [t(lin["wq"]), t(lin["s"]), t(lin["z"])]
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(b)).half().cuda()
+    want = dequant_gemm(x, *mats, b, 128)
+    W = O.dequantize(lin["wq"], lin["s"], lin["z"], b, 128, K).astype(np.float64)
+    assert rel_fro(want.double().cpu().numpy(), x.double().cpu().numpy() @ W) < 2.0 ** -11  # one rounding of the result
+    for which in range(3):
+        m = list(mats)
+        flat = torch.empty(m[which].numel() + 1, dtype=m[which].dtype, device="cuda")
+        m[which] = flat[1:].view_as(m[which]).copy_(m[which])
+        assert m[which].data_ptr() % 16 and torch.equal(dequant_gemm(x, *m, b, 128), want)
+    assert int(error_word(x.device).item()) == 0
