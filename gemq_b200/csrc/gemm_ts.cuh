@@ -100,7 +100,8 @@ struct alignas(64) Params {
   int staged;              // the words come through shared memory
 };
 
-// The TMA warp brings a stage's packed words, scales and offsets, too, up to three stages ahead of the producers.  The words
+// The TMA warp brings a stage's packed words, scales and offsets, too.  It asks for them once the stage is released; the group
+// that fills the stage comes from the one two before it, so they are about one stage ahead of it.  The words
 // of 128 k have a place of their own up to 3 bits; at 4 bits they take the quarter of the stage that tiles of up to 192
 // tokens leave free (above, the MMAs take longer anyway).
 constexpr int kStagedTokens = 192, kWordsAt = kStagedTokens / 2 * 2 * kRowBytes, kWordBytes = 14 * kCols * 4;
@@ -353,7 +354,7 @@ template <bool UP>
 struct TileWords {
   const CUtensorMap* map[2];
   const __half* scales[4];  // of the CTA's first column: [matrix][scales, offsets]
-  int bits, row0, col, bytes;
+  int bits, row0, col;
   uint32_t all, parts;      // bytes of a stage; of a row of scales
   size_t N;
   int G;
@@ -468,13 +469,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   constexpr uint32_t kWordStep = B == 4 ? kStageBytes : kWordBytes;
   const uint32_t words0 = (B == 4 ? smem_u32(S.b[0]) + kWordsAt : smem_u32(S.packed[0])) + mi * stage_rows(B) * kPitch + 4 * in_row;
   const uint32_t scales0 = smem_u32(S.scales[0]) + mi * 256 + 2 * in_row;
-  auto take = [&](Set& R) {
-    if (kb >= real) {
-#pragma unroll
-      for (int i = 0; i < NW; ++i) R.w[i] = 0u;
-      R.s = R.z = __float2half_rn(0.f);
-      return;
-    }
+  auto take = [&](Set& R) {  // whole stages: no block of zeros
     // The stage's release first.  The TMA warp flips words[s] in every use of the stage, these warps look at it in staged tiles only;
     // before the MMAs of its last use are complete, that use's own phase may be open, and the parity of the one before lets
     // the wait pass (a staged tile behind one that was not: words of another tile, or none).  They are complete only after the
@@ -529,25 +524,24 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
       take(ring[0]);
       put(ring[0]);
     }
-    return;
-  }
-  fetch(ring[0], kb);
+  } else {
+    fetch(ring[0], kb);
 #pragma unroll 1
-  for (;;) {
-    if constexpr (STAGED) {
-    } else if constexpr (B == 3) {  // one copy of the long body, the sets are moved
-      if (kb + kGroups < kb1) fetch(ring[1], kb + kGroups);
-      put(ring[0]);
-      kb += kGroups;
-      if (kb >= kb1) return;
-      ring[0] = ring[1];
-    } else {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (kb + kGroups < kb1) fetch(ring[u ^ 1], kb + kGroups);
-        put(ring[u]);
+    for (;;) {
+      if constexpr (B == 3) {  // one copy of the long body, the sets are moved
+        if (kb + kGroups < kb1) fetch(ring[1], kb + kGroups);
+        put(ring[0]);
         kb += kGroups;
         if (kb >= kb1) return;
+        ring[0] = ring[1];
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (kb + kGroups < kb1) fetch(ring[u ^ 1], kb + kGroups);
+          put(ring[u]);
+          kb += kGroups;
+          if (kb >= kb1) return;
+        }
       }
     }
   }
