@@ -139,8 +139,8 @@ def test_moe_large_tiles(rows, bits):
 
 @pytest.mark.parametrize("D,Fd,E", [(128, 10240, 16), (10240, 128, 32)])
 def test_moe_many_tiles_per_pair(D, Fd, E):
-    """More than sixteen tiles for every pair of CTAs, so the places through which a pair's tile numbers are handed over are
-    used again twice; k of one stage, the shortest there is."""
+    """More than sixteen tiles for every pair of CTAs with k of one stage, the shortest there is: barriers whose phases run through
+    the ring many times within a launch, tiles of all widths in turn (and in the other launch, k of eighty stages)."""
     bits = [1, 2, 3, 4] * (E // 4)
     layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=E, A=1, bits=bits, seed=11, gate_std=0.02)
     blk = MF.gpu_block(layer)
@@ -157,11 +157,11 @@ def test_moe_many_tiles_per_pair(D, Fd, E):
     assert torch.equal(out, blk._prefill(x.cuda(), 1, True, routing=(w.cuda(), sel.cuda()))[0])
 
 
-@pytest.mark.parametrize("rows", [[128, 129, 40, 7], [192, 193, 130, 33]])
-@pytest.mark.parametrize("bits", [[1, 2, 3, 4], [3, 4, 1, 2]])
+@pytest.mark.parametrize("rows", [[128, 129, 40, 7], [192, 193, 130, 33], [161, 177, 224, 192]])
+@pytest.mark.parametrize("bits", [[1, 2, 3, 4], [3, 4, 1, 2], [4, 4, 4, 3]])
 def test_moe_staged_words(rows, bits):
-    """Tiles up to and past the tokens whose stages also hold the packed words, reduction
-    lengths that end inside a 3-bit word."""
+    """4-bit tiles up to and past the 192 tokens whose stages also hold their packed words, among them those whose activations
+    end where the words begin (161 to 192 rows), the other widths at the same sizes; reduction lengths that end inside a 3-bit word."""
     g = torch.Generator().manual_seed(sum(rows))
     sel = torch.cat([torch.full((n,), e, dtype=torch.int64) for e, n in enumerate(rows)])
     T = sel.numel()
@@ -171,11 +171,12 @@ def test_moe_staged_words(rows, bits):
         layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=4, A=1, bits=bits, seed=5, gate_std=0.02)
         blk = MF.gpu_block(layer)
         w1, w3, w2, _ = MF.oracle_parts(layer)
-        x = torch.randn(T, D, generator=g).half()
-        out = blk._prefill(x.cuda(), 1, True, routing=(w.cuda(), sel.cuda()))[0]
-        assert blk.prefill_error_code(T) == 0
-        ref = O.moe_reference_fp32(x, w.float(), sel, w1, w3, w2).numpy()
-        assert rel_fro(out.float().cpu().numpy(), ref) < REL_FRO_TOL
+        for dtype in (torch.float16, torch.bfloat16):
+            x = torch.randn(T, D, generator=g).to(dtype)
+            out = blk._prefill(x.cuda(), 1, True, routing=(w.to(dtype).cuda(), sel.cuda()))[0]
+            assert blk.prefill_error_code(T) == 0
+            ref = O.moe_reference_fp32(x.float(), w.to(dtype).float(), sel, w1, w3, w2).numpy()
+            assert rel_fro(out.float().cpu().numpy(), ref) < REL_FRO_TOL
 
 
 def _reference(layer, x, w, sel):
