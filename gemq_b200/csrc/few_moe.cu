@@ -526,8 +526,9 @@ static bool init_attrs() {
 
 // Layers and batches this path takes: group 128, extents in whole groups, and on average at most
 // kFewAverage rows per expert (above, the tensor cores' de-quantised tiles, whose cost does not grow with the rows,
-// win): 24 rows per expert take 323 against 452 us (8 experts of 4096 x 14336), 214 against 239 (64 of
-// 2048 x 1408), 135 against 129 (32 of them); 32 rows 393 against 454, 266 against 259, 153 against 133.
+// win): 20 rows per expert take 295 against 363 us (8 experts of 4096 x 14336), 199 against 207 (64 of 2048 x 1408), 130 against 130
+// (32 of them), 109 against 121 (16 of 2048 x 3456); 24 rows 330 against 364, 220 against 209, 139 against 128, 120 against
+// 122; 32 rows 398 against 365, 266 against 214, 162 against 131, 142 against 124.
 constexpr int kFewAverage = 24;
 bool moe_few_rows_ok(const gemq_moe_layer_t* L, int tokens) {
   const int D = L->hidden, F = L->ffn, SF = L->shared_ffn;

@@ -56,7 +56,10 @@ int launch_down(const Params& P, int tiles_bound, cudaStream_t stream) { return 
 // A tile's time is its k-blocks': the de-quantisation of 256 columns (by bit width, whatever the tokens), or the MMAs of
 // many tokens.  Few tokens and few columns leave most of the 74 pairs without a tile, so the tokens go to smaller tiles
 // (more of them, each with its own de-quantisation) or k is split (fp32 parts through memory and a second launch),
-// whichever is estimated to end first.  4096 x 4096, 2 bits, 32 rows: 16.0 us unsplit, on 16 pairs; 14336 x 1024: 48, on 4.
+// whichever is estimated to end first.  4096 x 4096, 2 bits, 32 rows: 20.9 us unsplit, on 16 pairs, 11.1 as taken; 14336 x 1024:
+// 62.2, on 4, and 11.3.  The block times below are of the kernel whose producers loaded the words, back to back.  Now a block
+// takes 0.27, 0.28, 0.35, 0.29 us (1 to 4 bits, 32 rows; 0.30, 0.31, 0.38, 0.33 at 128 with every pair busy), so 1- and
+// 2-bit matrices are estimated too low: 256 rows of 4096 x 4096 are left whole, 21.9 us, where 3 and 4 bits in parts take 18.
 LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split) {
   static const float block_us[4] = {0.20f, 0.20f, 0.39f, 0.25f};
   const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, KB = K / kBK, ct = cdiv(N, 2 * kCols);
