@@ -51,14 +51,14 @@ constexpr int kRowBytes = kBK * 2;
 constexpr int kStages = 4;
 constexpr int kProducers = 16;
 constexpr int kGroups = kProducers / 4;
-constexpr int kTmaWarp = kProducers, kMmaWarp = kProducers + 1, kEpiWarp = kProducers + 2;
+constexpr int kTmaWarp = kProducers, kMmaWarp = kProducers + 1, kWordWarp = kProducers + 2, kEpiWarp = kProducers + 4;
 constexpr int kThreads = 32 * (kEpiWarp + 4);
-constexpr int kOutPitch = kCols * 2 + 16;  // bytes of a staged row: reads of a column of rows hit all banks
+constexpr int kOutPitch = kCols * 2;  // bytes of a staged row of results, its 16-byte pieces swizzled by the row
 constexpr int kStageBytes = kTokens / 2 * 2 * kRowBytes;  // half of the tokens
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemA = 256;   // A ring behind the accumulators: 64 columns per stage
 
-enum { kErrFull = 11, kErrEmpty = 13, kErrAcc = 14, kErrDrained = 15 };
+enum { kErrFull = 11, kErrEmpty = 13, kErrAcc = 14, kErrDrained = 15, kErrTile = 16 };
 enum { kOutUp = 0,      // silu(gate) * up, fp16, stored in the order of the down projection's words
        kOutDown = 1,    // times the row's routing weight, fp16
        kOutLinear = 2,  // activation type
@@ -100,21 +100,36 @@ struct alignas(64) Params {
   int staged;              // the words come through shared memory
 };
 
-// The TMA warp brings a stage's packed words, scales and offsets, too.  It asks for them once the stage is released; the group
-// that fills the stage comes from the one two before it, so they are about one stage ahead of it.  The words
-// of 128 k have a place of their own up to 3 bits; at 4 bits they take the quarter of the stage that tiles of up to 192
-// tokens leave free (above, the MMAs take longer anyway).
-constexpr int kStagedTokens = 192, kWordsAt = kStagedTokens / 2 * 2 * kRowBytes, kWordBytes = 14 * kCols * 4;
-static_assert(kWordsAt + 16 * kCols * 4 <= kStageBytes, "128 k of 4 bits");
+// Packed words, scales and offsets of 128 k have a ring of their own: a place is asked for again as soon as the producers hold
+// its words in registers, which is two to three thousand cycles before they are wanted.
+constexpr int kWordBytes = 16 * kCols * 4;  // 4 bits
 // Packed rows of 128 k; 3-bit rows from the one in which the first code lies.
 __host__ __device__ constexpr int stage_rows(int bits) { return bits == 3 ? 14 : 4 * bits; }
+
+// A tile of the launch, as one CTA of the pair sees it.
+struct alignas(16) Tile {
+  int fam, expert, row0, rows, col0;
+  int kb0, kbn, part;      // its k-blocks, its part of k
+  int bits, out_bits;      // of its matrices, of the matrix that reads h
+  int odd;                 // its matrices do not begin at whole rows and 16-byte boundaries
+  int woff, wrow;          // where its packed words begin: words, rows
+  long long zoff[2];       // ... its scales and offsets
+  // tokens of the MMA (32, 64, ..), of which each CTA brings half
+  __device__ __forceinline__ int n() const { return (rows + 31) & ~31; }
+  // first accumulator column of the CTA's tile number j
+  __device__ __forceinline__ int acc(uint32_t j) const { return rows <= kTokens / 2 ? static_cast<int>(j & 1) * (kTokens / 2) : 0; }
+};
+constexpr int kTileSlots = 8;
 
 struct Smem {
   alignas(1024) unsigned char b[kStages][kStageBytes];
   alignas(16) unsigned char out[kTokens * kOutPitch];  // accumulators rounded to 16 bits
   alignas(128) unsigned char packed[kStages][kWordBytes];
   alignas(16) unsigned char scales[kStages][kCols * 4];  // of the stage's group: [matrix][scales, offsets][columns]
-  alignas(8) unsigned long long full[kStages], empty[kStages], words[kStages], acc_full[2], drained[2];  // [2]: by the tile's parity
+  alignas(8) unsigned long long full[kStages], empty[kStages], words[kStages], freed[kStages];
+  unsigned long long acc_full[2], drained[2];  // by the tile's parity
+  unsigned long long tile_full[kTileSlots], tile_free[kTileSlots];
+  Tile tiles[kTileSlots];
   uint32_t tmem_base;
 };
 
@@ -289,110 +304,135 @@ __device__ __forceinline__ void dequant_b3(const Exps<3>& X, uint32_t (&pr)[40],
   }
 }
 
-// A tile of the launch, as one CTA of the pair sees it.
-struct Tile {
-  int fam, expert, row0, rows, col0;
-  int odd;             // its matrices do not begin at whole rows and 16-byte boundaries
-  int kb0, kbn, part;  // its k-blocks, its part of k
-  // tokens of the MMA (32, 64, ..), of which each CTA brings half
-  __device__ __forceinline__ int n() const { return (rows + 31) & ~31; }
-  // first accumulator column of the CTA's tile number j
-  __device__ __forceinline__ int acc(uint32_t j) const { return rows <= kTokens / 2 ? static_cast<int>(j & 1) * (kTokens / 2) : 0; }
+// The tiles of a launch, read from the list and the experts' tables by the second word warp of a CTA for all roles.  Each step uses
+// what the one before it has loaded: three reads from L2 in a row, 1500 to 2500 cycles where every role did them for itself
+// when it got to the tile, in which no MMA ran.
+template <int COLS, bool LINEAR>  // COLS: columns of a CTA along N (gate/up: 64)
+struct TileReader {
+  const Params& P;
+  const int rank;
+  int n_tiles;
+  Tile t;
+  int4 d;                            // step 0
+  int bits, out_bits, woff, zoff[2];  // step 1
+  __device__ __forceinline__ TileReader(const Params& p, int r) : P(p), rank(r) { n_tiles = LINEAR ? 0 : *P.n_tiles; }
+  __device__ __forceinline__ void find(int idx) {
+    t = Tile{};
+    if (LINEAR) {
+      t.kbn = P.fam[0].K / kBK;
+      if (P.splits > 1) {
+        t.part = idx % P.splits;
+        idx /= P.splits;
+        t.kb0 = t.part * P.split_kb;
+        t.kbn = min(P.split_kb, t.kbn - t.kb0);
+      }
+      const int ct = P.fam[0].col_tiles, mt = idx / ct;
+      t.col0 = (2 * (idx - mt * ct) + rank) * COLS;
+      d = make_int4(P.expert ? static_cast<int>(*P.expert) : 0, mt * P.tile_rows, min(P.tile_rows, P.rows - mt * P.tile_rows), 0);
+    } else {
+      const int sh = P.shared_tiles * P.fam[1].col_tiles;
+      t.fam = idx < sh ? 1 : 0;
+      const int i = t.fam ? idx : idx - sh, ct = P.fam[t.fam].col_tiles, mt = (t.fam ? 0 : P.shared_tiles) + i / ct;
+      t.kbn = P.fam[t.fam].K / kBK;
+      t.col0 = (2 * (i % ct) + rank) * COLS;
+      d = make_int4(0, 0, 0, 0);
+      if (mt < n_tiles) d = P.tiles[mt];
+    }
+  }
+  __device__ __forceinline__ void look_up() {
+    t.expert = d.x;
+    t.row0 = d.y;
+    t.rows = max(d.z, 0);
+    t.odd = d.w;
+    const Family& F = P.fam[t.fam];
+    const int e = t.expert;
+    bits = F.bits;
+    out_bits = F.out_bits;
+    woff = zoff[0] = zoff[1] = 0;
+    if (t.rows > 0 && e >= 0) {
+      if (F.nbits) bits = F.nbits[e];
+      if (F.out_nbits) out_bits = F.out_nbits[e];
+      if (F.wq_strides) woff = F.wq_strides[e];
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+        if (F.zs_strides[m]) zoff[m] = F.zs_strides[m][e];
+    }
+  }
+  __device__ __forceinline__ void finish() {
+    const Family& F = P.fam[t.fam];
+    t.bits = clamp_bits(bits);  // indexes the maps of packed words
+    t.out_bits = clamp_bits(out_bits);
+    t.woff = woff;
+    t.wrow = static_cast<int>(static_cast<unsigned>(woff) / static_cast<unsigned>(F.N));
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+      t.zoff[m] = t.expert < 0 ? 0 : (F.zs_strides[m] ? zoff[m] : static_cast<long long>(t.expert) * (F.K / F.G) * F.N);
+  }
+  // step 0, 1, 2 of the CTA's tile j, number idx of the launch; step 2 hands it over
+  __device__ __forceinline__ void step(Smem& S, int n, int idx, uint32_t j, int* err) {
+    if (n == 0) find(idx);
+    if (n == 1) look_up();
+    if (n == 2) {
+      finish();
+      const uint32_t s = j % kTileSlots;
+      mbar_sleep_wait(&S.tile_free[s], ((j / kTileSlots) & 1) ^ 1, err, kErrTile);
+      if ((threadIdx.x & 31) == 0) {
+        S.tiles[s] = t;
+        mbar_arrive(&S.tile_full[s]);
+      }
+      __syncwarp();
+    }
+  }
 };
 
-template <int COLS, bool LINEAR>  // COLS: columns of a CTA along N (gate/up: 64)
-__device__ __forceinline__ bool get_tile(const Params& P, int idx, int rank, Tile& t) {
-  if (LINEAR) {
-    const Family& F = P.fam[0];
-    t.part = 0;
-    t.kb0 = 0;
-    t.kbn = F.K / kBK;
-    if (P.splits > 1) {
-      t.part = idx % P.splits;
-      idx /= P.splits;
-      t.kb0 = t.part * P.split_kb;
-      t.kbn = min(P.split_kb, t.kbn - t.kb0);
-    }
-    const int mt = idx / F.col_tiles;
-    if (mt * P.tile_rows >= P.rows) return false;
-    t.fam = t.odd = 0;
-    t.expert = P.expert ? static_cast<int>(*P.expert) : 0;
-    t.row0 = mt * P.tile_rows;
-    t.rows = min(P.tile_rows, P.rows - t.row0);
-    t.col0 = (2 * (idx - mt * F.col_tiles) + rank) * COLS;
-    return true;
-  }
-  const int sh = P.shared_tiles * P.fam[1].col_tiles;
-  const int fam = idx < sh ? 1 : 0;
-  const int i = fam ? idx : idx - sh;
-  const int ct = P.fam[fam].col_tiles;
-  const int mt = (fam ? 0 : P.shared_tiles) + i / ct;
-  if (mt >= *P.n_tiles) return false;
-  const int4 d = P.tiles[mt];
-  t.fam = fam;
-  t.part = t.kb0 = 0;
-  t.kbn = P.fam[fam].K / kBK;
-  t.expert = d.x;
-  t.row0 = d.y;
-  t.rows = d.z;
-  t.odd = d.w;
-  t.col0 = (2 * (i % ct) + rank) * COLS;
-  return true;
+__device__ __forceinline__ bool staged(const Params& P, const Tile& t) { return P.staged && !t.odd; }
+
+// The launch's tiles in the CTA's order, as its tile warp leaves them; nullptr: no more.
+__device__ __forceinline__ const Tile* next_tile(Smem& S, uint32_t j, int* err) {
+  const uint32_t s = j % kTileSlots;
+  if (!mbar_sleep_wait(&S.tile_full[s], (j / kTileSlots) & 1, err, kErrTile)) return nullptr;
+  return S.tiles[s].rows > 0 ? &S.tiles[s] : nullptr;
+}
+__device__ __forceinline__ void done_tile(Smem& S, uint32_t j) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(&S.tile_free[j % kTileSlots]);
 }
 
-__device__ __forceinline__ int tile_bits(const Params& P, const Tile& t) {
-  const Family& F = P.fam[t.fam];
-  return clamp_bits(F.nbits && t.expert >= 0 ? F.nbits[t.expert] : F.bits);  // indexes the maps of packed words
-}
-
-__device__ __forceinline__ bool staged(const Params& P, const Tile& t, int bits) {
-  return P.staged && !t.odd && (bits <= 3 || t.rows <= kStagedTokens);
-}
-
-// Words, scales and offsets of a tile, as its CTA's TMA warp brings them into the stages.
+// What the two word warps bring into a CTA's stages of a tile: the first one the packed words of the (first) matrix as a tiled copy,
+// the second one the scales and offsets, 16 bytes a lane, and the words of the second matrix.  (Scales and offsets as bulk
+// copies cost the issuing lane 250 to 300 cycles each: with two or four a stage they set the pace of everything, 950 cycles.)
 template <bool UP>
 struct TileWords {
-  const CUtensorMap* map[2];
-  const __half* scales[4];  // of the CTA's first column: [matrix][scales, offsets]
+  static constexpr int kColumns = UP ? kCols / 2 : kCols;
+  const CUtensorMap* map;
+  const __half* sc;  // where the lane copies from
   int bits, row0, col;
-  uint32_t all, parts;      // bytes of a stage; of a row of scales
+  bool on;           // its columns exist
   size_t N;
-  int G;
-  __device__ __forceinline__ void init(const Params& P, const Tile& t) {
+  int at, per;       // stages since the group's first, of a group
+  __device__ __forceinline__ void init(const Params& P, const Tile& t, int which, int lane) {
     const Family& F = P.fam[t.fam];
-    bits = tile_bits(P, t);
+    bits = t.bits;
     N = F.N;
-    G = F.G;
+    per = F.G / kStageK;
     col = t.col0;
-    const bool stacked = t.expert >= 0 && F.wq_strides;
-    row0 = stacked ? static_cast<int>(static_cast<unsigned>(F.wq_strides[t.expert]) / static_cast<unsigned>(F.N)) : 0;
-    const int columns = UP ? kCols / 2 : kCols;
-    const int valid = min(max(F.N - col, 0), columns);
-    parts = 2 * valid;
-#pragma unroll
-    for (int m = 0; m < (UP ? 2 : 1); ++m) {
-      map[m] = &P.w_map[t.fam][m][bits - 1];
-      size_t off = col;
-      if (t.expert >= 0) off += F.zs_strides[m] ? static_cast<size_t>(F.zs_strides[m][t.expert]) : static_cast<size_t>(t.expert) * (F.K / F.G) * N;
-      scales[2 * m] = F.scales[m] + off;
-      scales[2 * m + 1] = F.zeros[m] + off;
-    }
-    all = (UP ? 2 : 1) * (stage_rows(bits) * columns * 4 + 2 * parts);
+    row0 = t.wrow;
+    map = &P.w_map[t.fam][UP ? which : 0][bits - 1];
+    const bool second = UP && lane >= 16, offsets = UP ? (lane >> 3) & 1 : lane >= 16;
+    const int c = 8 * (lane & (UP ? 7 : 15)), sb0 = t.kb0 / 2;
+    on = col + c < F.N;
+    at = sb0 % per;
+    const size_t off = static_cast<size_t>(t.zoff[second ? 1 : 0]) + col + c + static_cast<size_t>(sb0 / per) * N;
+    sc = (offsets ? (second ? F.zeros[1] : F.zeros[0]) : (second ? F.scales[1] : F.scales[0])) + off;
   }
-  __device__ __forceinline__ void load(unsigned char* at, unsigned char* sc, unsigned long long* bar, int kb) const {
-    const int k0 = kb * kBK, row = row0 + (bits == 3 ? k0 / 10 : k0 * bits / 32), g = k0 / G;
-    mbar_arrive_expect_tx(bar, all);
-#pragma unroll
-    for (int m = 0; m < (UP ? 2 : 1); ++m) {
-      tma_load_2d(at + m * stage_rows(bits) * kCols * 2, map[m], col, row, bar);
-#pragma unroll
-      for (int z = 0; z < 2; ++z)
-        if (parts)
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                           smem_u32(sc + m * 256 + z * (UP ? kCols : 2 * kCols))),
-                       "l"(scales[2 * m + z] + static_cast<size_t>(g) * N), "r"(parts), "r"(smem_u32(bar))
-                       : "memory");
-    }
+  __device__ __forceinline__ void load_words(unsigned char* dst, unsigned long long* bar, int kb) const {
+    const int k0 = kb * kBK;
+    mbar_arrive_expect_tx(bar, stage_rows(bits) * kColumns * 4);
+    tma_load_2d(dst, map, col, row0 + (bits == 3 ? k0 / 10 : k0 * bits / 32), bar);
+  }
+  __device__ __forceinline__ void load_scales(uint32_t dst) {  // stages in order
+    if (on) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(sc) : "memory");
+    if (++at == per) { at = 0; sc += N; }
   }
 };
 
@@ -410,13 +450,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   // columns past the end repeat the last one; their results are not stored
   const int col = UP ? T.col0 + 16 * (warp & 3) + (lane & 15) : min(T.col0 + 32 * (warp & 3) + lane, F.N - 1);
   const size_t N = F.N;
-  const int ngroups = F.K / F.G;
-  size_t woff = 0, zoff = 0;
-  if (T.expert >= 0 && F.wq_strides) woff = static_cast<size_t>(F.wq_strides[T.expert]);
-  if (T.expert >= 0) {
-    const int* zs = mi ? F.zs_strides[1] : F.zs_strides[0];
-    zoff = zs ? static_cast<size_t>(zs[T.expert]) : static_cast<size_t>(T.expert) * ngroups * N;
-  }
+  const size_t woff = static_cast<size_t>(T.woff), zoff = static_cast<size_t>(T.zoff[mi]);
   const uint32_t* wp = (mi ? F.wq[1] : F.wq[0]) + woff + col;
   const __half* sp = (mi ? F.scales[1] : F.scales[0]) + zoff + col;
   const __half* zp = (mi ? F.zeros[1] : F.zeros[0]) + zoff + col;
@@ -466,18 +500,25 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   // STAGED
   constexpr uint32_t kPitch = UP ? kCols * 2 : kCols * 4;
   const int in_row = UP ? 16 * (warp & 3) + (lane & 15) : 32 * (warp & 3) + lane;
-  constexpr uint32_t kWordStep = B == 4 ? kStageBytes : kWordBytes;
-  const uint32_t words0 = (B == 4 ? smem_u32(S.b[0]) + kWordsAt : smem_u32(S.packed[0])) + mi * stage_rows(B) * kPitch + 4 * in_row;
+  const uint32_t words0 = smem_u32(S.packed[0]) + mi * stage_rows(B) * kPitch + 4 * in_row;
   const uint32_t scales0 = smem_u32(S.scales[0]) + mi * 256 + 2 * in_row;
-  auto take = [&](Set& R) {  // whole stages: no block of zeros
-    // The stage's release first.  The TMA warp flips words[s] in every use of the stage, these warps look at it in staged tiles only;
-    // before the MMAs of its last use are complete, that use's own phase may be open, and the parity of the one before lets
-    // the wait pass (a staged tile behind one that was not: words of another tile, or none).  They are complete only after the
-    // TMA warp had arrived for that use.  It asks for the words of this one behind the same release: nothing is lost.
+  // The barriers of the words flip in every use of a stage, staged or not: a use and the one before it are the same warps'.
+  auto words_ready = [&]() { mbar_sleep_wait(&S.words[s], par ^ 1u, err, kErrFull); };
+  auto words_free = [&]() {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&S.freed[s]);
+  };
+  auto stage_free = [&]() {
+    if (!STAGED) {
+      words_ready();
+      words_free();
+    }
     mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
-    mbar_sleep_wait(&S.words[s], par ^ 1u, err, kErrFull);
+  };
+  auto take = [&](Set& R) {  // whole stages: no block of zeros
+    words_ready();
     const int row = B == 3 ? kb * kBK / 10 - (kb & ~1) * kBK / 10 : (kb & 1) * 2 * B;
-    const uint32_t w = words0 + s * kWordStep + row * kPitch, sc = scales0 + s * (kCols * 4);
+    const uint32_t w = words0 + s * kWordBytes + row * kPitch, sc = scales0 + s * (kCols * 4);
 #pragma unroll
     for (int i = 0; i < NW; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(R.w[i]) : "r"(w + i * kPitch) : "memory");
     unsigned short a, b;
@@ -485,6 +526,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(sc + kPitch / 2) : "memory");
     R.s = __ushort_as_half(a);
     R.z = __ushort_as_half(b);
+    words_free();
   };
   auto put = [&](const Set& cur) {
     const __half2 s2 = __half2half2(cur.s), z2 = __half2half2(cur.z);
@@ -492,7 +534,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
     if constexpr (B == 3) {
       uint32_t pr[40];
       dequant_b3<BF16>(X, pr, cur.w, s2, z2);
-      if (!STAGED) mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
+      stage_free();
       tc_fence_after_sync();
       switch ((kb * kBK % 10) >> 1) {  // uniform
         case 0: tmem_st32(dst, pr); break;
@@ -505,7 +547,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
       // in two halves: 16 result registers instead of 32
       uint32_t o[16];
       dequant_words<B, BF16, NAT, 0>(X, o, cur.w, s2, z2);
-      if (!STAGED) mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
+      stage_free();
       tc_fence_after_sync();
       tmem_st16(dst, o);
       dequant_words<B, BF16, NAT, 0>(X, o, cur.w + B, s2, z2);
@@ -548,7 +590,8 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
 }
 
 template <bool UP, bool BF16, bool NAT, bool STAGED>
-__device__ __forceinline__ void produce_bits(Smem& S, const Params& P, const Tile& T, int bits, uint32_t base, uint32_t tmem) {
+__device__ __forceinline__ void produce_bits(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
+  const int bits = T.bits;
   if (bits == 1) produce<UP, BF16, NAT, 1, STAGED>(S, P, T, base, tmem);
   else if (bits == 2) produce<UP, BF16, NAT, 2, STAGED>(S, P, T, base, tmem);
   else if (bits == 3) produce<UP, BF16, NAT, 3, STAGED>(S, P, T, base, tmem);
@@ -556,9 +599,8 @@ __device__ __forceinline__ void produce_bits(Smem& S, const Params& P, const Til
 }
 template <bool UP, bool BF16, bool NAT>
 __device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
-  const int bits = tile_bits(P, T);
-  if (staged(P, T, bits)) produce_bits<UP, BF16, NAT, true>(S, P, T, bits, base, tmem);
-  else produce_bits<UP, BF16, NAT, false>(S, P, T, bits, base, tmem);
+  if (staged(P, T)) produce_bits<UP, BF16, NAT, true>(S, P, T, base, tmem);
+  else produce_bits<UP, BF16, NAT, false>(S, P, T, base, tmem);
 }
 
 // ---- epilogue --------------------------------------------------------------------------------------
@@ -598,7 +640,8 @@ __device__ __forceinline__ uint32_t pack_act(uint32_t lo, uint32_t hi) {
 // conversions, two stores (a column's values one by one took 16 stores of two bytes).
 template <typename T>
 __device__ __forceinline__ void drain(Smem& S, uint32_t at, int rows, int lq, int lane) {
-  uint32_t dst = smem_u32(S.out) + (8 * (lane >> 4) + (lane & 7)) * kOutPitch + 2 * (32 * lq + 8 * ((lane >> 3) & 1));
+  uint32_t dst = smem_u32(S.out) + (8 * (lane >> 4) + (lane & 7)) * kOutPitch;
+  const uint32_t piece = 4 * lq + ((lane >> 3) & 1), at16[2] = {16 * (piece ^ (lane & 7)), 16 * ((piece + 2) ^ (lane & 7))};
 #pragma unroll 1
   for (int c = 0; c < rows; c += 16, dst += 16 * kOutPitch) {
     uint32_t d[2][8];
@@ -607,7 +650,7 @@ __device__ __forceinline__ void drain(Smem& S, uint32_t at, int rows, int lq, in
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst + 32 * h),
+      asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst + at16[h]),
                    "r"(pack_act<T>(d[h][0], d[h][1])), "r"(pack_act<T>(d[h][2], d[h][3])), "r"(pack_act<T>(d[h][4], d[h][5])),
                    "r"(pack_act<T>(d[h][6], d[h][7]))
                    : "memory");
@@ -645,19 +688,20 @@ __device__ __forceinline__ void word_order(const __half (&h)[32], uint32_t (&o)[
 // 16 columns each in two warps' worth of staged columns).
 __device__ __forceinline__ void finish_up(const Smem& S, const Params& P, const Tile& t, int tid) {
   const Family& F = P.fam[t.fam];
-  const int bits = clamp_bits(F.out_nbits && t.expert >= 0 ? F.out_nbits[t.expert] : F.out_bits);
+  const int bits = t.out_bits;
   const size_t pitch = F.N;
   __half* const out = static_cast<__half*>(F.out) + static_cast<size_t>(t.row0 - F.row0) * pitch + t.col0;
   const int rows = t.rows;
 #pragma unroll 1
   for (int i = tid; i < 2 * rows; i += 128) {
     const int grp = i >= rows ? 1 : 0, row = i - grp * rows;
-    const unsigned char* src = S.out + row * kOutPitch + 128 * grp;
+    const unsigned char* src = S.out + row * kOutPitch;
     __half h[32];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {  // eight columns each
-      const unsigned char* p = src + (q >> 1) * 64 + (q & 1) * 16;
-      const uint4 g = *reinterpret_cast<const uint4*>(p), u = *reinterpret_cast<const uint4*>(p + 32);
+      const int piece = 8 * grp + 4 * (q >> 1) + (q & 1);
+      const uint4 g = *reinterpret_cast<const uint4*>(src + 16 * (piece ^ (row & 7)));
+      const uint4 u = *reinterpret_cast<const uint4*>(src + 16 * ((piece + 2) ^ (row & 7)));
       const __half *gh = reinterpret_cast<const __half*>(&g), *uh = reinterpret_cast<const __half*>(&u);
 #pragma unroll
       for (int k = 0; k < 8; ++k)
@@ -692,7 +736,7 @@ __device__ __forceinline__ void finish_rows(const Smem& S, const Params& P, cons
   const int rows = t.rows;
 #pragma unroll 2
   for (int row = tid >> 4; row < rows; row += 8) {
-    uint4 v = *reinterpret_cast<const uint4*>(S.out + row * kOutPitch + 16 * q);
+    uint4 v = *reinterpret_cast<const uint4*>(S.out + row * kOutPitch + 16 * (q ^ (row & 7)));
     T* e = reinterpret_cast<T*>(&v);
     if (OUT == kOutDown) {
       if (rw) {
@@ -721,11 +765,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&S.full[s], 17);  // in the first CTA: two groups' warps of either CTA, the activation boxes
       mbar_init(&S.empty[s], 1);
-      mbar_init(&S.words[s], 1);
+      mbar_init(&S.words[s], UP ? 34 : 33);  // a tiled copy per matrix, the lanes that copy scales
+      mbar_init(&S.freed[s], 8);               // two groups' warps
     }
     for (int j = 0; j < 2; ++j) {
       mbar_init(&S.acc_full[j], 1);
       mbar_init(&S.drained[j], 8);  // in the first CTA: the epilogue warps of both
+    }
+    for (int j = 0; j < kTileSlots; ++j) {
+      mbar_init(&S.tile_full[j], 1);
+      mbar_init(&S.tile_free[j], kThreads / 32 - (rank == 0 ? 1 : 2));  // all other warps; the second CTA's MMA warp has no work
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -746,48 +795,85 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
   // a short one in the next.
   const int step = static_cast<int>(gridDim.x >> 1), first = static_cast<int>(blockIdx.x >> 1);
   auto tile_of = [&](int i) { return i * step + ((i & 1) ? step - 1 - first : first); };
-  Tile t;
+  int* const err = P.err;
   if (warp < kProducers) {
     uint32_t base = 0;
 #pragma unroll 1
-    for (int i = 0; get_tile<COLS, LINEAR>(P, tile_of(i), rank, t); ++i) {
-      produce_any<UP, BF16, LINEAR>(S, P, t, base, tmem);
-      base += (t.kbn + 1) & ~1;
+    for (uint32_t j = 0; const Tile* t = next_tile(S, j, err); ++j) {
+      produce_any<UP, BF16, LINEAR>(S, P, *t, base, tmem);
+      base += (t->kbn + 1) & ~1;
+      done_tile(S, j);
     }
   } else if (warp == kTmaWarp) {
     uint32_t c = 0;
     const uint32_t full0 = first_cta(&S.full[0]);
-    int* const err = P.err;
-    for (int i = 0; get_tile<COLS, LINEAR>(P, tile_of(i), rank, t); ++i) {
+    for (uint32_t j = 0; const Tile* at = next_tile(S, j, err); ++j) {
+      const Tile t = *at;
+      done_tile(S, j);
       const Family& F = P.fam[t.fam];
       const int SB = (t.kbn + 1) / 2, half = t.n() / 2;
       const int box = (half + 31) / 32;  // in 32 rows: an odd number of 16-row blocks brings the next 16 rows, too
       const uint32_t bytes = 2 * 32 * box * kRowBytes;
       const int row = t.row0 - F.row0 + rank * half;
       const CUtensorMap* const map = &P.b_map[t.fam][box - 1];
-      const bool with_words = staged(P, t, tile_bits(P, t));
-      TileWords<UP> words;
-      if (with_words) words.init(P, t);
       for (int sb = 0; sb < SB; ++sb, ++c) {
         const uint32_t s = c % kStages;
         mbar_sleep_wait(&S.empty[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&S.full[s], 2 * bytes);
-          if (with_words) words.load(words.bits == 4 ? S.b[s] + kWordsAt : S.packed[s], S.scales[s], &S.words[s], t.kb0 + 2 * sb);
-          else mbar_arrive(&S.words[s]);  // the barrier's phases follow the stages
           tma_load_pair(S.b[s], map, row, t.kb0 + 2 * sb, full0 + s * 8);
         }
         __syncwarp();
       }
     }
+  } else if (warp >= kWordWarp && warp < kEpiWarp) {
+    const int which = warp - kWordWarp, lane = static_cast<int>(threadIdx.x & 31);
+    constexpr uint32_t kTilesAhead = 1;
+    TileReader<COLS, LINEAR> reader(P, rank);
+    if (which)
+      for (uint32_t j = 0; j < kTilesAhead; ++j)
+        for (int n = 0; n < 3; ++n) reader.step(S, n, tile_of(j), j, err);
+    uint32_t c = 0;
+    for (uint32_t j = 0; const Tile* next = next_tile(S, j, err); ++j) {
+      const Tile t = *next;
+      done_tile(S, j);
+      int step = which ? 0 : 3;
+      const int SB = (t.kbn + 1) / 2;
+      const bool on = staged(P, t);  // the barrier's phases follow the stages, staged or not
+      TileWords<UP> words;
+      if (on) words.init(P, t, which, lane);
+      const uint32_t at = UP && which && on ? stage_rows(words.bits) * kCols * 2 : 0;
+      for (int sb = 0; sb < SB; ++sb, ++c) {
+        const uint32_t s = c % kStages;
+        const int kb = t.kb0 + 2 * sb;
+        mbar_sleep_wait(&S.freed[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
+        if (which) {
+          if (on) {
+            words.load_scales(smem_u32(S.scales[s]) + 16 * lane);
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&S.words[s])) : "memory");
+          } else {
+            mbar_arrive(&S.words[s]);
+          }
+        }
+        if ((UP || !which) && elect_one()) {
+          if (on) words.load_words(S.packed[s] + at, &S.words[s], kb);
+          else mbar_arrive(&S.words[s]);
+        }
+        __syncwarp();
+        if (step < 3) reader.step(S, step++, tile_of(j + kTilesAhead), j + kTilesAhead, err);
+      }
+      for (; step < 3; ++step) reader.step(S, step, tile_of(j + kTilesAhead), j + kTilesAhead, err);
+    }
   } else if (warp == kMmaWarp && rank == 0) {
     // The whole warp runs the loop and one elected lane issues: descriptors and addresses stay in uniform
     // registers.  (In a one-lane branch every tcgen05.mma cost 85 cycles to issue.)
     uint32_t s = 0, par = 0, j = 0;
+    const Tile* next;
     bool small = true;  // the tile before fits one half of the accumulators
     const uint64_t desc0 = umma_desc_k_sw128(smem_u32(S.b[0]));
-    int* const err = P.err;
-    for (; get_tile<COLS, LINEAR>(P, tile_of(j), rank, t); ++j) {
+    for (; (next = next_tile(S, j, err)) != nullptr; ++j) {
+      const Tile t = *next;
+      done_tile(S, j);
       const int SB = (t.kbn + 1) / 2;
       const uint32_t idesc = umma_idesc_f16(BF16 ? 1 : 0, 2 * kCols, t.n());
       const uint32_t second = ((t.n() / 2 + 31) / 32 * 32 * kRowBytes) >> 4;  // distance of a stage's second k-block
@@ -816,10 +902,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
   }
   if (warp >= kEpiWarp) {
     const int lq = warp & 3, tid = static_cast<int>(threadIdx.x) - 32 * kEpiWarp;
-    uint32_t j = 0;
 #pragma unroll 1
-    for (; get_tile<COLS, LINEAR>(P, tile_of(j), rank, t); ++j) {
-      mbar_sleep_wait(&S.acc_full[j & 1], (j >> 1) & 1, P.err, kErrAcc);
+    for (uint32_t j = 0; const Tile* next = next_tile(S, j, err); ++j) {
+      const Tile t = *next;
+      done_tile(S, j);
+      mbar_sleep_wait(&S.acc_full[j & 1], (j >> 1) & 1, err, kErrAcc);
       tc_fence_after_sync();
       const uint32_t at = tmem + (static_cast<uint32_t>(32 * lq) << 16) + t.acc(j);
       const int column = 32 * lq + static_cast<int>(threadIdx.x & 31);

@@ -29,6 +29,18 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, uint32_t 
       : "memory");
   return ok != 0;
 }
+// Looks once, without waiting.
+__device__ __forceinline__ bool mbar_test_wait(unsigned long long* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait: gives up after kSpinLimit polls, records `code` and returns.  A waiting warp
 // sleeps between polls so that it does not take issue slots from the warps that are working.
 __device__ __forceinline__ void mbar_wait(unsigned long long* bar, uint32_t parity, int* err, int code,
@@ -43,7 +55,8 @@ __device__ __forceinline__ void mbar_wait(unsigned long long* bar, uint32_t pari
 // Bounded wait of a warp that sleeps in hardware until the phase ends (at most 20 us a time, about a second in
 // all).  Without the time hint try_wait comes back after some tens of cycles, and warps that wait long -- for
 // the end of a tile, say -- spend the issue slots of the others.
-__device__ __forceinline__ void mbar_sleep_wait(unsigned long long* bar, uint32_t parity, int* err, int code) {
+__device__ __forceinline__ bool mbar_sleep_wait(unsigned long long* bar, uint32_t parity, int* err, int code) {
+  if (mbar_test_wait(bar, parity)) return true;
   for (int i = 0; i < (1 << 16); ++i) {
     uint32_t ok;
     asm volatile(
@@ -53,9 +66,10 @@ __device__ __forceinline__ void mbar_sleep_wait(unsigned long long* bar, uint32_
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(parity), "r"(20000)
         : "memory");
-    if (ok) return;
+    if (ok) return true;
   }
   atomicExch(err, code);
+  return false;
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 // Tiled TMA load of one box at element coordinates (x = column, y = row); x * element size
