@@ -100,8 +100,8 @@ struct alignas(64) Params {
   int staged;              // the words come through shared memory
 };
 
-// Packed words, scales and offsets of 128 k have a ring of their own: a place is asked for again as soon as the producers hold
-// its words in registers, which is two to three thousand cycles before they are wanted.
+// Packed words, scales and offsets of 128 k have a ring of their own: a place is asked for again as soon as the producers are
+// done with its words, not when the MMAs release the stage: about three stages before the next ones are wanted.
 constexpr int kWordBytes = 16 * kCols * 4;  // 4 bits
 // Packed rows of 128 k; 3-bit rows from the one in which the first code lies.
 __host__ __device__ constexpr int stage_rows(int bits) { return bits == 3 ? 14 : 4 * bits; }
@@ -526,7 +526,6 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(sc + kPitch / 2) : "memory");
     R.s = __ushort_as_half(a);
     R.z = __ushort_as_half(b);
-    words_free();
   };
   auto put = [&](const Set& cur) {
     const __half2 s2 = __half2half2(cur.s), z2 = __half2half2(cur.z);
@@ -553,6 +552,9 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
       dequant_words<B, BF16, NAT, 0>(X, o, cur.w + B, s2, z2);
       tmem_st16(dst + 16, o);
     }
+    // Behind the stores, which hold what came of the words: an arrival right behind the loads overtook them (shared-memory reads that
+    // wait behind the epilogue's; the next words were there before 4 to 32 lanes had read the last row).
+    if (STAGED) words_free();
     tmem_wait_st();
     tc_fence_before_sync();
     __syncwarp();
@@ -611,6 +613,13 @@ template <typename T> __device__ __forceinline__ T as_act(float v);
 template <> __device__ __forceinline__ __half as_act<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 as_act<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
+// Waits for the tensor-memory loads into r: what uses r stays behind it (the loads alone define the registers for the compiler).
+template <int N>
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[N]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i])::"memory");
+}
 // 32 lanes x 16 columns into registers.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -619,11 +628,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  tmem_wait_ld(r);
 }
 
 // 16 tokens of 16 lanes: two mma fragments (a thread has two neighbouring tokens of lanes l / 4 and l / 4 + 8) of 8 tokens each.
-__device__ __forceinline__ void tmem_ld_fragments(uint32_t taddr, uint32_t (&r)[8]) {
+__device__ __forceinline__ void tmem_ld_fragments(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr)
@@ -637,23 +646,30 @@ __device__ __forceinline__ uint32_t pack_act(uint32_t lo, uint32_t hi) {
 
 // The accumulators of a warp's 32 weight columns, rounded, to rows of tokens in shared memory.  What the MMAs of the next
 // tile wait for, so few instructions: fragments whose 8 x 8 blocks stmatrix transposes, per 16 tokens two loads, eight
-// conversions, two stores (a column's values one by one took 16 stores of two bytes).
+// conversions, two stores (a column's values one by one took 16 stores of two bytes), the loads of 32 tokens in flight.
 template <typename T>
 __device__ __forceinline__ void drain(Smem& S, uint32_t at, int rows, int lq, int lane) {
   uint32_t dst = smem_u32(S.out) + (8 * (lane >> 4) + (lane & 7)) * kOutPitch;
   const uint32_t piece = 4 * lq + ((lane >> 3) & 1), at16[2] = {16 * (piece ^ (lane & 7)), 16 * ((piece + 2) ^ (lane & 7))};
 #pragma unroll 1
-  for (int c = 0; c < rows; c += 16, dst += 16 * kOutPitch) {
-    uint32_t d[2][8];
-    tmem_ld_fragments(at + c, d[0]);
-    tmem_ld_fragments(at + (16u << 16) + c, d[1]);
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  for (int c = 0; c < rows; c += 32, dst += 32 * kOutPitch) {  // the MMAs' tokens are whole blocks of 32
+    uint32_t d[32];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-      asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst + at16[h]),
-                   "r"(pack_act<T>(d[h][0], d[h][1])), "r"(pack_act<T>(d[h][2], d[h][3])), "r"(pack_act<T>(d[h][4], d[h][5])),
-                   "r"(pack_act<T>(d[h][6], d[h][7]))
-                   : "memory");
+    for (int u = 0; u < 2; ++u) {
+      tmem_ld_fragments(at + c + 16 * u, d + 16 * u);
+      tmem_ld_fragments(at + (16u << 16) + c + 16 * u, d + 16 * u + 8);
+    }
+    tmem_wait_ld(d);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t* v = d + 16 * u + 8 * h;
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst + 16 * u * kOutPitch + at16[h]),
+                     "r"(pack_act<T>(v[0], v[1])), "r"(pack_act<T>(v[2], v[3])), "r"(pack_act<T>(v[4], v[5])),
+                     "r"(pack_act<T>(v[6], v[7]))
+                     : "memory");
+      }
   }
 }
 
@@ -684,6 +700,11 @@ __device__ __forceinline__ void word_order(const __half (&h)[32], uint32_t (&o)[
   }
 }
 
+// The quotient by reciprocal, good to two units of fp32's last place.  The epilogue of a gate/up tile is 16 K of these per CTA: with an
+// IEEE division and every product in fp32, its four warps took longer than the MMAs of a tile of 2048 k (waits of 9 to 15 thousand
+// cycles for the accumulators against 14 thousand of MMAs).
+__device__ __forceinline__ float silu_quick(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
+
 // h = F.silu(x1) * x3 on fp16 tensors, each step rounded: a thread takes 32 columns of a token (x1 and x3 of
 // 16 columns each in two warps' worth of staged columns).
 __device__ __forceinline__ void finish_up(const Smem& S, const Params& P, const Tile& t, int tid) {
@@ -696,16 +717,18 @@ __device__ __forceinline__ void finish_up(const Smem& S, const Params& P, const 
   for (int i = tid; i < 2 * rows; i += 128) {
     const int grp = i >= rows ? 1 : 0, row = i - grp * rows;
     const unsigned char* src = S.out + row * kOutPitch;
-    __half h[32];
+    alignas(4) __half h[32];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {  // eight columns each
       const int piece = 8 * grp + 4 * (q >> 1) + (q & 1);
       const uint4 g = *reinterpret_cast<const uint4*>(src + 16 * (piece ^ (row & 7)));
       const uint4 u = *reinterpret_cast<const uint4*>(src + 16 * ((piece + 2) ^ (row & 7)));
-      const __half *gh = reinterpret_cast<const __half*>(&g), *uh = reinterpret_cast<const __half*>(&u);
+      const __half2 *gh = reinterpret_cast<const __half2*>(&g), *uh = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        h[8 * q + k] = __float2half_rn(__half2float(__float2half_rn(silu_f32(__half2float(gh[k])))) * __half2float(uh[k]));
+      for (int k = 0; k < 4; ++k) {
+        const float2 v = __half22float2(gh[k]);
+        *reinterpret_cast<__half2*>(h + 8 * q + 2 * k) = __hmul2(__floats2half2_rn(silu_quick(v.x), silu_quick(v.y)), uh[k]);
+      }
     }
     uint32_t o[16];
     if (bits == 1) word_order<32>(h, o);
@@ -738,11 +761,11 @@ __device__ __forceinline__ void finish_rows(const Smem& S, const Params& P, cons
   for (int row = tid >> 4; row < rows; row += 8) {
     uint4 v = *reinterpret_cast<const uint4*>(S.out + row * kOutPitch + 16 * (q ^ (row & 7)));
     T* e = reinterpret_cast<T*>(&v);
-    if (OUT == kOutDown) {
+    if constexpr (OUT == kOutDown) {
       if (rw) {
-        const float f = __half2float(rw[row]);
+        const __half2 f = __half2half2(rw[row]);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) e[k] = as_act<T>(as_float<T>(e[k]) * f);
+        for (int k = 0; k < 4; ++k) reinterpret_cast<__half2*>(&v)[k] = __hmul2(reinterpret_cast<__half2*>(&v)[k], f);
       }
     } else if (has_bias) {
 #pragma unroll
@@ -774,7 +797,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     }
     for (int j = 0; j < kTileSlots; ++j) {
       mbar_init(&S.tile_full[j], 1);
-      mbar_init(&S.tile_free[j], kThreads / 32 - (rank == 0 ? 1 : 2));  // all other warps; the second CTA's MMA warp has no work
+      mbar_init(&S.tile_free[j], kThreads / 32 - (rank == 0 ? 0 : 1));  // every warp; the second CTA's MMA warp has no work
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
