@@ -398,9 +398,9 @@ __device__ __forceinline__ void done_tile(Smem& S, uint32_t j) {
   if ((threadIdx.x & 31) == 0) mbar_arrive(&S.tile_free[j % kTileSlots]);
 }
 
-// What the two word warps bring into a CTA's stages of a tile: the first one the packed words of the (first) matrix as a tiled copy,
-// the second one the scales and offsets, 16 bytes a lane, and the words of the second matrix.  (Scales and offsets as bulk
-// copies cost the issuing lane 250 to 300 cycles each: with two or four a stage they set the pace of everything, 950 cycles.)
+// What the two word warps bring into a CTA's stages of a tile: the first one the packed words as tiled copies, the second one
+// the scales and offsets, 16 bytes a lane.  (Scales and offsets as bulk copies cost the issuing lane 250 to 300 cycles each,
+// and a group's number by division as many: 950 cycles a stage.)
 template <bool UP>
 struct TileWords {
   static constexpr int kColumns = UP ? kCols / 2 : kCols;
@@ -410,14 +410,14 @@ struct TileWords {
   bool on;           // its columns exist
   size_t N;
   int at, per;       // stages since the group's first, of a group
-  __device__ __forceinline__ void init(const Params& P, const Tile& t, int which, int lane) {
+  __device__ __forceinline__ void init(const Params& P, const Tile& t, int lane) {
     const Family& F = P.fam[t.fam];
     bits = t.bits;
     N = F.N;
     per = F.G / kStageK;
     col = t.col0;
     row0 = t.wrow;
-    map = &P.w_map[t.fam][UP ? which : 0][bits - 1];
+    map = &P.w_map[t.fam][0][bits - 1];
     const bool second = UP && lane >= 16, offsets = UP ? (lane >> 3) & 1 : lane >= 16;
     const int c = 8 * (lane & (UP ? 7 : 15)), sb0 = t.kb0 / 2;
     on = col + c < F.N;
@@ -426,9 +426,10 @@ struct TileWords {
     sc = (offsets ? (second ? F.zeros[1] : F.zeros[0]) : (second ? F.scales[1] : F.scales[0])) + off;
   }
   __device__ __forceinline__ void load_words(unsigned char* dst, unsigned long long* bar, int kb) const {
-    const int k0 = kb * kBK;
-    mbar_arrive_expect_tx(bar, stage_rows(bits) * kColumns * 4);
-    tma_load_2d(dst, map, col, row0 + (bits == 3 ? k0 / 10 : k0 * bits / 32), bar);
+    const int k0 = kb * kBK, row = row0 + (bits == 3 ? k0 / 10 : k0 * bits / 32), bytes = stage_rows(bits) * kColumns * 4;
+    mbar_arrive_expect_tx(bar, UP ? 2 * bytes : bytes);
+    tma_load_2d(dst, map, col, row, bar);
+    if (UP) tma_load_2d(dst + bytes, map + 4, col, row, bar);  // the second matrix's maps come behind the four of the first
   }
   __device__ __forceinline__ void load_scales(uint32_t dst) {  // stages in order
     if (on) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(sc) : "memory");
@@ -775,6 +776,10 @@ __device__ __forceinline__ void finish_rows(const Smem& S, const Params& P, cons
   }
 }
 
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
+}
+
 template <int OUT, bool BF16>
 __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_constant__ Params P) {
   constexpr bool UP = OUT == kOutUp, LINEAR = OUT == kOutLinear || OUT == kOutPartial;
@@ -788,7 +793,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&S.full[s], 17);  // in the first CTA: two groups' warps of either CTA, the activation boxes
       mbar_init(&S.empty[s], 1);
-      mbar_init(&S.words[s], UP ? 34 : 33);  // a tiled copy per matrix, the lanes that copy scales
+      mbar_init(&S.words[s], 33);      // the words, the lanes that copy scales
       mbar_init(&S.freed[s], 8);               // two groups' warps
     }
     for (int j = 0; j < 2; ++j) {
@@ -802,6 +807,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) tmem_alloc_pair(&S.tmem_base, kTmemCols);
+  // The maps are launch parameters: their first use finds them in the cache.
+  const int lane = static_cast<int>(threadIdx.x & 31);
+  if (warp == kTmaWarp && lane < 4) prefetch_map(&P.b_map[0][lane]);
+  if (warp == kWordWarp && P.staged && lane < (LINEAR ? 1 : (UP ? 8 : 4)))
+    prefetch_map(LINEAR ? &P.w_map[0][0][clamp_bits(P.fam[0].bits) - 1] : &P.w_map[0][lane >> 2][lane & 3]);
   tc_fence_before_sync();
   __syncthreads();
   pair_sync();
@@ -850,7 +860,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       }
     }
   } else if (warp >= kWordWarp && warp < kEpiWarp) {
-    const int which = warp - kWordWarp, lane = static_cast<int>(threadIdx.x & 31);
+    const int which = warp - kWordWarp;
     constexpr uint32_t kTilesAhead = 1;
     TileReader<COLS, LINEAR> reader(P, rank);
     if (which)
@@ -864,8 +874,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const int SB = (t.kbn + 1) / 2;
       const bool on = staged(P, t);  // the barrier's phases follow the stages, staged or not
       TileWords<UP> words;
-      if (on) words.init(P, t, which, lane);
-      const uint32_t at = UP && which && on ? stage_rows(words.bits) * kCols * 2 : 0;
+      if (on) words.init(P, t, lane);
       for (int sb = 0; sb < SB; ++sb, ++c) {
         const uint32_t s = c % kStages;
         const int kb = t.kb0 + 2 * sb;
@@ -878,8 +887,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
             mbar_arrive(&S.words[s]);
           }
         }
-        if ((UP || !which) && elect_one()) {
-          if (on) words.load_words(S.packed[s] + at, &S.words[s], kb);
+        if (!which && elect_one()) {
+          if (on) words.load_words(S.packed[s], &S.words[s], kb);
           else mbar_arrive(&S.words[s]);
         }
         __syncwarp();
@@ -934,7 +943,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const uint32_t at = tmem + (static_cast<uint32_t>(32 * lq) << 16) + t.acc(j);
       const int column = 32 * lq + static_cast<int>(threadIdx.x & 31);
       if (OUT == kOutPartial) drain_partial(P, t, at, t.col0 + column);
-      else drain<T>(S, at, t.rows, lq, static_cast<int>(threadIdx.x & 31));
+      else drain<T>(S, at, t.rows, lq, lane);
       tc_fence_before_sync();
       __syncwarp();
       if ((threadIdx.x & 31) == 0) arrive_at(first_cta(&S.drained[j & 1]));  // a later tile's MMAs may overwrite them
