@@ -57,24 +57,24 @@ int launch_down(const Params& P, int tiles_bound, cudaStream_t stream) { return 
 // many tokens.  Few tokens and few columns leave most of the 74 pairs without a tile, so the tokens go to smaller tiles
 // (more of them, each with its own de-quantisation) or k is split (fp32 parts through memory and a second launch),
 // whichever is estimated to end first.  4096 x 4096, 2 bits, 32 rows: 20.9 us unsplit, on 16 pairs, 11.1 as taken; 14336 x 1024:
-// 62.2, on 4, and 11.3.  The block times below are of the kernel whose producers loaded the words, back to back.  Now a block
-// takes 0.27, 0.28, 0.35, 0.29 us (1 to 4 bits, 32 rows; 0.30, 0.31, 0.38, 0.33 at 128 with every pair busy), so 1- and
-// 2-bit matrices are estimated too low: 256 rows of 4096 x 4096 are left whole, 21.9 us, where 3 and 4 bits in parts take 18.
+// 62.2, on 4, and 11.3.  The constants are a fit (4 % rms) to 623 times of 64 to 1000 rows, 11 shapes of 512 to 14336 wide, 1 to 4
+// bits, one call behind the other on weights out of L2: 5.3 us for the start and the end; a block of 64 k its de-quantisation or its
+// MMAs; the epilogue of a tile by its rows; parts of k 1.3 us and their sums' way through memory.
 LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split) {
-  static const float block_us[4] = {0.20f, 0.20f, 0.39f, 0.25f};
+  static const float block_us[4] = {0.22f, 0.225f, 0.32f, 0.24f};
   const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, KB = K / kBK, ct = cdiv(N, 2 * kCols);
-  const float dequant = block_us[bits >= 1 && bits <= 4 ? bits - 1 : 1];
   LinearPlan best = {kTokens, 1, (KB + 1) & ~1, 1e30f};
   for (int tr = kTokens; tr >= 32; tr /= 2) {
     const long long tiles = static_cast<long long>(ct) * cdiv(M, tr);
-    const float mma = 0.37f * static_cast<float>(M < tr ? M : tr) / kTokens;
+    const float rows = static_cast<float>(M < tr ? M : tr);
+    const float mma = 0.37f * rows / kTokens, dequant = block_us[bits >= 1 && bits <= 4 ? bits - 1 : 1] + 0.0002f * rows;
     for (int sp = 1; sp == 1 || (may_split && sp <= 16 && tiles * sp <= pairs && KB / sp >= 8); ++sp) {
       const int kb = (cdiv(KB, sp) + 1) & ~1;
       if (sp > 1 && cdiv(KB, kb) != sp) continue;
       const float rounds = static_cast<float>((tiles * sp + pairs - 1) / pairs);
-      float us = 3.f + rounds * static_cast<float>(kb) * (mma > dequant ? mma : dequant);
-      if (sp > 1) us += 2.5f + 8e-6f / 4.f * static_cast<float>(sp) * static_cast<float>(M) * static_cast<float>(N);
-      if (us < 0.97f * best.us) best = {tr, sp, kb, us};
+      float us = 5.3f + rounds * (static_cast<float>(kb) * (mma > dequant ? mma : dequant) + 0.0056f * rows);
+      if (sp > 1) us += 1.3f + 1e-6f * static_cast<float>(sp) * static_cast<float>(M) * static_cast<float>(N);
+      if (us < 0.99f * best.us) best = {tr, sp, kb, us};
     }
   }
   return best;
