@@ -74,7 +74,7 @@ LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split) {
       const float rounds = static_cast<float>((tiles * sp + pairs - 1) / pairs);
       float us = 5.3f + rounds * (static_cast<float>(kb) * (mma > dequant ? mma : dequant) + 0.0056f * rows);
       if (sp > 1) us += 1.3f + 1e-6f * static_cast<float>(sp) * static_cast<float>(M) * static_cast<float>(N);
-      if (us < 0.99f * best.us) best = {tr, sp, kb, us};
+      if (us < (tr < best.tile_rows ? 0.94f : 0.99f) * best.us) best = {tr, sp, kb, us};  // more tiles, more copies of both operands
     }
   }
   return best;

@@ -220,6 +220,26 @@ def test_moe_staged_behind_unstaged_tiles(D, Fd, shared):
         assert torch.equal(out, blk._prefill(*args, routing=(w.cuda(), sel.cuda()))[0])
 
 
+@pytest.mark.parametrize("D,Fd,bits", [(128, 2048, [4, 3, 1]), (2048, 128, [2, 4, 3]), (4096, 128, [1, 3, 4])])
+def test_moe_many_short_tiles(D, Fd, bits):
+    """Gate/up or down tiles of one stage, up to 9 a pair of CTAs: the slots of tile descriptions and the ring of words go round
+    while a tile is over before the next one's description is made; rows of 1 to 256."""
+    g = torch.Generator().manual_seed(D + Fd)
+    layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=3, A=1, bits=bits, seed=5, gate_std=0.02)
+    sel = torch.tensor([0] * 5121 + [1] * 129 + [2] * 5000)
+    T = sel.numel()
+    blk = MF.gpu_block(layer)
+    sel = sel[torch.randperm(T, generator=g)].view(T, 1)
+    w = (torch.rand(T, 1, generator=g) * 0.5 + 0.5).half()
+    x = torch.randn(T, D, generator=g).half()
+    args = (x.cuda(), 1, True)
+    out = blk._prefill(*args, routing=(w.cuda(), sel.cuda()))[0]
+    assert blk.prefill_error_code(T) == 0
+    assert rel_fro(out.float().cpu().numpy(), _reference(layer, x, w, sel)) < REL_FRO_TOL
+    for _ in range(10):
+        assert torch.equal(out, blk._prefill(*args, routing=(w.cuda(), sel.cuda()))[0])
+
+
 @pytest.mark.parametrize("shared", [0, 2])
 def test_moe_few_rows_one_behind_the_other(shared):
     """Decode batches on one scratch with nothing in between but kernels that write their weights: the products read the plan, which
