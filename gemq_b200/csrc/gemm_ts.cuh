@@ -20,8 +20,11 @@
 //   16 producer warps  four groups that take 64-wide k-blocks in turn: packed words from shared memory (or loaded a
 //                      block of the group ahead), de-quantise 64 k x 32 columns per warp, store them to the A ring;
 //                      they never stop between tiles
-//   1 TMA warp         per stage an activation box (32 to 128 tokens x 128 k, 128B swizzle), and the packed words,
-//                      scales and offsets of its 128 k (509 Mixtral tokens 531 -> 455 us, 4096 2650 -> 2490)
+//   1 TMA warp         per stage an activation box (32 to 128 tokens x 128 k, 128B swizzle)
+//   2 word warps       packed words; scales, offsets and the next tile's description.  They run ahead of the stages in rings of
+//                      their own (words asked for when the MMAs release their stage: 1100 of a block's 1950 cycles a wait;
+//                      1000 rows of 4096 x 4096, 4 bits 35.3 -> 32.5 us, 509 Mixtral tokens 455 -> 408, 2000 DeepSeek-V2-Lite
+//                      tokens 391 -> 343, the epilogue's part in these named there)
 //   1 MMA warp         (first CTA) issues tcgen05.mma and the commits that free the ring stages
 //   4 epilogue warps   round the accumulators to 16 bits into shared memory, which frees them for the next
 //                      tile, then finish and store whole rows while it is computed.  Tiles of up to 128 tokens
@@ -375,7 +378,7 @@ struct TileReader {
     if (n == 2) {
       finish();
       const uint32_t s = j % kTileSlots;
-      mbar_sleep_wait(&S.tile_free[s], ((j / kTileSlots) & 1) ^ 1, err, kErrTile);
+      mbar_look_wait(&S.tile_free[s], ((j / kTileSlots) & 1) ^ 1, err, kErrTile);
       if ((threadIdx.x & 31) == 0) {
         S.tiles[s] = t;
         mbar_arrive(&S.tile_full[s]);
@@ -390,7 +393,7 @@ __device__ __forceinline__ bool staged(const Params& P, const Tile& t) { return 
 // The launch's tiles in the CTA's order, as its tile warp leaves them; nullptr: no more.
 __device__ __forceinline__ const Tile* next_tile(Smem& S, uint32_t j, int* err) {
   const uint32_t s = j % kTileSlots;
-  if (!mbar_sleep_wait(&S.tile_full[s], (j / kTileSlots) & 1, err, kErrTile)) return nullptr;
+  if (!mbar_look_wait(&S.tile_full[s], (j / kTileSlots) & 1, err, kErrTile)) return nullptr;
   return S.tiles[s].rows > 0 ? &S.tiles[s] : nullptr;
 }
 __device__ __forceinline__ void done_tile(Smem& S, uint32_t j) {
@@ -504,7 +507,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   const uint32_t words0 = smem_u32(S.packed[0]) + mi * stage_rows(B) * kPitch + 4 * in_row;
   const uint32_t scales0 = smem_u32(S.scales[0]) + mi * 256 + 2 * in_row;
   // The barriers of the words flip in every use of a stage, staged or not: a use and the one before it are the same warps'.
-  auto words_ready = [&]() { mbar_sleep_wait(&S.words[s], par ^ 1u, err, kErrFull); };
+  auto words_ready = [&]() { mbar_look_wait(&S.words[s], par ^ 1u, err, kErrFull); };
   auto words_free = [&]() {
     __syncwarp();
     if (lane == 0) mbar_arrive(&S.freed[s]);
@@ -514,7 +517,7 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
       words_ready();
       words_free();
     }
-    mbar_sleep_wait(&S.empty[s], par, err, kErrEmpty);
+    mbar_look_wait(&S.empty[s], par, err, kErrEmpty);
   };
   auto take = [&](Set& R) {  // whole stages: no block of zeros
     words_ready();
@@ -866,7 +869,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const CUtensorMap* const map = &P.b_map[t.fam][box - 1];
       for (int sb = 0; sb < SB; ++sb, ++c) {
         const uint32_t s = c % kStages;
-        mbar_sleep_wait(&S.empty[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
+        mbar_look_wait(&S.empty[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
         if (elect_one()) {
           if (rank == 0) mbar_arrive_expect_tx(&S.full[s], 2 * bytes);
           tma_load_pair(S.b[s], map, row, t.kb0 + 2 * sb, full0 + s * 8);
@@ -893,7 +896,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       for (int sb = 0; sb < SB; ++sb, ++c) {
         const uint32_t s = c % kStages;
         const int kb = t.kb0 + 2 * sb;
-        mbar_sleep_wait(&S.freed[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
+        mbar_look_wait(&S.freed[s], ((c / kStages) & 1) ^ 1, err, kErrEmpty);
         if (which) {
           if (on) {
             words.load_scales(smem_u32(S.scales[s]) + 16 * lane);
@@ -925,13 +928,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       const uint32_t idesc = umma_idesc_f16(BF16 ? 1 : 0, 2 * kCols, t.n());
       const uint32_t second = ((t.n() / 2 + 31) / 32 * 32 * kRowBytes) >> 4;  // distance of a stage's second k-block
       // The accumulators of the tile two back are out; with a tile over 128 tokens also those of the last.
-      mbar_sleep_wait(&S.drained[j & 1], ((j >> 1) & 1) ^ 1, err, kErrDrained);
+      mbar_look_wait(&S.drained[j & 1], ((j >> 1) & 1) ^ 1, err, kErrDrained);
       const bool now_small = t.rows <= kTokens / 2;
-      if (j > 0 && !(small && now_small)) mbar_sleep_wait(&S.drained[(j - 1) & 1], ((j - 1) >> 1) & 1, err, kErrDrained);
+      if (j > 0 && !(small && now_small)) mbar_look_wait(&S.drained[(j - 1) & 1], ((j - 1) >> 1) & 1, err, kErrDrained);
       small = now_small;
       const uint32_t acc = tmem + t.acc(j);
       for (int sb = 0; sb < SB; ++sb) {
-        mbar_sleep_wait(&S.full[s], par, err, kErrFull);
+        mbar_look_wait(&S.full[s], par, err, kErrFull);
         tc_fence_after_sync();
         const uint64_t bd = desc0 + s * (kStageBytes >> 4);
         const uint32_t a = tmem + kTmemA + s * 64;
@@ -953,7 +956,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     for (uint32_t j = 0; const Tile* next = tile_at(j, own); ++j) {
       const Tile t = *next;
       tile_done(j);
-      mbar_sleep_wait(&S.acc_full[j & 1], (j >> 1) & 1, err, kErrAcc);
+      mbar_look_wait(&S.acc_full[j & 1], (j >> 1) & 1, err, kErrAcc);
       tc_fence_after_sync();
       const uint32_t at = tmem + (static_cast<uint32_t>(32 * lq) << 16) + t.acc(j);
       const int column = 32 * lq + static_cast<int>(threadIdx.x & 31);
