@@ -196,8 +196,8 @@ def _reference(layer, x, w, sel):
 @pytest.mark.parametrize("shared", [False, True])
 @pytest.mark.parametrize("D,Fd", [(1280, 1024), (2560, 256)])
 def test_moe_staged_behind_unstaged_tiles(D, Fd, shared):
-    """Every pair of CTAs gets 4-bit tiles of 256 rows, whose packed words do not come through the stages, and then tiles whose
-    words do: routed experts of 2 and 1 bits behind a 4-bit one, or 3 bits behind the shared expert, whose tiles lead the list.
+    """Every pair of CTAs gets 4-bit tiles of 256 rows, whose packed words fill a whole place of the ring, and then tiles of
+    shorter words: routed experts of 2 and 1 bits behind a 4-bit one, or 3 bits behind the shared expert, whose tiles lead the list.
     Reduction lengths of two stages (a use of every second stage) to twenty."""
     g = torch.Generator().manual_seed(D)
     if shared:
