@@ -704,10 +704,10 @@ __device__ __forceinline__ void word_order(const __half (&h)[32], uint32_t (&o)[
   }
 }
 
-// The quotient by reciprocal, good to two units of fp32's last place.  Over all finite fp16 v, after the rounding to fp16: 1 of 63488 is not
-// the rounded fp64 value (3 with the division), the mean error is the same (3.74731e-5), infinities and NaN come out alike.  The epilogue of a gate/up tile is 16 K of these per CTA: with an
-// IEEE division and every product in fp32, its four warps took longer than the MMAs of a tile of 2048 k (waits of 9 to 15 thousand
-// cycles for the accumulators against 14 thousand of MMAs).
+// The quotient by reciprocal, good to two units of fp32's last place.  Over all finite fp16 v, after the rounding to fp16, 1 of 63488 is
+// not the rounded fp64 value (3 with the division), the mean error is the same (3.74731e-5), infinities and NaN come out alike.
+// The epilogue of a gate/up tile is 16 K of these per CTA: with an IEEE division and every product in fp32, its four warps took
+// longer than the MMAs of a tile of 2048 k (waits of 9 to 15 thousand cycles for the accumulators against 14 thousand of MMAs).
 __device__ __forceinline__ float silu_quick(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 
 // h = F.silu(x1) * x3 on fp16 tensors, each step rounded: a thread takes 32 columns of a token (x1 and x3 of
