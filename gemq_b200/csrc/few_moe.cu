@@ -524,14 +524,16 @@ static bool init_attrs() {
   return true;
 }
 
-// Layers and batches this path takes: group 128, extents in whole groups, and on average at most few_average rows per
-// expert (above, the tensor cores' de-quantised tiles, whose cost hardly grows with the rows, win).  us here and there:
+// Layers and batches this path takes: group 128, extents in whole groups, and on average at most kFewAverage rows per
+// expert.  Above, the GEMM takes over, whose cost hardly grows with the rows.  It would be the faster from 16 to 20 rows on, but
+// it rounds every weight to fp16 (and bf16 activations, which end at 65504 there), where these launches take the codes, scales and
+// offsets as they are: a faster call is no reason to move the line down.  us of a layer, here and by the GEMM:
 //   64 experts of 2048 x 1408    16 rows 174 173   18 rows 184 175   24 rows 218 177
 //   32 of them                   16 rows 108 112   18 rows 113 112   24 rows 136 114
 //   16 of 2048 x 3456            16 rows  97 103   18 rows 106 105   24 rows 117 105
 //   8 of 4096 x 7168             14 rows 129 143   16 rows 146 143   24 rows 165 145
-//   8 of 4096 x 14336            18 rows 269 295   20 rows 272 295   24 rows 320 295: large matrices keep these launches full
-static int few_average(const gemq_moe_layer_t* L) { return static_cast<long long>(L->hidden) * L->ffn > (32ll << 20) ? 21 : 17; }
+//   8 of 4096 x 14336            18 rows 269 295   20 rows 272 295   24 rows 320 295
+constexpr int kFewAverage = 24;
 bool moe_few_rows_ok(const gemq_moe_layer_t* L, int tokens) {
   const int D = L->hidden, F = L->ffn, SF = L->shared_ffn;
   if (L->group_size != kGroup || D % kGroup || F % kGroup || SF % kGroup || D > 32768) return false;
@@ -548,7 +550,7 @@ bool moe_few_rows_ok(const gemq_moe_layer_t* L, int tokens) {
       if (!aligned16(p)) return false;
   if (L->w1.wq_rows <= 0 || L->w3.wq_rows <= 0 || L->w2.wq_rows <= 0) return false;
   const long long R = static_cast<long long>(tokens) * L->top_k;
-  return R <= static_cast<long long>(few_average(L)) * L->n_experts && tokens <= 4096;
+  return R <= static_cast<long long>(kFewAverage) * L->n_experts && tokens <= 4096;
 }
 
 size_t moe_few_rows_bytes(const gemq_moe_layer_t* L, int tokens) { return moe_few_rows_layout(L, tokens, nullptr, nullptr); }

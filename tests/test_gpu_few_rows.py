@@ -336,6 +336,47 @@ def test_moe_experts_off_whole_rows(words, scales):
         assert blk.prefill_error_code(T) == 0
 
 
+def _takes_few_rows(layer, T, A):
+    """Whether a batch of T tokens takes the few-row launches: they report experts off a whole row, which the GEMM loads."""
+    blk = MF.gpu_block(layer)
+    _shift(blk, 5, 0)
+    D, E = layer["gate"].shape[1], layer["gate"].shape[0]
+    sel = (torch.arange(T * A).view(T, A) % E).cuda()
+    blk._prefill(torch.ones(T, D, dtype=torch.float16, device="cuda"), 1, True,
+                 routing=(torch.full((T, A), 0.5, dtype=torch.float16, device="cuda"), sel))
+    code = blk.prefill_error_code(T)
+    assert code in (0, 22)
+    return code == 22
+
+
+@pytest.mark.parametrize("rows", [17, 18, 21, 22, 24, 25])
+def test_moe_few_rows_line(rows):
+    """Up to 24 rows per expert on average the codes are used as they are: weights are not rounded to fp16, and bf16
+    activations beyond fp16's range count (gate and up weights of their group are 2^-8 of the others: h stays in range)."""
+    E, A, D, Fd = 4, 2, 256, 384
+    T = rows * E // A
+    layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=E, A=A, bits=[1, 2, 3, 4], seed=rows, gate_std=0.02)
+    assert _takes_few_rows(layer, T, A) == (rows <= 24)
+    if rows > 24:
+        return
+    for mats in (layer["w1"], layer["w3"]):
+        for lin in mats:
+            lin["s"][0] *= np.float16(2.0 ** -8)
+            lin["z"][0] *= np.float16(2.0 ** -8)
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(T, D, generator=g).bfloat16()
+    x[T // 2, 7] = 90000.0
+    sel = torch.stack([torch.randperm(E, generator=g)[:A] for _ in range(T)])
+    w = torch.softmax(torch.randn(T, A, generator=g), -1).bfloat16()
+    blk = MF.gpu_block(layer)
+    out = blk._prefill(x.cuda(), 1, True, routing=(w.cuda(), sel.cuda()))[0]
+    assert blk.prefill_error_code(T) == 0 and out.isfinite().all()
+    w1, w3, w2, _ = MF.oracle_parts(layer)
+    ref = O.moe_reference_fp32(x.float(), w.float(), sel, w1, w3, w2).numpy()
+    got, large = out.float().cpu().numpy(), np.arange(T) == T // 2
+    assert rel_fro(got[large], ref[large]) < REL_FRO_TOL and rel_fro(got[~large], ref[~large]) < REL_FRO_TOL
+
+
 @pytest.mark.parametrize("b", [1, 2, 3, 4])
 def test_gemm_of_unaligned_views(b):
     """A dense matrix whose words, scales or offsets begin off a 16-byte boundary is loaded by the GEMM's producers: the same sums."""
