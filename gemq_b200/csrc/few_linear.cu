@@ -270,17 +270,21 @@ static bool linear_split(int rows, int N, int K, int nbits, int* tile_rows, int*
 }
 
 // Estimates in us of what the two kernels were measured to take (1 to 64 rows of 14 shapes, 512 to 14336 wide).  The
-// GEMM: linear_plan; the few-row kernel: rounds of the chip, each with a start and a table of the k of a warp.  The 3-bit table
+// GEMM: linear_line_us; the few-row kernel: rounds of the chip, each with a start and a table of the k of a warp.  The 3-bit table
 // costs up to 2.5 times the others'.  Of 352 pairs (11 shapes, 1 to 4 bits, 4 to 64 rows, back to back) 52 take the one that is slower
 // by more than 5 %: mostly 1- and 2-bit matrices, whose GEMM is estimated too low (8 rows of 4096 x 4096, 1 bit:
 // few-row kernel 7.4 us, GEMM 10.2; the worst, 4 rows of 14336 x 14336, 1 bit: 36.6 and 61.1).
+// The line does not follow the constants that linear_plan has since: the kernels round differently (weights to the activation type
+// in the GEMM, not at all here), and drawn by those it is no better.  Of 518 calls that would come here 267 gain more than
+// 3 % and 179 lose as much (128 rows of 4096 x 576, 4 bits: GEMM 9.4 us, few-row kernel 17.1); 3 rows of 14336 x 2816, 3 bits, bf16, would
+// go to the GEMM and from an error of 1.65e-3 to 2.38e-3.
 extern "C" int gemq_linear_takes_gemm(int rows, int N, int K, int nbits) {
   int tr, splits, tab;
   size_t smem;
   const int sms = sm_count();
   if (rows <= 0 || N <= 0 || K <= 0 || nbits < 1 || nbits > 4 || sms <= 0) return rows >= 32;
   if (!linear_split(rows, N, K, nbits, &tr, &splits, &tab, &smem)) return 1;
-  const float gemm = ts::linear_plan(rows, N, K, nbits, true).us;
+  const float gemm = ts::linear_line_us(rows, N, K, nbits);
   const int per_sm = tr > 8 || 3 * (smem + 2048) > kMaxDyn ? (2 * (smem + 2048) > kMaxDyn ? 1 : 2) : 3;
   const int rounds = cdiv(cdiv(N, 64) * splits * cdiv(rows, tr), per_sm * sms);
   const float warp_k = static_cast<float>(K) / static_cast<float>(kCons * splits);

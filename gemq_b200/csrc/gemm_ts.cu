@@ -60,24 +60,35 @@ int launch_down(const Params& P, int tiles_bound, cudaStream_t stream) { return 
 // 62.2, on 4, and 11.3.  The constants are a fit (4 % rms) to 623 times of 64 to 1000 rows, 11 shapes of 512 to 14336 wide, 1 to 4
 // bits, one call behind the other on weights out of L2: 5.3 us for the start and the end; a block of 64 k its de-quantisation or its
 // MMAs; the epilogue of a tile by its rows; parts of k 1.3 us and their sums' way through memory.
-LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split) {
-  static const float block_us[4] = {0.22f, 0.225f, 0.32f, 0.24f};
+struct GemmTimes {
+  float start, block[4], block_row;  // us; of 64 k by bit width, and by row of the tile
+  float epilogue_row;                // of a tile
+  float parts, part_value;           // parts of k: their launch, a value of a part
+  float smaller, more;               // what smaller tiles, more parts have to come down to
+};
+static LinearPlan fastest(const GemmTimes& t, int M, int N, int K, int bits, bool may_split) {
   const int pairs = sm_count() / 2 > 0 ? sm_count() / 2 : 1, KB = K / kBK, ct = cdiv(N, 2 * kCols);
   LinearPlan best = {kTokens, 1, (KB + 1) & ~1, 1e30f};
   for (int tr = kTokens; tr >= 32; tr /= 2) {
     const long long tiles = static_cast<long long>(ct) * cdiv(M, tr);
     const float rows = static_cast<float>(M < tr ? M : tr);
-    const float mma = 0.37f * rows / kTokens, dequant = block_us[bits >= 1 && bits <= 4 ? bits - 1 : 1] + 0.0002f * rows;
+    const float mma = 0.37f * rows / kTokens, dequant = t.block[bits >= 1 && bits <= 4 ? bits - 1 : 1] + t.block_row * rows;
     for (int sp = 1; sp == 1 || (may_split && sp <= 16 && tiles * sp <= pairs && KB / sp >= 8); ++sp) {
       const int kb = (cdiv(KB, sp) + 1) & ~1;
       if (sp > 1 && cdiv(KB, kb) != sp) continue;
       const float rounds = static_cast<float>((tiles * sp + pairs - 1) / pairs);
-      float us = 5.3f + rounds * (static_cast<float>(kb) * (mma > dequant ? mma : dequant) + 0.0056f * rows);
-      if (sp > 1) us += 1.3f + 1e-6f * static_cast<float>(sp) * static_cast<float>(M) * static_cast<float>(N);
-      if (us < (tr < best.tile_rows ? 0.94f : 0.99f) * best.us) best = {tr, sp, kb, us};  // more tiles, more copies of both operands
+      float us = t.start + rounds * (static_cast<float>(kb) * (mma > dequant ? mma : dequant) + t.epilogue_row * rows);
+      if (sp > 1) us += t.parts + t.part_value * static_cast<float>(sp) * static_cast<float>(M) * static_cast<float>(N);
+      if (us < (tr < best.tile_rows ? t.smaller : t.more) * best.us) best = {tr, sp, kb, us};  // more tiles, more copies of both operands
     }
   }
   return best;
+}
+LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split) {
+  return fastest({5.3f, {0.22f, 0.225f, 0.32f, 0.24f}, 0.0002f, 0.0056f, 1.3f, 1e-6f, 0.94f, 0.99f}, M, N, K, bits, may_split);
+}
+float linear_line_us(int M, int N, int K, int bits) {
+  return fastest({3.f, {0.20f, 0.20f, 0.39f, 0.25f}, 0.f, 0.f, 2.5f, 2e-6f, 0.97f, 0.97f}, M, N, K, bits, true).us;
 }
 
 // The parts of k, in order, rounded and biased like the one launch does.  A thread takes four columns.

@@ -987,6 +987,8 @@ struct LinearPlan {
   float us;
 };
 LinearPlan linear_plan(int M, int N, int K, int bits, bool may_split);
+// What the line between the few-row kernel and the GEMM is drawn by (few_linear.cu): constants of their own.
+float linear_line_us(int M, int N, int K, int bits);
 
 // gemm_ts.cu; tiles_bound: most tiles the launch can have
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream);

@@ -90,6 +90,28 @@ def test_gemm_tile_edges(b, N, K):
     assert int(error_word(wq.device).item()) == 0
 
 
+@pytest.mark.parametrize("M,N,K,b,gemm", [(3, 2816, 14336, 3, 0), (4, 6912, 4224, 3, 0), (128, 576, 4096, 4, 1), (15, 1152, 384, 1, 1),
+                                          (21, 4096, 512, 1, 1), (13, 4096, 4096, 4, 0), (64, 4096, 4096, 4, 1)])
+def test_linear_line(M, N, K, b, gemm):
+    """Which kernel a linear takes decides how its weights are rounded.  Calls at which other constants of the GEMM's estimate
+    would draw the line elsewhere: on the few-row kernel a bf16 result carries one rounding of its own (2^-9 of a value at
+    most), in the GEMM one of every weight, too."""
+    from gemq_b200 import _capi
+    from gemq_b200.kernels.dequant_gemm import quant_linear
+    assert _capi.lib.gemq_linear_takes_gemm(M, N, K, b) == gemm
+    if gemm:
+        return
+    lin = MF.draw_linear(np.random.default_rng(N), N, K, b)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    wq, s, z = t(lin["wq"]), t(lin["s"]), t(lin["z"])
+    W = torch.from_numpy(O.dequantize(lin["wq"], lin["s"], lin["z"], b, 128, K).astype(np.float64)).cuda()
+    scale, zero = s.double().repeat_interleave(128, 0), z.double().repeat_interleave(128, 0)
+    W = ((W - zero) / scale).round() * scale + zero  # without the rounding to fp16
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).bfloat16().cuda()
+    y = quant_linear(x, wq, s, z, b, 128, None)
+    assert rel_fro(y.double().cpu().numpy(), (x.double() @ W).cpu().numpy()) < 2.0 ** -9
+
+
 @pytest.mark.parametrize("b", [1, 2, 3, 4])
 @pytest.mark.parametrize("N,K,M", [(288, 2176, 1), (96, 4096, 33), (1024, 5376, 100)])
 def test_gemm_split_k(b, N, K, M):
