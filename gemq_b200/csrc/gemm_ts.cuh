@@ -371,6 +371,12 @@ struct TileReader {
     for (int m = 0; m < 2; ++m)
       t.zoff[m] = t.expert < 0 ? 0 : (F.zs_strides[m] || t.expert == 0 ? zoff[m] : static_cast<long long>(t.expert) * (F.K / F.G) * F.N);
   }
+  // Of a linear whose words are staged: no expert, no tables, nothing to read.
+  __device__ __forceinline__ void finish_plain() {
+    t.row0 = d.y;
+    t.rows = max(d.z, 0);
+    t.bits = clamp_bits(P.fam[0].bits);
+  }
   // step 0, 1, 2 of the CTA's tile j, number idx of the launch; step 2 hands it over
   __device__ __forceinline__ void step(Smem& S, int n, int idx, uint32_t j, int* err) {
     if (n == 0) find(idx);
@@ -443,18 +449,21 @@ struct TileWords {
 // ---- producer ------------------------------------------------------------------------------------
 // All k-blocks of a tile; `base` = k-blocks this CTA has handled before the tile (even).  An odd number of
 // blocks is followed by one of zeros: the activations of its stage end in zeros, too.
-// (Out of line: inlined, the 88 registers of 22 warps spill in the k loop.)
-// STAGED: packed words, scales and offsets lie in the stage.
+// (Out of line: inlined, the 80 registers of 24 warps spill in the k loop.  What it reads of the tile comes by value: through a
+// pointer a linear's tile, which every role works out, lies in local memory: 10 rows of 512 x 576 6.1 us instead of 5.7, 1000 of
+// 4096 x 4096 27.3 instead of 27.0.)
+// STAGED: packed words, scales and offsets lie in the ring.
 template <bool UP, bool BF16, bool NAT, int B, bool STAGED>
-__device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
+__device__ __noinline__ void produce(Smem& S, const Params& P, int fam, int col0, int kb0, int kbn, int first_word, long long first_scale,
+                                     uint32_t base, uint32_t tmem) {
   constexpr int NW = B == 3 ? 8 : 2 * B;  // words of a 64-code window
-  const Family& F = P.fam[T.fam];
+  const Family& F = P.fam[NAT ? 0 : fam];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int mi = UP ? lane >> 4 : 0;
   // columns past the end repeat the last one; their results are not stored
-  const int col = UP ? T.col0 + 16 * (warp & 3) + (lane & 15) : min(T.col0 + 32 * (warp & 3) + lane, F.N - 1);
+  const int col = UP ? col0 + 16 * (warp & 3) + (lane & 15) : min(col0 + 32 * (warp & 3) + lane, F.N - 1);
   const size_t N = F.N;
-  const size_t woff = static_cast<size_t>(T.woff), zoff = static_cast<size_t>(T.zoff[mi]);
+  const size_t woff = static_cast<size_t>(first_word), zoff = static_cast<size_t>(first_scale);
   const uint32_t* wp = (mi ? F.wq[1] : F.wq[0]) + woff + col;
   const __half* sp = (mi ? F.scales[1] : F.scales[0]) + zoff + col;
   const __half* zp = (mi ? F.zeros[1] : F.zeros[0]) + zoff + col;
@@ -463,9 +472,9 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
   int* const err = P.err;
   const int gshift = (G & (G - 1)) == 0 ? __ffs(G) - 1 : -1;
   int kb = static_cast<int>(((warp >> 2) + kGroups - base % kGroups) % kGroups);  // first k-block of this warp's group
-  const int real = T.kb0 + T.kbn, kb1 = T.kb0 + ((T.kbn + 1) & ~1);
-  base -= T.kb0;  // base + kb counts the blocks this CTA has handled
-  kb += T.kb0;
+  const int real = kb0 + kbn, kb1 = kb0 + ((kbn + 1) & ~1);
+  base -= kb0;  // base + kb counts the blocks this CTA has handled
+  kb += kb0;
   if (kb >= kb1) return;
   struct Set { uint32_t w[NW]; __half s, z; };
   Set ring[STAGED ? 1 : 2];
@@ -598,10 +607,11 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, const Tile& T, ui
 template <bool UP, bool BF16, bool NAT, bool STAGED>
 __device__ __forceinline__ void produce_bits(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
   const int bits = T.bits;
-  if (bits == 1) produce<UP, BF16, NAT, 1, STAGED>(S, P, T, base, tmem);
-  else if (bits == 2) produce<UP, BF16, NAT, 2, STAGED>(S, P, T, base, tmem);
-  else if (bits == 3) produce<UP, BF16, NAT, 3, STAGED>(S, P, T, base, tmem);
-  else produce<UP, BF16, NAT, 4, STAGED>(S, P, T, base, tmem);
+  const long long zoff = T.zoff[UP ? (threadIdx.x >> 4) & 1 : 0];  // of the lane's matrix
+  if (bits == 1) produce<UP, BF16, NAT, 1, STAGED>(S, P, T.fam, T.col0, T.kb0, T.kbn, T.woff, zoff, base, tmem);
+  else if (bits == 2) produce<UP, BF16, NAT, 2, STAGED>(S, P, T.fam, T.col0, T.kb0, T.kbn, T.woff, zoff, base, tmem);
+  else if (bits == 3) produce<UP, BF16, NAT, 3, STAGED>(S, P, T.fam, T.col0, T.kb0, T.kbn, T.woff, zoff, base, tmem);
+  else produce<UP, BF16, NAT, 4, STAGED>(S, P, T.fam, T.col0, T.kb0, T.kbn, T.woff, zoff, base, tmem);
 }
 template <bool UP, bool BF16, bool NAT>
 __device__ __forceinline__ void produce_any(Smem& S, const Params& P, const Tile& T, uint32_t base, uint32_t tmem) {
@@ -804,18 +814,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
       mbar_init(&S.acc_full[j], 1);
       mbar_init(&S.drained[j], 8);  // in the first CTA: the epilogue warps of both
     }
-    for (int j = 0; j < kTileSlots; ++j) {
+    for (int j = 0; !LINEAR && j < kTileSlots; ++j) {
       mbar_init(&S.tile_full[j], 1);
       mbar_init(&S.tile_free[j], kThreads / 32 - (rank == 0 ? 0 : 1));  // every warp; the second CTA's MMA warp has no work
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) tmem_alloc_pair(&S.tmem_base, kTmemCols);
-  // The maps are launch parameters: their first use finds them in the cache.
+  // The maps are launch parameters: their first use finds them in the cache.  (A linear has one of each, and its tile at once: there
+  // this gains nothing and takes 0.1 us of a short call.)
   const int lane = static_cast<int>(threadIdx.x & 31);
-  if (warp == kTmaWarp && lane < 4) prefetch_map(&P.b_map[0][lane]);
-  if (warp == kWordWarp && P.staged && lane < (LINEAR ? 1 : (UP ? 8 : 4)))
-    prefetch_map(LINEAR ? &P.w_map[0][0][clamp_bits(P.fam[0].bits) - 1] : &P.w_map[0][lane >> 2][lane & 3]);
+  if (!LINEAR && warp == kTmaWarp && lane < 4) prefetch_map(&P.b_map[0][lane]);
+  if (!LINEAR && warp == kWordWarp && P.staged && lane < (UP ? 8 : 4)) prefetch_map(&P.w_map[0][lane >> 2][lane & 3]);
   tc_fence_before_sync();
   __syncthreads();
   pair_sync();
@@ -833,13 +843,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
   const int step = static_cast<int>(gridDim.x >> 1), first = static_cast<int>(blockIdx.x >> 1);
   auto tile_of = [&](int i) { return i * step + ((i & 1) ? step - 1 - first : first); };
   // The CTA's tile j.  A linear's needs no look at memory: every role works it out (through the slots, 1010 rows of 512 x 576
-  // took 8.7 us instead of 7.9).
+  // took 8.7 us instead of 7.9; with the steps that read the tables, 10 rows of 256 x 640 5.5 instead of 5.2).
   auto tile_at = [&](uint32_t j, Tile& own) -> const Tile* {
     if (!LINEAR) return next_tile(S, j, P.err);
     TileReader<COLS, LINEAR> reader(P, rank);
     reader.find(tile_of(j));
-    reader.look_up();
-    reader.finish();
+    if (P.staged) {
+      reader.finish_plain();
+    } else {
+      reader.look_up();
+      reader.finish();
+    }
     own = reader.t;
     return own.rows > 0 ? &own : nullptr;
   };
