@@ -43,7 +43,7 @@ __device__ __forceinline__ void consume_linear(State<NB>& A, LinearShared& S, co
   if (B == 3) build_b3<T>(R, tab, x, rows, lo, hi, lane);
   else build_pow2<T, B == 3 ? 2 : B>(R, tab, x, rows, lo, hi, lane);
   __syncwarp();
-  const uint32_t zero = smem_u32(S.zero), tab32 = smem_u32(tab), ring32 = smem_u32(ring);
+  const uint32_t zero = smem_u32(S.zero), tab32 = smem_u32(tab), ring32 = smem_u32(ring), none = lds32(zero);
   int slot = 0;
   uint32_t par = 0;
 #pragma unroll 1
@@ -54,8 +54,7 @@ __device__ __forceinline__ void consume_linear(State<NB>& A, LinearShared& S, co
     if (sg < hi)
       stage_any<B, NB, kStrip>(A, st + warp * 2 * kStrip, tab32 + it * table_stage_bytes(B, rows), zero, st + kWStage + warp * 1024,
                                rows, sg, P.K / kGroup, lane);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&S.empty[slot]);
+    release_stage<NB>(A, &S.empty[slot], none, lane);
     if (++slot == P.ring) { slot = 0; par ^= 1u; }
   }
 }

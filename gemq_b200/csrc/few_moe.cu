@@ -62,7 +62,7 @@ template <int MODE> constexpr int kStripStep = MODE == kUp ? kCons * kStrip : kS
 template <int MODE, int NB, int B>
 __device__ __forceinline__ void consume_moe(State<NB>& A, MoeShared& S, const MoeParams& P, uint32_t ring, int lo, int hi, int rows,
                                             int ngroups, int warp, int lane) {
-  const uint32_t zero = smem_u32(S.zero);
+  const uint32_t zero = smem_u32(S.zero), none = lds32(zero);
   int slot = 0;
   uint32_t par = 0;
 #pragma unroll 1
@@ -71,8 +71,7 @@ __device__ __forceinline__ void consume_moe(State<NB>& A, MoeShared& S, const Mo
     mbar_sleep_wait(&S.full[slot], par, P.err, kErrFewFull);
     stage_any<B, NB, kStripStep<MODE>>(A, st + (MODE == kUp ? 1 : 2) * warp * kStrip, st + kWStage + kMetaStage, zero,
                                        st + kWStage + warp * 1024, rows, sg, ngroups, lane);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&S.empty[slot]);
+    release_stage<NB>(A, &S.empty[slot], none, lane);
     if (++slot == P.ring) { slot = 0; par ^= 1u; }
   }
 }

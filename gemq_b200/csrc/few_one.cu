@@ -204,7 +204,7 @@ __device__ __forceinline__ void consume_one(State<1>& A, OneShared& S, const One
     else build_pair<B == 3 ? 2 : B>(tab, static_cast<const float*>(x), K, lo, hi, lane);
   }
   __syncwarp();
-  const uint32_t zero = smem_u32(S.zero), tab32 = smem_u32(tab), ring32 = smem_u32(ring);
+  const uint32_t zero = smem_u32(S.zero), tab32 = smem_u32(tab), ring32 = smem_u32(ring), none = lds32(zero);
   int slot = 0;
   uint32_t par = 0;
 #pragma unroll 1
@@ -214,8 +214,7 @@ __device__ __forceinline__ void consume_one(State<1>& A, OneShared& S, const One
     if (lo + it < hi)
       stage_any<B, 1, kStrip>(A, st + warp * 2 * kStrip, tab32 + it * table_stage_bytes(B, kRows), zero, st + kWStage + warp * 1024,
                               kRows, lo + it, K / kGroup, lane);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&S.empty[slot]);
+    release_stage<1>(A, &S.empty[slot], none, lane);
     if (++slot == P.ring) { slot = 0; par ^= 1u; }
   }
 }
