@@ -62,3 +62,35 @@ def gpu_block(layer, device="cuda"):
     s1, s2, s3 = layer["shared"]
     return QuantFusedDeepseekV2MoEBlock.from_linears(layer["cfg"], gate, p(layer["w1"]), p(layer["w2"]), p(layer["w3"]),
                                                      (to_packed(s1, device), to_packed(s2, device), to_packed(s3, device)))
+
+
+def shift_experts(blk, words, scales, which=None):
+    """The block's experts moved off their places: `words` int32 and `scales` fp16 elements ahead of each, or of those in
+    `which` only, the others at whole rows."""
+    for name in ("w1", "w2", "w3"):
+        for suffix, table, gap in (("wq", "wq_strides", words), ("scales", "zs_strides", scales), ("zeros", "zs_strides", scales)):
+            old = getattr(blk, f"{name}_{suffix}")
+            at, N = getattr(blk, f"{name}_{table}").tolist() + [old.numel()], old.shape[1]
+            places, end = [], 0
+            for e in range(len(at) - 1):
+                places.append(end + gap if which is None or e in which else -(-end // N) * N)
+                end = places[-1] + at[e + 1] - at[e]
+            new = torch.zeros(-(-end // N), N, dtype=old.dtype, device=old.device)
+            for e, p in enumerate(places):
+                new.view(-1)[p:p + at[e + 1] - at[e]] = old.reshape(-1)[at[e]:at[e + 1]]
+            setattr(blk, f"{name}_{suffix}", new)
+            if suffix != "scales":  # the offsets, next, lie like the scales
+                setattr(blk, f"{name}_{table}", torch.tensor(places, dtype=torch.int32, device=old.device))
+    blk._build_layer(blk._layer.route_mode, bool(blk._layer.renorm), blk._layer.shared_ffn)
+
+
+def takes_few_rows(layer, T):
+    """Whether a batch of T tokens takes the few-row launches: they report experts off a whole row, which the GEMM loads."""
+    blk, A = gpu_block(layer), layer["A"]
+    shift_experts(blk, 5, 0)
+    E, D = layer["gate"].shape
+    routing = (torch.full((T, A), 0.5, dtype=torch.float16, device="cuda"), (torch.arange(T * A).view(T, A) % E).cuda())
+    blk._prefill(torch.ones(T, D, dtype=torch.float16, device="cuda"), 1, True, routing=routing)
+    code = blk.prefill_error_code(T)
+    assert code in (0, 22)
+    return code == 22

@@ -282,20 +282,21 @@ def test_expert_id_out_of_range_is_reported_not_used():
     assert rc == 0
     assert blk.decode_error_code() == 7
     blk.reset_decode_scratch()
-    T = 40
-    xs = torch.randn(T, 256, generator=torch.Generator().manual_seed(42)).half().cuda()
-    sel = torch.randint(0, 4, (T, 2), generator=torch.Generator().manual_seed(43))
-    sel[:, 1] = (sel[:, 0] + 1) % 4
-    sel[3, 1] = -5
-    sel[7, 0] = 4
-    ws = torch.full((T, 2), 0.5, dtype=torch.float16)
-    out = blk._prefill(xs, 1, True, routing=(ws.cuda(), sel.cuda()))[0]
-    assert blk.prefill_error_code(T) == 21
     w1, w3, w2, _ = MF.oracle_parts(layer)
-    good = [t for t in range(T) if t not in (3, 7)]
-    ref = O.moe_reference_fp32(xs.cpu()[good], ws[good].float(), sel[good], w1, w3, w2).numpy()
-    got = out.float().cpu().numpy()[good]
-    assert rel_fro(got, ref) < REL_FRO_TOL and max_abs(got, ref) < MAX_ABS_TOL
+    for T in (40, 400):  # few-row launches and the GEMM
+        assert MF.takes_few_rows(layer, T) == (T == 40)
+        xs = torch.randn(T, 256, generator=torch.Generator().manual_seed(42)).half().cuda()
+        sel = torch.randint(0, 4, (T, 2), generator=torch.Generator().manual_seed(43))
+        sel[:, 1] = (sel[:, 0] + 1) % 4
+        sel[3, 1] = -5
+        sel[7, 0] = 4
+        ws = torch.full((T, 2), 0.5, dtype=torch.float16)
+        out = blk._prefill(xs, 1, True, routing=(ws.cuda(), sel.cuda()))[0]
+        assert blk.prefill_error_code(T) == 21
+        good = [t for t in range(T) if t not in (3, 7)]
+        ref = O.moe_reference_fp32(xs.cpu()[good], ws[good].float(), sel[good], w1, w3, w2).numpy()
+        got = out.float().cpu().numpy()[good]
+        assert rel_fro(got, ref) < REL_FRO_TOL and max_abs(got, ref) < MAX_ABS_TOL
 
 
 def test_torch_compile_traces_through_the_block():

@@ -182,8 +182,8 @@ def test_moe_many_tiles_per_pair(D, Fd, E):
 @pytest.mark.parametrize("rows", [[128, 129, 40, 7], [192, 193, 130, 33], [161, 177, 224, 192]])
 @pytest.mark.parametrize("bits", [[1, 2, 3, 4], [3, 4, 1, 2], [4, 4, 4, 3]])
 def test_moe_staged_words(rows, bits):
-    """4-bit tiles up to and past the 192 tokens whose stages also hold their packed words, among them those whose activations
-    end where the words begin (161 to 192 rows), the other widths at the same sizes; reduction lengths that end inside a 3-bit word."""
+    """Tiles of 7 to 224 rows, at and next to multiples of 32, whose packed words come through shared memory, every width at every
+    size; reduction lengths that end inside a 3-bit word."""
     g = torch.Generator().manual_seed(sum(rows))
     sel = torch.cat([torch.full((n,), e, dtype=torch.int64) for e, n in enumerate(rows)])
     T = sel.numel()
@@ -217,7 +217,7 @@ def _reference(layer, x, w, sel):
 
 @pytest.mark.parametrize("shared", [False, True])
 @pytest.mark.parametrize("D,Fd", [(1280, 1024), (2560, 256)])
-def test_moe_staged_behind_unstaged_tiles(D, Fd, shared):
+def test_moe_long_words_before_short(D, Fd, shared):
     """Every pair of CTAs gets 4-bit tiles of 256 rows, whose packed words fill a whole place of the ring, and then tiles of
     shorter words: routed experts of 2 and 1 bits behind a 4-bit one, or 3 bits behind the shared expert, whose tiles lead the list.
     Reduction lengths of two stages (a use of every second stage) to twenty."""
@@ -242,13 +242,15 @@ def test_moe_staged_behind_unstaged_tiles(D, Fd, shared):
         assert torch.equal(out, blk._prefill(*args, routing=(w.cuda(), sel.cuda()))[0])
 
 
-@pytest.mark.parametrize("D,Fd,bits", [(128, 2048, [4, 3, 1]), (2048, 128, [2, 4, 3]), (4096, 128, [1, 3, 4])])
+@pytest.mark.parametrize("D,Fd,bits", [(128, 2048, [4, 3, 1, 2, 4, 3]), (2048, 128, [2, 4, 3, 4, 1, 2]), (4096, 128, [1, 3, 4, 3, 2, 1])])
 def test_moe_many_short_tiles(D, Fd, bits):
-    """Gate/up or down tiles of one stage, up to 9 a pair of CTAs: the slots of tile descriptions and the ring of words go round
-    while a tile is over before the next one's description is made; rows of 1 to 256."""
+    """Gate/up or down tiles of one stage, some nine or more a pair of CTAs: the slots of tile descriptions and the ring of words go
+    round while a tile is over before the next one's description is made.  Tiles of 1, 17, 65 and 128 rows, which use the halves of
+    the accumulators in turn, between those of some 240 to 256, which take all of them."""
     g = torch.Generator().manual_seed(D + Fd)
-    layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=3, A=1, bits=bits, seed=5, gate_std=0.02)
-    sel = torch.tensor([0] * 5121 + [1] * 129 + [2] * 5000)
+    layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=6, A=1, bits=bits, seed=5, gate_std=0.02)
+    rows = (5121, 129, 5000, 1, 17, 128)
+    sel = torch.cat([torch.full((n,), e) for e, n in enumerate(rows)])
     T = sel.numel()
     blk = MF.gpu_block(layer)
     sel = sel[torch.randperm(T, generator=g)].view(T, 1)
@@ -312,6 +314,7 @@ def test_moe_bit_width_tables(T):
     """Widths on the device are clamped before they choose a map of packed words, and the shared expert's third matrix is read with
     the first one's width."""
     layer = MF.make_layer("deepseek", D=256, Fd=384, E=4, A=2, bits=[4, 4, 1, 4], seed=1, gate_std=0.02, n_shared=1)
+    assert MF.takes_few_rows(layer, T) == (T == 40)
     blk = MF.gpu_block(layer)
     x = torch.randn(T, 256, generator=torch.Generator().manual_seed(T)).half().cuda()
     want = blk._prefill(x, 2, False)[0].clone()
@@ -322,29 +325,13 @@ def test_moe_bit_width_tables(T):
     assert blk.prefill_error_code(T) == 0
 
 
-def _shift(blk, words, scales):
-    """The block's experts with `words` int32 and `scales` fp16 elements ahead of each."""
-    for name in ("w1", "w2", "w3"):
-        for suffix, table, gap in (("wq", "wq_strides", words), ("scales", "zs_strides", scales), ("zeros", "zs_strides", scales)):
-            old = getattr(blk, f"{name}_{suffix}")
-            at = getattr(blk, f"{name}_{table}").tolist() + [old.numel()]
-            new = torch.zeros(-(-(old.numel() + gap * len(at)) // old.shape[1]), old.shape[1], dtype=old.dtype, device=old.device)
-            for e in range(len(at) - 1):
-                new.view(-1)[at[e] + gap * (e + 1):at[e + 1] + gap * (e + 1)] = old.reshape(-1)[at[e]:at[e + 1]]
-            setattr(blk, f"{name}_{suffix}", new)
-        for table, gap in (("wq_strides", words), ("zs_strides", scales)):
-            t = getattr(blk, f"{name}_{table}")
-            setattr(blk, f"{name}_{table}", t + gap * torch.arange(1, t.numel() + 1, dtype=torch.int32, device=t.device))
-    blk._build_layer(blk._layer.route_mode, bool(blk._layer.renorm), blk._layer.shared_ffn)
-
-
 @pytest.mark.parametrize("words,scales", [(0, 8), (5, 0), (32, 0), (0, 3), (9, 1)])
 def test_moe_experts_off_whole_rows(words, scales):
     """Experts that begin off a whole row of words or a 16-byte boundary of scales: the GEMM's producers load them, few-row launches
     leave them out and say so.  Eight scales more are a boundary."""
     layer = MF.make_layer("mixtral", D=384, Fd=256, E=4, A=1, bits=[1, 2, 3, 4], seed=7, gate_std=0.02)
     blk, moved = MF.gpu_block(layer), MF.gpu_block(layer)
-    _shift(moved, words, scales)
+    MF.shift_experts(moved, words, scales)
     g = torch.Generator().manual_seed(words + scales)
     for T in (16, 300, 1200):
         x, w = torch.randn(T, 384, generator=g).half().cuda(), torch.rand(T, 1, generator=g).half().cuda()
@@ -358,19 +345,6 @@ def test_moe_experts_off_whole_rows(words, scales):
         assert blk.prefill_error_code(T) == 0
 
 
-def _takes_few_rows(layer, T, A):
-    """Whether a batch of T tokens takes the few-row launches: they report experts off a whole row, which the GEMM loads."""
-    blk = MF.gpu_block(layer)
-    _shift(blk, 5, 0)
-    D, E = layer["gate"].shape[1], layer["gate"].shape[0]
-    sel = (torch.arange(T * A).view(T, A) % E).cuda()
-    blk._prefill(torch.ones(T, D, dtype=torch.float16, device="cuda"), 1, True,
-                 routing=(torch.full((T, A), 0.5, dtype=torch.float16, device="cuda"), sel))
-    code = blk.prefill_error_code(T)
-    assert code in (0, 22)
-    return code == 22
-
-
 @pytest.mark.parametrize("rows", [17, 18, 21, 22, 24, 25])
 def test_moe_few_rows_line(rows):
     """Up to 24 rows per expert on average the codes are used as they are: weights are not rounded to fp16, and bf16
@@ -378,7 +352,7 @@ def test_moe_few_rows_line(rows):
     E, A, D, Fd = 4, 2, 256, 384
     T = rows * E // A
     layer = MF.make_layer("mixtral", D=D, Fd=Fd, E=E, A=A, bits=[1, 2, 3, 4], seed=rows, gate_std=0.02)
-    assert _takes_few_rows(layer, T, A) == (rows <= 24)
+    assert MF.takes_few_rows(layer, T) == (rows <= 24)
     if rows > 24:
         return
     for mats in (layer["w1"], layer["w3"]):
@@ -397,6 +371,26 @@ def test_moe_few_rows_line(rows):
     ref = O.moe_reference_fp32(x.float(), w.float(), sel, w1, w3, w2).numpy()
     got, large = out.float().cpu().numpy(), np.arange(T) == T // 2
     assert rel_fro(got[large], ref[large]) < REL_FRO_TOL and rel_fro(got[~large], ref[~large]) < REL_FRO_TOL
+
+
+@pytest.mark.parametrize("moved", [(0,), (1,), (0, 2), (1, 2), (0, 1, 2)])
+@pytest.mark.parametrize("D,Fd,shared", [(128, 2560, False), (256, 1280, True), (384, 2560, False), (2560, 1024, True)])
+def test_moe_staged_and_unstaged_tiles(D, Fd, shared, moved):
+    """Tiles of experts off their boundaries, whose words the producers load, before, between and behind those of experts (and of
+    the shared one, whose tiles lead) whose words come through shared memory, some eleven a pair of CTAs and of 1, 2, 3, 8, 10 and 20
+    stages: the two kinds pass the same barriers."""
+    g = torch.Generator().manual_seed(D + len(moved))
+    layer = MF.make_layer("deepseek" if shared else "mixtral", D=D, Fd=Fd, E=3, A=1, bits=[4, 3, 1], seed=3, gate_std=0.02, n_shared=int(shared))
+    blk, other = MF.gpu_block(layer), MF.gpu_block(layer)
+    MF.shift_experts(other, 5, 8, moved)
+    sel = torch.tensor([0] * 5120 + [1] * 2700 + [2] * 2420)
+    T = sel.numel()
+    args = (torch.randn(T, D, generator=g).half().cuda(), 1, True)
+    routing = ((torch.rand(T, 1, generator=g) * 0.5 + 0.5).half().cuda(), sel[torch.randperm(T, generator=g)].view(T, 1).cuda())
+    want = blk._prefill(*args, routing=routing)[0]
+    for _ in range(10):
+        assert torch.equal(other._prefill(*args, routing=routing)[0], want)
+    assert blk.prefill_error_code(T) == 0 and other.prefill_error_code(T) == 0
 
 
 @pytest.mark.parametrize("b", [1, 2, 3, 4])

@@ -74,6 +74,7 @@ def test_deepseek_decode_batch_rows():
 
 def test_mixtral_n_tokens_small():
     layer = MF.make_layer("mixtral", D=256, Fd=512, E=4, A=2, bits=[4, 1, 3, 2], seed=5, gate_std=0.02)
+    assert MF.takes_few_rows(layer, 37)
     blk = MF.gpu_block(layer)
     w1, w3, w2, _ = MF.oracle_parts(layer)
     x = torch.randn(37, 256, generator=torch.Generator().manual_seed(2)).half()
