@@ -362,7 +362,7 @@ __device__ __forceinline__ void stage_any(State<NB>& S, uint32_t W, uint32_t T, 
 }
 
 // Gives a stage back behind the sums that came of everything read from it.  The refill is written past the order of a warp's
-// shared-memory accesses (TMA): with the arrival right behind the reads, and sixteen other warps in bank conflicts, 22 % of the words
+// shared-memory accesses (TMA): with the arrival right behind the reads, and 22 other warps in bank conflicts, 22 % of the words
 // that a probe read were the next refill's; with an arrival whose address takes in what was read, none of 1.5e9.  (Refills by
 // stores or cp.async: none either way.)  `none` is a zero that the compiler does not know.  One fragment per strip and row block will
 // do, they share their loads.  Costs nothing (all of them: 1 % of 32 Mixtral rows).

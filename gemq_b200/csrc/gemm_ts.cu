@@ -56,10 +56,12 @@ int launch_down(const Params& P, int tiles_bound, cudaStream_t stream) { return 
 // A tile's time is its k-blocks': the de-quantisation of 256 columns (by bit width, whatever the tokens), or the MMAs of
 // many tokens.  Few tokens and few columns leave most of the 74 pairs without a tile, so the tokens go to smaller tiles
 // (more of them, each with its own de-quantisation) or k is split (fp32 parts through memory and a second launch),
-// whichever is estimated to end first.  4096 x 4096, 2 bits, 32 rows: 20.9 us unsplit, on 16 pairs, 11.1 as taken; 14336 x 1024:
-// 62.2, on 4, and 11.3.  The constants are a fit (4 % rms) to 623 times of 64 to 1000 rows, 11 shapes of 512 to 14336 wide, 1 to 4
-// bits, one call behind the other on weights out of L2: 5.3 us for the start and the end; a block of 64 k its de-quantisation or its
-// MMAs; the epilogue of a tile by its rows; parts of k 1.3 us and their sums' way through memory.
+// whichever is estimated to end first.  4096 x 4096, 2 bits, 32 rows: 19.4 us unsplit, on 16 pairs, 10.8 as taken; 14336 x 1024:
+// 56.4, on 4, and 11.2.  linear_plan's constants are a fit (4 % rms) to 623 times of 64 to 1000 rows, 11 shapes of 512 to 14336 wide, 1
+// to 4 bits, one call behind the other on weights out of L2: 5.3 us for the start and the end; a block of 64 k its de-quantisation or its
+// MMAs; the epilogue of a tile by its rows; parts of k 1.3 us and their sums' way through memory.  (Fewer rows are outside the fit.)  Of 401
+// calls of other shapes whose tiles or parts they changed, against the constants of linear_line_us on the GEMM before this one: 12 % less
+// time, 349 faster and 12 slower by more than 3 % (148 rows of 14336 x 1024, 3 bits, 16 parts instead of 14: 15.0 -> 16.8 us).
 struct GemmTimes {
   float start, block[4], block_row;  // us; of 64 k by bit width, and by row of the tile
   float epilogue_row;                // of a tile

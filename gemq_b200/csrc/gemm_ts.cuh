@@ -565,8 +565,8 @@ __device__ __noinline__ void produce(Smem& S, const Params& P, int fam, int col0
       dequant_words<B, BF16, NAT, 0>(X, o, cur.w + B, s2, z2);
       tmem_st16(dst + 16, o);
     }
-    // Behind the stores, which hold what came of the words: an arrival right behind the loads overtook them (shared-memory reads that
-    // wait behind the epilogue's; the next words were there before 4 to 32 lanes had read the last row).
+    // Behind the stores, which hold what came of the words: an arrival does not wait for the shared-memory reads ahead of it, and TMA
+    // writes past them (reads that waited behind the epilogue's: the next words were there before 4 to 32 lanes had read the last row).
     if (STAGED) words_free();
     tmem_wait_st();
     tc_fence_before_sync();
@@ -807,8 +807,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_ts_kernel(const __grid_const
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&S.full[s], 17);  // in the first CTA: two groups' warps of either CTA, the activation boxes
       mbar_init(&S.empty[s], 1);
-      mbar_init(&S.words[s], 33);      // the words, the lanes that copy scales
-      mbar_init(&S.freed[s], 8);               // two groups' warps
+      mbar_init(&S.words[s], 33);  // the words, the lanes that copy scales
+      mbar_init(&S.freed[s], 8);   // two groups' warps
     }
     for (int j = 0; j < 2; ++j) {
       mbar_init(&S.acc_full[j], 1);
@@ -1008,8 +1008,8 @@ float linear_line_us(int M, int N, int K, int bits);
 int launch_up(const Params& P, int tiles_bound, cudaStream_t stream);
 int launch_down(const Params& P, int tiles_bound, cudaStream_t stream);
 bool activation_maps(CUtensorMap (&maps)[4], const void* x, int K, long long rows);
-// Maps of a matrix's packed words (rows of N; all widths, or one) and whether words, scales and offsets can be staged: bulk copies
-// want 16-byte boundaries, a stage one group.
+// Maps of a matrix's packed words (rows of N; all widths, or one) and whether words, scales and offsets can be staged: tiled copies
+// and copies of 16 bytes a lane want 16-byte boundaries, a stage one group.
 bool word_maps(CUtensorMap (&maps)[4], const void* wq, const void* scales, const void* zeros, int N, long long rows, int G, int bits,
                int columns);
 

@@ -81,7 +81,9 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(Plan pl, con
     }
   }
   __syncthreads();
-  // Experts with the longest tiles first: cycles of 128 k by the tile's MMAs, or by the de-quantisation.  (By bit width alone
+  // Experts with the longest tiles first: cycles of 128 k by the tile's MMAs, or by the de-quantisation, as they were when the producers
+  // waited for their words.  Since the words have a ring of their own they are 590 to 770 at 1, 2 and 4 bits, 850 to 1030 at 3 and
+  // 880 to 1025 for 225 to 256 rows of any width, so 3-bit tiles of few rows stand too far ahead; not fitted anew.  (By bit width alone
   // the pairs' shares differed by a quarter where 400 tokens meet 32 experts unevenly.)  E <= 256: one expert a thread.
   if (tid < E) {
     const int n = count[tid], nt = (n + kTile - 1) / kTile, rows = nt ? (n + nt - 1) / nt : 0;
